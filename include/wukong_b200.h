@@ -263,7 +263,9 @@ int wk_store_build_device(wk_ctx* ctx, const uint32_t* triples, uint64_t n_tripl
  * (WK_E_CAPACITY).  No reference counterpart. */
 int wk_store_export(wk_ctx* ctx, void* slots, uint64_t slots_cap, uint32_t* edges, uint64_t edges_cap,
                     wk_seg_meta* segs, uint32_t segs_cap, uint64_t* n_slots, uint64_t* n_edges, uint32_t* n_segs);
-/* Device bytes held by the store (slots + edges + segment table). */
+/* Device bytes held by the store (slots + edges + segment table).  The lookup tables derived from
+ * it at load time (vertex directories, at most a quarter of the then free memory; the original
+ * words of one-entry lists) are not counted. */
 int wk_store_bytes(const wk_ctx* ctx, uint64_t* bytes);
 
 /* ---------------------------------------------------------------- result tables */
@@ -444,7 +446,8 @@ int wk_debug_device_allocs(uint64_t* count);
 /* Tile-schedule knobs of the exploration launch (what the autotuner sets).
  *   knob 0: lanes per probe group of the single-query path (1: one thread per row reading its
  *           home bucket's first 32 bytes; 2, 4 or 8: a group of lanes staging 32-, 64- or
- *           128-byte bucket slices per request);
+ *           128-byte bucket slices per request).  A store with vertex directories (dense ids:
+ *           built when it is loaded) is looked up by one thread per row whatever the knob says;
  *   knob 1: the same for batches and serving;
  *   knob 2: the list length above which a row's output is written as 2,048-row slices by every
  *           CTA (block-per-row) instead of by the CTA that probed it (group-per-row); 8 to

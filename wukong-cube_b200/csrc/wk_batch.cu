@@ -356,12 +356,12 @@ int enqueue_batch(wk_ctx* ctx, BatchState* b, const Plan& P, ProfHooks* ph = nul
     WKB_CUDA(ctx, cudaMemsetAsync(b->d_qfirst, 0xFF, 8ull * L * n, s));
     WKB_CUDA(ctx, cudaMemsetAsync(b->d_qcount, 0, 8ull * L * n, s));
     if (ph) WKB_CUDA(ctx, cudaEventRecord(ph->extra[1], s));
-    const int lanes = ctx->batch_lanes;
+    const int lanes = ctx->probe_lanes(ctx->batch_lanes);
     for (int k = 0; k < L; ++k) {
         wk::ExploreArgs a{};
         a.store = ctx->dev_store();
-        a.seg_index[0] = ctx->seg_of(0, 0, wk::kIn);
-        a.seg_index[1] = ctx->seg_of(0, 0, wk::kOut);
+        a.seg_index[0] = ctx->seg_id(0, 0, wk::kIn);
+        a.seg_index[1] = ctx->seg_id(0, 0, wk::kOut);
         a.desc = b->d_desc + (size_t)k * n;
         a.n_queries = n;
         a.virtual_rows = k == 0;
@@ -480,7 +480,7 @@ int launch_batch(wk_ctx* ctx, BatchState* b, const Plan& P) {
     put(&ctx->batch_slice_rows, 4);
     put(&ctx->batch_flat, 4);
     put(&b->d_flat, sizeof(void*));
-    put(&ctx->d_slots, sizeof(void*));
+    put(&ctx->store_gen, 8);
     if (shape != b->shape || !b->exec) {
         if (b->exec) cudaGraphExecDestroy(b->exec);
         b->exec = nullptr;

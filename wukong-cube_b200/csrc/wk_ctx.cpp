@@ -12,6 +12,7 @@
 
 #include "wk_batch.h"
 #include "wk_ctx.h"
+#include "wk_dir.h"
 
 #define WK_CUDA(ctx, call)                                   \
     do {                                                     \
@@ -150,6 +151,36 @@ int wk_ctx::ensure_status(uint64_t tiles) {
     status_cap = cap;
     drop_graphs();   // captured launches hold the old status pointer
     return WK_SUCCESS;
+}
+
+// Free the store and everything derived from it; the serving lanes, which hold its addresses, go
+// too (the next serving run makes them again).  A lane's own store belongs to its parent.
+void wk_ctx::drop_store() {
+    for (wk_ctx* lane : lanes) wk_ctx_destroy(lane);
+    lanes.clear();
+    drop_graphs();
+    ++store_gen;
+    has_store = false;
+    if (!borrowed_store) {
+        cudaFree(d_slots);
+        cudaFree(d_edges);
+        cudaFree(d_pseg);
+        cudaFree(d_inline_orig);
+        cudaFree(d_segs);
+        cudaFree(d_dir_blocks);
+        cudaFree(d_dir_words);
+    }
+    d_slots = nullptr;
+    d_edges = nullptr;
+    d_pseg = nullptr;
+    d_inline_orig = nullptr;
+    d_segs = nullptr;
+    d_dir_blocks = nullptr;
+    d_dir_words = nullptr;
+    n_slots = n_edges = n_inline = 0;
+    n_pseg = 0;
+    has_dir = false;
+    seg_desc.clear();
 }
 
 void wk_ctx::drop_graphs() {
@@ -396,8 +427,8 @@ int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* 
     if (!in || st.in_cols <= 0) return WK_E_BADARG;
     ExploreArgs a{};
     a.store = ctx->dev_store();
-    a.seg_index[0] = ctx->seg_of(0, 0, kIn);
-    a.seg_index[1] = ctx->seg_of(0, 0, kOut);
+    a.seg_index[0] = ctx->seg_id(0, 0, kIn);
+    a.seg_index[1] = ctx->seg_id(0, 0, kOut);
     a.one = make_step_desc(ctx, st);
     a.desc = nullptr;
     a.n_queries = 1;
@@ -437,6 +468,8 @@ int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* 
         f.store = a.store;
         f.seg_index[0] = a.seg_index[0];
         f.seg_index[1] = a.seg_index[1];
+        f.seg = ctx->seg_of(st.kind == PlanStep::kI2K || (st.kind == PlanStep::kC2K && st.start_const == 0) ? 0 : 1,
+                            st.kind == PlanStep::kI2K ? st.start_const : st.pid, st.dir);
         f.step = a.one;
         f.in_rows = a.in_rows;
         f.in = a.in;
@@ -475,36 +508,36 @@ StepDesc make_step_desc(const wk_ctx* ctx, const PlanStep& s) {
     case PlanStep::kIndex:
         d.op = kXStart;
         d.start_key = make_key(0, s.start_const, s.dir);
-        d.seg = ctx->seg_of(0, s.start_const, s.dir);
+        d.seg = ctx->seg_id(0, s.start_const, s.dir);
         break;
     case PlanStep::kConst:
         d.op = kXStart;
         d.start_key = make_key(s.start_const, s.pid, s.dir);
-        d.seg = ctx->seg_of(s.start_const, s.pid, s.dir);
+        d.seg = ctx->seg_id(s.start_const, s.pid, s.dir);
         break;
     case PlanStep::kK2U:
         d.op = kXK2U;
         d.type_index = (s.pid == kTypeId && s.dir == kIn) ? 1 : 0;
-        d.seg = ctx->seg_of(1, s.pid, s.dir);   // any nonzero vid: the normal segment
+        d.seg = ctx->seg_id(1, s.pid, s.dir);   // any nonzero vid: the normal segment
         break;
     case PlanStep::kK2K:
         d.op = kXK2K;
-        d.seg = ctx->seg_of(1, s.pid, s.dir);
+        d.seg = ctx->seg_id(1, s.pid, s.dir);
         break;
     case PlanStep::kC2K:
         d.op = kXC2K;
         d.start_key = make_key(s.start_const, s.pid, s.dir);
-        d.seg = ctx->seg_of(s.start_const, s.pid, s.dir);
+        d.seg = ctx->seg_id(s.start_const, s.pid, s.dir);
         break;
     case PlanStep::kI2K:
         d.op = kXI2K;
         d.start_key = make_key(0, s.start_const, s.dir);
-        d.seg = ctx->seg_of(0, s.start_const, s.dir);
+        d.seg = ctx->seg_id(0, s.start_const, s.dir);
         d.mt = (uint32_t)(s.mt_tid & 0xFFFF) | ((uint32_t)(s.mt_factor & 0xFFFF) << 16);
         break;
     default:
         d.op = kXK2C;
-        d.seg = ctx->seg_of(1, s.pid, s.dir);
+        d.seg = ctx->seg_id(1, s.pid, s.dir);
         break;
     }
     return d;
@@ -564,6 +597,10 @@ int wk::ctx_make_child(wk_ctx* parent, const CtaUse& beside_use, int beside_ctas
     ctx->n_edges = parent->n_edges;
     ctx->segs = parent->segs;
     ctx->index = parent->index;
+    ctx->seg_desc = parent->seg_desc;
+    ctx->d_segs = parent->d_segs;
+    ctx->d_dir_words = parent->d_dir_words;
+    ctx->has_dir = parent->has_dir;
     ctx->has_store = parent->has_store;
     ctx->versatile = parent->versatile;
     ctx->d_pseg = parent->d_pseg;
@@ -622,18 +659,13 @@ extern "C" int wk_ctx_destroy(wk_ctx* ctx) {
     if (!ctx) return WK_E_BADARG;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (wk_ctx* lane : ctx->lanes) wk_ctx_destroy(lane);   // they read this context's store
-    ctx->lanes.clear();
     wk_batch_release(ctx);
     ctx->drop_graphs();
     for (auto& t : ctx->rbuf) {
         if (t.d) cudaFree(t.d);
         if (t.d_rows) cudaFree(t.d_rows);
     }
-    if (ctx->d_slots && !ctx->borrowed_store) cudaFree(ctx->d_slots);
-    if (ctx->d_edges && !ctx->borrowed_store) cudaFree(ctx->d_edges);
-    if (ctx->d_pseg && !ctx->borrowed_store) cudaFree(ctx->d_pseg);
-    if (ctx->d_inline_orig && !ctx->borrowed_store) cudaFree(ctx->d_inline_orig);
+    ctx->drop_store();
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->d_heavy) cudaFree(ctx->d_heavy);
     if (ctx->d_flat) cudaFree(ctx->d_flat);
@@ -680,11 +712,7 @@ extern "C" int wk_store_upload(wk_ctx* ctx, const wk_seg_meta* segs, uint32_t n_
     }
     WK_CUDA(ctx, cudaSetDevice(ctx->device));
     WK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->d_slots) cudaFree(ctx->d_slots);
-    if (ctx->d_edges) cudaFree(ctx->d_edges);
-    ctx->d_slots = nullptr;
-    ctx->d_edges = nullptr;
-    ctx->has_store = false;
+    ctx->drop_store();
     if (wk::dev_malloc(&ctx->d_slots, std::max<uint64_t>(n_slots, wk::kAssoc) * sizeof(wk::Slot)) != cudaSuccess ||
         wk::dev_malloc(&ctx->d_edges, (n_edges + kPadWords) * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();
@@ -700,8 +728,143 @@ extern "C" int wk_store_upload(wk_ctx* ctx, const wk_seg_meta* segs, uint32_t n_
     return wk::store_adopt(ctx, ds, n_slots, de, n_edges, sv);
 }
 
-// Make device arrays the context's store: segment lookup, predicate segment table, the
-// sorted-list check.  The context owns the arrays from here on, on failure too.
+// The segment and predicate segment tables on the device, from seg_desc.
+static int store_tables(wk_ctx* ctx) {
+    const uint32_t n_segs = (uint32_t)ctx->segs.size();
+    std::vector<wk::SegDesc> sd(1 + (size_t)n_segs, wk::SegDesc{});
+    std::copy(ctx->seg_desc.begin(), ctx->seg_desc.end(), sd.begin() + 1);
+    // the predicate segments by pid * 2 + dir, for the versatile steps' list walks; a
+    // vertex-predicate segment (pid PREDICATE_ID) makes the store versatile
+    std::vector<wk::PredSeg> ps;
+    ctx->versatile = false;
+    for (uint32_t i = 0; i < n_segs; ++i) {
+        const wk_seg_meta& m = ctx->segs[i];
+        if (m.index || m.pid >= (1u << wk::kNbitsIdx)) continue;
+        if (m.pid == wk::kPredicateId) ctx->versatile = true;
+        ps.push_back(wk::PredSeg{m.pid * 2 + (uint32_t)m.dir, i, ctx->seg_desc[i]});
+    }
+    std::sort(ps.begin(), ps.end(), [](const wk::PredSeg& a, const wk::PredSeg& b) { return a.key < b.key; });
+    ctx->n_pseg = (uint32_t)ps.size();
+    if (!ctx->d_segs && wk::dev_malloc(&ctx->d_segs, sd.size() * sizeof(wk::SegDesc)) != cudaSuccess) {
+        cudaGetLastError();
+        return ctx->fail(WK_E_OOM, "segment table");
+    }
+    if (!ctx->d_pseg &&
+        wk::dev_malloc(&ctx->d_pseg, std::max<size_t>(ps.size(), 1) * sizeof(wk::PredSeg)) != cudaSuccess) {
+        cudaGetLastError();
+        return ctx->fail(WK_E_OOM, "predicate segment table");
+    }
+    WK_CUDA(ctx, cudaMemcpy(ctx->d_segs, sd.data(), sd.size() * sizeof(wk::SegDesc), cudaMemcpyHostToDevice));
+    if (!ps.empty())
+        WK_CUDA(ctx, cudaMemcpy(ctx->d_pseg, ps.data(), ps.size() * sizeof(wk::PredSeg), cudaMemcpyHostToDevice));
+    return WK_SUCCESS;
+}
+
+// Which segments get a directory: normal segments whose blocks (16 bytes per 64 vertex ids from
+// the lowest to the highest) take no more room than their buckets, when no two segments share
+// buckets and the whole (blocks, and a word per key) fits a quarter of the free device memory.
+// At the default load factor a key has about 180 bytes of buckets, so a segment with a key per
+// 700 ids still gets one: its 16-byte blocks are read from L2 where its buckets are not, and a
+// thinner one reads about as many distinct lines either way.  `vid` holds each segment's lowest
+// and highest id; the segments come back by bucket, with the total of their main buckets and
+// blocks.
+static std::vector<wk::DirSeg> dir_plan(const std::vector<wk_seg_meta>& segs, const std::vector<wk::SegDesc>& desc,
+                                        const std::vector<uint32_t>& vid_of_seg, uint64_t free_bytes,
+                                        std::vector<uint32_t>* which, uint64_t* n_buckets, uint64_t* n_blocks) {
+    std::vector<uint32_t> order;
+    for (uint32_t i = 0; i < segs.size(); ++i)
+        if (segs[i].num_buckets) order.push_back(i);
+    std::sort(order.begin(), order.end(),
+              [&](uint32_t a, uint32_t b) { return segs[a].bucket_start < segs[b].bucket_start; });
+    *n_buckets = *n_blocks = 0;
+    which->clear();
+    std::vector<wk::DirSeg> out;
+    uint64_t end = 0, keys = 0;
+    for (uint32_t i : order) {
+        const wk_seg_meta& m = segs[i];
+        if (m.bucket_start < end) return {};
+        end = m.bucket_start + m.num_buckets;
+        const uint32_t lo = vid_of_seg[2 * i], hi = vid_of_seg[2 * i + 1];
+        if (m.index || lo > hi || hi - lo == 0xFFFFFFFFu) continue;
+        const uint64_t blocks = ((uint64_t)(hi - lo) + 64) / 64;
+        if (blocks * sizeof(wk::DirBlock) > m.num_buckets * wk::kAssoc * sizeof(wk::Slot)) continue;
+        wk::DirSeg d{};
+        d.first = *n_buckets;
+        d.block0 = *n_blocks;
+        d.seg = desc[i];
+        d.seg.vid_lo = lo;
+        d.seg.vid_span = hi - lo + 1;
+        d.key = m.pid * 2 + (uint32_t)m.dir;
+        *n_buckets += m.num_buckets;
+        *n_blocks += blocks;
+        keys += m.num_keys;
+        which->push_back(i);
+        out.push_back(d);
+    }
+    if (*n_blocks * sizeof(wk::DirBlock) + keys * 8 > free_bytes / 4) return {};
+    return out;
+}
+
+// The vertex directories of a store (see wk_dir.cu).  A store that cannot have them (or whose
+// device has no room) keeps the hash probes: that is no error.
+static int build_directories(wk_ctx* ctx, const std::vector<uint32_t>& vid_of_seg, wk::StoreScan* d_scan) {
+    size_t free_b = 0, total_b = 0;
+    WK_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
+    std::vector<uint32_t> which;
+    uint64_t n_buckets = 0, n_blocks = 0;
+    std::vector<wk::DirSeg> ds = dir_plan(ctx->segs, ctx->seg_desc, vid_of_seg, free_b, &which, &n_buckets, &n_blocks);
+    if (ds.empty()) return WK_SUCCESS;
+    const uint64_t n_sums = (n_blocks + wk::kDirScanBlocks - 1) / wk::kDirScanBlocks;
+    wk::DirSeg* d_ds = nullptr;
+    uint64_t* d_sums = nullptr;
+    wk::DirBlock* blocks = nullptr;
+    uint64_t* words = nullptr;
+    auto drop = [&](int rc) {
+        cudaFree(d_ds);
+        cudaFree(d_sums);
+        cudaFree(blocks);
+        cudaFree(words);
+        return rc;
+    };
+    if (wk::dev_malloc(&d_ds, ds.size() * sizeof(wk::DirSeg)) != cudaSuccess ||
+        wk::dev_malloc(&d_sums, (n_sums + 1) * 8) != cudaSuccess ||
+        wk::dev_malloc(&blocks, n_blocks * sizeof(wk::DirBlock)) != cudaSuccess) {
+        cudaGetLastError();
+        return drop(WK_SUCCESS);
+    }
+    for (auto& d : ds) d.seg.dir = blocks + d.block0;
+    cudaStream_t s = ctx->stream;
+    uint64_t n_words = 0;
+    wk::StoreScan h{};
+    cudaError_t e = cudaMemcpyAsync(d_ds, ds.data(), ds.size() * sizeof(wk::DirSeg), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(blocks, 0, n_blocks * sizeof(wk::DirBlock), s);
+    if (e == cudaSuccess)
+        e = wk::launch_dir_bits(ctx->dev_store(), d_ds, (uint32_t)ds.size(), n_buckets, blocks, n_blocks, d_sums, d_scan,
+                                ctx->sm_count, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&n_words, d_sums + n_sums, 8, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_scan, sizeof(h), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return drop(ctx->cuda_fail(e, "vertex directories"));
+    if (h.flags & (wk::kStoreBadChain | wk::kStoreDupKey)) return drop(WK_SUCCESS);
+    if (wk::dev_malloc(&words, std::max<uint64_t>(n_words, 1) * 8) != cudaSuccess) {
+        cudaGetLastError();
+        return drop(WK_SUCCESS);
+    }
+    e = wk::launch_dir_fill(ctx->dev_store(), d_ds, (uint32_t)ds.size(), n_buckets, words, d_scan, ctx->sm_count, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return drop(ctx->cuda_fail(e, "vertex directories"));
+    ctx->d_dir_blocks = blocks;
+    ctx->d_dir_words = words;
+    blocks = nullptr;
+    words = nullptr;
+    ctx->has_dir = true;
+    for (size_t k = 0; k < ds.size(); ++k) ctx->seg_desc[which[k]] = ds[k].seg;
+    return drop(store_tables(ctx));
+}
+
+// Make device arrays the context's store: segment lookup, predicate segment table, the list
+// checks, the one-entry lists, the vertex directories.  The context owns the arrays from here
+// on, on failure too.
 int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_edges, uint64_t n_edges,
                     const std::vector<wk_seg_meta>& segs) {
     ctx->d_slots = d_slots;
@@ -712,29 +875,10 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
     const uint32_t n_segs = (uint32_t)segs.size();
     ctx->segs = segs;
     ctx->index.build(ctx->segs.data(), n_segs);
-    {
-        // the predicate segments by pid * 2 + dir, for the versatile steps' list walks; a
-        // vertex-predicate segment (pid PREDICATE_ID) makes the store versatile
-        std::vector<wk::PredSeg> ps;
-        ctx->versatile = false;
-        for (uint32_t i = 0; i < n_segs; ++i) {
-            const wk_seg_meta& m = segs[i];
-            if (m.index || m.pid >= (1u << wk::kNbitsIdx)) continue;
-            if (m.pid == wk::kPredicateId) ctx->versatile = true;
-            ps.push_back(wk::PredSeg{m.pid * 2 + (uint32_t)m.dir, 0, wk::to_desc(m)});
-        }
-        std::sort(ps.begin(), ps.end(), [](const wk::PredSeg& a, const wk::PredSeg& b) { return a.key < b.key; });
-        if (ctx->d_pseg) cudaFree(ctx->d_pseg);
-        ctx->d_pseg = nullptr;
-        ctx->n_pseg = 0;
-        if (wk::dev_malloc(&ctx->d_pseg, std::max<size_t>(ps.size(), 1) * sizeof(wk::PredSeg)) != cudaSuccess) {
-            cudaGetLastError();
-            return ctx->fail(WK_E_OOM, "predicate segment table");
-        }
-        if (!ps.empty())
-            WK_CUDA(ctx, cudaMemcpy(ctx->d_pseg, ps.data(), ps.size() * sizeof(wk::PredSeg), cudaMemcpyHostToDevice));
-        ctx->n_pseg = (uint32_t)ps.size();
-    }
+    ctx->seg_desc.clear();
+    for (auto& m : segs) ctx->seg_desc.push_back(to_desc(m));
+    int rc = store_tables(ctx);
+    if (rc) return rc;
     {
         // the index lists' lengths (the keys [0|tpid|dir] of the two index segments: a few
         // buckets per predicate and type), which the serving admission projects from
@@ -759,65 +903,63 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
             }
         }
     }
+    // one pass over the slots: are all lists inside the edge array, ascending and unique (which
+    // lets the filters binary-search long lists); the one-entry lists counted; each segment's
+    // vertex ids
+    cudaStream_t s = ctx->stream;
+    const uint32_t np = ctx->n_pseg;
+    struct Scan {   // the scan's results, behind them the segments' id ranges, then the chunks
+        StoreScan* d = nullptr;
+        ~Scan() { cudaFree(d); }
+    } scan;
+    const size_t scan_bytes = sizeof(StoreScan) + 8ull * np;
+    const size_t chunks_at = (scan_bytes + 15) & ~(size_t)15;
+    const uint32_t max_chunks = store_scan_chunks(n_edges);
+    std::vector<unsigned char> hs(scan_bytes, 0);
+    uint32_t* hv = reinterpret_cast<uint32_t*>(hs.data() + sizeof(StoreScan));
+    for (uint32_t i = 0; i < np; ++i) hv[2 * i] = 0xFFFFFFFFu;
+    if (dev_malloc(&scan.d, chunks_at + 16ull * max_chunks) != cudaSuccess) {
+        cudaGetLastError();
+        return ctx->fail(WK_E_OOM, "store check");
+    }
+    uint32_t* d_vid = reinterpret_cast<uint32_t*>(scan.d + 1);
+    cudaError_t e = cudaMemcpyAsync(scan.d, hs.data(), scan_bytes, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess && n_slots)
+        e = launch_store_scan(ctx->dev_store(), ctx->d_pseg, np, d_vid, scan.d,
+                              reinterpret_cast<ulonglong2*>(reinterpret_cast<char*>(scan.d) + chunks_at), max_chunks,
+                              ctx->sm_count, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hs.data(), scan.d, scan_bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return ctx->cuda_fail(e, "store check");
+    StoreScan found;
+    std::memcpy(&found, hs.data(), sizeof(found));
+    if (found.flags & kStoreBadList) return ctx->fail(WK_E_CORRUPT, "a key's list lies outside the edge array");
+    ctx->sorted_lists = (found.flags & kStoreUnsorted) ? 0 : 1;
+    if (found.flags & kStoreInlineType)
+        return ctx->fail(WK_E_UNSUPPORTED, "a pointer word of type 3 (attribute values are not served)");
+    // one-entry lists into their keys' pointer words, the original words kept aside
+    if (found.n_inline) {
+        if (dev_malloc(&ctx->d_inline_orig, found.n_inline * 16) != cudaSuccess) {
+            cudaGetLastError();
+            return ctx->fail(WK_E_OOM, "one-entry list table");
+        }
+        ctx->n_inline = found.n_inline;
+        e = cudaMemsetAsync(&scan.d->n_inline, 0, sizeof(scan.d->n_inline), s);
+        if (e == cudaSuccess) e = launch_inline(ctx->dev_store(), &scan.d->n_inline, ctx->d_inline_orig, ctx->sm_count, s);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "one-entry lists");
+    }
+    if (!(found.flags & kStoreBadChain)) {
+        std::vector<uint32_t> vid(2ull * n_segs);
+        for (uint32_t i = 0; i < n_segs; ++i) vid[2 * i] = 0xFFFFFFFFu;
+        std::vector<PredSeg> ps(np);   // which segment each range belongs to
+        if (np) WK_CUDA(ctx, cudaMemcpy(ps.data(), ctx->d_pseg, np * sizeof(PredSeg), cudaMemcpyDeviceToHost));
+        for (uint32_t i = 0; i < np; ++i) std::memcpy(&vid[2ull * ps[i].seg_no], hv + 2 * i, 8);
+        rc = build_directories(ctx, vid, scan.d);
+        if (rc) return rc;
+    }
+    e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return ctx->cuda_fail(e, "one-entry lists");
     ctx->has_store = true;
-    {
-        // are all lists ascending + unique?  (lets the filters binary-search long lists)
-        unsigned* d_flag = nullptr;
-        WK_CUDA(ctx, wk::dev_malloc(&d_flag, sizeof(unsigned)));
-        WK_CUDA(ctx, cudaMemsetAsync(d_flag, 0, sizeof(unsigned), ctx->stream));
-        cudaError_t e = wk::launch_sorted_check(ctx->dev_store(), d_flag, ctx->stream);
-        unsigned flag = 0;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&flag, d_flag, sizeof(flag), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        cudaFree(d_flag);
-        if (e != cudaSuccess) return ctx->cuda_fail(e, "sorted-list check");
-        if (flag & 2u) {
-            ctx->has_store = false;
-            return ctx->fail(WK_E_CORRUPT, "a key's list lies outside the edge array");
-        }
-        ctx->sorted_lists = (flag & 1u) ? 0 : 1;
-    }
-    {
-        // one-entry lists into their keys' pointer words, the original words kept aside: count,
-        // then convert
-        if (ctx->d_inline_orig) cudaFree(ctx->d_inline_orig);
-        ctx->d_inline_orig = nullptr;
-        ctx->n_inline = 0;
-        struct Counts {
-            unsigned long long n;
-            unsigned clash, pad;
-        };
-        Counts* d_c = nullptr;
-        Counts h_c{};
-        WK_CUDA(ctx, wk::dev_malloc(&d_c, sizeof(Counts)));
-        cudaError_t e = cudaMemsetAsync(d_c, 0, sizeof(Counts), ctx->stream);
-        if (e == cudaSuccess) e = wk::launch_inline(ctx->dev_store(), &d_c->n, &d_c->clash, nullptr, ctx->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h_c, d_c, sizeof(Counts), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e == cudaSuccess && !h_c.clash && h_c.n) {
-            if (wk::dev_malloc(&ctx->d_inline_orig, h_c.n * 16) != cudaSuccess) {
-                cudaGetLastError();
-                cudaFree(d_c);
-                ctx->has_store = false;
-                return ctx->fail(WK_E_OOM, "one-entry list table");
-            }
-            e = cudaMemsetAsync(d_c, 0, sizeof(Counts), ctx->stream);
-            if (e == cudaSuccess)
-                e = wk::launch_inline(ctx->dev_store(), &d_c->n, &d_c->clash, ctx->d_inline_orig, ctx->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-            ctx->n_inline = h_c.n;
-        }
-        cudaFree(d_c);
-        if (e != cudaSuccess) {
-            ctx->has_store = false;
-            return ctx->cuda_fail(e, "one-entry lists");
-        }
-        if (h_c.clash) {
-            ctx->has_store = false;
-            return ctx->fail(WK_E_UNSUPPORTED, "a pointer word of type 3 (attribute values are not served)");
-        }
-    }
-    ctx->drop_graphs();
     return WK_SUCCESS;
 }
 

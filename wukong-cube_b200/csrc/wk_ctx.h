@@ -88,6 +88,13 @@ struct wk_ctx {
     uint64_t n_edges = 0;
     std::vector<wk_seg_meta> segs;
     wk::SegIndex index;
+    std::vector<wk::SegDesc> seg_desc;   // of each segment, with its directory
+    wk::SegDesc* d_segs = nullptr;       // DevStore::segs: an absent segment, then seg_desc
+    wk::DirBlock* d_dir_blocks = nullptr;   // vertex directories (wk_dir.cu)
+    uint64_t* d_dir_words = nullptr;
+    bool has_dir = false;                // some segment has a directory
+    uint64_t store_gen = 0;              // stores this context has held (captured launches hold
+                                         // the addresses of theirs)
     bool has_store = false;
     bool versatile = false;           // the store holds the vertex-predicate lists
     wk::PredSeg* d_pseg = nullptr;    // predicate segments by pid * 2 + dir (versatile steps)
@@ -152,13 +159,18 @@ struct wk_ctx {
         s.n_buckets = n_slots / wk::kAssoc;
         s.edges = d_edges;
         s.n_edges = n_edges;
+        s.segs = d_segs;
+        s.dir_words = d_dir_words;
         return s;
     }
     wk::SegDesc seg_of(uint64_t vid, uint32_t pid, int dir) const {
-        int32_t i = index.find(vid, pid, dir);
-        wk::SegDesc d{0, 0, 0, 0};
-        if (i >= 0 && pid < (1u << wk::kNbitsIdx)) d = wk::to_desc(segs[i]);
-        return d;
+        const uint32_t i = seg_id(vid, pid, dir);
+        return i ? seg_desc[i - 1] : wk::SegDesc{};
+    }
+    // its entry in DevStore::segs (0: absent)
+    uint32_t seg_id(uint64_t vid, uint32_t pid, int dir) const {
+        const int32_t i = index.find(vid, pid, dir);
+        return i >= 0 && pid < (1u << wk::kNbitsIdx) ? (uint32_t)i + 1 : 0;
     }
     int fail(int code, const std::string& msg) {
         last_error = msg;
@@ -169,15 +181,20 @@ struct wk_ctx {
         return WK_E_CUDA;
     }
     int blocks_per_sm(int op, int cols, int lanes);
+    // Lanes per probe group of a launch that asks for `lanes`: a store with vertex directories is
+    // looked up by one thread per row (a directory lookup is one block and one word, so a group
+    // has nothing to share); the group widths serve stores without.
+    int probe_lanes(int lanes) const { return has_dir ? 1 : lanes; }
     // lanes per probe group for (op, cols): the tuned choice, else 2 (one 32-byte sector)
     int lanes_for(int op, int cols) const {
         auto it = tuned_lanes.find(op * 1000 + cols);
-        return it != tuned_lanes.end() ? it->second : default_lanes;
+        return probe_lanes(it != tuned_lanes.end() ? it->second : default_lanes);
     }
     void drop_graphs();
     int ensure_status(uint64_t tiles);
     int ensure_heavy(uint64_t out_rows_cap);
     int ensure_flat(uint64_t in_rows_cap);
+    void drop_store();
     int final_scratch_reserve(size_t bytes);
     int table_reserve(wk_table* t, uint64_t elems);
     int read_ctl(uint32_t* err, uint64_t* need);

@@ -152,6 +152,17 @@ __device__ __forceinline__ uint32_t list_at(const uint32_t* edges, uint64_t off,
     return (off & kInlineTag) ? (uint32_t)off : __ldg(edges + off + k);
 }
 
+// ---------------------------------------------------------------- vertex directory
+// Pointer word of id `i` of a directory (i < vid_span) whose block is `b`; 0 when absent.
+__device__ __forceinline__ ulonglong2 dir_block(const SegDesc& s, uint32_t i) {
+    return __ldg(reinterpret_cast<const ulonglong2*>(s.dir) + (i >> 6));
+}
+__device__ __forceinline__ uint64_t dir_word(const DevStore& st, ulonglong2 b, uint32_t i) {
+    const unsigned long long bit = 1ull << (i & 63);
+    return (b.x & bit) ? __ldg(reinterpret_cast<const unsigned long long*>(st.dir_words) + b.y + __popcll(b.x & (bit - 1)))
+                       : 0;
+}
+
 // Probe kUnroll keys per group of L lanes.  Every lane of the warp must call this (ballots and
 // shuffles are warp-wide).  On entry bucket[u] is the key's home bucket and pending[u] says
 // whether to look; on return ptr[u] is the slot's pointer word in every lane of the group, or 0
@@ -260,11 +271,53 @@ __device__ __forceinline__ uint64_t thread_probe(const DevStore& st, uint64_t ke
     return 0;
 }
 
-// Is `target` in the list edges[off, off + deg)?  Binary search when lists are sorted.  `off`
-// may be a tagged single entry.
+// thread_probe from the key's home bucket, out of line: in a kernel whose lookups go by directory
+// it is the rare case, and inlined it costs the others their registers.
+__device__ __noinline__ uint64_t hash_lookup(const Slot* slots, uint64_t n_buckets, uint64_t bucket_start,
+                                             uint64_t num_buckets, uint64_t magic, uint64_t key, unsigned* err) {
+    DevStore st{};
+    st.slots = slots;
+    st.n_buckets = n_buckets;
+    return thread_probe(st, key, bucket_start + mod_barrett(hash_u64(key), num_buckets, magic), err);
+}
+__device__ __forceinline__ uint64_t hash_lookup(const DevStore& st, const SegDesc& sg, uint64_t key, unsigned* err) {
+    return hash_lookup(st.slots, st.n_buckets, sg.bucket_start, sg.num_buckets, sg.magic, key, err);
+}
+
+// Pointer word of `key`, whose vertex is `vid` and whose segment is `sg` (num_buckets != 0, key
+// != 0): by the segment's directory where it has one, else by hash.
+__device__ __forceinline__ uint64_t seg_lookup(const DevStore& st, const SegDesc& sg, uint64_t key, uint32_t vid,
+                                               unsigned* err) {
+    if (sg.vid_span) {
+        const uint32_t i = vid - sg.vid_lo;
+        return i < sg.vid_span ? dir_word(st, dir_block(sg, i), i) : 0;
+    }
+    return hash_lookup(st, sg, key, err);
+}
+
+// Is `target` in the list edges[off, off + deg)?  A short list is compared whole, through the
+// aligned 16-byte quads that hold it, two in flight (one or two round trips where a binary search
+// of five entries makes three or four; the edge array is padded past its end); a longer one by
+// binary search when lists are sorted.  `off` may be a tagged single entry.
+constexpr uint64_t kQuadList = 12;
 __device__ __forceinline__ bool thread_member(const uint32_t* edges, uint64_t off, uint64_t deg,
                                               uint32_t target, bool sorted) {
     if (off & kInlineTag) return deg == 1 && (uint32_t)off == target;
+    if (deg <= kQuadList) {
+        const uint4* q = reinterpret_cast<const uint4*>(edges) + (off >> 2);
+        const int lo = (int)(off & 3), hi = lo + (int)deg;   // the list's words among the quads'
+        bool hit = false;
+        for (int k = 0; k < hi && !hit; k += 8) {
+            const uint4 a = __ldg(q + (k >> 2));
+            uint4 b = make_uint4(0, 0, 0, 0);
+            if (k + 4 < hi) b = __ldg(q + (k >> 2) + 1);
+            hit = (a.x == target && k >= lo && k < hi) || (a.y == target && k + 1 >= lo && k + 1 < hi) ||
+                  (a.z == target && k + 2 >= lo && k + 2 < hi) || (a.w == target && k + 3 >= lo && k + 3 < hi) ||
+                  (b.x == target && k + 4 < hi) || (b.y == target && k + 5 < hi) ||
+                  (b.z == target && k + 6 < hi) || (b.w == target && k + 7 < hi);
+        }
+        return hit;
+    }
     const uint32_t* p = edges + off;
     if (sorted) {
         uint64_t lo = 0, hi = deg;

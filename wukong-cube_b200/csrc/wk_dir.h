@@ -1,0 +1,60 @@
+// Load-time passes over a store on the device (wk_dir.cu): the checks of its lists, the
+// one-entry lists moved into their keys' slots, and the vertex directories.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "wk_kernels.h"
+#include "wk_versatile.h"
+
+namespace wk {
+
+// What the first pass finds.
+enum : uint32_t {
+    kStoreUnsorted = 1u,   // a list is not strictly ascending
+    kStoreBadList = 2u,    // a list lies outside the edge array
+    kStoreInlineType = 4u, // a pointer word already carries the inline type
+    kStoreBadChain = 8u,   // a chain link past the slot array, or a chain that does not end
+    kStoreDupKey = 16u,    // a key twice in one chain
+};
+struct StoreScan {
+    unsigned long long n_inline;   // keys whose list has one entry
+    unsigned int flags;
+    unsigned int n_chunks;         // chunks of long lists
+};
+constexpr uint64_t kChunkList = 8192;   // entries of a long list checked by one warp
+inline uint32_t store_scan_chunks(uint64_t n_edges) {   // room for every chunk of disjoint lists
+    return (uint32_t)(2 * n_edges / kChunkList) + 1;
+}
+
+// Pass over every slot: the checks, the one-entry lists counted, and the lowest and highest
+// vertex id of each predicate segment's keys (vid[2 * i], vid[2 * i + 1] for pseg[i]; the
+// caller sets them to 0xFFFFFFFF and 0; ids of 2^32 or more are left out).  `chunks`:
+// store_scan_chunks(n_edges) entries of scratch.
+cudaError_t launch_store_scan(const DevStore& st, const PredSeg* pseg, uint32_t n_pseg, uint32_t* vid, StoreScan* out,
+                              ulonglong2* chunks, uint32_t max_chunks, int sm_count, cudaStream_t s);
+// One-entry lists into their keys' pointer words; the original words (slot index, word) go to
+// orig, counted in *n (0 on entry).
+cudaError_t launch_inline(const DevStore& st, unsigned long long* n, uint64_t* orig, int sm_count, cudaStream_t s);
+
+// A segment whose directory is built: its main buckets (disjoint from every other's), the keys'
+// predicate and direction, and where its blocks start among all blocks.
+struct DirSeg {
+    uint64_t first;          // main buckets of the segments before it in the table
+    uint64_t block0;
+    SegDesc seg;             // vid_lo, vid_span and (for the fill) dir set
+    uint32_t key;            // pid * 2 + dir
+    uint32_t pad;
+};
+// Set the presence bits of every key a probe of its segment finds (flags: kStoreBadChain,
+// kStoreDupKey), then each block's base: blocks[] and sums[] (one per kDirScanBlocks blocks, plus
+// the total, which *words receives) on the device.
+constexpr uint32_t kDirScanBlocks = 2048;
+cudaError_t launch_dir_bits(const DevStore& st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets,
+                            DirBlock* blocks, uint64_t n_blocks, uint64_t* sums, StoreScan* out, int sm_count,
+                            cudaStream_t s);
+// Put every key's pointer word in its place.
+cudaError_t launch_dir_fill(const DevStore& st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets,
+                            uint64_t* words, StoreScan* out, int sm_count, cudaStream_t s);
+
+}  // namespace wk

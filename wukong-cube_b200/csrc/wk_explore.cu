@@ -68,7 +68,7 @@ __shared__ long long s_ph_t;
 #endif
 
 // The step every row of a finished query runs: nothing.
-__constant__ StepDesc c_done = {{0, 0, 0, 0}, 0, 0, 0, kXDone, 0, 0, 0, 0, 0, 0, 0, 0};
+__constant__ StepDesc c_done = {0, 0, 0, 0, kXDone, 0, 0, 0, 0, 0, 0, 0, 0};
 
 // Rows with more output rows than this are written as slices from the queue.  At most 2^23, so
 // a tile's short-row outputs (256 rows) stay below 2^31 and their scan fits 32 bits.
@@ -168,15 +168,14 @@ __device__ __forceinline__ TileBuf tile_buf(uint32_t* base, int wi) {
     return b;
 }
 
-// Setup of one row of a tile: its step (descriptor), probe key, home bucket and filter target,
-// and the flag op | valid << 8 | pending << 9 | cin << 16 | cout << 24; records the row's meta.
-__device__ __forceinline__ void row_setup(const ExploreArgs& a, const TileBuf& B, int row, int wi,
-                                          uint64_t* key_out, uint32_t* bkt_out, uint32_t* tgt_out,
-                                          uint32_t* flag_out) {
+// Setup of one row of a tile: its step (descriptor), probe key, segment and filter target, and the
+// flag op | valid << 8 | pending << 9 | cin << 16 | cout << 24; records the row's meta.
+__device__ __forceinline__ const SegDesc* row_setup(const ExploreArgs& a, const TileBuf& B, int row, int wi,
+                                                    uint64_t* key_out, uint32_t* tgt_out, uint32_t* flag_out) {
     const StepDesc* d = step_desc(a, B.q[row]);
     const uint32_t op = d->op;
     bool valid = op != kXDone;
-    const SegDesc* sg = &d->seg;
+    const SegDesc* sg = a.store.segs + d->seg;
     uint32_t target = d->end_const;
     uint64_t key = 0;
     if (op == kXStart) {
@@ -192,21 +191,21 @@ __device__ __forceinline__ void row_setup(const ExploreArgs& a, const TileBuf& B
         if (op == kXK2U && d->type_index) {
             // get_index(cur, IN) (sparql.hpp:342-345); only 17-bit ids can be keys
             key = make_key(0, cur, kIn);
-            sg = &a.seg_index[kIn];
+            sg = a.store.segs + a.seg_index[kIn];
             if (cur >= (1u << kNbitsIdx)) valid = false;
         } else {
             key = make_key(cur, d->pid, d->dir);
-            if (cur == 0) sg = &a.seg_index[d->dir & 1];   // vid 0 names the index
+            if (cur == 0) sg = a.store.segs + (d->dir & 1 ? a.seg_index[1] : a.seg_index[0]);   // vid 0 names the index
         }
         if (cur == kBlankId) valid = false;
     }
     const bool pending = valid && sg->num_buckets != 0 && key != 0;
     const uint32_t cin = d->cin, cout = d->cout;
     *key_out = key;
-    *bkt_out = pending ? (uint32_t)bucket_of(key, *sg) : 0;   // 32 bits (stores are refused at 2^32)
     *tgt_out = target;
     *flag_out = op | (valid ? 0x100u : 0u) | (pending ? 0x200u : 0u) | (cin << 16) | (cout << 24);
     B.meta[row] = op | (cin << 8) | (cout << 16);
+    return sg;
 }
 
 // A row's count and list offset (an edge-array offset or a tagged single entry) once its list
@@ -227,48 +226,49 @@ __device__ __forceinline__ uint32_t row_count(const ExploreArgs& a, const TileBu
     return cnt;
 }
 
-// One thread per row (the L = 1 launch): each thread sets up its tile rows, loads every row's
-// home sector (slots 0 and 1, 32 bytes) before comparing any, and walks on from slot 2 only
-// where that sector does not settle the key; filters then search the list themselves.  No
-// ballots or shuffles.
+// One thread per row (the L = 1 launch): each thread sets up its tile rows, then looks each row's
+// key up: by its segment's vertex directory (every row's block loaded before any word), or, for a
+// segment without one, by its home bucket's first sector and the walk.  Filters then search the
+// list themselves.  No ballots or shuffles.
 __device__ __forceinline__ void tile_probe_rows(const ExploreArgs& a, const TileBuf& B, TileState& S, int n, int wi,
                                                 unsigned long long& acc_alg, unsigned long long& acc_sd) {
     constexpr int kRows = kTileRows / kStepThreads;
     uint64_t key[kRows];
-    uint32_t bkt[kRows], tgt[kRows], flag[kRows];
+    uint32_t tgt[kRows], flag[kRows], id[kRows];
+    const SegDesc* sg[kRows];
+    ulonglong2 blk[kRows];
+    constexpr uint32_t kNoDir = 0xFFFFFFFFu;   // the row's segment has no directory
 #pragma unroll
     for (int k = 0; k < kRows; ++k) {
         const int row = threadIdx.x + k * kStepThreads;
         key[k] = 0;
-        bkt[k] = 0;
         tgt[k] = 0;
+        id[k] = 0;
         flag[k] = kXDone;
-        if (row < n) row_setup(a, B, row, wi, &key[k], &bkt[k], &tgt[k], &flag[k]);
-        if ((flag[k] & 0x200u) && bkt[k] >= a.store.n_buckets) {
-            atomicOr(&a.ctl->err, kErrCorrupt);
-            flag[k] &= ~0x200u;
+        blk[k] = make_ulonglong2(0, 0);
+        if (row < n) sg[k] = row_setup(a, B, row, wi, &key[k], &tgt[k], &flag[k]);
+        if (flag[k] & 0x200u) {
+            const uint32_t span = __ldg(&sg[k]->vid_span);
+            id[k] = (uint32_t)key_vid(key[k]) - __ldg(&sg[k]->vid_lo);
+            if (!span) id[k] = kNoDir;
+            else if (id[k] < span) blk[k] = dir_block(*sg[k], id[k]);
+            else id[k] = 0;   // outside the directory: no key (blk stays empty)
         }
     }
-    ulonglong2 s0[kRows], s1[kRows];
+    uint64_t p[kRows];
 #pragma unroll
     for (int k = 0; k < kRows; ++k) {
-        s0[k] = make_ulonglong2(0, 0);
-        s1[k] = make_ulonglong2(0, 0);
-        if (flag[k] & 0x200u) load_sector(a.store.slots + (uint64_t)bkt[k] * kAssoc, &s0[k], &s1[k]);
+        p[k] = 0;
+        if (!(flag[k] & 0x200u)) continue;
+        if (id[k] != kNoDir) p[k] = dir_word(a.store, blk[k], id[k]);
+        else p[k] = hash_lookup(a.store, *sg[k], key[k], &a.ctl->err);
     }
 #pragma unroll
     for (int k = 0; k < kRows; ++k) {
         const int row = threadIdx.x + k * kStepThreads;
         if (row >= n || !(flag[k] & 0x100u)) continue;
-        uint64_t p = 0;
-        if (flag[k] & 0x200u) {
-            if (s0[k].x == key[k]) p = s0[k].y;
-            else if (s0[k].x == 0) p = 0;   // first empty slot: absent (insert-only store)
-            else if (s1[k].x == key[k]) p = s1[k].y;
-            else if (s1[k].x != 0) p = thread_probe(a.store, key[k], bkt[k], &a.ctl->err, 2);
-        }
         uint64_t off, deg;
-        list_of_ptr(p, a.store.n_edges, &a.ctl->err, &off, &deg);
+        list_of_ptr(p[k], a.store.n_edges, &a.ctl->err, &off, &deg);
         const uint32_t op = flag[k] & 0xFFu;
         if (op == kXI2K) {   // index_to_known reads its mt slice of the list (a one-entry list
             uint64_t lo, hi;   // keeps its entry: its slice starts at 0)
@@ -337,7 +337,11 @@ __device__ __forceinline__ void tile_front(const ExploreArgs& a, const TileBuf& 
             mbkt[j] = 0;
             mtgt[j] = 0;
             mflag[j] = kXDone;
-            if (u < kUnroll && row < n) row_setup(a, B, row, wi, &mkey[j], &mbkt[j], &mtgt[j], &mflag[j]);
+            if (u < kUnroll && row < n) {
+                const SegDesc* sg = row_setup(a, B, row, wi, &mkey[j], &mtgt[j], &mflag[j]);
+                // 32 bits: stores of 2^32 buckets or more are refused
+                if (mflag[j] & 0x200u) mbkt[j] = (uint32_t)bucket_of(mkey[j], *sg);
+            }
         }
         uint64_t key[kUnroll], ptr[kUnroll];
         uint32_t bucket[kUnroll];

@@ -19,10 +19,10 @@ __host__ __device__ inline bool is_filter_op(uint32_t op) {
     return op == kXK2K || op == kXK2C || op == kXC2K || op == kXI2K;
 }
 
-// One query's step at one level (64 bytes).
+// One query's step at one level (32 bytes).
 struct StepDesc {
-    SegDesc seg;            // segment of the step's normal key, or of the start key
     uint64_t start_key;     // kXStart: the constant / index key whose list starts the table
+    uint32_t seg;           // DevStore::segs entry of the step's normal key, or of the start key
     uint32_t pid;
     uint32_t end_const;     // kXK2C
     uint8_t op, dir, cin, cout;
@@ -38,7 +38,7 @@ __host__ __device__ inline void mt_slice(uint32_t mt, uint64_t deg, uint64_t* lo
     *lo = (tid % factor) * len;
     *hi = (tid % factor) == factor - 1 ? deg : *lo + len;
 }
-static_assert(sizeof(StepDesc) == 64, "StepDesc is 64 bytes");
+static_assert(sizeof(StepDesc) == 32, "StepDesc is 32 bytes");
 
 // A slice of a long neighbour list.  Rows whose count exceeds kHeavyRows are not written by
 // the CTA that scanned them: it queues them as kHeavyChunk-row slices, and CTAs that run out of
@@ -61,7 +61,7 @@ constexpr int kPhaseSlots = 12;  // phase cycle counters of an instrumented buil
 
 struct ExploreArgs {
     DevStore store;
-    SegDesc seg_index[2];        // index segment of each direction
+    uint32_t seg_index[2];       // DevStore::segs entries of the two index segments
     StepDesc one;                // the step of every row when desc is null
     const StepDesc* desc;        // [n_queries] this level's step per query, or null
     // Continuous batching: when desc_stride > 0, query q's step is

@@ -118,57 +118,50 @@ __device__ __forceinline__ bool last_count_cta(StepCtl* ctl) {
     return s_last != 0;
 }
 
-// Key of a row of the count pass: the step's start key (const_to_known / index_to_known) or
-// [cur|pid|dir] (the index key of get_index for the TYPE_ID/IN form, and for vid 0); *look is
-// false where there is nothing to probe.
-__device__ __forceinline__ uint64_t count_key(const FlatArgs& a, const StepDesc& d, bool from_const, uint32_t cur,
-                                              bool* valid, bool* look, uint64_t* bucket) {
-    uint64_t key;
-    SegDesc sg = d.seg;   // by value: registers, not a pointer into the parameter block
+// Pointer word of a row of the count pass: of the step's start key (const_to_known /
+// index_to_known) or of [cur|pid|dir] (the index key of get_index for the TYPE_ID/IN form, and for
+// vid 0); *valid is false for a row that takes no part.  kDir: the step's segment has a directory.
+template <bool kDir>
+__device__ __forceinline__ uint64_t count_ptr(const FlatArgs& a, const StepDesc& d, bool from_const, uint32_t cur,
+                                              bool* valid) {
     *valid = from_const || cur != kBlankId;
-    if (from_const) {
-        key = d.start_key;
-    } else if (d.op == kXK2U && d.type_index) {
-        // get_index(cur, IN) (sparql.hpp:342-345); only 17-bit ids can be keys
-        key = make_key(0, cur, kIn);
-        sg = a.seg_index[kIn];
-        if (cur >= (1u << kNbitsIdx)) *valid = false;
-    } else {
-        key = make_key(cur, d.pid, d.dir);
-        if (cur == 0) sg = a.seg_index[d.dir & 1];   // vid 0 names the index
+    if (!*valid) return 0;
+    if (!from_const && !(d.op == kXK2U && d.type_index) && cur != 0) {
+        if (kDir) {
+            const uint32_t i = cur - a.seg.vid_lo;
+            return i < a.seg.vid_span ? dir_word(a.store, dir_block(a.seg, i), i) : 0;
+        }
+        if (a.seg.num_buckets == 0) return 0;
+        const uint64_t key = make_key(cur, d.pid, d.dir);
+        return thread_probe(a.store, key, bucket_of(key, a.seg), &a.ctl->err);
     }
-    *look = *valid && sg.num_buckets != 0 && key != 0;
-    *bucket = *look ? bucket_of(key, sg) : 0;
-    if (*look && *bucket >= a.store.n_buckets) {
-        atomicOr(&a.ctl->err, kErrCorrupt);
-        *look = false;
+    uint64_t key = d.start_key;
+    uint64_t b0 = a.seg.bucket_start, nb = a.seg.num_buckets, magic = a.seg.magic;
+    if (!from_const) {
+        // get_index(cur, IN) (sparql.hpp:342-345), only 17-bit ids can be keys; else vid 0, which
+        // names the index
+        const bool type = d.op == kXK2U && d.type_index;
+        const int dir = type ? kIn : (d.dir & 1);
+        key = make_key(0, type ? cur : d.pid, dir);
+        const SegDesc* sg = a.store.segs + (dir ? a.seg_index[1] : a.seg_index[0]);
+        b0 = sg->bucket_start;
+        nb = sg->num_buckets;
+        magic = sg->magic;
+        if (type && cur >= (1u << kNbitsIdx)) *valid = false;
     }
-    return key;
+    if (!*valid || nb == 0 || key == 0) return 0;
+    return hash_lookup(a.store.slots, a.store.n_buckets, b0, nb, magic, key, &a.ctl->err);
 }
 
-// Pointer word of `key` given its home bucket's slots 0 and 1 (one 32-byte sector, loaded
-// together); the walk goes on from slot 2 only when they do not settle the key.
-__device__ __forceinline__ uint64_t settle_slot(const DevStore& st, uint64_t key, uint64_t b, ulonglong2 s0,
-                                                ulonglong2 s1, unsigned* err) {
-    if (s0.x == key) return s0.y;
-    if (s0.x == 0) return 0;   // first empty slot: absent (insert-only store)
-    if (s1.x == key) return s1.y;
-    if (s1.x == 0) return 0;
-    return thread_probe(st, key, b, err, 2);
-}
-
-// kRowsPerThread rows per thread at a time: their keys are worked out and their home slots
-// loaded before any is compared, and the neighbour words of their one-to-one rows are loaded
-// before any output row is written, so a thread has that many random reads in flight.
-// Registers are capped for kCountCtas CTAs per SM.  One row per thread at 8 CTAs (2,048 threads
-// per SM) measured best: more rows per thread at fewer CTAs (2-8 rows, 2-6 CTAs) ran 1-35%
-// slower on the heavy star and triangle, so resident warps, not reads per thread, set the rate.
+// One row per thread at a time, registers capped for kCountCtas CTAs per SM (2,048 threads): the
+// lookups are independent reads, and resident warps, not reads per thread, set their rate (two to
+// eight rows per thread at fewer CTAs ran 1-35% slower on the heavy star and triangle when every
+// lookup was a hash probe).
 // kFilter: the membership steps (known_to_known, known_to_const, const_to_known,
 // index_to_known); the other instance (starts and known_to_unknown) carries no membership search.
-constexpr int kRowsPerThread = 1;
 constexpr int kCountCtas = 8;
 
-template <bool kFilter>
+template <bool kFilter, bool kDir>
 __global__ void __launch_bounds__(kFlatThreads, kCountCtas) flat_count_kernel(const FlatArgs a) {
     __shared__ uint64_t s_warp[kFlatThreads / 32];
     const uint64_t R = flat_rows(a);
@@ -181,76 +174,41 @@ __global__ void __launch_bounds__(kFlatThreads, kCountCtas) flat_count_kernel(co
     uint64_t sum = 0, sd = 0, nvalid = 0;
     bool ones = true;   // every row of this thread has exactly one output row
     const bool spec = R <= a.out_cap_rows;   // output row r exists: one-to-one rows written here
-    constexpr int K = kRowsPerThread;
-    constexpr uint64_t kStride = (uint64_t)K * kFlatThreads;
-    for (uint64_t r0 = lo + threadIdx.x; r0 < hi; r0 += kStride) {
-        uint64_t key[K], bkt[K], p[K];
-        bool valid[K], look[K];
-        ulonglong2 s0[K], s1[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const uint64_t r = r0 + (uint64_t)k * kFlatThreads;
-            const uint32_t cur = r < hi ? __ldg(a.in + r * (uint64_t)a.w_in + d.cs) : kBlankId;
-            key[k] = count_key(a, d, from_const, cur, &valid[k], &look[k], &bkt[k]);
-            if (r >= hi) valid[k] = look[k] = false;
+    for (uint64_t r = lo + threadIdx.x; r < hi; r += kFlatThreads) {
+        const uint32_t* src = a.in + r * (uint64_t)a.w_in;
+        bool valid;
+        const uint64_t p = count_ptr<kDir>(a, d, from_const, __ldg(src + d.cs), &valid);
+        uint64_t off, deg;
+        list_of_ptr(p, a.store.n_edges, &a.ctl->err, &off, &deg);
+        if (d.op == kXI2K && valid) {   // index_to_known reads its mt slice of the list
+            uint64_t s_lo, s_hi;
+            mt_slice(d.mt, deg, &s_lo, &s_hi);
+            off += s_lo;
+            deg = s_hi - s_lo;
         }
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            s0[k] = s1[k] = make_ulonglong2(0, 0);
-            if (look[k]) load_sector(a.store.slots + bkt[k] * kAssoc, &s0[k], &s1[k]);
+        uint32_t c = (uint32_t)deg;
+        if (kFilter && valid && deg) {
+            // the membership target shares the row's sector with its start column
+            const uint32_t target = tcol >= 0 ? __ldg(src + tcol) : d.end_const;
+            c = thread_member(a.store.edges, off, deg, target, a.sorted_lists != 0) ? 1u : 0u;
         }
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            p[k] = look[k] ? settle_slot(a.store, key[k], bkt[k], s0[k], s1[k], &a.ctl->err) : 0;
-        // counts and list offsets
-        uint32_t c[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const uint64_t r = r0 + (uint64_t)k * kFlatThreads;
-            uint64_t off, deg;
-            list_of_ptr(p[k], a.store.n_edges, &a.ctl->err, &off, &deg);
-            if (d.op == kXI2K && valid[k]) {   // index_to_known reads its mt slice of the list
-                uint64_t s_lo, s_hi;
-                mt_slice(d.mt, deg, &s_lo, &s_hi);
-                off += s_lo;
-                deg = s_hi - s_lo;
-            }
-            c[k] = (uint32_t)deg;
-            if (kFilter && valid[k] && deg) {
-                // the membership target shares the row's sector with its start column
-                const uint32_t target = tcol >= 0 ? __ldg(a.in + r * (uint64_t)a.w_in + tcol) : d.end_const;
-                c[k] = thread_member(a.store.edges, off, deg, target, a.sorted_lists != 0) ? 1u : 0u;
-            }
-            if (!valid[k]) c[k] = 0;
-            p[k] = off;   // from here on p holds the list offset
-            if (r < hi) {
-                a.pos[r] = c[k];   // the count; flat_place_kernel turns it into the row's position
-                if (!kFilter) a.off[r] = off;
-                if (c[k] != 1) ones = false;
-                sum += c[k];
-            }
-            if (valid[k]) {
-                sd += deg;
-                ++nvalid;
-            }
+        if (!valid) c = 0;
+        a.pos[r] = c;   // the count; flat_place_kernel turns it into the row's position
+        if (!kFilter) a.off[r] = off;
+        if (c != 1) ones = false;
+        sum += c;
+        if (valid) {
+            sd += deg;
+            ++nvalid;
         }
-        if (!kFilter && spec) {
+        if (!kFilter && spec && c == 1) {
             // A row with exactly one output row writes it now, at output row r: when every row
             // has one (a functional predicate), that is the step's output and the place and
-            // expand passes return at once; otherwise expand overwrites these rows.  The rows'
-            // neighbour words are all loaded before any row is written.
-            uint32_t nb[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) nb[k] = c[k] == 1 ? list_at(a.store.edges, p[k], 0) : 0;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                if (c[k] != 1) continue;
-                const uint64_t r = r0 + (uint64_t)k * kFlatThreads;
-                const uint32_t* src = a.in + r * (uint64_t)a.w_in;
-                uint32_t* dst = a.out + r * (uint64_t)a.w_out;
-                for (int j = 0; j < d.cin; ++j) dst[j] = __ldg(src + j);
-                dst[d.cin] = nb[k];
-            }
+            // expand passes return at once; otherwise expand overwrites these rows.
+            uint32_t* dst = a.out + r * (uint64_t)a.w_out;
+            const uint32_t nb = list_at(a.store.edges, off, 0);
+            for (int j = 0; j < d.cin; ++j) dst[j] = __ldg(src + j);
+            dst[d.cin] = nb;
         }
     }
     const bool all_ones = __syncthreads_and(ones);
@@ -444,96 +402,61 @@ __device__ void flat_level_scan_parts(const FlatLevelArgs& a, uint32_t nparts, u
     }
 }
 
-// kRowsPerThread rows per thread at a time, their home slots loaded before any is compared (as
-// in flat_count_kernel).
 __global__ void __launch_bounds__(kFlatThreads, kCountCtas) flat_level_count_kernel(const FlatLevelArgs a) {
     __shared__ uint64_t s_warp[kFlatThreads / 32];
     const uint64_t R = level_rows(a);
     uint64_t lo, hi;
     chunk_of(R, &lo, &hi);
     uint64_t sum = 0, sd = 0, alg = 0;
-    constexpr int K = kRowsPerThread;
-    constexpr uint64_t kStride = (uint64_t)K * kFlatThreads;
-    for (uint64_t r0 = lo + threadIdx.x; r0 < hi; r0 += kStride) {
-        uint64_t key[K], bkt[K];
-        uint32_t target[K];
-        bool valid[K], look[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const uint64_t r = r0 + (uint64_t)k * kFlatThreads;
-            key[k] = 0;
-            bkt[k] = 0;
-            target[k] = 0;
-            valid[k] = look[k] = false;
-            if (r >= hi) continue;
-            const StepDesc* d = a.desc + level_owner(a, r);
-            const uint32_t op = d->op;
-            const SegDesc* sg = &d->seg;
-            bool v = op != kXDone;
-            target[k] = d->end_const;
-            if (v && op == kXStart) {
-                key[k] = d->start_key;
-            } else if (v && (op == kXC2K || op == kXI2K)) {   // one list for every row
-                key[k] = d->start_key;
-                target[k] = __ldg(a.in + r * (uint64_t)a.w_in + d->ce);
-            } else if (v) {
-                const uint32_t* row = a.in + r * (uint64_t)a.w_in;
-                const uint32_t cur = __ldg(row + d->cs);
-                if (op == kXK2K) target[k] = __ldg(row + d->ce);
-                if (cur == kBlankId) v = false;
-                if (op == kXK2U && d->type_index) {
-                    // get_index(cur, IN) (sparql.hpp:342-345); only 17-bit ids can be keys
-                    key[k] = make_key(0, cur, kIn);
-                    sg = &a.seg_index[kIn];
-                    if (cur >= (1u << kNbitsIdx)) v = false;
-                } else {
-                    key[k] = make_key(cur, d->pid, d->dir);
-                    if (cur == 0) sg = &a.seg_index[d->dir & 1];   // vid 0 names the index
-                }
-            }
-            valid[k] = v;
-            look[k] = v && sg->num_buckets != 0 && key[k] != 0;
-            if (look[k]) bkt[k] = bucket_of(key[k], *sg);
-            if (look[k] && bkt[k] >= a.store.n_buckets) {
-                atomicOr(&a.ctl->err, kErrCorrupt);
-                look[k] = false;
+    for (uint64_t r = lo + threadIdx.x; r < hi; r += kFlatThreads) {
+        const StepDesc* d = a.desc + level_owner(a, r);
+        const uint32_t op = d->op;
+        const uint32_t* row = a.in + r * (uint64_t)a.w_in;
+        const SegDesc* sg = a.store.segs + d->seg;
+        bool valid = op != kXDone;
+        uint64_t key = 0;
+        uint32_t target = d->end_const;
+        if (valid && op == kXStart) {
+            key = d->start_key;
+        } else if (valid && (op == kXC2K || op == kXI2K)) {   // one list for every row
+            key = d->start_key;
+            target = __ldg(row + d->ce);
+        } else if (valid) {
+            const uint32_t cur = __ldg(row + d->cs);
+            if (op == kXK2K) target = __ldg(row + d->ce);
+            if (cur == kBlankId) valid = false;
+            if (op == kXK2U && d->type_index) {
+                // get_index(cur, IN) (sparql.hpp:342-345); only 17-bit ids can be keys
+                key = make_key(0, cur, kIn);
+                sg = a.store.segs + a.seg_index[kIn];
+                if (cur >= (1u << kNbitsIdx)) valid = false;
+            } else {
+                key = make_key(cur, d->pid, d->dir);
+                if (cur == 0) sg = a.store.segs + (d->dir & 1 ? a.seg_index[1] : a.seg_index[0]);   // vid 0 names the index
             }
         }
-        ulonglong2 s0[K], s1[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            s0[k] = s1[k] = make_ulonglong2(0, 0);
-            if (look[k]) load_sector(a.store.slots + bkt[k] * kAssoc, &s0[k], &s1[k]);
+        uint64_t off = 0, deg = 0;
+        if (valid && sg->num_buckets != 0 && key != 0) {
+            const uint64_t p = seg_lookup(a.store, *sg, key, (uint32_t)key_vid(key), &a.ctl->err);
+            list_of_ptr(p, a.store.n_edges, &a.ctl->err, &off, &deg);
+            if (op == kXI2K) {
+                uint64_t s_lo, s_hi;
+                mt_slice(d->mt, deg, &s_lo, &s_hi);
+                off += s_lo;
+                deg = s_hi - s_lo;
+            }
         }
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const uint64_t r = r0 + (uint64_t)k * kFlatThreads;
-            if (r >= hi) continue;
-            const StepDesc* d = a.desc + level_owner(a, r);
-            const uint32_t op = d->op;
-            uint64_t off = 0, deg = 0;
-            if (look[k]) {
-                const uint64_t p = settle_slot(a.store, key[k], bkt[k], s0[k], s1[k], &a.ctl->err);
-                list_of_ptr(p, a.store.n_edges, &a.ctl->err, &off, &deg);
-                if (op == kXI2K) {
-                    uint64_t s_lo, s_hi;
-                    mt_slice(d->mt, deg, &s_lo, &s_hi);
-                    off += s_lo;
-                    deg = s_hi - s_lo;
-                }
-            }
-            const bool filt = is_filter_op(op);
-            uint32_t c = (uint32_t)deg;
-            if (filt) c = (valid[k] && deg && thread_member(a.store.edges, off, deg, target[k], a.sorted_lists != 0)) ? 1u : 0u;
-            if (!valid[k]) c = 0;
-            a.pos[r] = c;   // the count; flat_level_place_kernel turns it into the row's position
-            a.off[r] = off;
-            sum += c;
-            if (valid[k]) {
-                const uint32_t cin = op == kXStart ? 0u : d->cin;
-                sd += deg;
-                alg += cin * 4ull + 16 + deg * 4 + (uint64_t)c * d->cout * 4;
-            }
+        const bool filt = is_filter_op(op);
+        uint32_t c = (uint32_t)deg;
+        if (filt) c = (valid && deg && thread_member(a.store.edges, off, deg, target, a.sorted_lists != 0)) ? 1u : 0u;
+        if (!valid) c = 0;
+        a.pos[r] = c;   // the count; flat_level_place_kernel turns it into the row's position
+        a.off[r] = off;
+        sum += c;
+        if (valid) {
+            const uint32_t cin = op == kXStart ? 0u : d->cin;
+            sd += deg;
+            alg += cin * 4ull + 16 + deg * 4 + (uint64_t)c * d->cout * 4;
         }
     }
     sum = block_sum(sum, s_warp);
@@ -674,25 +597,33 @@ __global__ void __launch_bounds__(kFlatThreads) flat_level_expand_kernel(const F
 
 int flat_grid(int sm_count) { return sm_count * (2048 / kFlatThreads); }
 
+namespace {
+using CountKernel = void (*)(const FlatArgs);
+CountKernel count_kernel(bool filter, bool dir) {
+    return filter ? (dir ? flat_count_kernel<true, true> : flat_count_kernel<true, false>)
+                  : (dir ? flat_count_kernel<false, true> : flat_count_kernel<false, false>);
+}
+}  // namespace
+
 int flat_grid_beside(int sm_count, const CtaUse& other, int other_ctas) {
-    cudaFuncAttributes fa{}, fb{};
-    int regs = 255;
-    if (cudaFuncGetAttributes(&fa, flat_count_kernel<true>) == cudaSuccess &&
-        cudaFuncGetAttributes(&fb, flat_count_kernel<false>) == cudaSuccess)
-        regs = std::max(fa.numRegs, fb.numRegs);
-    int dev = 0, reserved = 0;
+    int regs = 0, dev = 0, reserved = 0;
+    size_t smem = 0;
+    for (int k = 0; k < 4; ++k) {
+        cudaFuncAttributes fa{};
+        if (cudaFuncGetAttributes(&fa, count_kernel(k & 1, k & 2)) != cudaSuccess) fa.numRegs = 255;
+        regs = std::max(regs, fa.numRegs);
+        smem = std::max(smem, fa.sharedSizeBytes);
+    }
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-    CtaUse me{(size_t)std::max(fa.sharedSizeBytes, fb.sharedSizeBytes) + (size_t)reserved,
-              ((regs * 32 + 255) / 256) * 256 * (kFlatThreads / 32), kFlatThreads};
+    CtaUse me{smem + (size_t)reserved, ((regs * 32 + 255) / 256) * 256 * (kFlatThreads / 32), kFlatThreads};
     const int alone = 2048 / kFlatThreads;
     return blocks_beside(me, alone, other, other_ctas) * sm_count;
 }
 
 cudaError_t launch_flat(const FlatArgs& a, int grid, cudaStream_t s) {
     // its last CTA scans the totals
-    if (is_filter_op(a.step.op)) flat_count_kernel<true><<<grid, kFlatThreads, 0, s>>>(a);
-    else flat_count_kernel<false><<<grid, kFlatThreads, 0, s>>>(a);
+    count_kernel(is_filter_op(a.step.op), a.seg.vid_span != 0 && !a.step.type_index)<<<grid, kFlatThreads, 0, s>>>(a);
     flat_place_kernel<<<grid, kFlatThreads, 0, s>>>(a, (uint32_t)grid);
     if (a.step.op == kXK2U) flat_expand_kernel<<<grid, kFlatThreads, 0, s>>>(a, (uint32_t)grid);
     return cudaGetLastError();
@@ -707,8 +638,8 @@ cudaError_t launch_flat_level(const FlatLevelArgs& a, int grid, cudaStream_t s) 
 
 cudaError_t flat_kernel_attrs() {
     cudaError_t e;
-    if ((e = use_max_shared_carveout(flat_count_kernel<true>)) != cudaSuccess) return e;
-    if ((e = use_max_shared_carveout(flat_count_kernel<false>)) != cudaSuccess) return e;
+    for (int k = 0; k < 4; ++k)
+        if ((e = use_max_shared_carveout(count_kernel(k & 1, k & 2))) != cudaSuccess) return e;
     if ((e = use_max_shared_carveout(flat_place_kernel)) != cudaSuccess) return e;
     if ((e = use_max_shared_carveout(flat_expand_kernel)) != cudaSuccess) return e;
     if ((e = use_max_shared_carveout(flat_level_count_kernel)) != cudaSuccess) return e;

@@ -9,7 +9,8 @@ namespace wk {
 
 struct FlatArgs {
     DevStore store;
-    SegDesc seg_index[2];        // index segment of each direction
+    uint32_t seg_index[2];       // DevStore::segs entries of the two index segments
+    SegDesc seg;                 // the step's segment
     StepDesc step;               // a known_to_unknown / known_to_known / known_to_const step
     const uint64_t* in_rows;     // device row count of the input
     const uint32_t* in;
@@ -46,7 +47,7 @@ cudaError_t flat_kernel_attrs();
 // caller has reset).  Level 0 has virtual rows: row r is query r's start.
 struct FlatLevelArgs {
     DevStore store;
-    SegDesc seg_index[2];
+    uint32_t seg_index[2];
     const StepDesc* desc;        // [n_queries] this level's step per query
     uint32_t n_queries;
     int32_t virtual_rows;

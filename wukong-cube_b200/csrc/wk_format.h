@@ -77,12 +77,24 @@ static_assert(sizeof(Slot) == 16, "slot must be 16 bytes");
 
 // Where one segment lives inside the uploaded slot and edge arrays.  Only the fields the
 // probe needs; the rest of rdf_seg_meta_t (segment_meta.hpp:87-154) is bookkeeping.
+struct DirBlock;
 struct SegDesc {
     uint64_t bucket_start;   // absolute bucket id of the segment's main-header region
     uint64_t num_buckets;    // hash space of the segment (0 = segment absent / empty)
     uint64_t magic;          // floor((2^64 - 1) / num_buckets): Barrett reciprocal of the modulo
-    uint64_t num_edges;      // number of edges of the segment (informational)
+    const DirBlock* dir;     // the segment's directory on the device (null when it has none)
+    uint32_t vid_lo;         // its first vertex id
+    uint32_t vid_span;       // vertex ids it covers (0: no directory, keys are probed by hash)
 };
+
+// 64 vertex ids of a segment's directory: which of them have a key, and the place of the first
+// one's pointer word in the store's word array (the others follow in vertex order).  Built on
+// the device when the store is loaded (wk_dir.cu); not part of the exported store.
+struct alignas(16) DirBlock {
+    uint64_t bits;
+    uint64_t base;
+};
+static_assert(sizeof(DirBlock) == 16, "directory blocks are 16 bytes");
 
 WK_HD uint64_t barrett_magic(uint64_t nb) { return nb ? ~0ull / nb : 0; }
 

@@ -1041,13 +1041,7 @@ extern "C" int wk_store_build_device(wk_ctx* ctx, const uint32_t* triples, uint6
     WKG_CUDA(ctx, cudaSetDevice(ctx->device));
     WKG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     // the old store goes first: a build needs the room
-    if (ctx->d_slots) cudaFree(ctx->d_slots);
-    if (ctx->d_edges) cudaFree(ctx->d_edges);
-    ctx->d_slots = nullptr;
-    ctx->d_edges = nullptr;
-    ctx->n_slots = ctx->n_edges = 0;
-    ctx->has_store = false;
-    ctx->drop_graphs();
+    ctx->drop_store();
     wk::Slot* slots = nullptr;
     uint32_t* edges = nullptr;
     uint64_t n_slots = 0, n_edges = 0;

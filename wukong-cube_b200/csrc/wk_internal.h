@@ -47,11 +47,10 @@ struct SegIndex {
 };
 
 inline SegDesc to_desc(const wk_seg_meta& m) {
-    SegDesc d;
+    SegDesc d{};   // without a directory
     d.bucket_start = m.bucket_start;
     d.num_buckets = m.num_buckets;
     d.magic = barrett_magic(m.num_buckets);
-    d.num_edges = m.num_edges;
     return d;
 }
 

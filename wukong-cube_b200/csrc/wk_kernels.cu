@@ -1,5 +1,5 @@
 // Small kernels of the single-query path: the start-list copy of index_to_unknown /
-// const_to_unknown, and the upload-time check that every neighbour list is sorted.
+// const_to_unknown, and the random-read calibration.
 //
 // The exploration launch itself is in wk_explore.cu.
 #include <cuda_runtime.h>
@@ -60,53 +60,6 @@ __global__ void list_kernel(const ListArgs a) {
     for (; i < n; i += stride) a.out[i] = __ldg(srcp + i);
 }
 
-// Checks that every key's list is strictly ascending (the loader's sort + dedup), which lets
-// the filters binary-search long lists.
-// One warp per slot; the lanes walk the slot's list together (coalesced), so a hub list costs
-// len/32 steps of one warp instead of len steps of one thread.
-__global__ void sorted_check_kernel(const Slot* slots, uint64_t n_slots, const uint32_t* edges,
-                                    uint64_t n_edges, unsigned* unsorted) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
-    for (uint64_t i = blockIdx.x * (uint64_t)(blockDim.x / 32) + threadIdx.x / 32; i < n_slots; i += warps) {
-        if ((i & (kAssoc - 1)) == kAssoc - 1) continue;   // chain link
-        const Slot s = slots[i];
-        if (s.key == 0) continue;
-        if (ptr_is_inline(s.ptr)) continue;   // a one-entry list (none before inline_kernel)
-        const uint64_t off = ptr_off(s.ptr), sz = ptr_size(s.ptr);
-        if (off + sz > n_edges) {
-            if (lane == 0) atomicOr(unsorted, 2u);
-            continue;
-        }
-        bool bad = false;
-        for (uint64_t k = 1 + lane; k < sz && !bad; k += 32) bad = __ldg(edges + off + k - 1) >= __ldg(edges + off + k);
-        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(unsorted, 1u);
-    }
-}
-
-// One-entry lists into their keys' own pointer words (see kInlinePtrType): for every data slot
-// (slots 0-6) whose list has one entry, the original pointer word goes to the side table
-// `orig` (slot index, pointer word; wk_store_export puts them back) and the slot's pointer word
-// becomes the entry with the inline type.  With orig null the kernel only counts such slots
-// (into *n) and whether any pointer word already carries type 3 (into *clash; the store is then
-// refused, since that type cannot be told apart).
-__global__ void inline_kernel(Slot* slots, uint64_t n_slots, const uint32_t* edges, uint64_t n_edges,
-                              unsigned long long* n, unsigned* clash, uint64_t* orig) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_slots; i += stride) {
-        if ((i & (kAssoc - 1)) == kAssoc - 1) continue;   // chain link
-        const Slot sl = slots[i];
-        if (sl.key == 0) continue;
-        if (!orig && ptr_is_inline(sl.ptr)) atomicOr(clash, 1u);
-        if ((sl.ptr >> 62) != 0 || ptr_size(sl.ptr) != 1 || ptr_off(sl.ptr) >= n_edges) continue;
-        const unsigned long long at = atomicAdd(n, 1ull);
-        if (!orig) continue;
-        orig[2 * at] = i;
-        orig[2 * at + 1] = sl.ptr;
-        slots[i].ptr = make_inline_ptr(__ldg(edges + ptr_off(sl.ptr)));
-    }
-}
-
 // Random-read calibration: every thread makes `per` independent 16-byte reads at pseudo-random
 // 16-byte-aligned positions of buf (the splitmix64 finaliser of thread and read index), eight in
 // flight at a time, in the probes' own load form (no L1 allocation, first out of L2).  With buf
@@ -144,22 +97,6 @@ cudaError_t launch_list(const ListArgs& a, int grid, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_sorted_check(const DevStore& st, unsigned* d_flag, cudaStream_t s) {
-    sorted_check_kernel<<<4096, 256, 0, s>>>(st.slots, st.n_buckets * kAssoc, st.edges, st.n_edges, d_flag);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_inline(const DevStore& st, unsigned long long* n, unsigned* clash, uint64_t* orig,
-                          cudaStream_t s) {
-    if (st.n_buckets)
-        inline_kernel<<<4096, 256, 0, s>>>(const_cast<Slot*>(st.slots), st.n_buckets * kAssoc, st.edges, st.n_edges,
-                                           n, clash, orig);
-    return cudaGetLastError();
-}
-
-cudaError_t small_kernel_attrs() {
-    cudaError_t e = use_max_shared_carveout(list_kernel);
-    return e != cudaSuccess ? e : use_max_shared_carveout(sorted_check_kernel);
-}
+cudaError_t small_kernel_attrs() { return use_max_shared_carveout(list_kernel); }
 
 }  // namespace wk

@@ -42,6 +42,8 @@ struct DevStore {
     uint64_t n_buckets;   // slots / 8
     const uint32_t* edges;
     uint64_t n_edges;
+    const SegDesc* segs;         // [n_segs + 1]: entry 0 an absent segment, i + 1 segment i
+    const uint64_t* dir_words;   // the directories' pointer words
 };
 
 struct ListArgs {
@@ -60,13 +62,6 @@ constexpr int kStepThreads = 128;
 constexpr int kTileRows = 256;
 
 cudaError_t launch_list(const ListArgs& a, int grid, cudaStream_t s);
-cudaError_t launch_sorted_check(const DevStore& st, unsigned* d_flag, cudaStream_t s);
-// One-entry lists into their keys' pointer words (inline_kernel): with orig null, counts them
-// into *n and flags pointer words that already carry the inline type in *clash; with orig (two
-// words per counted slot), converts them and keeps the original pointer words there.  *n must
-// be 0 on entry.
-cudaError_t launch_inline(const DevStore& st, unsigned long long* n, unsigned* clash, uint64_t* orig,
-                          cudaStream_t s);
 // `grid` CTAs of 256 threads, `per` random 16-byte reads each from a `bytes`-byte buffer.
 cudaError_t launch_random_reads(const void* buf, uint64_t bytes, int per, uint64_t seed,
                                 uint32_t* sink, int grid, cudaStream_t s);

@@ -136,8 +136,8 @@ extern "C" int wk_step_known_to_unknown_noalloc(wk_ctx* ctx, const wk_table* in,
     st.out_cols = in->cols + 1;
     wk::ExploreArgs a{};
     a.store = ctx->dev_store();
-    a.seg_index[0] = ctx->seg_of(0, 0, wk::kIn);
-    a.seg_index[1] = ctx->seg_of(0, 0, wk::kOut);
+    a.seg_index[0] = ctx->seg_id(0, 0, wk::kIn);
+    a.seg_index[1] = ctx->seg_id(0, 0, wk::kOut);
     a.one = wk::make_step_desc(ctx, st);
     a.n_queries = 1;
     a.in_rows = in->d_rows;

@@ -257,8 +257,8 @@ struct Serve {
     ExploreArgs explore_args(uint32_t iter, int cur) const {
         ExploreArgs a{};
         a.store = ctx->dev_store();
-        a.seg_index[0] = ctx->seg_of(0, 0, kIn);
-        a.seg_index[1] = ctx->seg_of(0, 0, kOut);
+        a.seg_index[0] = ctx->seg_id(0, 0, kIn);
+        a.seg_index[1] = ctx->seg_id(0, 0, kOut);
         a.desc = d_plans;
         a.desc_stride = kMaxSteps;
         a.iter = iter;
@@ -275,7 +275,7 @@ struct Serve {
         a.ctl = ctx->d_ctl;
         a.status = ctx->d_status;
         a.sorted_lists = ctx->sorted_lists;
-        a.lanes = ctx->batch_lanes;
+        a.lanes = ctx->probe_lanes(ctx->batch_lanes);
         a.slice_rows = ctx->batch_slice_rows;
         a.spin_limit = ctx->spin_limit;
         return a;
@@ -304,7 +304,7 @@ struct Serve {
             d_qfirst, d_qcount, slots_n, d_total + cur, d_plans, d_admit, d_stage, d_new, n_new, iter);
         WKS_CUDA(ctx, cudaGetLastError());
         const int light = light_ctas();
-        const int grid = std::min(explore_blocks_per_sm(w, w, ctx->batch_lanes), light) * ctx->sm_count;
+        const int grid = std::min(explore_blocks_per_sm(w, w, ctx->probe_lanes(ctx->batch_lanes)), light) * ctx->sm_count;
         if (has_cont) {
             ExploreArgs a = explore_args(iter, cur);
             a.n_queries = slots_n;
@@ -323,7 +323,7 @@ struct Serve {
             a.virtual_rows = 1;
             a.virt_owner = d_new;
             a.out_base_rows = d_total + cur;
-            const int g0 = std::min(explore_blocks_per_sm(0, w, ctx->batch_lanes), light) * ctx->sm_count;
+            const int g0 = std::min(explore_blocks_per_sm(0, w, ctx->probe_lanes(ctx->batch_lanes)), light) * ctx->sm_count;
             cudaError_t e = launch_explore(a, g0, s);
             if (e != cudaSuccess) return ctx->cuda_fail(e, "serving start launch");
         }
@@ -538,8 +538,8 @@ extern "C" int wk_serve_run_open_loop(wk_ctx* ctx, const wk_serve_config* cfg_in
         // Lanes leave room on every SM for the iteration launches' CTAs (the larger of the two
         // launch shapes, one CTA of margin), so both persistent launches stay resident at once
         // and neither waits for the other to finish.
-        const wk::CtaUse a = wk::explore_cta_use(S.w, S.w, ctx->batch_lanes);
-        const wk::CtaUse b = wk::explore_cta_use(0, S.w, ctx->batch_lanes);
+        const wk::CtaUse a = wk::explore_cta_use(S.w, S.w, ctx->probe_lanes(ctx->batch_lanes));
+        const wk::CtaUse b = wk::explore_cta_use(0, S.w, ctx->probe_lanes(ctx->batch_lanes));
         const wk::CtaUse light{std::max(a.smem, b.smem), std::max(a.regs, b.regs),
                                std::max(a.threads, b.threads)};
         const uint64_t lane_bytes =

@@ -55,7 +55,9 @@ __device__ __forceinline__ void list_of(const VersArgs& a, uint64_t vid, uint32_
     *deg = 0;
     const uint64_t key = make_key(vid, pid, a.dir);
     if (sg.num_buckets == 0 || key == 0) return;
-    const uint64_t p = thread_probe(a.store, key, bucket_of(key, sg), &a.ctl->err);
+    // (vid 0 names no vertex, so no directory holds it)
+    const uint64_t p = vid ? seg_lookup(a.store, sg, key, (uint32_t)vid, &a.ctl->err)
+                           : hash_lookup(a.store, sg, key, &a.ctl->err);
     list_of_ptr(p, a.store.n_edges, &a.ctl->err, off, deg);   // *off may be a tagged entry
 }
 

@@ -13,7 +13,7 @@ enum VersOp : int32_t { kVKUU = 0, kVKUC = 1, kVCUU = 2, kVCUC = 3 };
 // store's table of these is sorted by key.
 struct PredSeg {
     uint32_t key;
-    uint32_t pad;
+    uint32_t seg_no;   // its place in the segment list
     SegDesc seg;
 };
 

@@ -179,8 +179,9 @@ void wk_ctx::drop_store() {
     d_dir_words = nullptr;
     n_slots = n_edges = n_inline = 0;
     n_pseg = 0;
-    has_dir = false;
+    has_dir = no_fuse = false;
     seg_desc.clear();
+    seg_longest.clear();
 }
 
 void wk_ctx::drop_graphs() {
@@ -360,7 +361,7 @@ int resolve_plan(const wk_query& q, int max_cols, std::vector<PlanStep>& steps, 
 }
 
 int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* out,
-                 int32_t mt_tid, int32_t mt_factor, cudaStream_t s, int grid_override, int flat_mode) {
+                 int32_t mt_tid, int32_t mt_factor, cudaStream_t s) {
     out->cols = st.out_cols;
     if (st.kind == PlanStep::kIndex || st.kind == PlanStep::kConst) {
         ListArgs a{};
@@ -382,8 +383,7 @@ int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* 
         a.ctl = ctx->d_ctl;
         // index lists are long (every instance of a type, every subject of a predicate): a
         // full-occupancy grid; a constant's list is usually short
-        int grid = st.kind == PlanStep::kIndex ? ctx->sm_count * 8 : std::min(ctx->sm_count * 2, 512);
-        if (grid_override > 0) grid = grid_override;
+        const int grid = st.kind == PlanStep::kIndex ? ctx->sm_count * 8 : std::min(ctx->sm_count * 2, 512);
         cudaError_t e = launch_list(a, grid, s);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "list kernel launch");
         return WK_SUCCESS;
@@ -452,45 +452,126 @@ int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* 
     a.lanes = ctx->lanes_for(a.one.op, st.in_cols);
     a.slice_rows = ctx->slice_rows;
     a.spin_limit = ctx->spin_limit;
-    // The flat pipeline needs its scratch sized for this input; without it the tile launch runs.
-    if (!ctx->flat_min_rows || !ctx->d_flat || a.in_cap_rows > ctx->flat_cap_rows ||
-        a.in_cap_rows < ctx->flat_min_rows || grid_override > 0)
-        flat_mode = kTileOnly;
-    if (flat_mode != kFlatOnly) {
-        if (flat_mode == kFlatAuto) a.max_rows = ctx->flat_min_rows;
-        int grid = grid_override > 0 ? grid_override
-                                     : ctx->blocks_per_sm(a.one.op, st.in_cols, a.lanes) * ctx->sm_count;
-        cudaError_t e = launch_explore(a, grid, s);
-        if (e != cudaSuccess) return ctx->cuda_fail(e, "exploration launch");
+    const int grid = ctx->blocks_per_sm(a.one.op, st.in_cols, a.lanes) * ctx->sm_count;
+    cudaError_t e = launch_explore(a, grid, s);
+    if (e != cudaSuccess) return ctx->cuda_fail(e, "exploration launch");
+    return WK_SUCCESS;
+}
+
+namespace {
+
+bool is_start(const PlanStep& s) { return s.kind == PlanStep::kIndex || s.kind == PlanStep::kConst; }
+bool is_filter(const PlanStep& s) {
+    return s.kind == PlanStep::kK2K || s.kind == PlanStep::kK2C || s.kind == PlanStep::kC2K ||
+           s.kind == PlanStep::kI2K;
+}
+// known_to_unknown whose lists all have at most one entry
+bool is_functional(const wk_ctx* ctx, const PlanStep& s) {
+    if (s.kind != PlanStep::kK2U || (s.pid == kTypeId && s.dir == kIn)) return false;
+    const uint32_t id = ctx->seg_id(1, s.pid, s.dir);
+    return id == 0 || ctx->seg_longest[id - 1] <= 1;
+}
+
+}  // namespace
+
+std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>& steps, bool fuse) {
+    std::vector<PlanPass> out;
+    const int n = (int)steps.size();
+    for (int i = 0; i < n;) {
+        const bool start = is_start(steps[i]);
+        int j = i + (start ? 1 : 0);
+        int ops = 0, cols = 0;
+        bool pipe = false;
+        for (; j < n && !is_start(steps[j]) && !is_versatile_step(steps[j].kind); ++j) {
+            const bool func = is_functional(ctx, steps[j]) && fuse;
+            if (is_filter(steps[j]) || func) {
+                if (ops == kMaxPipeOps || (func && cols == kMaxPipeCols)) break;
+                ++ops;
+                cols += func;
+                pipe = true;
+                if (fuse) continue;
+            } else {
+                pipe = true;   // a step that multiplies rows ends the pass
+            }
+            ++j;
+            break;
+        }
+        if (!pipe) j = i + 1;
+        out.push_back(PlanPass{i, j - i, pipe});
+        i = j;
     }
-    if (flat_mode != kTileOnly) {
-        FlatArgs f{};
-        f.store = a.store;
-        f.seg_index[0] = a.seg_index[0];
-        f.seg_index[1] = a.seg_index[1];
-        f.seg = ctx->seg_of(st.kind == PlanStep::kI2K || (st.kind == PlanStep::kC2K && st.start_const == 0) ? 0 : 1,
-                            st.kind == PlanStep::kI2K ? st.start_const : st.pid, st.dir);
-        f.step = a.one;
-        f.in_rows = a.in_rows;
-        f.in = a.in;
-        f.w_in = a.w_in;
-        f.in_cap_rows = a.in_cap_rows;
-        f.out = a.out;
-        f.w_out = a.w_out;
-        f.out_cap_rows = a.out_cap_rows;
-        f.out_rows = a.out_rows;
-        f.min_rows = flat_mode == kFlatAuto ? ctx->flat_min_rows : 0;
-        // a serving lane leaves room on every SM for the iteration launches' CTAs beside it
-        const int grid = ctx->beside_ctas > 0 ? flat_grid_beside(ctx->sm_count, ctx->beside_use, ctx->beside_ctas)
-                                              : flat_grid(ctx->sm_count);
-        f.pos = reinterpret_cast<uint64_t*>(ctx->d_flat);
-        f.off = f.pos + ctx->flat_cap_rows + 1;
-        f.part = f.off + ctx->flat_cap_rows;
-        f.ctl = ctx->d_ctl;
-        f.sorted_lists = ctx->sorted_lists;
-        cudaError_t e = launch_flat(f, grid, s);
-        if (e != cudaSuccess) return ctx->cuda_fail(e, "flat pipeline launch");
+    return out;
+}
+
+int enqueue_pass(wk_ctx* ctx, const std::vector<PlanStep>& steps, const PlanPass& p, const wk_table* in, wk_table* out,
+                 int32_t mt_tid, int32_t mt_factor, bool fuse, cudaStream_t s, bool account) {
+    if (!p.pipe) return enqueue_step(ctx, steps[p.first], in, out, mt_tid, mt_factor, s);
+    PipeArgs a{};
+    a.store = ctx->dev_store();
+    a.seg_index[0] = ctx->seg_id(0, 0, kIn);
+    a.seg_index[1] = ctx->seg_id(0, 0, kOut);
+    int i = p.first;
+    if (is_start(steps[i])) {
+        const PlanStep& st = steps[i++];
+        const bool index = st.kind == PlanStep::kIndex;
+        a.from_list = 1;
+        a.src_key = index ? make_key(0, st.start_const, st.dir) : make_key(st.start_const, st.pid, st.dir);
+        auto it = ctx->index_ptr.find(st.start_const * 2 + (uint32_t)st.dir);
+        if (index && it != ctx->index_ptr.end()) {
+            a.src_known = 1;
+            a.src_off = ptr_off(it->second);
+            a.src_len = ptr_size(it->second);
+        }
+        a.src_seg = index ? ctx->seg_of(0, st.start_const, st.dir) : ctx->seg_of(st.start_const, st.pid, st.dir);
+        a.mt_tid = index ? mt_tid : 0;
+        a.mt_factor = index && mt_factor > 0 ? mt_factor : 1;
+        a.w_in = 1;
+    } else {
+        if (!in || steps[i].in_cols <= 0) return WK_E_BADARG;
+        a.w_in = steps[i].in_cols;
+        a.in_rows = in->d_rows;
+        a.in = in->d;
+        a.in_cap_rows = in->cap / steps[i].in_cols;
     }
+    for (; i < p.first + p.n; ++i) {
+        const PlanStep& st = steps[i];
+        const StepDesc d = make_step_desc(ctx, st);
+        PipeOp o{};
+        o.start_key = d.start_key;
+        if (d.seg) o.seg = ctx->seg_desc[d.seg - 1];
+        o.pid = d.pid;
+        o.end_const = d.end_const;
+        o.mt = d.mt;
+        o.op = d.op;
+        o.dir = d.dir;
+        o.cs = d.cs;
+        o.ce = d.ce;
+        o.type_index = d.type_index;
+        if (is_filter(st) || (fuse && is_functional(ctx, st))) {
+            a.ops[a.n_ops++] = o;
+        } else {
+            a.last = o;
+            a.has_last = 1;
+        }
+    }
+    out->cols = steps[p.first + p.n - 1].out_cols;
+    a.out = out->d;
+    a.w_out = out->cols;
+    a.out_cap_rows = out->cap / out->cols;
+    a.out_rows = out->d_rows;
+    a.heavy = ctx->d_heavy;
+    a.heavy_cap = ctx->heavy_cap;
+    a.ctl = ctx->d_ctl;
+    a.status = ctx->d_status;
+    a.sorted_lists = ctx->sorted_lists;
+    a.slice_rows = ctx->slice_rows;
+    a.spin_limit = ctx->spin_limit;
+    a.account = account ? 1 : 0;
+    // a serving lane leaves room on every SM for the iteration launches' CTAs beside it
+    const int grid = ctx->beside_ctas > 0 ? pipe_grid_beside(ctx->sm_count, ctx->beside_use, ctx->beside_ctas)
+                                          : pipe_grid(ctx->sm_count);
+    cudaError_t e = launch_pipe(a, grid, s);
+    if (e != cudaSuccess) return ctx->cuda_fail(e, "fused pass launch");
     return WK_SUCCESS;
 }
 
@@ -598,8 +679,9 @@ int wk::ctx_make_child(wk_ctx* parent, const CtaUse& beside_use, int beside_ctas
     ctx->segs = parent->segs;
     ctx->index = parent->index;
     ctx->seg_desc = parent->seg_desc;
+    ctx->seg_longest = parent->seg_longest;
+    ctx->index_ptr = parent->index_ptr;
     ctx->d_segs = parent->d_segs;
-    ctx->d_dir_words = parent->d_dir_words;
     ctx->has_dir = parent->has_dir;
     ctx->has_store = parent->has_store;
     ctx->versatile = parent->versatile;
@@ -636,6 +718,7 @@ static int ctx_init_device(wk_ctx* ctx, bool low_priority) {
     if (e == cudaSuccess) e = wk::batch_kernel_attrs();
     if (e == cudaSuccess) e = wk::serve_kernel_attrs();
     if (e == cudaSuccess) e = wk::flat_kernel_attrs();
+    if (e == cudaSuccess) e = wk::pipe_kernel_attrs();
     if (e == cudaSuccess) e = wk::final_kernel_attrs();
     if (e == cudaSuccess) e = wk::versatile_kernel_attrs();
     if (e == cudaSuccess) e = wk::gbuild_kernel_attrs();
@@ -760,16 +843,16 @@ static int store_tables(wk_ctx* ctx) {
     return WK_SUCCESS;
 }
 
-// Which segments get a directory: normal segments whose blocks (16 bytes per 64 vertex ids from
+// Which segments get a directory: normal segments whose blocks (8 bytes per 32 vertex ids from
 // the lowest to the highest) take no more room than their buckets, when no two segments share
 // buckets and the whole (blocks, and a word per key) fits a quarter of the free device memory.
 // At the default load factor a key has about 180 bytes of buckets, so a segment with a key per
-// 700 ids still gets one: its 16-byte blocks are read from L2 where its buckets are not, and a
-// thinner one reads about as many distinct lines either way.  `vid` holds each segment's lowest
+// 700 ids still gets one: its 8-byte blocks are read from L2 where its buckets are not, and a
+// thinner one reads about as many distinct lines either way.  `of_seg` holds each segment's lowest
 // and highest id; the segments come back by bucket, with the total of their main buckets and
 // blocks.
 static std::vector<wk::DirSeg> dir_plan(const std::vector<wk_seg_meta>& segs, const std::vector<wk::SegDesc>& desc,
-                                        const std::vector<uint32_t>& vid_of_seg, uint64_t free_bytes,
+                                        const std::vector<wk::SegScan>& of_seg, uint64_t free_bytes,
                                         std::vector<uint32_t>* which, uint64_t* n_buckets, uint64_t* n_blocks) {
     std::vector<uint32_t> order;
     for (uint32_t i = 0; i < segs.size(); ++i)
@@ -784,9 +867,9 @@ static std::vector<wk::DirSeg> dir_plan(const std::vector<wk_seg_meta>& segs, co
         const wk_seg_meta& m = segs[i];
         if (m.bucket_start < end) return {};
         end = m.bucket_start + m.num_buckets;
-        const uint32_t lo = vid_of_seg[2 * i], hi = vid_of_seg[2 * i + 1];
+        const uint32_t lo = of_seg[i].vid_lo, hi = of_seg[i].vid_hi;
         if (m.index || lo > hi || hi - lo == 0xFFFFFFFFu) continue;
-        const uint64_t blocks = ((uint64_t)(hi - lo) + 64) / 64;
+        const uint64_t blocks = ((uint64_t)(hi - lo) + 32) / 32;
         if (blocks * sizeof(wk::DirBlock) > m.num_buckets * wk::kAssoc * sizeof(wk::Slot)) continue;
         wk::DirSeg d{};
         d.first = *n_buckets;
@@ -794,9 +877,10 @@ static std::vector<wk::DirSeg> dir_plan(const std::vector<wk_seg_meta>& segs, co
         d.seg = desc[i];
         d.seg.vid_lo = lo;
         d.seg.vid_span = hi - lo + 1;
+        d.seg.dir_values = of_seg[i].longest == 1;
         d.key = m.pid * 2 + (uint32_t)m.dir;
         *n_buckets += m.num_buckets;
-        *n_blocks += blocks;
+        *n_blocks += (blocks + wk::kDirScanBlocks - 1) / wk::kDirScanBlocks * wk::kDirScanBlocks;
         keys += m.num_keys;
         which->push_back(i);
         out.push_back(d);
@@ -807,18 +891,18 @@ static std::vector<wk::DirSeg> dir_plan(const std::vector<wk_seg_meta>& segs, co
 
 // The vertex directories of a store (see wk_dir.cu).  A store that cannot have them (or whose
 // device has no room) keeps the hash probes: that is no error.
-static int build_directories(wk_ctx* ctx, const std::vector<uint32_t>& vid_of_seg, wk::StoreScan* d_scan) {
+static int build_directories(wk_ctx* ctx, const std::vector<wk::SegScan>& of_seg, wk::StoreScan* d_scan) {
     size_t free_b = 0, total_b = 0;
     WK_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
     std::vector<uint32_t> which;
     uint64_t n_buckets = 0, n_blocks = 0;
-    std::vector<wk::DirSeg> ds = dir_plan(ctx->segs, ctx->seg_desc, vid_of_seg, free_b, &which, &n_buckets, &n_blocks);
+    std::vector<wk::DirSeg> ds = dir_plan(ctx->segs, ctx->seg_desc, of_seg, free_b, &which, &n_buckets, &n_blocks);
     if (ds.empty()) return WK_SUCCESS;
-    const uint64_t n_sums = (n_blocks + wk::kDirScanBlocks - 1) / wk::kDirScanBlocks;
+    const uint64_t n_sums = n_blocks / wk::kDirScanBlocks;
     wk::DirSeg* d_ds = nullptr;
     uint64_t* d_sums = nullptr;
     wk::DirBlock* blocks = nullptr;
-    uint64_t* words = nullptr;
+    char* words = nullptr;
     auto drop = [&](int rc) {
         cudaFree(d_ds);
         cudaFree(d_sums);
@@ -834,23 +918,33 @@ static int build_directories(wk_ctx* ctx, const std::vector<uint32_t>& vid_of_se
     }
     for (auto& d : ds) d.seg.dir = blocks + d.block0;
     cudaStream_t s = ctx->stream;
-    uint64_t n_words = 0;
+    std::vector<uint64_t> sums(n_sums + 1);
     wk::StoreScan h{};
     cudaError_t e = cudaMemcpyAsync(d_ds, ds.data(), ds.size() * sizeof(wk::DirSeg), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(blocks, 0, n_blocks * sizeof(wk::DirBlock), s);
     if (e == cudaSuccess)
         e = wk::launch_dir_bits(ctx->dev_store(), d_ds, (uint32_t)ds.size(), n_buckets, blocks, n_blocks, d_sums, d_scan,
                                 ctx->sm_count, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&n_words, d_sums + n_sums, 8, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(sums.data(), d_sums, sums.size() * 8, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_scan, sizeof(h), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return drop(ctx->cuda_fail(e, "vertex directories"));
     if (h.flags & (wk::kStoreBadChain | wk::kStoreDupKey)) return drop(WK_SUCCESS);
-    if (wk::dev_malloc(&words, std::max<uint64_t>(n_words, 1) * 8) != cudaSuccess) {
+    // each segment's words, on 16 bytes
+    std::vector<uint64_t> at(ds.size() + 1, 0);
+    for (size_t k = 0; k < ds.size(); ++k) {
+        const uint64_t b1 = k + 1 < ds.size() ? ds[k + 1].block0 : n_blocks;
+        const uint64_t n = sums[b1 / wk::kDirScanBlocks] - sums[ds[k].block0 / wk::kDirScanBlocks];
+        at[k + 1] = at[k] + (n * (ds[k].seg.dir_values ? 4 : 8) + 15) / 16 * 16;
+    }
+    if (wk::dev_malloc(&words, std::max<uint64_t>(at.back(), 16)) != cudaSuccess) {
         cudaGetLastError();
         return drop(WK_SUCCESS);
     }
-    e = wk::launch_dir_fill(ctx->dev_store(), d_ds, (uint32_t)ds.size(), n_buckets, words, d_scan, ctx->sm_count, s);
+    for (size_t k = 0; k < ds.size(); ++k) ds[k].seg.dir_words = words + at[k];
+    e = cudaMemcpyAsync(d_ds, ds.data(), ds.size() * sizeof(wk::DirSeg), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+        e = wk::launch_dir_fill(ctx->dev_store(), d_ds, (uint32_t)ds.size(), n_buckets, d_scan, ctx->sm_count, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return drop(ctx->cuda_fail(e, "vertex directories"));
     ctx->d_dir_blocks = blocks;
@@ -880,9 +974,10 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
     int rc = store_tables(ctx);
     if (rc) return rc;
     {
-        // the index lists' lengths (the keys [0|tpid|dir] of the two index segments: a few
-        // buckets per predicate and type), which the serving admission projects from
-        ctx->index_len.clear();
+        // the index lists (the keys [0|tpid|dir] of the two index segments: a few
+        // buckets per predicate and type): where plans start, and what the serving admission
+        // projects from
+        ctx->index_ptr.clear();
         const uint64_t nb = n_slots / wk::kAssoc;
         std::vector<wk::Slot> bk;
         for (int d = 0; d < 2; ++d) {
@@ -898,7 +993,7 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
                 for (size_t k = 0; k < bk.size(); ++k) {
                     const uint64_t key = bk[k].key;
                     if (k % wk::kAssoc == wk::kAssoc - 1 || key == 0 || wk::key_vid(key) != 0) continue;
-                    ctx->index_len[wk::key_pid(key) * 2 + wk::key_dir(key)] = wk::ptr_size(bk[k].ptr);
+                    ctx->index_ptr.emplace(wk::key_pid(key) * 2 + wk::key_dir(key), bk[k].ptr);
                 }
             }
         }
@@ -912,20 +1007,21 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
         StoreScan* d = nullptr;
         ~Scan() { cudaFree(d); }
     } scan;
-    const size_t scan_bytes = sizeof(StoreScan) + 8ull * np;
+    const size_t scan_bytes = sizeof(StoreScan) + sizeof(SegScan) * (size_t)np;
     const size_t chunks_at = (scan_bytes + 15) & ~(size_t)15;
     const uint32_t max_chunks = store_scan_chunks(n_edges);
     std::vector<unsigned char> hs(scan_bytes, 0);
-    uint32_t* hv = reinterpret_cast<uint32_t*>(hs.data() + sizeof(StoreScan));
-    for (uint32_t i = 0; i < np; ++i) hv[2 * i] = 0xFFFFFFFFu;
+    SegScan* hv = reinterpret_cast<SegScan*>(hs.data() + sizeof(StoreScan));
+    const SegScan no_key{0xFFFFFFFFu, 0, 0, 0};
+    std::fill(hv, hv + np, no_key);
     if (dev_malloc(&scan.d, chunks_at + 16ull * max_chunks) != cudaSuccess) {
         cudaGetLastError();
         return ctx->fail(WK_E_OOM, "store check");
     }
-    uint32_t* d_vid = reinterpret_cast<uint32_t*>(scan.d + 1);
+    SegScan* d_per_seg = reinterpret_cast<SegScan*>(scan.d + 1);
     cudaError_t e = cudaMemcpyAsync(scan.d, hs.data(), scan_bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && n_slots)
-        e = launch_store_scan(ctx->dev_store(), ctx->d_pseg, np, d_vid, scan.d,
+        e = launch_store_scan(ctx->dev_store(), ctx->d_pseg, np, d_per_seg, scan.d,
                               reinterpret_cast<ulonglong2*>(reinterpret_cast<char*>(scan.d) + chunks_at), max_chunks,
                               ctx->sm_count, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(hs.data(), scan.d, scan_bytes, cudaMemcpyDeviceToHost, s);
@@ -948,13 +1044,14 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
         if (e == cudaSuccess) e = launch_inline(ctx->dev_store(), &scan.d->n_inline, ctx->d_inline_orig, ctx->sm_count, s);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "one-entry lists");
     }
+    std::vector<SegScan> of_seg(n_segs, no_key);
+    std::vector<PredSeg> ps(np);   // which segment each entry belongs to
+    if (np) WK_CUDA(ctx, cudaMemcpy(ps.data(), ctx->d_pseg, np * sizeof(PredSeg), cudaMemcpyDeviceToHost));
+    for (uint32_t i = 0; i < np; ++i) of_seg[ps[i].seg_no] = hv[i];
+    ctx->seg_longest.clear();
+    for (auto& x : of_seg) ctx->seg_longest.push_back(x.longest);
     if (!(found.flags & kStoreBadChain)) {
-        std::vector<uint32_t> vid(2ull * n_segs);
-        for (uint32_t i = 0; i < n_segs; ++i) vid[2 * i] = 0xFFFFFFFFu;
-        std::vector<PredSeg> ps(np);   // which segment each range belongs to
-        if (np) WK_CUDA(ctx, cudaMemcpy(ps.data(), ctx->d_pseg, np * sizeof(PredSeg), cudaMemcpyDeviceToHost));
-        for (uint32_t i = 0; i < np; ++i) std::memcpy(&vid[2ull * ps[i].seg_no], hv + 2 * i, 8);
-        rc = build_directories(ctx, vid, scan.d);
+        rc = build_directories(ctx, of_seg, scan.d);
         if (rc) return rc;
     }
     e = cudaStreamSynchronize(s);
@@ -1105,7 +1202,7 @@ static int run_step_sync(wk_ctx* ctx, const wk::PlanStep& st, const wk_table* in
         int rc = ctx->ensure_flat(in && in->cols > 0 ? in->cap / in->cols : 1);
         if (rc) return rc;
     }
-    int flat = wk::kTileOnly;
+    bool pipe = false;
     if (in && in->cols > 0 && !wk::is_versatile_step(st.kind)) {
         int rc = ctx->ensure_status(in->cap / in->cols / wk::kTileRows + 2);
         if (rc) return rc;
@@ -1116,16 +1213,14 @@ static int run_step_sync(wk_ctx* ctx, const wk::PlanStep& st, const wk_table* in
         // a row count past the capacity marks a table whose writing step overflowed
         if (rows * (uint64_t)in->cols > in->cap)
             return ctx->fail(WK_E_CORRUPT, "input row count beyond table capacity");
-        if (ctx->flat_min_rows && rows >= ctx->flat_min_rows) {
-            rc = ctx->ensure_flat(in->cap / in->cols);
-            if (rc) return rc;
-            flat = wk::kFlatOnly;
-        }
+        pipe = ctx->flat_min_rows && rows >= ctx->flat_min_rows;
     }
+    const std::vector<wk::PlanStep> one{st};
+    bool fuse = true;
     for (int attempt = 0; attempt < 8; ++attempt) {
         int rc = ctx->ensure_heavy(out->cap);
         if (rc) return rc;
-        rc = wk::enqueue_step(ctx, st, in, out, mt_tid, mt_factor, ctx->stream, 0, flat);
+        rc = wk::enqueue_pass(ctx, one, wk::PlanPass{0, 1, pipe}, in, out, mt_tid, mt_factor, fuse, ctx->stream);
         if (rc) return rc;
         uint32_t err = 0;
         uint64_t need = 0;
@@ -1137,6 +1232,7 @@ static int run_step_sync(wk_ctx* ctx, const wk::PlanStep& st, const wk_table* in
         if (err & wk::kErrCorrupt) return ctx->fail(WK_E_CORRUPT, "key table chain out of range");
         if (err & wk::kErrTimeout) return ctx->fail(WK_E_TIMEOUT, "tile look-back timed out");
         if (err & wk::kErrStatus) return ctx->fail(WK_E_CAPACITY, "status array too small");
+        if (err & wk::kErrUnfuse) fuse = false;   // an input row of vertex 0
         if (err & wk::kErrOverflow) {
             // `need` counts rows (the list copy of a start step has one column)
             const uint64_t elems = need * (uint64_t)std::max(st.out_cols, 1);
@@ -1327,33 +1423,46 @@ static std::string plan_key(const std::vector<wk::PlanStep>& steps, const wk_que
     put(&ctx->d_flat, sizeof(ctx->d_flat));
     put(&ctx->flat_cap_rows, sizeof(ctx->flat_cap_rows));
     put(&ctx->flat_min_rows, sizeof(ctx->flat_min_rows));
+    put(&ctx->no_fuse, sizeof(ctx->no_fuse));
     return k;
 }
 
-// Plans that start from an index build large tables: their steps launch both the tile launch
-// and the flat pipeline, and the device picks by the row count.
-static int plan_flat_mode(const std::vector<wk::PlanStep>& steps) {
-    return (!steps.empty() && steps[0].kind == wk::PlanStep::kIndex) ? wk::kFlatAuto : wk::kTileOnly;
+// The launches of a plan run back to back: fused passes, or (knob 4 at 0) one launch per step.
+static std::vector<wk::PlanPass> query_passes(const wk_ctx* ctx, const std::vector<wk::PlanStep>& steps) {
+    if (ctx->flat_min_rows) return wk::plan_passes(ctx, steps, !ctx->no_fuse);
+    std::vector<wk::PlanPass> out;
+    for (size_t i = 0; i < steps.size(); ++i) out.push_back(wk::PlanPass{(int)i, 1, false});
+    return out;
+}
+static wk_table* final_table(wk_ctx* ctx, const std::vector<wk::PlanPass>& passes) {
+    return &ctx->rbuf[passes.empty() ? 0 : (passes.size() - 1) & 1];
 }
 
-// Flat scratch for every step input of a plan (the rbuf capacities bound the row counts).
-static int plan_ensure_flat(wk_ctx* ctx, const std::vector<wk::PlanStep>& steps) {
+// Scratch of the versatile steps' inputs (the rbuf capacities bound the row counts), and status
+// words for the rows of an index list, which no table's capacity bounds.
+static int plan_scratch(wk_ctx* ctx, const std::vector<wk::PlanStep>& steps) {
     bool vers = false;
     for (auto& s : steps) vers |= wk::is_versatile_step(s.kind);
-    if (!vers && (plan_flat_mode(steps) == wk::kTileOnly || !ctx->flat_min_rows)) return WK_SUCCESS;
+    if (!steps.empty() && steps[0].kind == wk::PlanStep::kIndex) {
+        auto it = ctx->index_ptr.find(steps[0].start_const * 2 + (uint32_t)steps[0].dir);
+        if (it != ctx->index_ptr.end()) {
+            int rc = ctx->ensure_status(wk::ptr_size(it->second) / wk::kPipeMaxTileRows + 4ull * wk::pipe_grid(ctx->sm_count));
+            if (rc) return rc;
+        }
+    }
+    if (!vers) return WK_SUCCESS;
     uint64_t rows = 1;
-    for (size_t i = 1; i < steps.size(); ++i)
-        if (steps[i].in_cols > 0) rows = std::max<uint64_t>(rows, ctx->rbuf[(i - 1) & 1].cap / steps[i].in_cols);
-    // the versatile steps always use the scratch; the flat passes only from their threshold on
-    return (vers || rows >= ctx->flat_min_rows) ? ctx->ensure_flat(rows) : WK_SUCCESS;
+    for (auto& s : steps)
+        if (s.in_cols > 0) rows = std::max<uint64_t>(rows, std::max(ctx->rbuf[0].cap, ctx->rbuf[1].cap) / s.in_cols);
+    return ctx->ensure_flat(rows);
 }
 
-static int enqueue_plan(wk_ctx* ctx, const std::vector<wk::PlanStep>& steps, const wk_query& q) {
-    const int fm = plan_flat_mode(steps);
-    for (size_t i = 0; i < steps.size(); ++i) {
+static int enqueue_plan(wk_ctx* ctx, const std::vector<wk::PlanStep>& steps, const std::vector<wk::PlanPass>& passes,
+                        const wk_query& q) {
+    for (size_t i = 0; i < passes.size(); ++i) {
         const wk_table* in = i ? &ctx->rbuf[(i - 1) & 1] : nullptr;
-        wk_table* out = &ctx->rbuf[i & 1];
-        int rc = wk::enqueue_step(ctx, steps[i], in, out, q.mt_tid, q.mt_factor, ctx->stream, 0, fm);
+        int rc = wk::enqueue_pass(ctx, steps, passes[i], in, &ctx->rbuf[i & 1], q.mt_tid, q.mt_factor, !ctx->no_fuse,
+                                  ctx->stream);
         if (rc) return rc;
     }
     return WK_SUCCESS;
@@ -1384,6 +1493,7 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
         }
         *out_table = &ctx->rbuf[(steps.size() - 1) & 1];
     } else {
+        std::vector<wk::PlanPass> passes;
         for (int attempt = 0;; ++attempt) {
             if (attempt >= 8) return ctx->fail(WK_E_CAPACITY, "results kept overflowing");
             uint64_t mx = std::max(ctx->rbuf[0].cap, ctx->rbuf[1].cap);
@@ -1391,8 +1501,9 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
             if (rc) return rc;
             rc = ctx->ensure_heavy(mx);
             if (rc) return rc;
-            rc = plan_ensure_flat(ctx, steps);
+            rc = plan_scratch(ctx, steps);
             if (rc) return rc;
+            passes = query_passes(ctx, steps);
             if (mode == WK_MODE_GRAPH) {
                 std::string key = plan_key(steps, *q, ctx);
                 auto it = ctx->graphs.find(key);
@@ -1400,7 +1511,7 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
                     if (ctx->graphs.size() > 256) ctx->drop_graphs();
                     cudaGraph_t graph;
                     WK_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-                    int erc = enqueue_plan(ctx, steps, *q);
+                    int erc = enqueue_plan(ctx, steps, passes, *q);
                     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
                     if (erc) return erc;
                     if (ce != cudaSuccess) return ctx->cuda_fail(ce, "end capture");
@@ -1412,7 +1523,7 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
                 }
                 WK_CUDA(ctx, cudaGraphLaunch(it->second.exec, ctx->stream));
             } else {
-                rc = enqueue_plan(ctx, steps, *q);
+                rc = enqueue_plan(ctx, steps, passes, *q);
                 if (rc) return rc;
             }
             uint32_t err = 0;
@@ -1424,6 +1535,7 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
             if (rc) return rc;
             if (err & wk::kErrCorrupt) return ctx->fail(WK_E_CORRUPT, "key table chain out of range");
             if (err & wk::kErrTimeout) return ctx->fail(WK_E_TIMEOUT, "tile look-back timed out");
+            if (err & wk::kErrUnfuse) ctx->no_fuse = true;   // vid 0 in the store's lists
             if (err & (wk::kErrOverflow | wk::kErrStatus)) {
                 int wmax = 1;
                 for (auto& s : steps) wmax = std::max(wmax, s.out_cols);
@@ -1435,10 +1547,11 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
                 }
             }
         }
-        *out_table = &ctx->rbuf[(steps.size() - 1) & 1];
+        // a replayed graph does not run enqueue_pass, so set the final table's width here
+        wk_table* t = final_table(ctx, passes);
+        t->cols = steps.back().out_cols;
+        *out_table = t;
     }
-    // a replayed graph does not run enqueue_step, so set the final table's width here
-    if (!steps.empty()) ctx->rbuf[(steps.size() - 1) & 1].cols = steps.back().out_cols;
     if (col_num) *col_num = cm.col_num;
     if (v2c_map)
         for (int i = 0; i < q->nvars; ++i) v2c_map[i] = cm.v2c[i];
@@ -1491,7 +1604,6 @@ int wk::lane_prepare(wk_ctx* lane, uint64_t elems) {
     const uint64_t mx = std::max(lane->rbuf[0].cap, lane->rbuf[1].cap);
     int rc = lane->ensure_status(mx / kTileRows + 2);
     if (!rc) rc = lane->ensure_heavy(mx);
-    if (!rc && lane->flat_min_rows) rc = lane->ensure_flat(mx);
     return rc;
 }
 
@@ -1515,10 +1627,10 @@ extern "C" int wk_query_enqueue(wk_ctx* ctx, const wk_query* q, int32_t mode) {
         auto it = ctx->graphs.find(plan_key(steps, *q, ctx));
         if (it == ctx->graphs.end()) return ctx->fail(WK_E_BADARG, "plan not captured yet");
         WK_CUDA(ctx, cudaGraphLaunch(it->second.exec, ctx->stream));
-        if (!steps.empty()) ctx->rbuf[(steps.size() - 1) & 1].cols = steps.back().out_cols;
+        if (!steps.empty()) final_table(ctx, query_passes(ctx, steps))->cols = steps.back().out_cols;
         return WK_SUCCESS;
     }
-    return enqueue_plan(ctx, steps, *q);
+    return enqueue_plan(ctx, steps, query_passes(ctx, steps), *q);
 }
 
 // Sticky device-side error bits of the context stream (0 = none); clears them.
@@ -1567,9 +1679,12 @@ extern "C" int wk_query_profile(wk_ctx* ctx, const wk_query* q, int32_t iters, w
     const wk_table* t = nullptr;
     rc = query_run(ctx, q, WK_MODE_PLAIN, &t, nullptr, nullptr);   // sizes the buffers
     if (rc) return rc;
-    rc = plan_ensure_flat(ctx, steps);
+    rc = plan_scratch(ctx, steps);
     if (rc) return rc;
-    const int fm = plan_flat_mode(steps);
+    // each known_to_* step as a pass of its own where the query runs fused passes
+    auto pass_of = [&](size_t i) {
+        return wk::PlanPass{(int)i, 1, ctx->flat_min_rows && !wk::is_versatile_step(steps[i].kind) && steps[i].in_cols > 0};
+    };
     cudaEvent_t e0, e1;
     WK_CUDA(ctx, cudaEventCreate(&e0));
     WK_CUDA(ctx, cudaEventCreate(&e1));
@@ -1580,7 +1695,8 @@ extern "C" int wk_query_profile(wk_ctx* ctx, const wk_query* q, int32_t iters, w
             wk_table* o = &ctx->rbuf[i & 1];
             WK_CUDA(ctx, cudaMemsetAsync(&ctx->d_ctl->sum_deg, 0, 16, ctx->stream));
             WK_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
-            rc = wk::enqueue_step(ctx, steps[i], in, o, q->mt_tid, q->mt_factor, ctx->stream, 0, fm);
+            rc = wk::enqueue_pass(ctx, steps, pass_of(i), in, o, q->mt_tid, q->mt_factor, !ctx->no_fuse, ctx->stream,
+                                  true);
             if (rc) return rc;
             WK_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
             WK_CUDA(ctx, cudaEventSynchronize(e1));

@@ -10,6 +10,7 @@
 #include "wk_internal.h"
 #include "wk_explore.h"
 #include "wk_flat.h"
+#include "wk_pipe.h"
 #include "wk_kernels.h"
 #include "wk_versatile.h"
 
@@ -89,9 +90,11 @@ struct wk_ctx {
     std::vector<wk_seg_meta> segs;
     wk::SegIndex index;
     std::vector<wk::SegDesc> seg_desc;   // of each segment, with its directory
+    std::vector<uint32_t> seg_longest;   // entries of each segment's longest list
+    bool no_fuse = false;                // a query met vid 0 in a functional step (kErrUnfuse)
     wk::SegDesc* d_segs = nullptr;       // DevStore::segs: an absent segment, then seg_desc
     wk::DirBlock* d_dir_blocks = nullptr;   // vertex directories (wk_dir.cu)
-    uint64_t* d_dir_words = nullptr;
+    void* d_dir_words = nullptr;
     bool has_dir = false;                // some segment has a directory
     uint64_t store_gen = 0;              // stores this context has held (captured launches hold
                                          // the addresses of theirs)
@@ -99,7 +102,7 @@ struct wk_ctx {
     bool versatile = false;           // the store holds the vertex-predicate lists
     wk::PredSeg* d_pseg = nullptr;    // predicate segments by pid * 2 + dir (versatile steps)
     uint32_t n_pseg = 0;
-    std::map<uint32_t, uint64_t> index_len;   // tpid * 2 + dir -> length of its index list
+    std::map<uint32_t, uint64_t> index_ptr;   // tpid * 2 + dir -> pointer word of its index list
     uint64_t* d_inline_orig = nullptr;   // (slot index, original pointer word) of every slot
     uint64_t n_inline = 0;               // whose one-entry list is kept in the slot itself
     bool borrowed_store = false;   // a serving lane: the store belongs to its parent context
@@ -160,7 +163,6 @@ struct wk_ctx {
         s.edges = d_edges;
         s.n_edges = n_edges;
         s.segs = d_segs;
-        s.dir_words = d_dir_words;
         return s;
     }
     wk::SegDesc seg_of(uint64_t vid, uint32_t pid, int dir) const {
@@ -202,16 +204,22 @@ struct wk_ctx {
 };
 
 namespace wk {
-// How a known_to_* step of a single query is launched.
-enum FlatMode {
-    kTileOnly = 0,   // the tile launch (wk_explore.cu)
-    kFlatAuto = 1,   // both, each guarded on the device by flat_min_rows: one of them runs
-    kFlatOnly = 2,   // the flat pipeline (wk_flat.cu); needs ensure_flat for the input
-};
-// Enqueue one resolved step reading `in` (may be null for index/const starts) into `out`.
+// Enqueue one resolved step reading `in` (may be null for index/const starts) into `out`: a
+// start or versatile step by its own launch, a known_to_* step by the tile launch.
 int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* out,
-                 int32_t mt_tid, int32_t mt_factor, cudaStream_t s, int grid_override,
-                 int flat_mode = kTileOnly);
+                 int32_t mt_tid, int32_t mt_factor, cudaStream_t s);
+// Consecutive steps [first, first + n) of a plan that run as one launch: a fused pass
+// (wk_pipe.cu), or (pipe false) one step by enqueue_step.
+struct PlanPass {
+    int first, n;
+    bool pipe;
+};
+// The passes of a plan; `fuse` false: one step each (a start list still joins its first step).
+std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>& steps, bool fuse);
+// Enqueue one pass reading `in` (null when it starts the plan) into `out`.  `fuse` as above;
+// `account`: the steps' bytes and list entries are added to the control block (a profile).
+int enqueue_pass(wk_ctx* ctx, const std::vector<PlanStep>& steps, const PlanPass& p, const wk_table* in, wk_table* out,
+                 int32_t mt_tid, int32_t mt_factor, bool fuse, cudaStream_t s, bool account = false);
 // The device descriptor of a resolved step.
 StepDesc make_step_desc(const wk_ctx* ctx, const PlanStep& s);
 

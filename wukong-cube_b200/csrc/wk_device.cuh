@@ -5,7 +5,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include "wk_kernels.h"
+#include "wk_explore.h"
 
 namespace wk {
 namespace dev {
@@ -153,14 +153,20 @@ __device__ __forceinline__ uint32_t list_at(const uint32_t* edges, uint64_t off,
 }
 
 // ---------------------------------------------------------------- vertex directory
-// Pointer word of id `i` of a directory (i < vid_span) whose block is `b`; 0 when absent.
-__device__ __forceinline__ ulonglong2 dir_block(const SegDesc& s, uint32_t i) {
-    return __ldg(reinterpret_cast<const ulonglong2*>(s.dir) + (i >> 6));
+// Block of id `i` of a directory (i < vid_span); whether the id has a key; its word's place.
+__device__ __forceinline__ uint2 dir_block(const SegDesc& s, uint32_t i) {
+    return __ldg(reinterpret_cast<const uint2*>(s.dir) + (i >> 5));
 }
-__device__ __forceinline__ uint64_t dir_word(const DevStore& st, ulonglong2 b, uint32_t i) {
-    const unsigned long long bit = 1ull << (i & 63);
-    return (b.x & bit) ? __ldg(reinterpret_cast<const unsigned long long*>(st.dir_words) + b.y + __popcll(b.x & (bit - 1)))
-                       : 0;
+__device__ __forceinline__ bool dir_has(uint2 b, uint32_t i) { return (b.x >> (i & 31)) & 1; }
+__device__ __forceinline__ uint32_t dir_place(uint2 b, uint32_t i) {
+    return b.y + __popc(b.x & ((1u << (i & 31)) - 1));
+}
+// Pointer word of id `i` whose block is `b`; 0 when absent.
+__device__ __forceinline__ uint64_t dir_word(const SegDesc& s, uint2 b, uint32_t i) {
+    if (!dir_has(b, i)) return 0;
+    const uint32_t at = dir_place(b, i);
+    return s.dir_values ? make_inline_ptr(__ldg(static_cast<const uint32_t*>(s.dir_words) + at))
+                        : __ldg(static_cast<const unsigned long long*>(s.dir_words) + at);
 }
 
 // Probe kUnroll keys per group of L lanes.  Every lane of the warp must call this (ballots and
@@ -290,7 +296,7 @@ __device__ __forceinline__ uint64_t seg_lookup(const DevStore& st, const SegDesc
                                                unsigned* err) {
     if (sg.vid_span) {
         const uint32_t i = vid - sg.vid_lo;
-        return i < sg.vid_span ? dir_word(st, dir_block(sg, i), i) : 0;
+        return i < sg.vid_span ? dir_word(sg, dir_block(sg, i), i) : 0;
     }
     return hash_lookup(st, sg, key, err);
 }
@@ -383,17 +389,33 @@ __device__ __forceinline__ uint64_t block_scan(const uint32_t* s_cnt, uint64_t* 
 }
 
 // Decoupled look-back (Merrill & Garland, "Single-pass Parallel Prefix Scan with Decoupled
-// Look-back", 2016) by one warp: each round reads the 32 nearest unvisited predecessors at once,
-// waits until all of them have published at least their aggregate, adds the aggregates up to
-// the nearest inclusive prefix and stops there.  Tiles are claimed in order from the tile
-// counter, so every predecessor is held by a running CTA and the wait ends; it is still bounded.
+// Look-back", 2016) by one warp: it reads the 32 nearest unvisited predecessors (coalesced), adds
+// up the leading ones that have been published and stops at the nearest inclusive prefix among
+// them; once all 32 are there and none holds a prefix it reads kLookWide groups of 32 at a time (a
+// wave of CTAs in step leaves a thousand aggregates before the nearest prefix, an L2 round trip
+// per group otherwise).  Tiles are claimed in order from the tile counter, so every predecessor is
+// held by a running CTA and the wait ends; it is still bounded.
 // The tile's own entry is published first (publish_aggregate, by one thread, as soon as the
 // tile's total is known) and resolved later (resolve_prefix, by all 32 lanes of one warp, which
 // returns the exclusive prefix in every lane).
+constexpr int kLookWide = 8;
 __device__ __forceinline__ void publish_aggregate(unsigned long long* status, uint64_t tile,
                                                   uint64_t agg, unsigned epoch) {
     volatile unsigned long long* st = status;
     st[tile] = pack_status(epoch, tile == 0 ? kFlagPrefix : kFlagAgg, agg);
+}
+
+// Add the published ones of the 32 predecessors p = base - lane, whose words are s, to *v (each
+// lane its own) up to the nearest prefix: 32 when all counted, -1 when a prefix ended the search,
+// else how many counted before one that is not published.
+__device__ __forceinline__ int look_group(unsigned long long s, unsigned epoch, uint64_t* v) {
+    const int lane = threadIdx.x & 31;
+    const unsigned long long flag = (s >> 46) & 3ull;
+    const bool ready = (unsigned)(s >> 48) == epoch && flag != 0;
+    const unsigned pm = __ballot_sync(kFull, ready && flag == kFlagPrefix), mm = __ballot_sync(kFull, !ready);
+    const int fp = pm ? __ffs(pm) - 1 : 32, fm = mm ? __ffs(mm) - 1 : 32;
+    if (lane <= (fp < fm ? fp : fm - 1)) *v += s & kValMask;
+    return fp < fm ? -1 : fm;
 }
 
 __device__ uint64_t resolve_prefix(unsigned long long* status, StepCtl* ctl, uint64_t tile,
@@ -401,33 +423,92 @@ __device__ uint64_t resolve_prefix(unsigned long long* status, StepCtl* ctl, uin
     volatile unsigned long long* st = status;
     const int lane = threadIdx.x & 31;
     if (tile == 0) return 0;   // tile 0 published its inclusive prefix already
-    uint64_t excl = 0;
-    int64_t base = (int64_t)tile - 1;
+    const unsigned long long before_all = pack_status(epoch, kFlagPrefix, 0);   // before tile 0
+    uint64_t v = 0;
+    int64_t base = (int64_t)tile - 1 - lane;
     unsigned long long spins = 0;
-    for (;;) {
-        const int64_t p = base - lane;
-        const unsigned long long s = p >= 0 ? st[p] : pack_status(epoch, kFlagPrefix, 0);
-        const unsigned long long flag = (s >> 46) & 3ull;
-        const bool ready = (unsigned)(s >> 48) == epoch && flag != 0;
-        if (!__all_sync(kFull, ready)) {
+    int n = 0;
+    while (n >= 0) {
+        n = look_group(base >= 0 ? st[base] : before_all, epoch, &v);
+        if (n < 0) break;
+        base -= n;
+        if (n == 0) {   // the nearest one is not there yet
             if (++spins > spin_limit) {
                 if (lane == 0) atomicOr(&ctl->err, kErrTimeout);
                 break;
             }
             if (spins > 32) __nanosleep(32);
+        }
+        while (n == 32) {   // a run of aggregates: several groups in flight
+            unsigned long long s[kLookWide];
+#pragma unroll
+            for (int j = 0; j < kLookWide; ++j) s[j] = base - 32 * j >= 0 ? st[base - 32 * j] : before_all;
+#pragma unroll
+            for (int j = 0; j < kLookWide; ++j)
+                if (n == 32) {
+                    n = look_group(s[j], epoch, &v);
+                    if (n > 0) base -= n;
+                }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    if (lane == 0) st[tile] = pack_status(epoch, kFlagPrefix, v + agg);
+    return v;
+}
+
+// ---------------------------------------------------------------- long-list slice queue
+// Queue the `count`-entry list at `off` of input row in_row (owner q), whose outputs start at
+// out_pos, as kHeavyChunk-row slices: fields first, then the epoch tag.
+__device__ __forceinline__ void push_slices(StepCtl* ctl, HeavyItem* heavy, uint64_t heavy_cap, unsigned epoch,
+                                            uint64_t in_row, uint64_t off, uint64_t out_pos, uint32_t count,
+                                            uint32_t q) {
+    const uint32_t nch = (count + kHeavyChunk - 1) / kHeavyChunk;
+    const unsigned long long at = atomicAdd(&ctl->heavy_n, (unsigned long long)nch);
+    for (uint32_t k = 0; k < nch; ++k) {
+        if (at + k >= heavy_cap) {
+            atomicOr(&ctl->err, kErrOverflow);
+            break;
+        }
+        HeavyItem* it = heavy + at + k;
+        it->in_row = in_row;
+        it->off = off + (uint64_t)k * kHeavyChunk;
+        it->out_pos = out_pos + (uint64_t)k * kHeavyChunk;
+        it->count = min((uint32_t)kHeavyChunk, count - k * kHeavyChunk);
+        it->q = q;
+        __threadfence();
+        *(volatile uint32_t*)&it->tag = epoch;
+    }
+}
+
+// One thread of a CTA out of tiles: claim the next queued slice.  A claimed index either gets
+// reserved by a tile still running (wait for its tag) or lies past the final count once every tile
+// is done (~0: the queue is drained).  The wait is bounded.
+__device__ __forceinline__ unsigned long long claim_slice(StepCtl* ctl, const HeavyItem* heavy, uint64_t heavy_cap,
+                                                          uint64_t ntiles, unsigned epoch,
+                                                          unsigned long long spin_limit) {
+    const unsigned long long idx = atomicAdd(&ctl->heavy_claim, 1ull);
+    unsigned long long spins = 0;
+    for (;;) {
+        unsigned long long hn = *(volatile unsigned long long*)&ctl->heavy_n;
+        if (idx < hn) {
+            if (idx >= heavy_cap) return ~0ull;   // the queue overflowed; kErrOverflow is already set
+            if (*(volatile const uint32_t*)&heavy[idx].tag == epoch) {
+                __threadfence();
+                return idx;
+            }
+        } else if (*(volatile unsigned long long*)&ctl->tiles_done >= ntiles) {
+            __threadfence();
+            hn = *(volatile unsigned long long*)&ctl->heavy_n;
+            if (idx >= hn) return ~0ull;
             continue;
         }
-        const unsigned pm = __ballot_sync(kFull, flag == kFlagPrefix);
-        const int first = pm ? __ffs(pm) - 1 : 32;   // nearest predecessor holding a prefix
-        uint64_t v = lane <= first ? (s & kValMask) : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-        excl += v;
-        if (pm) break;
-        base -= 32;
+        if (++spins > spin_limit) {
+            atomicOr(&ctl->err, kErrTimeout);
+            return ~0ull;
+        }
+        if (spins > 32) __nanosleep(64);
     }
-    if (lane == 0) st[tile] = pack_status(epoch, kFlagPrefix, excl + agg);
-    return excl;
 }
 
 // Copy `count` words from shared memory to global memory with 16-byte stores where aligned.
@@ -454,15 +535,16 @@ __device__ __forceinline__ void store_words(uint32_t* dst, const uint32_t* src, 
 // The last CTA to leave resets the tile/exit counters and advances the epoch; when the 16-bit
 // epoch wraps it clears the status array first so no stale word can match the next epoch.
 // `tags` / `tag_stride` / `n_tags`: epoch-tagged words of the long-list slice queue, cleared with
-// the status array when the epoch wraps.
+// the status array when the epoch wraps.  n_ctas: how many CTAs of the launch get here.
 __device__ void exit_protocol(StepCtl* ctl, unsigned long long* status, unsigned epoch,
-                              unsigned* tags, unsigned tag_stride, unsigned long long n_tags) {
+                              unsigned* tags, unsigned tag_stride, unsigned long long n_tags,
+                              unsigned n_ctas = gridDim.x) {
     __shared__ int s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned prev = atomicAdd(&ctl->exit_counter, 1u);
-        s_last = (prev == gridDim.x - 1);
+        s_last = (prev == n_ctas - 1);
     }
     __syncthreads();
     if (!s_last) return;

@@ -4,11 +4,12 @@
 // a probe of a distinct key moves a whole DRAM line for the 16 bytes it reads, however near the
 // vertex ids are to each other.  Wukong's ids are dense (its string server hands them out in
 // order of appearance), so each (predicate, direction) segment also gets a directory by vertex id
-// on the device: one 16-byte block per 64 ids (which of them have a key, and where the first
-// one's pointer word is) and the keys' pointer words in vertex order.  A lookup reads its block
-// and, where the bit is set, one word.  Neighbouring vertices share both, absent keys are settled
-// by the bit, and at 10,000 organisations a segment's blocks (11 MB) stay in L2.  The words are
-// the slots' own, so a lookup answers what the probe answers; segments whose ids are too thin for
+// on the device: one 8-byte block per 32 ids (which of them have a key, and where the first one's
+// word is) and the keys' words in vertex order: their pointer words, or, for a segment whose lists
+// all have one entry, those entries.  A lookup reads its block and, where the bit is set, one word.
+// Neighbouring vertices share both, absent keys are settled by the bit, and at 10,000 organisations
+// a segment's blocks (11 MB) stay in L2.  The words are the slots' own, so a lookup answers what
+// the probe answers; segments whose ids are too thin for
 // one (see dir_plan in wk_ctx.cpp) keep the hash probe.  Measured against probing by hash, whole
 // calls: the triangle at 10,000 organisations 868 -> 449 us (its first two count passes 305 and
 // 119 -> 103 us each, where the writes now bound them), the star over a Zipf graph of 3,001 198 ->
@@ -42,10 +43,13 @@ __device__ __forceinline__ uint32_t pseg_find(const PredSeg* ps, uint32_t n, uin
     return lo < n && __ldg(&ps[lo].key) == key ? lo : n;
 }
 
-__device__ __forceinline__ void flush_range(uint32_t* vid, uint32_t seg, uint32_t n_pseg, uint32_t lo, uint32_t hi) {
-    if (seg >= n_pseg || lo > hi) return;
-    atomicMin(vid + 2 * seg, lo);
-    atomicMax(vid + 2 * seg + 1, hi);
+__device__ __forceinline__ void flush_range(SegScan* out, uint32_t seg, uint32_t n_pseg, uint32_t lo, uint32_t hi,
+                                            uint32_t longest) {
+    if (seg >= n_pseg) return;
+    if (longest) atomicMax(&out[seg].longest, longest);
+    if (lo > hi) return;
+    atomicMin(&out[seg].vid_lo, lo);
+    atomicMax(&out[seg].vid_hi, hi);
 }
 
 // One thread per slot, each warp over a contiguous share, four slots loaded before any is looked
@@ -56,7 +60,7 @@ __device__ __forceinline__ void flush_range(uint32_t* vid, uint32_t seg, uint32_
 // this check cost on that store.
 constexpr int kScanUnroll = 4;
 __global__ void __launch_bounds__(kLoadThreads)
-store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, uint32_t* vid, StoreScan* out,
+store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, SegScan* per_seg, StoreScan* out,
                   ulonglong2* chunks, uint32_t max_chunks) {
     const uint64_t n_slots = st.n_buckets * kAssoc;
     const int lane = threadIdx.x & 31;
@@ -65,7 +69,7 @@ store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, uint3
     constexpr uint64_t kStep = 32 * kScanUnroll;
     const uint64_t share = ((n_slots + warps - 1) / warps + kStep - 1) / kStep * kStep;
     const uint64_t lo = min(n_slots, w * share), hi = min(n_slots, lo + share);
-    uint32_t flags = 0, seg = n_pseg, seg_key = 0xFFFFFFFFu, vlo = 0xFFFFFFFFu, vhi = 0;
+    uint32_t flags = 0, seg = n_pseg, seg_key = 0xFFFFFFFFu, vlo = 0xFFFFFFFFu, vhi = 0, longest = 0;
     unsigned long long ones = 0;
     for (uint64_t b = lo; b < hi; b += kStep) {
         Slot sl[kScanUnroll];
@@ -84,13 +88,14 @@ store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, uint3
                 const uint64_t v = key_vid(sl[u].key);
                 const uint32_t k = key_pid(sl[u].key) * 2 + key_dir(sl[u].key);
                 if (k != seg_key) {
-                    flush_range(vid, seg, n_pseg, vlo, vhi);
+                    flush_range(per_seg, seg, n_pseg, vlo, vhi, longest);
                     seg_key = k;
                     seg = pseg_find(pseg, n_pseg, k);
                     vlo = 0xFFFFFFFFu;
-                    vhi = 0;
+                    vhi = longest = 0;
                 }
-                if (v != 0 && v <= 0xFFFFFFFFull) {
+                if (v != 0) longest = max(longest, (uint32_t)ptr_size(sl[u].ptr));   // vid 0: an index list
+                if (v != 0 && v < kBlankId) {
                     vlo = min(vlo, (uint32_t)v);
                     vhi = max(vhi, (uint32_t)v);
                 }
@@ -138,9 +143,10 @@ store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, uint3
     if (__all_sync(kFull, seg == seg0)) {
         vlo = __reduce_min_sync(kFull, vlo);
         vhi = __reduce_max_sync(kFull, vhi);
-        if (lane == 0) flush_range(vid, seg, n_pseg, vlo, vhi);
+        longest = __reduce_max_sync(kFull, longest);
+        if (lane == 0) flush_range(per_seg, seg, n_pseg, vlo, vhi, longest);
     } else {
-        flush_range(vid, seg, n_pseg, vlo, vhi);
+        flush_range(per_seg, seg, n_pseg, vlo, vhi, longest);
     }
     flags = __reduce_or_sync(kFull, flags);
     for (int o = 16; o > 0; o >>= 1) ones += __shfl_xor_sync(kFull, ones, o);
@@ -246,7 +252,7 @@ __device__ __forceinline__ void dir_walk(const DevStore& st, const DirSeg* segs,
                         end = false;
                     } else {
                         const uint64_t v = key_vid(key);
-                        if (v != 0 && v <= 0xFFFFFFFFull && key_pid(key) * 2 + key_dir(key) == d.key &&
+                        if (v != 0 && v < kBlankId && key_pid(key) * 2 + key_dir(key) == d.key &&
                             bucket_of(key, d.seg) == home)
                             f(d, (uint32_t)v, ptr);
                     }
@@ -262,33 +268,37 @@ __device__ __forceinline__ void dir_walk(const DevStore& st, const DirSeg* segs,
 __global__ void __launch_bounds__(kLoadThreads)
 dir_bits_kernel(const DevStore st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets, DirBlock* blocks,
                 unsigned* flags) {
-    dir_walk(st, segs, n_segs, n_buckets, flags, [&](const DirSeg& d, uint32_t vid, uint64_t) {
+    dir_walk(st, segs, n_segs, n_buckets, flags, [&](const DirSeg& d, uint32_t vid, uint64_t ptr) {
+        if (ptr_size(ptr) == 0) return;   // an empty list is no key to any step
         const uint32_t i = vid - d.seg.vid_lo;
         if (i >= d.seg.vid_span) return;   // the scan saw every key, so none is outside
-        unsigned* half = reinterpret_cast<unsigned*>(&blocks[d.block0 + (i >> 6)].bits) + ((i >> 5) & 1);
         const unsigned bit = 1u << (i & 31);
-        if (atomicOr(half, bit) & bit) atomicOr(flags, (unsigned)kStoreDupKey);
+        if (atomicOr(&blocks[d.block0 + (i >> 5)].bits, bit) & bit) atomicOr(flags, (unsigned)kStoreDupKey);
     });
 }
 
 __global__ void __launch_bounds__(kLoadThreads)
-dir_fill_kernel(const DevStore st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets, uint64_t* words,
-                unsigned* flags) {
+dir_fill_kernel(const DevStore st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets, unsigned* flags) {
     dir_walk(st, segs, n_segs, n_buckets, flags, [&](const DirSeg& d, uint32_t vid, uint64_t ptr) {
         const uint32_t i = vid - d.seg.vid_lo;
-        if (i >= d.seg.vid_span) return;
-        const DirBlock b = d.seg.dir[i >> 6];
-        words[b.base + __popcll(b.bits & ((1ull << (i & 63)) - 1))] = ptr;
+        if (i >= d.seg.vid_span || ptr_size(ptr) == 0) return;
+        const uint32_t at = dir_place(dir_block(d.seg, i), i);
+        if (d.seg.dir_values)
+            static_cast<uint32_t*>(const_cast<void*>(d.seg.dir_words))[at] =
+                ptr_is_inline(ptr) ? (uint32_t)(ptr >> kNbitsSize) : __ldg(st.edges + ptr_off(ptr));
+        else
+            static_cast<uint64_t*>(const_cast<void*>(d.seg.dir_words))[at] = ptr;
     });
 }
 
-// Each block's base: the keys of the blocks before it.  kDirScanBlocks blocks per CTA; the CTAs'
-// sums are scanned by one CTA in between.
-__global__ void __launch_bounds__(kLoadThreads) dir_sum_kernel(const DirBlock* blocks, uint64_t n, uint64_t* sums) {
+// Each block's base: the keys of its segment's blocks before it.  kDirScanBlocks blocks per CTA
+// (segments start at multiples of that many blocks); the CTAs' sums are scanned by one CTA in
+// between.
+__global__ void __launch_bounds__(kLoadThreads) dir_sum_kernel(const DirBlock* blocks, uint64_t* sums) {
     __shared__ uint64_t s_warp[kLoadThreads / 32];
-    const uint64_t b0 = (uint64_t)blockIdx.x * kDirScanBlocks, b1 = min(n, b0 + kDirScanBlocks);
+    const uint64_t b0 = (uint64_t)blockIdx.x * kDirScanBlocks;
     uint64_t c = 0;
-    for (uint64_t i = b0 + threadIdx.x; i < b1; i += kLoadThreads) c += __popcll(blocks[i].bits);
+    for (uint32_t i = threadIdx.x; i < kDirScanBlocks; i += kLoadThreads) c += __popc(blocks[b0 + i].bits);
     const uint64_t ex = block_exclusive_sum<kLoadThreads>(c, s_warp);
     if (threadIdx.x == kLoadThreads - 1) sums[blockIdx.x] = ex + c;
 }
@@ -311,20 +321,27 @@ __global__ void __launch_bounds__(kLoadThreads) dir_scan_kernel(uint64_t* sums, 
     if (threadIdx.x == 0) sums[n] = s_carry;
 }
 
-__global__ void __launch_bounds__(kLoadThreads) dir_base_kernel(DirBlock* blocks, uint64_t n, const uint64_t* sums) {
+__global__ void __launch_bounds__(kLoadThreads)
+dir_base_kernel(DirBlock* blocks, const uint64_t* sums, const DirSeg* segs, uint32_t n_segs) {
     __shared__ uint64_t s_warp[kLoadThreads / 32];
     constexpr int kPer = kDirScanBlocks / kLoadThreads;   // consecutive blocks per thread
     const uint64_t b0 = (uint64_t)blockIdx.x * kDirScanBlocks + threadIdx.x * kPer;
-    uint64_t c[kPer], sum = 0;
+    uint32_t lo = 0, hi = n_segs - 1;   // the segment these blocks belong to
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (__ldg(&segs[mid].block0) <= b0) lo = mid; else hi = mid - 1;
+    }
+    const uint64_t first = sums[segs[lo].block0 / kDirScanBlocks];
+    uint32_t c[kPer], sum = 0;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        c[k] = b0 + k < n ? __popcll(blocks[b0 + k].bits) : 0;
+        c[k] = __popc(blocks[b0 + k].bits);
         sum += c[k];
     }
-    uint64_t at = sums[blockIdx.x] + block_exclusive_sum<kLoadThreads>(sum, s_warp);
+    uint32_t at = (uint32_t)(sums[blockIdx.x] - first + block_exclusive_sum<kLoadThreads>(sum, s_warp));
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        if (b0 + k < n) blocks[b0 + k].base = at;
+        blocks[b0 + k].base = at;
         at += c[k];
     }
 }
@@ -333,9 +350,9 @@ int load_grid(int sm_count) { return sm_count * (2048 / kLoadThreads); }
 
 }  // namespace
 
-cudaError_t launch_store_scan(const DevStore& st, const PredSeg* pseg, uint32_t n_pseg, uint32_t* vid, StoreScan* out,
-                              ulonglong2* chunks, uint32_t max_chunks, int sm_count, cudaStream_t s) {
-    store_scan_kernel<<<load_grid(sm_count), kLoadThreads, 0, s>>>(st, pseg, n_pseg, vid, out, chunks, max_chunks);
+cudaError_t launch_store_scan(const DevStore& st, const PredSeg* pseg, uint32_t n_pseg, SegScan* per_seg,
+                              StoreScan* out, ulonglong2* chunks, uint32_t max_chunks, int sm_count, cudaStream_t s) {
+    store_scan_kernel<<<load_grid(sm_count), kLoadThreads, 0, s>>>(st, pseg, n_pseg, per_seg, out, chunks, max_chunks);
     chunk_check_kernel<<<load_grid(sm_count), kLoadThreads, 0, s>>>(st.edges, chunks, max_chunks, out);
     return cudaGetLastError();
 }
@@ -349,17 +366,17 @@ cudaError_t launch_inline(const DevStore& st, unsigned long long* n, uint64_t* o
 cudaError_t launch_dir_bits(const DevStore& st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets,
                             DirBlock* blocks, uint64_t n_blocks, uint64_t* sums, StoreScan* out, int sm_count,
                             cudaStream_t s) {
-    const uint32_t n_sums = (uint32_t)((n_blocks + kDirScanBlocks - 1) / kDirScanBlocks);
+    const uint32_t n_sums = (uint32_t)(n_blocks / kDirScanBlocks);
     dir_bits_kernel<<<load_grid(sm_count), kLoadThreads, 0, s>>>(st, segs, n_segs, n_buckets, blocks, &out->flags);
-    dir_sum_kernel<<<n_sums, kLoadThreads, 0, s>>>(blocks, n_blocks, sums);
+    dir_sum_kernel<<<n_sums, kLoadThreads, 0, s>>>(blocks, sums);
     dir_scan_kernel<<<1, kLoadThreads, 0, s>>>(sums, n_sums);
-    dir_base_kernel<<<n_sums, kLoadThreads, 0, s>>>(blocks, n_blocks, sums);
+    dir_base_kernel<<<n_sums, kLoadThreads, 0, s>>>(blocks, sums, segs, n_segs);
     return cudaGetLastError();
 }
 
 cudaError_t launch_dir_fill(const DevStore& st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets,
-                            uint64_t* words, StoreScan* out, int sm_count, cudaStream_t s) {
-    dir_fill_kernel<<<load_grid(sm_count), kLoadThreads, 0, s>>>(st, segs, n_segs, n_buckets, words, &out->flags);
+                            StoreScan* out, int sm_count, cudaStream_t s) {
+    dir_fill_kernel<<<load_grid(sm_count), kLoadThreads, 0, s>>>(st, segs, n_segs, n_buckets, &out->flags);
     return cudaGetLastError();
 }
 

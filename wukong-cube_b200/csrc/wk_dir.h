@@ -27,12 +27,18 @@ inline uint32_t store_scan_chunks(uint64_t n_edges) {   // room for every chunk 
     return (uint32_t)(2 * n_edges / kChunkList) + 1;
 }
 
-// Pass over every slot: the checks, the one-entry lists counted, and the lowest and highest
-// vertex id of each predicate segment's keys (vid[2 * i], vid[2 * i + 1] for pseg[i]; the
-// caller sets them to 0xFFFFFFFF and 0; ids of 2^32 or more are left out).  `chunks`:
-// store_scan_chunks(n_edges) entries of scratch.
-cudaError_t launch_store_scan(const DevStore& st, const PredSeg* pseg, uint32_t n_pseg, uint32_t* vid, StoreScan* out,
-                              ulonglong2* chunks, uint32_t max_chunks, int sm_count, cudaStream_t s);
+// What it finds of each predicate segment.
+struct SegScan {
+    uint32_t vid_lo, vid_hi;   // lowest and highest vertex id of its keys (the blank id and
+                               // above left out); 0xFFFFFFFF and 0 when there is none
+    uint32_t longest;          // entries of its longest list
+    uint32_t pad;
+};
+
+// Pass over every slot: the checks, the one-entry lists counted, and per_seg[i] for pseg[i] (set
+// by the caller to no key, 0).  `chunks`: store_scan_chunks(n_edges) entries of scratch.
+cudaError_t launch_store_scan(const DevStore& st, const PredSeg* pseg, uint32_t n_pseg, SegScan* per_seg,
+                              StoreScan* out, ulonglong2* chunks, uint32_t max_chunks, int sm_count, cudaStream_t s);
 // One-entry lists into their keys' pointer words; the original words (slot index, word) go to
 // orig, counted in *n (0 on entry).
 cudaError_t launch_inline(const DevStore& st, unsigned long long* n, uint64_t* orig, int sm_count, cudaStream_t s);
@@ -42,19 +48,20 @@ cudaError_t launch_inline(const DevStore& st, unsigned long long* n, uint64_t* o
 struct DirSeg {
     uint64_t first;          // main buckets of the segments before it in the table
     uint64_t block0;
-    SegDesc seg;             // vid_lo, vid_span and (for the fill) dir set
+    SegDesc seg;             // vid_lo, vid_span, dir, dir_values and (for the fill) dir_words set
     uint32_t key;            // pid * 2 + dir
     uint32_t pad;
 };
 // Set the presence bits of every key a probe of its segment finds (flags: kStoreBadChain,
-// kStoreDupKey), then each block's base: blocks[] and sums[] (one per kDirScanBlocks blocks, plus
-// the total, which *words receives) on the device.
-constexpr uint32_t kDirScanBlocks = 2048;
+// kStoreDupKey), then each block's base.  block0 and n_blocks are multiples of kDirScanBlocks;
+// sums[k] becomes the keys of the blocks before k * kDirScanBlocks (n_blocks / kDirScanBlocks + 1
+// entries).
+constexpr uint32_t kDirScanBlocks = 512;
 cudaError_t launch_dir_bits(const DevStore& st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets,
                             DirBlock* blocks, uint64_t n_blocks, uint64_t* sums, StoreScan* out, int sm_count,
                             cudaStream_t s);
-// Put every key's pointer word in its place.
+// Put every key's word in its place (seg.dir_words).
 cudaError_t launch_dir_fill(const DevStore& st, const DirSeg* segs, uint32_t n_segs, uint64_t n_buckets,
-                            uint64_t* words, StoreScan* out, int sm_count, cudaStream_t s);
+                            StoreScan* out, int sm_count, cudaStream_t s);
 
 }  // namespace wk

@@ -236,7 +236,7 @@ __device__ __forceinline__ void tile_probe_rows(const ExploreArgs& a, const Tile
     uint64_t key[kRows];
     uint32_t tgt[kRows], flag[kRows], id[kRows];
     const SegDesc* sg[kRows];
-    ulonglong2 blk[kRows];
+    uint2 blk[kRows];
     constexpr uint32_t kNoDir = 0xFFFFFFFFu;   // the row's segment has no directory
 #pragma unroll
     for (int k = 0; k < kRows; ++k) {
@@ -245,7 +245,7 @@ __device__ __forceinline__ void tile_probe_rows(const ExploreArgs& a, const Tile
         tgt[k] = 0;
         id[k] = 0;
         flag[k] = kXDone;
-        blk[k] = make_ulonglong2(0, 0);
+        blk[k] = make_uint2(0, 0);
         if (row < n) sg[k] = row_setup(a, B, row, wi, &key[k], &tgt[k], &flag[k]);
         if (flag[k] & 0x200u) {
             const uint32_t span = __ldg(&sg[k]->vid_span);
@@ -260,7 +260,7 @@ __device__ __forceinline__ void tile_probe_rows(const ExploreArgs& a, const Tile
     for (int k = 0; k < kRows; ++k) {
         p[k] = 0;
         if (!(flag[k] & 0x200u)) continue;
-        if (id[k] != kNoDir) p[k] = dir_word(a.store, blk[k], id[k]);
+        if (id[k] != kNoDir) p[k] = dir_word(*sg[k], blk[k], id[k]);
         else p[k] = hash_lookup(a.store, *sg[k], key[k], &a.ctl->err);
     }
 #pragma unroll
@@ -440,27 +440,12 @@ __device__ __forceinline__ void tile_back(const ExploreArgs& a, const TileBuf& B
             if (i == n - 1 || B.q[i + 1] != q) atomicAdd(a.qcount + q, (unsigned long long)(excl + B.pre[i + 1]));
         }
     }
-    // long lists -> slices on the queue (fields first, then the epoch tag)
+    // long lists -> slices on the queue
     if (S.has_heavy && fits) {
         for (int i = threadIdx.x; i < n; i += kStepThreads) {
             const uint32_t c = B.cnt[i];
             if (c <= slice_threshold(a)) continue;
-            const uint32_t nch = (c + kHeavyChunk - 1) / kHeavyChunk;
-            const unsigned long long at = atomicAdd(&a.ctl->heavy_n, (unsigned long long)nch);
-            for (uint32_t k = 0; k < nch; ++k) {
-                if (at + k >= a.heavy_cap) {
-                    atomicOr(&a.ctl->err, kErrOverflow);
-                    break;
-                }
-                HeavyItem* it = a.heavy + at + k;
-                it->in_row = r0 + i;
-                it->off = B.off[i] + (uint64_t)k * kHeavyChunk;
-                it->out_pos = excl + B.pre[i] + (uint64_t)k * kHeavyChunk;
-                it->count = min((uint32_t)kHeavyChunk, c - k * kHeavyChunk);
-                it->q = B.q[i];
-                __threadfence();
-                *(volatile uint32_t*)&it->tag = epoch;
-            }
+            push_slices(a.ctl, a.heavy, a.heavy_cap, epoch, r0 + i, B.off[i], excl + B.pre[i], c, B.q[i]);
         }
     }
     WK_PH(5);
@@ -538,16 +523,15 @@ __global__ void __launch_bounds__(kStepThreads, explore_min_blocks(L)) explore_k
     // an input count past its capacity means the step before overflowed (and said so): its rows
     // were never written, so this step does no work and reports no size of its own
     if (!a.virtual_rows && R > a.in_cap_rows) R = 0;
-    const bool handed_off = !a.virtual_rows && a.max_rows && R >= a.max_rows;   // flat pipeline's
-    const Tiling T = make_tiling(handed_off ? 0 : R, a.ctl->status_cap);
+    const Tiling T = make_tiling(R, a.ctl->status_cap);
     uint64_t ntiles = T.ntiles;
     if (ntiles > a.ctl->status_cap) {
         if (threadIdx.x == 0) atomicOr(&a.ctl->err, kErrStatus);
         ntiles = 0;
     }
     const uint64_t obase = a.out_base_rows ? *(volatile const uint64_t*)a.out_base_rows : 0;
-    if (ntiles == 0 && !handed_off && blockIdx.x == 0 && threadIdx.x == 0) *a.out_rows = obase;
-    // Nothing to do (an empty input, or the flat passes run this step): leave at once.  No CTA
+    if (ntiles == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.out_rows = obase;
+    // Nothing to do (an empty input): leave at once.  No CTA
     // claims a tile or a slice or publishes a status word, so the counters stay as the last
     // launch reset them and the epoch need not move (it tags only published words).  A launch
     // that returns at once costs a few microseconds instead of every CTA's counter atomics.
@@ -587,44 +571,11 @@ __global__ void __launch_bounds__(kStepThreads, explore_min_blocks(L)) explore_k
     }
 
     // Out of tiles: write queued long-list slices until every tile is done and the queue is
-    // drained.  A claimed index either gets reserved by a tile still running (wait for its
-    // tag) or lies past the final count (stop).  Every wait is bounded.
+    // drained.
     __syncthreads();
     for (;;) {
-        if (threadIdx.x == 0) {
-            const unsigned long long idx = atomicAdd(&a.ctl->heavy_claim, 1ull);
-            int state = 0;
-            unsigned long long spins = 0;
-            for (;;) {
-                unsigned long long hn = *(volatile unsigned long long*)&a.ctl->heavy_n;
-                if (idx < hn) {
-                    if (idx >= a.heavy_cap) {
-                        state = 2;   // the queue overflowed; kErrOverflow is already set
-                        break;
-                    }
-                    if (*(volatile uint32_t*)&a.heavy[idx].tag == epoch) {
-                        __threadfence();
-                        state = 1;
-                        break;
-                    }
-                } else if (*(volatile unsigned long long*)&a.ctl->tiles_done >= ntiles) {
-                    __threadfence();
-                    hn = *(volatile unsigned long long*)&a.ctl->heavy_n;
-                    if (idx >= hn) {
-                        state = 2;
-                        break;
-                    }
-                    continue;
-                }
-                if (++spins > spin_limit(a)) {
-                    atomicOr(&a.ctl->err, kErrTimeout);
-                    state = 2;
-                    break;
-                }
-                if (spins > 32) __nanosleep(64);
-            }
-            s_claim = state == 1 ? idx : ~0ull;
-        }
+        if (threadIdx.x == 0)
+            s_claim = claim_slice(a.ctl, a.heavy, a.heavy_cap, ntiles, epoch, spin_limit(a));
         __syncthreads();
         const unsigned long long idx = s_claim;
         if (idx == ~0ull) break;

@@ -95,9 +95,6 @@ struct ExploreArgs {
     // shorter ones are written by the CTA that scanned them.  0 means kHeavyRows; values below
     // kMinSliceRows are raised to it (the queues of a context are sized for that).
     uint32_t slice_rows;
-    // When nonzero and the input has at least this many rows, the launch does nothing (the
-    // flat pipeline of wk_flat.cu runs the step instead).
-    uint64_t max_rows;
     // Polls a look-back on a predecessor tile or a wait for the slice queue makes before it
     // gives up and sets kErrTimeout (0: kDefaultSpinLimit).  Tests lower it to make the waits
     // run out; the wait for the launch's own bulk copies keeps its fixed limit.

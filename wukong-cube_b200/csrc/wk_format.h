@@ -83,18 +83,21 @@ struct SegDesc {
     uint64_t num_buckets;    // hash space of the segment (0 = segment absent / empty)
     uint64_t magic;          // floor((2^64 - 1) / num_buckets): Barrett reciprocal of the modulo
     const DirBlock* dir;     // the segment's directory on the device (null when it has none)
+    const void* dir_words;   // its keys in vertex order: their pointer words, or (dir_values) the
+                             // one entry of each one's list
     uint32_t vid_lo;         // its first vertex id
     uint32_t vid_span;       // vertex ids it covers (0: no directory, keys are probed by hash)
+    uint32_t dir_values;     // every list of the segment has one entry: dir_words is uint32
+    uint32_t pad;
 };
 
-// 64 vertex ids of a segment's directory: which of them have a key, and the place of the first
-// one's pointer word in the store's word array (the others follow in vertex order).  Built on
-// the device when the store is loaded (wk_dir.cu); not part of the exported store.
-struct alignas(16) DirBlock {
-    uint64_t bits;
-    uint64_t base;
+// 32 vertex ids of a segment's directory: which of them have a key, and the place of the first
+// one's word (the others follow in vertex order).  Built on the device when the store is loaded
+// (wk_dir.cu); not part of the exported store.
+struct alignas(8) DirBlock {
+    uint32_t bits;
+    uint32_t base;
 };
-static_assert(sizeof(DirBlock) == 16, "directory blocks are 16 bytes");
 
 WK_HD uint64_t barrett_magic(uint64_t nb) { return nb ? ~0ull / nb : 0; }
 

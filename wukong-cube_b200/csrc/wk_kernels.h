@@ -14,6 +14,7 @@ enum : uint32_t {
     kErrCorrupt = 4u,    // a key-table chain left the slot array or exceeded the hop limit
     kErrStatus = 8u,     // more tiles than the status array holds (host grows it and reruns)
     kErrResult = 16u,    // a result gather did not fit its buffer (host grows it and reruns)
+    kErrUnfuse = 32u,    // a step taken for functional gave a row several (host reruns unfused)
 };
 
 // Per-stream control block of the single-pass scan.  Kernels that use it reset the tile and
@@ -43,7 +44,6 @@ struct DevStore {
     const uint32_t* edges;
     uint64_t n_edges;
     const SegDesc* segs;         // [n_segs + 1]: entry 0 an absent segment, i + 1 segment i
-    const uint64_t* dir_words;   // the directories' pointer words
 };
 
 struct ListArgs {

@@ -126,8 +126,8 @@ uint64_t plan_projection(const wk_ctx* ctx, const std::vector<PlanStep>& plan) {
         const double in_bytes = rows * cols * 4.0;
         switch (s.kind) {
             case PlanStep::kIndex: {
-                auto it = ctx->index_len.find(s.start_const * 2 + (uint32_t)s.dir);
-                rows = it == ctx->index_len.end() ? 0.0 : (double)it->second;
+                auto it = ctx->index_ptr.find(s.start_const * 2 + (uint32_t)s.dir);
+                rows = it == ctx->index_ptr.end() ? 0.0 : (double)ptr_size(it->second);
                 break;
             }
             case PlanStep::kConst: rows = mean_deg(s.pid, s.dir); break;

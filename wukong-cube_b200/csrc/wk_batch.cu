@@ -191,7 +191,7 @@ int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, uint64_t ro
     WKB_CUDA(ctx, cudaDeviceSynchronize());
     free_state(b);
     auto dm = [&](void** p, size_t bytes) {
-        if (wk::dev_malloc(p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+        if (wk::ctx_malloc(ctx, p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }

@@ -93,7 +93,7 @@ int wk_ctx::ensure_heavy(uint64_t out_rows_cap) {
     if (d_heavy) cudaFree(d_heavy);
     d_heavy = nullptr;
     heavy_cap = 0;
-    if (wk::dev_malloc(&d_heavy, cap * sizeof(wk::HeavyItem)) != cudaSuccess) {
+    if (wk::ctx_malloc(this, &d_heavy, cap * sizeof(wk::HeavyItem)) != cudaSuccess) {
         cudaGetLastError();
         return fail(WK_E_OOM, "long-list slice queue");
     }
@@ -109,7 +109,7 @@ int wk_ctx::ensure_flat(uint64_t in_rows_cap) {
     if (d_flat) cudaFree(d_flat);
     d_flat = nullptr;
     flat_cap_rows = 0;
-    if (wk::dev_malloc(&d_flat, wk::flat_scratch_bytes(rows, wk::flat_grid(sm_count))) != cudaSuccess) {
+    if (wk::ctx_malloc(this, &d_flat, wk::flat_scratch_bytes(rows, wk::flat_grid(sm_count))) != cudaSuccess) {
         cudaGetLastError();
         return fail(WK_E_OOM, "flat pipeline scratch");
     }
@@ -125,7 +125,7 @@ int wk_ctx::final_scratch_reserve(size_t bytes) {
     d_final_scratch = nullptr;
     final_scratch_bytes = 0;
     const size_t cap = bytes + bytes / 4;
-    if (wk::dev_malloc(&d_final_scratch, cap) != cudaSuccess) {
+    if (wk::ctx_malloc(this, &d_final_scratch, cap) != cudaSuccess) {
         cudaGetLastError();
         return fail(WK_E_OOM, "post-pattern scratch");
     }
@@ -139,7 +139,7 @@ int wk_ctx::ensure_status(uint64_t tiles) {
     WK_CUDA(this, cudaStreamSynchronize(stream));
     if (d_status) WK_CUDA(this, cudaFree(d_status));
     d_status = nullptr;
-    if (wk::dev_malloc(&d_status, cap * sizeof(unsigned long long)) != cudaSuccess) {
+    if (wk::ctx_malloc(this, &d_status, cap * sizeof(unsigned long long)) != cudaSuccess) {
         cudaGetLastError();
         status_cap = 0;
         return fail(WK_E_OOM, "status array");
@@ -197,7 +197,7 @@ int wk_ctx::table_reserve(wk_table* t, uint64_t elems) {
     if (t->d) cudaFree(t->d);
     t->d = nullptr;
     t->cap = 0;
-    if (wk::dev_malloc(&t->d, (elems + kPadWords) * sizeof(uint32_t)) != cudaSuccess) {
+    if (wk::ctx_malloc(this, &t->d, (elems + kPadWords) * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();
         return fail(WK_E_OOM, "result table of " + std::to_string(elems) + " elements");
     }
@@ -212,12 +212,19 @@ int wk_ctx::table_reserve(wk_table* t, uint64_t elems) {
     return WK_SUCCESS;
 }
 
-int wk_ctx::read_ctl(uint32_t* err, uint64_t* need) {
-    WK_CUDA(this, cudaMemcpyAsync(h_ctl, d_ctl, sizeof(wk::StepCtl), cudaMemcpyDeviceToHost, stream));
+// The control block (and, with `t`, that table's row count), after everything enqueued so far.
+int wk_ctx::read_ctl(uint32_t* err, uint64_t* need, const wk_table* t) {
+    WK_CUDA(this, cudaMemcpyAsync(h_ctl, d_ctl, wk::kCtlBlockBytes, cudaMemcpyDeviceToHost, stream));
+    const bool own = t == &rbuf[0] || t == &rbuf[1];
+    if (t && !own) WK_CUDA(this, cudaMemcpyAsync(h_rows, t->d_rows, 8, cudaMemcpyDeviceToHost, stream));
     WK_CUDA(this, cudaStreamSynchronize(stream));
     *err = h_ctl->err | inject_err;   // a failure staged by wk_debug_fail_next counts once
     *need = h_ctl->need;
     inject_err = 0;
+    if (t && !*err) {
+        t->rows = own ? reinterpret_cast<const uint64_t*>(h_ctl + 1)[t - rbuf] : h_rows[0];
+        t->rows_known = true;
+    }
     return WK_SUCCESS;
 }
 
@@ -363,6 +370,7 @@ int resolve_plan(const wk_query& q, int max_cols, std::vector<PlanStep>& steps, 
 int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* out,
                  int32_t mt_tid, int32_t mt_factor, cudaStream_t s) {
     out->cols = st.out_cols;
+    out->written();
     if (st.kind == PlanStep::kIndex || st.kind == PlanStep::kConst) {
         ListArgs a{};
         a.store = ctx->dev_store();
@@ -555,6 +563,7 @@ int enqueue_pass(wk_ctx* ctx, const std::vector<PlanStep>& steps, const PlanPass
         }
     }
     out->cols = steps[p.first + p.n - 1].out_cols;
+    out->written();
     a.out = out->d;
     a.w_out = out->cols;
     a.out_cap_rows = out->cap / out->cols;
@@ -723,10 +732,16 @@ static int ctx_init_device(wk_ctx* ctx, bool low_priority) {
     if (e == cudaSuccess) e = wk::versatile_kernel_attrs();
     if (e == cudaSuccess) e = wk::gbuild_kernel_attrs();
     if (e != cudaSuccess) return bail(e, "kernel attributes");
-    e = wk::dev_malloc(&ctx->d_ctl, sizeof(wk::StepCtl));
+    e = wk::dev_malloc(&ctx->d_ctl, wk::kCtlBlockBytes);
     if (e != cudaSuccess) return bail(e, "control block");
-    e = cudaMallocHost(&ctx->h_ctl, sizeof(wk::StepCtl));
+    ctx->rbuf[0].d_rows = reinterpret_cast<uint64_t*>(ctx->d_ctl + 1);
+    ctx->rbuf[1].d_rows = ctx->rbuf[0].d_rows + 1;
+    e = cudaMemset(ctx->rbuf[0].d_rows, 0, 16);
+    if (e != cudaSuccess) return bail(e, "control init");
+    e = cudaMallocHost(&ctx->h_ctl, wk::kCtlBlockBytes);
     if (e != cudaSuccess) return bail(e, "pinned control block");
+    e = cudaMallocHost(&ctx->h_small, wk::kSmallElems * 4);
+    if (e != cudaSuccess) return bail(e, "pinned result head");
     e = cudaMallocHost(&ctx->h_rows, sizeof(uint64_t) * 4);
     if (e != cudaSuccess) return bail(e, "pinned rows");
     wk::StepCtl init{};
@@ -743,11 +758,9 @@ extern "C" int wk_ctx_destroy(wk_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     wk_batch_release(ctx);
+    ctx->release_serve();
     ctx->drop_graphs();
-    for (auto& t : ctx->rbuf) {
-        if (t.d) cudaFree(t.d);
-        if (t.d_rows) cudaFree(t.d_rows);
-    }
+    for (auto& t : ctx->rbuf) cudaFree(t.d);   // (their row counts are in the control block)
     ctx->drop_store();
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->d_heavy) cudaFree(ctx->d_heavy);
@@ -755,6 +768,7 @@ extern "C" int wk_ctx_destroy(wk_ctx* ctx) {
     if (ctx->d_final_scratch) cudaFree(ctx->d_final_scratch);
     if (ctx->d_ctl) cudaFree(ctx->d_ctl);
     if (ctx->h_ctl) cudaFreeHost(ctx->h_ctl);
+    if (ctx->h_small) cudaFreeHost(ctx->h_small);
     if (ctx->h_rows) cudaFreeHost(ctx->h_rows);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -796,8 +810,8 @@ extern "C" int wk_store_upload(wk_ctx* ctx, const wk_seg_meta* segs, uint32_t n_
     WK_CUDA(ctx, cudaSetDevice(ctx->device));
     WK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     ctx->drop_store();
-    if (wk::dev_malloc(&ctx->d_slots, std::max<uint64_t>(n_slots, wk::kAssoc) * sizeof(wk::Slot)) != cudaSuccess ||
-        wk::dev_malloc(&ctx->d_edges, (n_edges + kPadWords) * sizeof(uint32_t)) != cudaSuccess) {
+    if (wk::ctx_malloc(ctx, &ctx->d_slots, std::max<uint64_t>(n_slots, wk::kAssoc) * sizeof(wk::Slot)) != cudaSuccess ||
+        wk::ctx_malloc(ctx, &ctx->d_edges, (n_edges + kPadWords) * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();
         return ctx->fail(WK_E_OOM, "store upload");
     }
@@ -1035,7 +1049,7 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
         return ctx->fail(WK_E_UNSUPPORTED, "a pointer word of type 3 (attribute values are not served)");
     // one-entry lists into their keys' pointer words, the original words kept aside
     if (found.n_inline) {
-        if (dev_malloc(&ctx->d_inline_orig, found.n_inline * 16) != cudaSuccess) {
+        if (ctx_malloc(ctx, &ctx->d_inline_orig, found.n_inline * 16) != cudaSuccess) {
             cudaGetLastError();
             return ctx->fail(WK_E_OOM, "one-entry list table");
         }
@@ -1141,18 +1155,26 @@ extern "C" int wk_table_upload(wk_ctx* ctx, wk_table* t, const uint32_t* host, u
     if (rc) return rc;
     if (n) WK_CUDA(ctx, cudaMemcpyAsync(t->d, host, n * 4, cudaMemcpyHostToDevice, ctx->stream));
     ctx->h_rows[0] = cols ? rows : 0;
+    t->written();
     WK_CUDA(ctx, cudaMemcpyAsync(t->d_rows, ctx->h_rows, 8, cudaMemcpyHostToDevice, ctx->stream));
     WK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     t->cols = cols;
+    t->rows = ctx->h_rows[0];
+    t->rows_known = true;
     return WK_SUCCESS;
 }
 
-static int table_rows(wk_ctx* ctx, const wk_table* t, uint64_t* rows) {
-    WK_CUDA(ctx, cudaMemcpyAsync(ctx->h_rows, t->d_rows, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    WK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    *rows = ctx->h_rows[0];
+int wk::table_rows(wk_ctx* ctx, const wk_table* t, uint64_t* rows) {
+    if (!t->rows_known) {
+        WK_CUDA(ctx, cudaMemcpyAsync(ctx->h_rows, t->d_rows, 8, cudaMemcpyDeviceToHost, ctx->stream));
+        WK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        t->rows = ctx->h_rows[0];
+        t->rows_known = true;
+    }
+    *rows = t->rows;
     return WK_SUCCESS;
 }
+using wk::table_rows;
 
 extern "C" int wk_table_shape(wk_ctx* ctx, const wk_table* t, uint64_t* rows, int32_t* cols) {
     if (!ctx || !t) return WK_E_BADARG;
@@ -1224,7 +1246,7 @@ static int run_step_sync(wk_ctx* ctx, const wk::PlanStep& st, const wk_table* in
         if (rc) return rc;
         uint32_t err = 0;
         uint64_t need = 0;
-        rc = ctx->read_ctl(&err, &need);
+        rc = ctx->read_ctl(&err, &need, out);
         if (rc) return rc;
         if (!err) return WK_SUCCESS;
         rc = ctx->clear_ctl_err();
@@ -1468,8 +1490,10 @@ static int enqueue_plan(wk_ctx* ctx, const std::vector<wk::PlanStep>& steps, con
     return WK_SUCCESS;
 }
 
+// `head`: bring the first elements of the final table with the control block (h_small).
 static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_table** out_table,
-                     int32_t* v2c_map, int32_t* col_num) {
+                     int32_t* v2c_map, int32_t* col_num, bool head = false) {
+    ctx->small_elems = 0;
     if (!ctx->has_store) return ctx->fail(WK_E_NOSTORE, "no store uploaded");
     std::vector<wk::PlanStep> steps;
     wk::ColMap cm(q->nvars);
@@ -1481,6 +1505,7 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
         if (rc) return rc;
     }
     if (steps.empty()) {
+        ctx->rbuf[0].written();
         WK_CUDA(ctx, cudaMemsetAsync(ctx->rbuf[0].d_rows, 0, 8, ctx->stream));
         ctx->rbuf[0].cols = 0;
         *out_table = &ctx->rbuf[0];
@@ -1521,16 +1546,24 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
                     if (ce != cudaSuccess) return ctx->cuda_fail(ce, "graph instantiate");
                     it = ctx->graphs.emplace(key, ge).first;
                 }
+                for (auto& t : ctx->rbuf) t.written();
                 WK_CUDA(ctx, cudaGraphLaunch(it->second.exec, ctx->stream));
             } else {
                 rc = enqueue_plan(ctx, steps, passes, *q);
                 if (rc) return rc;
             }
+            const wk_table* ft = final_table(ctx, passes);
+            const uint64_t n_head = head ? std::min(ft->cap, wk::kSmallElems) : 0;
+            if (n_head)
+                WK_CUDA(ctx, cudaMemcpyAsync(ctx->h_small, ft->d, n_head * 4, cudaMemcpyDeviceToHost, ctx->stream));
             uint32_t err = 0;
             uint64_t need = 0;
-            rc = ctx->read_ctl(&err, &need);
+            rc = ctx->read_ctl(&err, &need, ft);
             if (rc) return rc;
-            if (!err) break;
+            if (!err) {
+                ctx->small_elems = n_head;
+                break;
+            }
             rc = ctx->clear_ctl_err();
             if (rc) return rc;
             if (err & wk::kErrCorrupt) return ctx->fail(WK_E_CORRUPT, "key table chain out of range");
@@ -1580,8 +1613,14 @@ extern "C" int wk_query_execute_host(wk_ctx* ctx, const wk_query* q, int32_t mod
     if (!ctx || !q || mode < 0 || mode > 2 || (!host_out && cap_elems)) return WK_E_BADARG;
     std::lock_guard<std::mutex> lk(ctx->mu);
     const wk_table* t = nullptr;
-    int rc = query_run(ctx, q, mode, &t, v2c_map, col_num);
+    int rc = query_run(ctx, q, mode, &t, v2c_map, col_num, true);
     if (rc) return rc;
+    const uint64_t n = t->rows_known ? t->rows * (uint64_t)t->cols : ~0ull;
+    if (n <= ctx->small_elems && n <= cap_elems) {   // the whole table came with the control block
+        if (n) std::memcpy(host_out, ctx->h_small, n * 4);
+        if (rows) *rows = t->rows;
+        return WK_SUCCESS;
+    }
     return table_download(ctx, t, host_out, cap_elems, rows);
 }
 
@@ -1626,6 +1665,7 @@ extern "C" int wk_query_enqueue(wk_ctx* ctx, const wk_query* q, int32_t mode) {
     if (mode == WK_MODE_GRAPH) {
         auto it = ctx->graphs.find(plan_key(steps, *q, ctx));
         if (it == ctx->graphs.end()) return ctx->fail(WK_E_BADARG, "plan not captured yet");
+        for (auto& t : ctx->rbuf) t.written();
         WK_CUDA(ctx, cudaGraphLaunch(it->second.exec, ctx->stream));
         if (!steps.empty()) final_table(ctx, query_passes(ctx, steps))->cols = steps.back().out_cols;
         return WK_SUCCESS;

@@ -20,6 +20,11 @@ struct wk_table {
     uint64_t cap = 0;          // elements held
     uint64_t* d_rows = nullptr;// row count, written by the kernels
     int32_t cols = 0;
+    // The row count where the host has read it since the last launch that writes the table (every
+    // such launch goes through written()), so that it is not read again.
+    mutable bool rows_known = false;
+    mutable uint64_t rows = 0;
+    void written() { rows_known = false; }
 };
 
 namespace wk {
@@ -129,7 +134,9 @@ struct wk_ctx {
     uint64_t heavy_cap = 0;
     unsigned long long* d_status = nullptr;
     uint64_t status_cap = 0;
-    wk::StepCtl* h_ctl = nullptr;     // pinned
+    wk::StepCtl* h_ctl = nullptr;     // pinned; as d_ctl it is followed by the row counts of rbuf
+    uint32_t* h_small = nullptr;      // pinned: the first elements of a query's table, which come
+    uint64_t small_elems = 0;         // with its control block (how many the last query brought)
     uint64_t* h_rows = nullptr;       // pinned
     uint32_t inject_err = 0;          // error bits the next control-block read reports (tests)
 
@@ -151,6 +158,7 @@ struct wk_ctx {
     void* batch = nullptr;
     void* batch2 = nullptr;
     void* batch_host = nullptr;   // plans, streams and events reused by every batch call
+    void* serve = nullptr;        // buffers kept between serving runs (wk_serve.cu)
     // serving lanes, kept between serving runs so their tables stay grown (wk_serve.cu)
     std::vector<wk_ctx*> lanes;
     wk::CtaUse lanes_use{0, 0, 0};
@@ -199,11 +207,27 @@ struct wk_ctx {
     void drop_store();
     int final_scratch_reserve(size_t bytes);
     int table_reserve(wk_table* t, uint64_t elems);
-    int read_ctl(uint32_t* err, uint64_t* need);
+    int read_ctl(uint32_t* err, uint64_t* need, const wk_table* t = nullptr);
+    void release_serve();
     int clear_ctl_err();
 };
 
 namespace wk {
+// Device block of a context's control words: StepCtl, then the row counts of rbuf[0] and rbuf[1], so
+// that one copy brings all of them.
+constexpr size_t kCtlBlockBytes = sizeof(StepCtl) + 2 * sizeof(uint64_t);
+constexpr uint64_t kSmallElems = 4096;
+// dev_malloc that gives the kept serving buffers back and tries again when the device is full.
+template <class T>
+cudaError_t ctx_malloc(wk_ctx* ctx, T** p, size_t bytes) {
+    cudaError_t e = dev_malloc(p, bytes);
+    if (e != cudaSuccess && ctx->serve) {
+        cudaGetLastError();
+        ctx->release_serve();
+        e = dev_malloc(p, bytes);
+    }
+    return e;
+}
 // Enqueue one resolved step reading `in` (may be null for index/const starts) into `out`: a
 // start or versatile step by its own launch, a known_to_* step by the tile launch.
 int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* out,
@@ -231,6 +255,8 @@ int ctx_make_child(wk_ctx* parent, const CtaUse& beside_use, int beside_ctas, wk
 // Run a whole query (mode: WK_MODE_RESIDENT or WK_MODE_GRAPH) and report its final table and row
 // count (host sync).
 int query_run_rows(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_table** t, uint64_t* rows);
+// A table's row count (host sync, unless the host knows it already).
+int table_rows(wk_ctx* ctx, const wk_table* t, uint64_t* rows);
 // Copy `elems` elements of a device table to host memory (host sync).
 int table_copy_out(wk_ctx* ctx, const wk_table* t, uint64_t elems, uint32_t* host);
 // Size a serving lane's tables and scan scratch for `elems`-element tables up front.

@@ -526,9 +526,8 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
     const int cols = in->cols;
     cudaStream_t s = ctx->stream;
     uint64_t R = 0;
-    WKF_CUDA(ctx, cudaMemcpyAsync(ctx->h_rows, in->d_rows, 8, cudaMemcpyDeviceToHost, s));
-    WKF_CUDA(ctx, cudaStreamSynchronize(s));
-    R = ctx->h_rows[0];
+    int rrc = table_rows(ctx, in, &R);
+    if (rrc) return rrc;
     // a row count past the capacity marks a table whose writing step overflowed: refused before
     // any launch (and before any scratch is sized from it), as wk_table_download refuses it
     if (cols > 0 && R > in->cap / (uint64_t)cols)
@@ -537,6 +536,7 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
         int rc = ctx->table_reserve(out, 1);
         if (rc) return rc;
         out->cols = cols;
+        out->written();
         WKF_CUDA(ctx, cudaMemsetAsync(out->d_rows, 0, 8, s));
         WKF_CUDA(ctx, cudaStreamSynchronize(s));
         return WK_SUCCESS;
@@ -696,10 +696,13 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
     const int rc = ctx->table_reserve(out, std::max<uint64_t>(count * n_keep, 1));
     if (rc) return done(rc);
     out->cols = n_keep;
+    out->written();
     const int pgrid = std::max(1, std::min<int>(ctx->sm_count * 8, (int)((count * n_keep + 255) / 256)));
     project_kernel<<<pgrid, kFinThreads, 0, s>>>(table_src, cols, d_keep, n_keep, idx, start, count, out->d,
                                                  out->d_rows);
     if ((e = cudaGetLastError()) != cudaSuccess) return done(ctx->cuda_fail(e, "projection launch"));
+    out->rows = count;
+    out->rows_known = true;
     return done(WK_SUCCESS);
 }
 
@@ -711,17 +714,18 @@ extern "C" int wk_table_filter_bound(wk_ctx* ctx, const wk_table* in, const int3
     if (n_bound > 64) return ctx->fail(WK_E_BADARG, "at most 64 bound columns");
     const int cols = in->cols;
     cudaStream_t s = ctx->stream;
-    WKF_CUDA(ctx, cudaMemcpyAsync(ctx->h_rows, in->d_rows, 8, cudaMemcpyDeviceToHost, s));
-    WKF_CUDA(ctx, cudaStreamSynchronize(s));
-    const uint64_t R = ctx->h_rows[0];
+    uint64_t R = 0;
+    int rc = table_rows(ctx, in, &R);
+    if (rc) return rc;
     if (cols > 0 && R > in->cap / (uint64_t)cols)
         return ctx->fail(WK_E_CORRUPT, "row count beyond table capacity");
     for (int k = 0; k < n_bound; ++k)
         if (bound_cols[k] < 0 || bound_cols[k] >= cols) return ctx->fail(WK_E_BADARG, "bound column out of range");
     if (R >= (1ull << 32)) return ctx->fail(WK_E_CAPACITY, "table too long for the filter stage");
-    int rc = ctx->table_reserve(out, std::max<uint64_t>(R * (uint64_t)std::max(cols, 1), 1));
+    rc = ctx->table_reserve(out, std::max<uint64_t>(R * (uint64_t)std::max(cols, 1), 1));
     if (rc) return rc;
     out->cols = cols;
+    out->written();
     if (R == 0 || n_bound == 0) {   // nothing to drop: the table as it is
         if (R) WKF_CUDA(ctx, cudaMemcpyAsync(out->d, in->d, R * (uint64_t)cols * 4, cudaMemcpyDeviceToDevice, s));
         WKF_CUDA(ctx, cudaMemcpyAsync(out->d_rows, in->d_rows, 8, cudaMemcpyDeviceToDevice, s));

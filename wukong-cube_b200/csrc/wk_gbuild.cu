@@ -803,7 +803,7 @@ int gbuild_segments(wk_ctx* ctx, Builder& bd, DirItems* D, unsigned long long* s
 
     // ---- edges and key records
     uint32_t* d_edges = nullptr;
-    if (wk::dev_malloc(&d_edges, (n_edges + 16) * sizeof(uint32_t)) != cudaSuccess) {
+    if (wk::ctx_malloc(ctx, &d_edges, (n_edges + 16) * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();
         return ctx->fail(WK_E_OOM, "store edges");
     }
@@ -916,7 +916,7 @@ int gbuild_segments(wk_ctx* ctx, Builder& bd, DirItems* D, unsigned long long* s
 
     const uint64_t n_slots = (main_buckets + n_ext) * kAssoc;
     Slot* d_slots = nullptr;
-    if (wk::dev_malloc(&d_slots, std::max<uint64_t>(n_slots, kAssoc) * sizeof(Slot)) != cudaSuccess) {
+    if (wk::ctx_malloc(ctx, &d_slots, std::max<uint64_t>(n_slots, kAssoc) * sizeof(Slot)) != cudaSuccess) {
         cudaGetLastError();
         return ctx->fail(WK_E_OOM, "store slots");
     }
@@ -1042,6 +1042,7 @@ extern "C" int wk_store_build_device(wk_ctx* ctx, const uint32_t* triples, uint6
     WKG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     // the old store goes first: a build needs the room
     ctx->drop_store();
+    ctx->release_serve();   // (a build needs the room)
     wk::Slot* slots = nullptr;
     uint32_t* edges = nullptr;
     uint64_t n_slots = 0, n_edges = 0;

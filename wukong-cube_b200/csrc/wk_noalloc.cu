@@ -157,6 +157,7 @@ extern "C" int wk_step_known_to_unknown_noalloc(wk_ctx* ctx, const wk_table* in,
     a.slice_rows = ctx->slice_rows;
     a.spin_limit = ctx->spin_limit;
     out->cols = st.out_cols;
+    out->written();
     // the same launch shape as wk_step_known_to_unknown's tile launch (a serving lane's context
     // leaves room on every SM for the iteration launches)
     const int grid = ctx->blocks_per_sm(a.one.op, st.in_cols, a.lanes) * ctx->sm_count;

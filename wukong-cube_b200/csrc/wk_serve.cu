@@ -25,6 +25,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <deque>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -156,9 +157,11 @@ struct QSlot {
 struct Serve {
     wk_ctx* ctx;
     wk_serve_config cfg;
-    uint32_t slots_n = 0;
+    uint32_t slots_n = 0;                     // of this run; the buffers hold slots_cap
+    uint32_t slots_cap = 0;
     int w = 1;
-    uint64_t rows_cap[2] = {0, 0};
+    uint64_t rows_cap[2] = {0, 0};            // rows of w columns an arena holds
+    uint64_t arena_elems[2] = {0, 0}, owner_rows[2] = {0, 0};   // what is allocated
     StepDesc* d_plans = nullptr;
     uint32_t* d_admit = nullptr;
     uint32_t* d_arena[2] = {nullptr, nullptr};
@@ -185,26 +188,37 @@ struct Serve {
         return sizeof(StepDesc) * kMaxSteps * (size_t)n_new + 4ull * (n_new + 2ull * n_fin);
     }
 
-    ~Serve() {
-        auto f = [](void* p) { if (p) cudaFree(p); };
-        auto fh = [](void* p) { if (p) cudaFreeHost(p); };
+    ~Serve() { release(); }
+    void release() {
+        auto f = [](auto& p) { cudaFree(p); p = nullptr; };
+        auto fh = [](auto& p) { if (p) cudaFreeHost(p); p = nullptr; };
         f(d_plans); f(d_admit); f(d_arena[0]); f(d_arena[1]); f(d_owner[0]); f(d_owner[1]);
         f(d_total); f(d_qfirst); f(d_qcount); f(d_in); f(d_pkt); f(d_result);
         fh(h_in); fh(h_pkt); fh(h_result);
+        slots_cap = 0;
+        for (int k = 0; k < 2; ++k) rows_cap[k] = arena_elems[k] = owner_rows[k] = 0;
+        result_cap = 0;
+    }
+    // device bytes of the buffers that grow
+    uint64_t kept_bytes() const {
+        return 4 * (arena_elems[0] + arena_elems[1] + owner_rows[0] + owner_rows[1] + result_cap) +
+               sizeof(StepDesc) * kMaxSteps * 2ull * slots_cap;
     }
 
     int alloc_arena(int k, uint64_t rows) {
-        if (d_arena[k]) cudaFree(d_arena[k]);
-        if (d_owner[k]) cudaFree(d_owner[k]);
+        cudaFree(d_arena[k]);
+        cudaFree(d_owner[k]);
         d_arena[k] = nullptr;
         d_owner[k] = nullptr;
+        rows_cap[k] = arena_elems[k] = owner_rows[k] = 0;
         rows = (rows + 15) & ~15ull;
         if (wk::dev_malloc(&d_arena[k], rows * w * 4 + 256) != cudaSuccess ||
             wk::dev_malloc(&d_owner[k], rows * 4 + 64) != cudaSuccess) {
             cudaGetLastError();
             return ctx->fail(WK_E_OOM, "serving arena");
         }
-        rows_cap[k] = rows;
+        rows_cap[k] = owner_rows[k] = rows;
+        arena_elems[k] = rows * w;
         return WK_SUCCESS;
     }
 
@@ -225,6 +239,16 @@ struct Serve {
     int init(uint32_t slots, int width) {
         slots_n = slots;
         w = std::max(width, 1);
+        // the buffers of the run before, where they are large enough
+        const uint64_t want = std::max<uint64_t>(cfg.arena_bytes / (4ull * w), 1 << 16);
+        if (slots_cap) {
+            for (int k = 0; k < 2; ++k) rows_cap[k] = std::min(owner_rows[k], arena_elems[k] / w) & ~15ull;
+            if (slots <= slots_cap && want <= rows_cap[0] && want <= rows_cap[1]) {
+                WKS_CUDA(ctx, cudaMemsetAsync(d_total, 0, 16, ctx->stream));
+                return WK_SUCCESS;
+            }
+            release();
+        }
         auto dm = [&](void** p, size_t bytes) {
             if (wk::dev_malloc(p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
                 cudaGetLastError();
@@ -243,12 +267,12 @@ struct Serve {
         new_slots.reserve(slots);
         fin_slots.reserve(slots);
         fin_cols.reserve(slots);
-        const uint64_t rows = std::max<uint64_t>(cfg.arena_bytes / (4ull * w), 1 << 16);
-        int rc = alloc_arena(0, rows);
-        if (!rc) rc = alloc_arena(1, rows);
+        int rc = alloc_arena(0, want);
+        if (!rc) rc = alloc_arena(1, want);
         if (!rc) rc = alloc_result(1 << 22);
         if (rc) return rc;
-        WKS_CUDA(ctx, cudaMemset(d_total, 0, 16));
+        slots_cap = slots;
+        WKS_CUDA(ctx, cudaMemsetAsync(d_total, 0, 16, ctx->stream));
         return WK_SUCCESS;
     }
 
@@ -442,6 +466,11 @@ struct HeavyLanes {
     }
 };
 
+// Device bytes of serving buffers a context keeps between runs (two default arenas and their
+// owners fit); larger ones go back at the end of the run.  Allocating and freeing them cost 30 to
+// 300 ms a run, many times a burst's own work.
+constexpr uint64_t kKeepServeBytes = 4ull << 30;
+
 }  // namespace
 
 cudaError_t serve_kernel_attrs() {
@@ -454,6 +483,11 @@ cudaError_t serve_kernel_attrs() {
 
 }  // namespace wk
 
+void wk_ctx::release_serve() {
+    delete static_cast<wk::Serve*>(serve);
+    serve = nullptr;
+}
+
 using Clock = std::chrono::steady_clock;
 
 extern "C" int wk_serve_run_open_loop(wk_ctx* ctx, const wk_serve_config* cfg_in, const wk_query* queries,
@@ -464,7 +498,11 @@ extern "C" int wk_serve_run_open_loop(wk_ctx* ctx, const wk_serve_config* cfg_in
     std::lock_guard<std::mutex> lk(ctx->mu);
     if (!ctx->has_store) return ctx->fail(WK_E_NOSTORE, "no store uploaded");
     if (n == 0) return WK_SUCCESS;
-    wk::Serve S;
+    // the buffers kept from the run before; a run that fails gives them back
+    std::unique_ptr<wk::Serve> kept(static_cast<wk::Serve*>(ctx->serve));
+    ctx->serve = nullptr;
+    if (!kept) kept.reset(new wk::Serve());
+    wk::Serve& S = *kept;
     S.ctx = ctx;
     S.cfg = cfg_in ? *cfg_in : wk_serve_config{};
     if (!S.cfg.working_set_cap_bytes) S.cfg.working_set_cap_bytes = 40ull << 30;
@@ -622,6 +660,7 @@ extern "C" int wk_serve_run_open_loop(wk_ctx* ctx, const wk_serve_config* cfg_in
             }
             (plans[q][0].kind == wk::PlanStep::kIndex ? wait_heavy : wait_light).push_back(q);
         }
+        if (done >= n) break;   // (the last one came back from a lane: nothing is left to wait for)
         // 2. admission, FIFO within each class; a class stops at the first query that does not
         // fit under the working-set cap (unless nothing at all is resident)
         while (!wait_heavy.empty() && heavy_inflight < S.cfg.max_heavy_inflight &&
@@ -739,5 +778,6 @@ extern "C" int wk_serve_run_open_loop(wk_ctx* ctx, const wk_serve_config* cfg_in
         finished.clear();
         ++iter;
     }
+    if (S.kept_bytes() <= wk::kKeepServeBytes) ctx->serve = kept.release();
     return WK_SUCCESS;
 }

@@ -2,7 +2,9 @@
 //
 // No counterpart in the reference, which serves one query per GPU agent at a time
 // (gpu_agent.hpp:173-246) and leaves light queries to the CPU engines
-// (console_proxy.hpp:387-392).  Level k's input is level k-1's output: every query's rows,
+// (console_proxy.hpp:387-392).  On a store with vertex directories a level is a fused launch
+// (wk_level.cu) that runs several steps of each query; else, and where the flat passes are asked
+// for (knob 5), it is one pattern of every query:  Level k's input is level k-1's output: every query's rows,
 // contiguous and in query order, each tagged with its owner query.  One exploration launch per
 // level (wk_explore.cu: a persistent launch whose CTAs claim tiles from a device counter) runs
 // each row's own query step, and records each query's output range (qfirst, qcount); rows of
@@ -20,6 +22,7 @@
 #include "wk_batch.h"
 #include "wk_ctx.h"
 #include "wk_device.cuh"
+#include "wk_level.h"
 
 namespace wk {
 namespace {
@@ -130,13 +133,13 @@ struct BatchState {
     int l_cap = 0;
     uint64_t rows_cap = 0;     // rows per level region
     int w_cap = 0;             // widest row the regions were sized for
-    wk::StepDesc* d_desc = nullptr;       // [l_cap][n_cap]
+    int s_cap = 0;             // steps of a query the plan block holds
+    // The batch's plans, in one block that goes up in one copy (PlanLayout).
+    unsigned char* d_plan = nullptr;
     uint32_t* d_owner = nullptr;          // [l_cap][rows_cap]
     uint64_t* d_total_out = nullptr;      // [l_cap]
     unsigned long long* d_qfirst = nullptr;   // [l_cap][n_cap]
     unsigned long long* d_qcount = nullptr;   // [l_cap][n_cap]
-    uint32_t* d_nsteps = nullptr;         // [n_cap]
-    uint32_t* d_final_cols = nullptr;     // [n_cap]
     int32_t* d_final_level = nullptr;     // [n_cap]
     uint64_t* d_final_base = nullptr;     // [n_cap]
     uint64_t* d_final_rows = nullptr;     // [n_cap]
@@ -147,9 +150,7 @@ struct BatchState {
     uint64_t* d_flat = nullptr;           // flat-level scratch: pos, off, part (wk_flat.h)
     uint64_t flat_rows = 0;               // rows it is sized for: max(rows_cap, n_cap)
     // pinned host staging
-    wk::StepDesc* h_desc = nullptr;
-    uint32_t* h_nsteps = nullptr;
-    uint32_t* h_final_cols = nullptr;
+    unsigned char* h_plan = nullptr;
     uint64_t* h_final_rows = nullptr;
     uint64_t* h_res_off = nullptr;
     wk::StepCtl* h_ctl = nullptr;         // control block snapshot after this state's batch
@@ -158,13 +159,28 @@ struct BatchState {
     std::string shape;
 };
 
+// Places in the plan block of a batch of n queries in L levels: each query's level count and final
+// columns, then (fused) its runs [L][n] and the steps of all queries, or (a pattern per level) the
+// step descriptors [L][n].
+struct PlanLayout {
+    size_t final_cols, runs, steps;
+    PlanLayout(uint32_t n, int L, bool fused) {
+        final_cols = 4ull * n;
+        runs = 8ull * n;
+        steps = (runs + (fused ? sizeof(wk::LevelRun) * (size_t)L * n : 0) + 15) / 16 * 16;
+    }
+    static size_t bytes(uint32_t n, int L, int s) {   // room for either form
+        return 8ull * n + 16 + sizeof(wk::LevelRun) * (size_t)L * n + sizeof(wk::StepDesc) * (size_t)std::max(s, L) * n;
+    }
+};
+
 void free_state(BatchState* b) {
     auto f = [](void* p) { if (p) cudaFree(p); };
-    f(b->d_desc); f(b->d_owner); f(b->d_total_out); f(b->d_qfirst); f(b->d_qcount);
-    f(b->d_nsteps); f(b->d_final_cols); f(b->d_final_level); f(b->d_final_base);
+    f(b->d_plan); f(b->d_owner); f(b->d_total_out); f(b->d_qfirst); f(b->d_qcount);
+    f(b->d_final_level); f(b->d_final_base);
     f(b->d_final_rows); f(b->d_res_off); f(b->d_arena); f(b->d_result); f(b->d_flat);
     auto fh = [](void* p) { if (p) cudaFreeHost(p); };
-    fh(b->h_desc); fh(b->h_nsteps); fh(b->h_final_cols); fh(b->h_final_rows); fh(b->h_res_off);
+    fh(b->h_plan); fh(b->h_final_rows); fh(b->h_res_off);
     fh(b->h_ctl);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     *b = BatchState();
@@ -176,14 +192,15 @@ void free_state(BatchState* b) {
         if (e_ != cudaSuccess) return (ctx)->cuda_fail(e_, #call); \
     } while (0)
 
-int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, uint64_t rows_cap, int w,
+int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, int steps, uint64_t rows_cap, int w,
                  uint64_t result_cap) {
     rows_cap = (rows_cap + 15) & ~15ull;   // keeps every level region 16-byte aligned
-    if (n <= b->n_cap && levels <= b->l_cap && rows_cap <= b->rows_cap && w <= b->w_cap &&
+    if (n <= b->n_cap && levels <= b->l_cap && steps <= b->s_cap && rows_cap <= b->rows_cap && w <= b->w_cap &&
         result_cap <= b->result_cap)
         return WK_SUCCESS;
     n = std::max(n, b->n_cap);
     levels = std::max(levels, b->l_cap);
+    steps = std::max(steps, b->s_cap);
     rows_cap = std::max(rows_cap, b->rows_cap);
     w = std::max(w, b->w_cap);
     result_cap = std::max(result_cap, b->result_cap);
@@ -200,17 +217,16 @@ int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, uint64_t ro
     auto hm = [&](void** p, size_t bytes) {
         return cudaMallocHost(p, std::max<size_t>(bytes, 16)) == cudaSuccess;
     };
-    bool ok = dm((void**)&b->d_desc, sizeof(wk::StepDesc) * levels * (size_t)n) &&
+    const size_t plan_bytes = PlanLayout::bytes(n, levels, steps);
+    bool ok = dm((void**)&b->d_plan, plan_bytes) &&
               dm((void**)&b->d_owner, 4ull * levels * rows_cap) &&
               dm((void**)&b->d_total_out, 8ull * levels) &&
               dm((void**)&b->d_qfirst, 8ull * levels * n) && dm((void**)&b->d_qcount, 8ull * levels * n) &&
-              dm((void**)&b->d_nsteps, 4ull * n) && dm((void**)&b->d_final_cols, 4ull * n) &&
               dm((void**)&b->d_final_level, 4ull * n) && dm((void**)&b->d_final_base, 8ull * n) &&
               dm((void**)&b->d_final_rows, 8ull * n) && dm((void**)&b->d_res_off, 8ull * (n + 1)) &&
               dm((void**)&b->d_arena, 4ull * levels * rows_cap * w + 256) &&
               dm((void**)&b->d_result, 4ull * result_cap + 64) &&
-              hm((void**)&b->h_desc, sizeof(wk::StepDesc) * levels * (size_t)n) &&
-              hm((void**)&b->h_nsteps, 4ull * n) && hm((void**)&b->h_final_cols, 4ull * n) &&
+              hm((void**)&b->h_plan, plan_bytes) &&
               hm((void**)&b->h_final_rows, 8ull * n) && hm((void**)&b->h_res_off, 8ull * (n + 1)) &&
               hm((void**)&b->h_ctl, sizeof(wk::StepCtl));
     const uint64_t frows = std::max<uint64_t>(rows_cap, n);
@@ -222,6 +238,7 @@ int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, uint64_t ro
     b->flat_rows = frows;
     b->n_cap = n;
     b->l_cap = levels;
+    b->s_cap = steps;
     b->rows_cap = rows_cap;
     b->w_cap = w;
     b->result_cap = result_cap;
@@ -230,12 +247,36 @@ int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, uint64_t ro
 
 struct Plan {
     uint32_t n = 0;
-    int levels = 0;
+    int levels = 0;                     // launches
+    bool fused = false;
+    size_t up_bytes = 0;                // of the plan block
     int width[kMaxBatchLevels] = {0};
     std::vector<int32_t> status;
     std::vector<wk::PlanStep> steps;    // [n][kMaxBatchLevels]
     std::vector<uint8_t> nsteps;        // [n]
+    std::vector<uint32_t> first;        // [n] each query's first step (fused)
+    const PlanLayout layout() const { return PlanLayout(n, levels, fused); }
 };
+
+// The levels of one query's steps: fused runs (one level starts the rows, then as many steps per
+// level as give a row at most one output row and one that multiplies rows), with `put(level, first
+// step, steps, last)` for each.  Returns how many.
+template <class Put>
+int query_levels(const wk_ctx* ctx, const wk::PlanStep* st, int ns, Put put) {
+    int level = 0;
+    for (int i = 0; i < ns; ++level) {
+        int j = i, cols = 0;
+        bool last = false;
+        for (; j < ns && !last; ++j) {
+            const bool one = wk::step_gives_one(ctx, st[j]);
+            if (one && st[j].kind == wk::PlanStep::kK2U && ++cols > wk::kMaxLevelCols) break;
+            last = !one;
+        }
+        put(level, i, j - i, last);
+        i = j;
+    }
+    return level;
+}
 
 // Host-side state kept between batch calls of a context: the plans (their arrays are large,
 // and touching fresh pages for them cost 0.4 ms per 16,384-query batch) and the pipelined
@@ -271,11 +312,14 @@ int build_plan(wk_ctx* ctx, BatchState* b, const wk_query* queries, uint32_t n, 
     P.nsteps.assign(n, 0);
     const int max_cols = ctx->cfg.max_cols;
     const bool versatile = ctx->versatile;
+    // fused levels look vertices up in directories; a store without them keeps a pattern per level
+    P.fused = ctx->has_dir && !ctx->no_fuse && !ctx->batch_flat;
+    int steps_max = 0;
 #pragma omp parallel if (n >= 2048)
     {
         std::vector<wk::PlanStep> st;
         st.reserve(kMaxBatchLevels + 4);
-        int levels = 0, width[kMaxBatchLevels] = {0};
+        int levels = 0, longest = 0, width[kMaxBatchLevels] = {0};
 #pragma omp for schedule(static) nowait
         for (int64_t qi = 0; qi < (int64_t)n; ++qi) {
             const uint32_t q = (uint32_t)qi;
@@ -292,30 +336,69 @@ int build_plan(wk_ctx* ctx, BatchState* b, const wk_query* queries, uint32_t n, 
             }
             P.nsteps[q] = (uint8_t)st.size();
             std::copy(st.begin(), st.end(), P.steps.begin() + (size_t)q * kMaxBatchLevels);
-            levels = std::max<int>(levels, (int)st.size());
-            for (size_t k = 0; k < st.size(); ++k) width[k] = std::max(width[k], st[k].out_cols);
+            longest = std::max<int>(longest, (int)st.size());
+            if (P.fused) {
+                const int nl = query_levels(ctx, st.data(), (int)st.size(), [&](int l, int i, int k, bool) {
+                    width[l] = std::max(width[l], st[i + k - 1].out_cols);
+                });
+                levels = std::max(levels, nl);
+            } else {
+                levels = std::max<int>(levels, (int)st.size());
+                for (size_t k = 0; k < st.size(); ++k) width[k] = std::max(width[k], st[k].out_cols);
+            }
         }
 #pragma omp critical
         {
             P.levels = std::max(P.levels, levels);
+            steps_max = std::max(steps_max, longest);
             for (int k = 0; k < kMaxBatchLevels; ++k) P.width[k] = std::max(P.width[k], width[k]);
         }
     }
     int w = 1;
     for (int k = 0; k < P.levels; ++k) w = std::max(w, P.width[k]);
-    int rc = ensure_state(ctx, b, n, std::max(P.levels, 1), std::max<uint64_t>(b->rows_cap, 1 << 20),
-                          std::max(b->w_cap, std::max(w, 8)), std::max<uint64_t>(b->result_cap, 1 << 22));
+    int rc = ensure_state(ctx, b, n, std::max(P.levels, 1), std::max(steps_max, 1),
+                          std::max<uint64_t>(b->rows_cap, 1 << 20), std::max(b->w_cap, std::max(w, 8)),
+                          std::max<uint64_t>(b->result_cap, 1 << 22));
     if (rc) return rc;
     const int L = P.levels;
+    const PlanLayout at = P.layout();
+    uint32_t* h_levels = reinterpret_cast<uint32_t*>(b->h_plan);
+    uint32_t* h_final_cols = reinterpret_cast<uint32_t*>(b->h_plan + at.final_cols);
+    wk::LevelRun* h_runs = reinterpret_cast<wk::LevelRun*>(b->h_plan + at.runs);
+    wk::StepDesc* h_steps = reinterpret_cast<wk::StepDesc*>(b->h_plan + at.steps);
+    size_t n_steps = (size_t)L * n;
+    if (P.fused) {
+        P.first.resize(n);
+        n_steps = 0;
+        for (uint32_t q = 0; q < n; ++q) {
+            P.first[q] = (uint32_t)n_steps;
+            n_steps += P.nsteps[q];
+        }
+    }
+    P.up_bytes = at.steps + sizeof(wk::StepDesc) * n_steps;
 #pragma omp parallel for schedule(static) if (n >= 2048)
     for (int64_t qi = 0; qi < (int64_t)n; ++qi) {
         const uint32_t q = (uint32_t)qi;
         const int ns = P.nsteps[q];
         const wk::PlanStep* st = P.steps.data() + (size_t)q * kMaxBatchLevels;
-        b->h_nsteps[q] = (uint32_t)ns;
-        b->h_final_cols[q] = ns ? (uint32_t)st[ns - 1].out_cols : 0;
+        h_levels[q] = (uint32_t)ns;
+        h_final_cols[q] = ns ? (uint32_t)st[ns - 1].out_cols : 0;
+        if (P.fused) {
+            for (int k = 0; k < ns; ++k) h_steps[P.first[q] + k] = wk::make_step_desc(ctx, st[k]);
+            const int nl = query_levels(ctx, st, ns, [&](int l, int i, int k, bool last) {
+                wk::LevelRun r{};
+                r.first = P.first[q] + (uint32_t)i;
+                r.n_ops = (uint8_t)(k - (last ? 1 : 0));
+                r.flags = (uint8_t)((last ? wk::kRunLast : 0) | (i + k == ns ? wk::kRunFinal : 0));
+                r.cin = (uint8_t)st[i].in_cols;
+                h_runs[(size_t)l * n + q] = r;
+            });
+            for (int l = nl; l < L; ++l) h_runs[(size_t)l * n + q] = wk::LevelRun{};
+            h_levels[q] = (uint32_t)nl;
+            continue;
+        }
         for (int k = 0; k < L; ++k) {
-            wk::StepDesc& d = b->h_desc[(size_t)k * n + q];
+            wk::StepDesc& d = h_steps[(size_t)k * n + q];
             if (k >= ns) {
                 std::memset(&d, 0, sizeof(d));
                 d.op = wk::kXDone;
@@ -327,14 +410,10 @@ int build_plan(wk_ctx* ctx, BatchState* b, const wk_query* queries, uint32_t n, 
     return WK_SUCCESS;
 }
 
-// Copy the batch's descriptors from the pinned staging to the device.
+// Copy the batch's plans from the pinned staging to the device.
 int upload_plan(wk_ctx* ctx, BatchState* b, const Plan& P, cudaStream_t s = nullptr) {
-    const uint32_t n = P.n;
     if (!s) s = ctx->stream;
-    WKB_CUDA(ctx, cudaMemcpyAsync(b->d_desc, b->h_desc, sizeof(wk::StepDesc) * (size_t)P.levels * n,
-                                  cudaMemcpyHostToDevice, s));
-    WKB_CUDA(ctx, cudaMemcpyAsync(b->d_nsteps, b->h_nsteps, 4ull * n, cudaMemcpyHostToDevice, s));
-    WKB_CUDA(ctx, cudaMemcpyAsync(b->d_final_cols, b->h_final_cols, 4ull * n, cudaMemcpyHostToDevice, s));
+    WKB_CUDA(ctx, cudaMemcpyAsync(b->d_plan, b->h_plan, P.up_bytes, cudaMemcpyHostToDevice, s));
     return WK_SUCCESS;
 }
 
@@ -357,12 +436,13 @@ int enqueue_batch(wk_ctx* ctx, BatchState* b, const Plan& P, ProfHooks* ph = nul
     WKB_CUDA(ctx, cudaMemsetAsync(b->d_qcount, 0, 8ull * L * n, s));
     if (ph) WKB_CUDA(ctx, cudaEventRecord(ph->extra[1], s));
     const int lanes = ctx->probe_lanes(ctx->batch_lanes);
+    const PlanLayout at = P.layout();
     for (int k = 0; k < L; ++k) {
         wk::ExploreArgs a{};
         a.store = ctx->dev_store();
         a.seg_index[0] = ctx->seg_id(0, 0, wk::kIn);
         a.seg_index[1] = ctx->seg_id(0, 0, wk::kOut);
-        a.desc = b->d_desc + (size_t)k * n;
+        a.desc = reinterpret_cast<const wk::StepDesc*>(b->d_plan + at.steps) + (P.fused ? 0 : (size_t)k * n);
         a.n_queries = n;
         a.virtual_rows = k == 0;
         a.in_rows = k > 0 ? b->d_total_out + (k - 1) : nullptr;
@@ -391,7 +471,38 @@ int enqueue_batch(wk_ctx* ctx, BatchState* b, const Plan& P, ProfHooks* ph = nul
             WKB_CUDA(ctx, cudaEventRecord(ph->ev[2 * k], s));
         }
         cudaError_t e;
-        if ((ctx->batch_flat >> k) & 1) {   // the four flat passes (wk_flat.cu), not the tile launch
+        if (P.fused) {
+            wk::LevelArgs f{};
+            f.store = a.store;
+            f.n_segs = (uint32_t)ctx->segs.size();
+            f.seg_index[0] = a.seg_index[0];
+            f.seg_index[1] = a.seg_index[1];
+            f.steps = a.desc;
+            f.runs = reinterpret_cast<const wk::LevelRun*>(b->d_plan + at.runs) + (size_t)k * n;
+            f.n_queries = n;
+            f.virtual_rows = a.virtual_rows;
+            f.in_rows = a.in_rows;
+            f.owner_in = a.owner_in;
+            f.in = a.in;
+            f.w_in = a.w_in;
+            f.in_cap_rows = a.in_cap_rows;
+            f.out = a.out;
+            f.w_out = a.w_out;
+            f.out_cap_rows = a.out_cap_rows;
+            f.out_rows = a.out_rows;
+            f.owner_out = a.owner_out;
+            f.qfirst = a.qfirst;
+            f.qcount = a.qcount;
+            f.heavy = a.heavy;
+            f.heavy_cap = a.heavy_cap;
+            f.ctl = a.ctl;
+            f.status = a.status;
+            f.sorted_lists = a.sorted_lists;
+            f.account = ph ? 1 : 0;
+            f.slice_rows = a.slice_rows;
+            f.spin_limit = a.spin_limit;
+            e = wk::launch_level(f, wk::level_grid(ctx->sm_count), s);
+        } else if ((ctx->batch_flat >> k) & 1) {   // the flat passes (wk_flat.cu), not the tile launch
             wk::FlatLevelArgs f{};
             f.store = a.store;
             f.seg_index[0] = a.seg_index[0];
@@ -429,10 +540,10 @@ int enqueue_batch(wk_ctx* ctx, BatchState* b, const Plan& P, ProfHooks* ph = nul
     }
     wk::ResultScanArgs ra{};
     ra.n = n;
-    ra.nsteps = b->d_nsteps;
+    ra.nsteps = reinterpret_cast<const uint32_t*>(b->d_plan);
     ra.qfirst = b->d_qfirst;
     ra.qcount = b->d_qcount;
-    ra.final_cols = b->d_final_cols;
+    ra.final_cols = reinterpret_cast<const uint32_t*>(b->d_plan + at.final_cols);
     ra.final_level = b->d_final_level;
     ra.final_base = b->d_final_base;
     ra.final_rows = b->d_final_rows;
@@ -446,7 +557,7 @@ int enqueue_batch(wk_ctx* ctx, BatchState* b, const Plan& P, ProfHooks* ph = nul
     ga.final_level = b->d_final_level;
     ga.final_base = b->d_final_base;
     ga.final_rows = b->d_final_rows;
-    ga.final_cols = b->d_final_cols;
+    ga.final_cols = ra.final_cols;
     ga.res_off = b->d_res_off;
     for (int k = 0; k < L; ++k) {
         ga.region[k] = b->d_arena + region_off[k];
@@ -469,6 +580,8 @@ int launch_batch(wk_ctx* ctx, BatchState* b, const Plan& P) {
     put(&P.n, 4);
     put(&P.levels, 4);
     put(P.width, sizeof(P.width));
+    put(&P.fused, sizeof(P.fused));
+    put(&b->d_plan, sizeof(void*));
     put(&b->d_arena, sizeof(void*));
     put(&b->d_result, sizeof(void*));
     put(&b->rows_cap, 8);
@@ -530,10 +643,11 @@ int run_batch(wk_ctx* ctx, BatchState* b, const wk_query* queries, uint32_t n, P
         ctx->clear_ctl_err();
         if (err & wk::kErrCorrupt) return ctx->fail(WK_E_CORRUPT, "key table chain out of range");
         if (err & wk::kErrTimeout) return ctx->fail(WK_E_TIMEOUT, "batch look-back timed out");
+        if (err & wk::kErrUnfuse) ctx->no_fuse = true;   // vid 0 in the store's lists
         uint64_t rows = b->rows_cap, res = b->result_cap;
         if (err & (wk::kErrOverflow | wk::kErrStatus)) rows = std::max<uint64_t>(rows * 2, need + need / 4);
         if (total_elems > res) res = total_elems + total_elems / 4 + 1024;
-        rc = ensure_state(ctx, b, n, P.levels, rows, b->w_cap, res);
+        rc = ensure_state(ctx, b, n, std::max(P.levels, b->l_cap), b->s_cap, rows, b->w_cap, res);
         if (rc) return rc;
         rc = build_plan(ctx, b, queries, n, P);   // staging was reallocated
         if (rc) return rc;
@@ -610,12 +724,13 @@ extern "C" int wk_batch_execute_stream(wk_ctx* ctx, const wk_query* queries, uin
             total = b->h_res_off[cnt[k]];
         }
         if (out_used + total > cap_elems) return rc = ctx->fail(WK_E_CAPACITY, "host buffer too small");
+        const uint32_t* final_cols = reinterpret_cast<const uint32_t*>(b->h_plan + P[k].layout().final_cols);
         for (uint32_t i = 0; i < cnt[k]; ++i) {
             wk_qresult& r = results[off[k] + i];
             std::memset(&r, 0, sizeof(r));
             r.status = P[k].status[i];
             r.rows = r.status ? 0 : b->h_final_rows[i];
-            r.cols = (int32_t)b->h_final_cols[i];
+            r.cols = (int32_t)final_cols[i];
             r.elem_offset = out_used + b->h_res_off[i];
         }
         if (cu(cudaStreamWaitEvent(cs, ready[k], 0), "copy wait")) return rc;
@@ -695,12 +810,13 @@ extern "C" int wk_batch_execute(wk_ctx* ctx, const wk_query* queries, uint32_t n
     int rc = run_batch(ctx, b, queries, n, P);
     if (rc) return rc;
     const uint64_t total = b->h_res_off[n];
+    const uint32_t* final_cols = reinterpret_cast<const uint32_t*>(b->h_plan + P.layout().final_cols);
     for (uint32_t q = 0; q < n; ++q) {
         wk_qresult& r = results[q];
         std::memset(&r, 0, sizeof(r));
         r.status = P.status[q];
         r.rows = P.status[q] ? 0 : b->h_final_rows[q];
-        r.cols = (int32_t)b->h_final_cols[q];
+        r.cols = (int32_t)final_cols[q];
         r.elem_offset = b->h_res_off[q];
     }
     if (total > cap_elems) return ctx->fail(WK_E_CAPACITY, "host buffer too small");

@@ -13,6 +13,7 @@
 #include "wk_batch.h"
 #include "wk_ctx.h"
 #include "wk_dir.h"
+#include "wk_level.h"
 
 #define WK_CUDA(ctx, call)                                   \
     do {                                                     \
@@ -482,6 +483,8 @@ bool is_functional(const wk_ctx* ctx, const PlanStep& s) {
 
 }  // namespace
 
+bool step_gives_one(const wk_ctx* ctx, const PlanStep& s) { return is_filter(s) || is_functional(ctx, s); }
+
 std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>& steps, bool fuse) {
     std::vector<PlanPass> out;
     const int n = (int)steps.size();
@@ -728,6 +731,7 @@ static int ctx_init_device(wk_ctx* ctx, bool low_priority) {
     if (e == cudaSuccess) e = wk::serve_kernel_attrs();
     if (e == cudaSuccess) e = wk::flat_kernel_attrs();
     if (e == cudaSuccess) e = wk::pipe_kernel_attrs();
+    if (e == cudaSuccess) e = wk::level_kernel_attrs();
     if (e == cudaSuccess) e = wk::final_kernel_attrs();
     if (e == cudaSuccess) e = wk::versatile_kernel_attrs();
     if (e == cudaSuccess) e = wk::gbuild_kernel_attrs();

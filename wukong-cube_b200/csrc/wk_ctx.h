@@ -238,6 +238,9 @@ struct PlanPass {
     int first, n;
     bool pipe;
 };
+// Whether a step gives each row at most one output row: a filter, or known_to_unknown on a
+// predicate whose lists all have at most one entry.
+bool step_gives_one(const wk_ctx* ctx, const PlanStep& s);
 // The passes of a plan; `fuse` false: one step each (a start list still joins its first step).
 std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>& steps, bool fuse);
 // Enqueue one pass reading `in` (null when it starts the plan) into `out`.  `fuse` as above;

@@ -20,7 +20,7 @@ __host__ __device__ inline bool is_filter_op(uint32_t op) {
 }
 
 // One query's step at one level (32 bytes).
-struct StepDesc {
+struct alignas(16) StepDesc {
     uint64_t start_key;     // kXStart: the constant / index key whose list starts the table
     uint32_t seg;           // DevStore::segs entry of the step's normal key, or of the start key
     uint32_t pid;

@@ -78,10 +78,7 @@ static_assert(sizeof(Slot) == 16, "slot must be 16 bytes");
 // Where one segment lives inside the uploaded slot and edge arrays.  Only the fields the
 // probe needs; the rest of rdf_seg_meta_t (segment_meta.hpp:87-154) is bookkeeping.
 struct DirBlock;
-struct SegDesc {
-    uint64_t bucket_start;   // absolute bucket id of the segment's main-header region
-    uint64_t num_buckets;    // hash space of the segment (0 = segment absent / empty)
-    uint64_t magic;          // floor((2^64 - 1) / num_buckets): Barrett reciprocal of the modulo
+struct alignas(16) SegDesc {
     const DirBlock* dir;     // the segment's directory on the device (null when it has none)
     const void* dir_words;   // its keys in vertex order: their pointer words, or (dir_values) the
                              // one entry of each one's list
@@ -89,7 +86,12 @@ struct SegDesc {
     uint32_t vid_span;       // vertex ids it covers (0: no directory, keys are probed by hash)
     uint32_t dir_values;     // every list of the segment has one entry: dir_words is uint32
     uint32_t pad;
+    uint64_t bucket_start;   // absolute bucket id of the segment's main-header region
+    uint64_t num_buckets;    // hash space of the segment (0 = segment absent / empty)
+    uint64_t magic;          // floor((2^64 - 1) / num_buckets): Barrett reciprocal of the modulo
+    uint64_t pad2;
 };
+static_assert(sizeof(SegDesc) == 64, "a segment's directory and its buckets are two 32-byte halves");
 
 // 32 vertex ids of a segment's directory: which of them have a key, and the place of the first
 // one's word (the others follow in vertex order).  Built on the device when the store is loaded

@@ -486,7 +486,6 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __g
         const uint64_t w0 = tile * tile_rows + (uint64_t)warp * warp_rows + lane;   // the warp's rows
         uint64_t total = 0;           // output rows of the warp
         uint64_t o0 = 0;              // its next output row
-        unsigned long long next = 0;
         // t < 0 counts round t + rounds, t >= 0 writes round t (one body for both); the look-back
         // lies between
 #pragma unroll 1
@@ -505,17 +504,11 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __g
                 if (warp == 0) {
                     if (lane == 0) publish_aggregate(a.status, tile, all, epoch);
                     __syncwarp();
-                    unsigned long long claim = ntiles;
-                    if (lane == 0 && ntiles > active) claim = atomicAdd(&a.ctl->tile_counter, 1ull);   // the next chunk
                     const uint64_t ex = resolve_prefix(a.status, a.ctl, tile, all, epoch, spin);
-                    if (lane == 0) {
-                        s_excl = ex;
-                        s_claim = claim;
-                    }
+                    if (lane == 0) s_excl = ex;
                 }
                 __syncthreads();
                 const uint64_t excl = s_excl;
-                next = s_claim;
                 o0 = excl + before;
                 if (tile == ntiles - 1 && threadIdx.x == 0) *a.out_rows = excl + all;
                 if (excl + all > a.out_cap_rows) {
@@ -714,7 +707,12 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __g
             }
             __syncwarp();
         }
-        tile = next;
+        // The next chunk: claimed only now, since the CTAs behind it wait for its count (claimed a
+        // look-back ahead it held them up by this one's writing), and whatever the grid, so that a
+        // launch never needs its last CTAs to be resident.
+        if (threadIdx.x == 0) s_claim = atomicAdd(&a.ctl->tile_counter, 1ull);
+        __syncthreads();
+        tile = s_claim;
     }
 
     if (kLast) {

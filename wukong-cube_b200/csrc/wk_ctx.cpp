@@ -156,13 +156,33 @@ int wk_ctx::ensure_status(uint64_t tiles) {
 
 // Free the store and everything derived from it; the serving lanes, which hold its addresses, go
 // too (the next serving run makes them again).  A lane's own store belongs to its parent.
-void wk_ctx::drop_store() {
+void wk_ctx::drop_spare() {
+    cudaFree(spare_slots.p);
+    cudaFree(spare_edges.p);
+    spare_slots = spare_edges = Spare{};
+}
+
+void wk_ctx::drop_store(bool spare) {
     for (wk_ctx* lane : lanes) wk_ctx_destroy(lane);
     lanes.clear();
     drop_graphs();
     ++store_gen;
     has_store = false;
+    drop_spare();
     if (!borrowed_store) {
+        // A store built again in the same context mostly needs the same arrays (freeing and mapping
+        // them took most of a small build); they are kept for it when a build's scratch, a few times
+        // the edges, cannot run short of the room they take.
+        size_t free_b = 0, total_b = 0;
+        if (spare && d_slots && slots_bytes && edges_bytes && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+            slots_bytes + edges_bytes <= free_b / 8) {
+            cudaDeviceSynchronize();   // (as freeing them would: other streams' work on the old store)
+            spare_slots = Spare{d_slots, slots_bytes};
+            spare_edges = Spare{d_edges, edges_bytes};
+            d_slots = nullptr;
+            d_edges = nullptr;
+        }
+        slots_bytes = edges_bytes = 0;
         cudaFree(d_slots);
         cudaFree(d_edges);
         cudaFree(d_pseg);

@@ -204,7 +204,19 @@ struct wk_ctx {
     int ensure_status(uint64_t tiles);
     int ensure_heavy(uint64_t out_rows_cap);
     int ensure_flat(uint64_t in_rows_cap);
-    void drop_store();
+    // Free the store (`spare`: its slots and edges kept aside for the build that follows, when the
+    // device has plenty of room).
+    void drop_store(bool spare = false);
+    void drop_spare();
+    struct Spare {
+        void* p = nullptr;
+        size_t bytes = 0;
+    };
+    Spare spare_slots, spare_edges;
+    size_t slots_bytes = 0, edges_bytes = 0;   // what d_slots and d_edges were allocated with
+    // A store array: the spare one where it is large enough (and at most twice as large).
+    template <class T>
+    cudaError_t store_malloc(Spare& sp, T** p, size_t bytes);
     int final_scratch_reserve(size_t bytes);
     int table_reserve(wk_table* t, uint64_t elems);
     int read_ctl(uint32_t* err, uint64_t* need, const wk_table* t = nullptr);
@@ -228,6 +240,23 @@ cudaError_t ctx_malloc(wk_ctx* ctx, T** p, size_t bytes) {
     }
     return e;
 }
+}  // namespace wk
+
+template <class T>
+cudaError_t wk_ctx::store_malloc(Spare& sp, T** p, size_t bytes) {
+    const size_t have = sp.bytes;
+    if (sp.p && have >= bytes && have / 2 <= bytes) {
+        *p = static_cast<T*>(sp.p);
+        sp = Spare{};
+        (&sp == &spare_slots ? slots_bytes : edges_bytes) = have;
+        return cudaSuccess;
+    }
+    drop_spare();
+    (&sp == &spare_slots ? slots_bytes : edges_bytes) = bytes;
+    return wk::ctx_malloc(this, p, bytes);
+}
+
+namespace wk {
 // Enqueue one resolved step reading `in` (may be null for index/const starts) into `out`: a
 // start or versatile step by its own launch, a known_to_* step by the tile launch.
 int enqueue_step(wk_ctx* ctx, const PlanStep& st, const wk_table* in, wk_table* out,

@@ -52,12 +52,14 @@ __device__ __forceinline__ void flush_range(SegScan* out, uint32_t seg, uint32_t
     atomicMax(&out[seg].vid_hi, hi);
 }
 
-// One thread per slot, each warp over a contiguous share, four slots loaded before any is looked
-// at.  Bound by the read of the table (16 bytes a slot, most of them empty at the default load
-// factor) and by the short lists' sectors.  Lists past kChunkList entries (the type and predicate
-// indexes: 1.5e6 entries in one list at 500 organisations) go to a queue as chunks that a second
-// kernel checks with every warp; walked by the one warp that met them, they took 21 of the 22 ms
-// this check cost on that store.
+// One thread per slot, a warp over shares of 1,024 slots, four slots loaded before any is looked
+// at.  The shares are dealt round: a segment's keys lie together, and with one contiguous share a
+// warp the few warps that met the segments with lists of hundreds of entries (the members of 9,000
+// departments) ran long after the others (1.78 -> 0.49 ms at 500 organisations).  Bound by the read of the table (16 bytes a slot, most of
+// them empty at the default load factor) and by the short lists' sectors.  Lists past kChunkList
+// entries (the type and predicate indexes: 1.5e6 entries in one list at 500 organisations) go to a
+// queue as chunks that a second kernel checks with every warp; walked by the one warp that met
+// them, they took 21 of the 22 ms this check cost on that store.
 constexpr int kScanUnroll = 4;
 __global__ void __launch_bounds__(kLoadThreads)
 store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, SegScan* per_seg, StoreScan* out,
@@ -66,87 +68,112 @@ store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, SegSc
     const int lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t)gridDim.x * (kLoadThreads / 32);
     const uint64_t w = (uint64_t)blockIdx.x * (kLoadThreads / 32) + threadIdx.x / 32;
-    constexpr uint64_t kStep = 32 * kScanUnroll;
-    const uint64_t share = ((n_slots + warps - 1) / warps + kStep - 1) / kStep * kStep;
-    const uint64_t lo = min(n_slots, w * share), hi = min(n_slots, lo + share);
+    constexpr uint64_t kStep = 32 * kScanUnroll, kShare = 8 * kStep;
     uint32_t flags = 0, seg = n_pseg, seg_key = 0xFFFFFFFFu, vlo = 0xFFFFFFFFu, vhi = 0, longest = 0;
     unsigned long long ones = 0;
-    for (uint64_t b = lo; b < hi; b += kStep) {
-        Slot sl[kScanUnroll];
-#pragma unroll
-        for (int u = 0; u < kScanUnroll; ++u) {
-            const uint64_t i = b + 32 * u + lane;
-            sl[u] = i < hi ? st.slots[i] : Slot{0, 0};
+    // one set of atomics a warp where its lanes met one segment or none; leaves the lanes' range empty
+    auto flush = [&] {
+        const unsigned any = __ballot_sync(kFull, seg < n_pseg);
+        if (!any) return;
+        const uint32_t seg0 = __shfl_sync(kFull, seg, __ffs(any) - 1);
+        if (__all_sync(kFull, seg == seg0 || seg >= n_pseg)) {
+            const uint32_t l = __reduce_min_sync(kFull, vlo), h = __reduce_max_sync(kFull, vhi);
+            const uint32_t len = __reduce_max_sync(kFull, longest);
+            if (lane == 0) flush_range(per_seg, seg0, n_pseg, l, h, len);
+        } else {
+            flush_range(per_seg, seg, n_pseg, vlo, vhi, longest);
         }
+        vlo = 0xFFFFFFFFu;
+        vhi = longest = 0;
+        seg = n_pseg;
+        seg_key = 0xFFFFFFFFu;
+    };
+    for (uint64_t b0 = w * kShare; b0 < n_slots; b0 += warps * kShare) {
+        const uint64_t hi = min(n_slots, b0 + kShare);
+        for (uint64_t b = b0; b < hi; b += kStep) {
+            Slot sl[kScanUnroll];
 #pragma unroll
-        for (int u = 0; u < kScanUnroll; ++u) {
-            const uint64_t i = b + 32 * u + lane;
-            uint64_t off = 0, sz = 0;
-            if (sl[u].key != 0 && (i & (kAssoc - 1)) == kAssoc - 1) {   // chain link
-                if (key_vid(sl[u].key) >= st.n_buckets) flags |= kStoreBadChain;
-            } else if (sl[u].key != 0) {
-                const uint64_t v = key_vid(sl[u].key);
-                const uint32_t k = key_pid(sl[u].key) * 2 + key_dir(sl[u].key);
-                if (k != seg_key) {
-                    flush_range(per_seg, seg, n_pseg, vlo, vhi, longest);
-                    seg_key = k;
-                    seg = pseg_find(pseg, n_pseg, k);
-                    vlo = 0xFFFFFFFFu;
-                    vhi = longest = 0;
-                }
-                if (v != 0) longest = max(longest, (uint32_t)ptr_size(sl[u].ptr));   // vid 0: an index list
-                if (v != 0 && v < kBlankId) {
-                    vlo = min(vlo, (uint32_t)v);
-                    vhi = max(vhi, (uint32_t)v);
-                }
-                off = ptr_off(sl[u].ptr);
-                sz = ptr_size(sl[u].ptr);
-                if ((sl[u].ptr >> 62) == 0 && sz == 1 && off < st.n_edges) ++ones;
-                if (ptr_is_inline(sl[u].ptr)) {
-                    flags |= kStoreInlineType;
-                    sz = 0;
-                } else if (off + sz > st.n_edges) {
-                    flags |= kStoreBadList;
-                    sz = 0;
-                } else if (sz <= kSerialList) {
-                    for (uint64_t e = 1; e < sz; ++e)
-                        if (__ldg(st.edges + off + e - 1) >= __ldg(st.edges + off + e)) flags |= kStoreUnsorted;
-                    sz = 0;
-                }
+            for (int u = 0; u < kScanUnroll; ++u) {
+                const uint64_t i = b + 32 * u + lane;
+                sl[u] = i < hi ? st.slots[i] : Slot{0, 0};
             }
-            // the long lists of the warp's slots, one after the other, 32 entries at a time
-            for (unsigned m = __ballot_sync(kFull, sz > 0); m; m &= m - 1) {
-                const int src = __ffs(m) - 1;
-                const uint64_t o = __shfl_sync(kFull, off, src), n = __shfl_sync(kFull, sz, src);
-                if (n > kChunkList) {
-                    const uint32_t nc = (uint32_t)((n + kChunkList - 1) / kChunkList);
-                    unsigned at = 0;
-                    if (lane == 0) at = atomicAdd(&out->n_chunks, nc);
-                    at = __shfl_sync(kFull, at, 0);
-                    if (at + nc <= max_chunks) {   // (lists that overlap may ask for more)
-                        for (uint32_t c = lane; c < nc; c += 32) {
-                            // a chunk begins with the last entry of the one before it
-                            const uint64_t c0 = (uint64_t)c * kChunkList - (c ? 1 : 0);
-                            chunks[at + c] = make_ulonglong2(o + c0, min(n, (uint64_t)(c + 1) * kChunkList) - c0);
-                        }
-                        continue;
+#pragma unroll
+            for (int u = 0; u < kScanUnroll; ++u) {
+                const uint64_t i = b + 32 * u + lane;
+                uint64_t off = 0, sz = 0;
+                if (sl[u].key != 0 && (i & (kAssoc - 1)) == kAssoc - 1) {   // chain link
+                    if (key_vid(sl[u].key) >= st.n_buckets) flags |= kStoreBadChain;
+                } else if (sl[u].key != 0) {
+                    const uint64_t v = key_vid(sl[u].key);
+                    const uint32_t k = key_pid(sl[u].key) * 2 + key_dir(sl[u].key);
+                    if (k != seg_key) {
+                        flush_range(per_seg, seg, n_pseg, vlo, vhi, longest);
+                        seg_key = k;
+                        seg = pseg_find(pseg, n_pseg, k);
+                        vlo = 0xFFFFFFFFu;
+                        vhi = longest = 0;
                     }
-                    for (uint32_t c = lane; c < nc && at + c < max_chunks; c += 32) chunks[at + c] = make_ulonglong2(0, 0);
+                    if (v != 0) longest = max(longest, (uint32_t)ptr_size(sl[u].ptr));   // vid 0: an index list
+                    if (v != 0 && v < kBlankId) {
+                        vlo = min(vlo, (uint32_t)v);
+                        vhi = max(vhi, (uint32_t)v);
+                    }
+                    off = ptr_off(sl[u].ptr);
+                    sz = ptr_size(sl[u].ptr);
+                    if ((sl[u].ptr >> 62) == 0 && sz == 1 && off < st.n_edges) ++ones;
+                    if (ptr_is_inline(sl[u].ptr)) {
+                        flags |= kStoreInlineType;
+                        sz = 0;
+                    } else if (off + sz > st.n_edges) {
+                        flags |= kStoreBadList;
+                        sz = 0;
+                    } else if (sz <= kSerialList) {
+                        uint32_t prev = 0;
+                        const int n = (int)sz;
+                        for (int e0 = 0; n > 1 && e0 < n; e0 += 8) {   // eight entries in flight
+                            uint32_t x[8];
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                if (e0 + j < n) x[j] = __ldg(st.edges + off + e0 + j);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                if (e0 + j >= n) continue;
+                                if (e0 + j && prev >= x[j]) flags |= kStoreUnsorted;
+                                prev = x[j];
+                            }
+                        }
+                        sz = 0;
+                    }
                 }
-                for (uint64_t e = 1 + lane; e < n; e += 32)
-                    if (__ldg(st.edges + o + e - 1) >= __ldg(st.edges + o + e)) flags |= kStoreUnsorted;
+                // the long lists of the warp's slots, one after the other, 32 entries at a time
+                for (unsigned m = __ballot_sync(kFull, sz > 0); m; m &= m - 1) {
+                    const int src = __ffs(m) - 1;
+                    const uint64_t o = __shfl_sync(kFull, off, src), n = __shfl_sync(kFull, sz, src);
+                    if (n > kChunkList) {
+                        const uint32_t nc = (uint32_t)((n + kChunkList - 1) / kChunkList);
+                        unsigned at = 0;
+                        if (lane == 0) at = atomicAdd(&out->n_chunks, nc);
+                        at = __shfl_sync(kFull, at, 0);
+                        if (at + nc <= max_chunks) {   // (lists that overlap may ask for more)
+                            for (uint32_t c = lane; c < nc; c += 32) {
+                                // a chunk begins with the last entry of the one before it
+                                const uint64_t c0 = (uint64_t)c * kChunkList - (c ? 1 : 0);
+                                chunks[at + c] = make_ulonglong2(o + c0, min(n, (uint64_t)(c + 1) * kChunkList) - c0);
+                            }
+                            continue;
+                        }
+                        for (uint32_t c = lane; c < nc && at + c < max_chunks; c += 32)
+                            chunks[at + c] = make_ulonglong2(0, 0);
+                    }
+                    bool bad = false;
+#pragma unroll 8
+                    for (uint64_t e = 1 + lane; e < n; e += 32)
+                        bad |= __ldg(st.edges + o + e - 1) >= __ldg(st.edges + o + e);
+                    if (bad) flags |= kStoreUnsorted;
+                }
             }
         }
-    }
-    // most warps end in one segment: one pair of atomics a warp
-    const uint32_t seg0 = __shfl_sync(kFull, seg, 0);
-    if (__all_sync(kFull, seg == seg0)) {
-        vlo = __reduce_min_sync(kFull, vlo);
-        vhi = __reduce_max_sync(kFull, vhi);
-        longest = __reduce_max_sync(kFull, longest);
-        if (lane == 0) flush_range(per_seg, seg, n_pseg, vlo, vhi, longest);
-    } else {
-        flush_range(per_seg, seg, n_pseg, vlo, vhi, longest);
+        flush();
     }
     flags = __reduce_or_sync(kFull, flags);
     for (int o = 16; o > 0; o >>= 1) ones += __shfl_xor_sync(kFull, ones, o);

@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <vector>
 
 #include "wk_ctx.h"
@@ -126,7 +127,7 @@ struct Pass {
     uint64_t n;
     int shift;
     int from_value;
-    uint32_t* hist;   // [kDigits][grid], digit-major
+    uint32_t* hist;   // [kDigits][grid], digit-major; then each digit's total [kDigits]
 };
 
 __device__ __forceinline__ uint32_t digit(const Pass& a, uint64_t i) {
@@ -139,7 +140,15 @@ __global__ void __launch_bounds__(kT) hist_kernel(const Pass a) {
     __syncthreads();
     uint64_t lo, hi;
     span_of(a.n, &lo, &hi);
-    for (uint64_t i = lo + threadIdx.x; i < hi; i += kT) atomicAdd(&s_h[digit(a, i)], 1u);
+    constexpr int kU = 8;   // digits loaded together, then counted
+    for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += kU * kT) {
+        uint32_t d[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) d[u] = i0 + u * kT < hi ? digit(a, i0 + u * kT) : 0xFFFFFFFFu;
+#pragma unroll
+        for (int u = 0; u < kU; ++u)
+            if (d[u] < kDigits) atomicAdd(&s_h[d[u]], 1u);
+    }
     __syncthreads();
     a.hist[threadIdx.x * gridDim.x + blockIdx.x] = s_h[threadIdx.x];
 }
@@ -162,12 +171,37 @@ __global__ void __launch_bounds__(1024) scan32_kernel(uint32_t* v, uint32_t n) {
     }
 }
 
+// One CTA per digit scans that digit's row of the histogram (one word per CTA of the pass) in place
+// and leaves the digit's total behind the rows; the scatter CTAs add the smaller digits' totals
+// themselves (4.9 us; one CTA over all the rows took 224 us, three quarters of a pass at 6e6 items).
+__global__ void __launch_bounds__(kT) digit_rows_kernel(uint32_t* hist, uint32_t grid) {
+    __shared__ uint64_t s_warp[kT / 32];
+    __shared__ uint64_t s_carry;
+    uint32_t* row = hist + (size_t)blockIdx.x * grid;
+    if (threadIdx.x == 0) s_carry = 0;
+    __syncthreads();
+    for (uint32_t b0 = 0; b0 < grid; b0 += kT) {
+        const uint32_t b = b0 + threadIdx.x;
+        const uint64_t x = b < grid ? row[b] : 0;
+        const uint64_t ex = block_exclusive_sum<kT>(x, s_warp);
+        const uint64_t carry = s_carry;
+        if (b < grid) row[b] = (uint32_t)(carry + ex);
+        __syncthreads();
+        if (threadIdx.x == kT - 1) s_carry = carry + ex + x;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) hist[(size_t)kDigits * grid + blockIdx.x] = (uint32_t)s_carry;
+}
+
 __global__ void __launch_bounds__(kT) scatter_kernel(const Pass a) {
+    __shared__ uint64_t s_warp[kT / 32];
     __shared__ uint32_t s_run[kDigits];
     __shared__ uint32_t s_cnt[kT / 32][kDigits];
     __shared__ uint32_t s_tile[kDigits];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    s_run[threadIdx.x] = a.hist[threadIdx.x * gridDim.x + blockIdx.x];
+    static_assert(kT == kDigits, "one thread per digit");
+    s_run[threadIdx.x] = a.hist[threadIdx.x * gridDim.x + blockIdx.x] +
+                         (uint32_t)block_exclusive_sum<kT>(a.hist[(size_t)kDigits * gridDim.x + threadIdx.x], s_warp);
     uint64_t lo, hi;
     span_of(a.n, &lo, &hi);
     for (uint64_t base = lo; base < hi; base += kT) {
@@ -466,6 +500,7 @@ cudaError_t gbuild_kernel_attrs() {
     if (e == cudaSuccess) e = use_max_shared_carveout(hist_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(scatter_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(scan32_kernel);
+    if (e == cudaSuccess) e = use_max_shared_carveout(digit_rows_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(compact_count_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(compact_place_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(values_kernel);
@@ -488,16 +523,52 @@ using wk::KeyRec;
         if (e_ != cudaSuccess) return (ctx)->cuda_fail(e_, #call); \
     } while (0)
 
-// Device buffers of one build, freed together at the end, or one by one (release) as soon as
+// Device buffers of one build, given back together at the end, or one by one (release) as soon as
 // nothing reads them any more, so the build's peak stays within the device at a billion keys.
+// In a build of up to kSlabTriples triples they are cut from slabs, and what is released in a slab is
+// used again: such a build takes 40 buffers, and allocating and freeing each took longer than its
+// kernels, with a device-wide wait per free.  Larger builds spend their time in kernels and need
+// every released buffer's room.  Work runs in order on one stream, so a buffer may be used again
+// as soon as it is released.
 struct Bufs {
-    std::vector<void*> ptrs;
+    static constexpr uint64_t kSlabBytes = 256ull << 20, kSlabTriples = 1ull << 24, kAlign = 256;
+    struct Slab {
+        char* base;
+        std::map<uint64_t, uint64_t> free_at;   // offset -> bytes
+    };
+    wk_ctx* ctx;
+    bool use_slabs;
+    std::vector<void*> ptrs;                                  // whole allocations
+    std::vector<Slab> slabs;
+    std::map<const void*, std::pair<size_t, uint64_t>> cut;   // buffer -> slab, bytes
+    Bufs(wk_ctx* c, uint64_t n_triples) : ctx(c), use_slabs(n_triples <= kSlabTriples) {}
     ~Bufs() {
         for (void* p : ptrs) cudaFree(p);
+        for (auto& s : slabs) cudaFree(s.base);
     }
-    // Frees p (one of this set's buffers; cudaFree waits for the work that may still read it).
+    // Gives p (one of this set's buffers) back; a cudaFree waits for the work that may still read it.
     void release(const void* p) {
         if (!p) return;
+        auto it = cut.find(p);
+        if (it != cut.end()) {
+            Slab& s = slabs[it->second.first];
+            uint64_t at = (uint64_t)(static_cast<const char*>(p) - s.base), n = it->second.second;
+            cut.erase(it);
+            auto next = s.free_at.lower_bound(at);
+            if (next != s.free_at.end() && next->first == at + n) {
+                n += next->second;
+                next = s.free_at.erase(next);
+            }
+            if (next != s.free_at.begin()) {
+                auto prev = std::prev(next);
+                if (prev->first + prev->second == at) {
+                    prev->second += n;
+                    return;
+                }
+            }
+            s.free_at[at] = n;
+            return;
+        }
         for (size_t i = 0; i < ptrs.size(); ++i)
             if (ptrs[i] == p) {
                 cudaFree(ptrs[i]);
@@ -505,14 +576,45 @@ struct Bufs {
                 return;
             }
     }
+    void* cut_from(size_t i, uint64_t bytes) {
+        for (auto f = slabs[i].free_at.begin(); f != slabs[i].free_at.end(); ++f) {
+            if (f->second < bytes) continue;
+            const uint64_t at = f->first, left = f->second - bytes;
+            slabs[i].free_at.erase(f);
+            if (left) slabs[i].free_at[at + bytes] = left;
+            void* p = slabs[i].base + at;
+            cut[p] = {i, bytes};
+            return p;
+        }
+        return nullptr;
+    }
     template <class T>
     bool get(T** p, uint64_t n) {
+        const uint64_t bytes = (std::max<uint64_t>(n, 1) * sizeof(T) + kAlign - 1) / kAlign * kAlign;
         void* q = nullptr;
-        if (wk::dev_malloc(&q, std::max<uint64_t>(n, 1) * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
+        if (use_slabs && bytes <= kSlabBytes) {
+            for (size_t i = 0; i < slabs.size() && !q; ++i) q = cut_from(i, bytes);
+            if (!q) {
+                char* base = nullptr;
+                if (wk::dev_malloc(&base, kSlabBytes) == cudaSuccess) {
+                    slabs.push_back(Slab{base, {{0, kSlabBytes}}});
+                    q = cut_from(slabs.size() - 1, bytes);
+                } else {
+                    cudaGetLastError();   // (no room for a slab: the buffer alone)
+                }
+            }
         }
-        ptrs.push_back(q);
+        if (!q) {
+            if (wk::dev_malloc(&q, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                ctx->drop_spare();   // (the old store's arrays, kept for the new one's)
+                if (wk::dev_malloc(&q, bytes) != cudaSuccess) {
+                    cudaGetLastError();
+                    return false;
+                }
+            }
+            ptrs.push_back(q);
+        }
         *p = static_cast<T*>(q);
         return true;
     }
@@ -544,7 +646,7 @@ struct Builder {
         auto pass = [&](int shift, int from_value) {
             wk::Pass p{ka, va, kb, vb, n, shift, from_value, hist};
             wk::hist_kernel<<<grid, wk::kT, 0, s>>>(p);
-            wk::scan32_kernel<<<1, 1024, 0, s>>>(hist, (uint32_t)(wk::kDigits * grid));
+            wk::digit_rows_kernel<<<wk::kDigits, wk::kT, 0, s>>>(hist, (uint32_t)grid);
             wk::scatter_kernel<<<grid, wk::kT, 0, s>>>(p);
             std::swap(ka, kb);
             std::swap(va, vb);
@@ -803,7 +905,7 @@ int gbuild_segments(wk_ctx* ctx, Builder& bd, DirItems* D, unsigned long long* s
 
     // ---- edges and key records
     uint32_t* d_edges = nullptr;
-    if (wk::ctx_malloc(ctx, &d_edges, (n_edges + 16) * sizeof(uint32_t)) != cudaSuccess) {
+    if (ctx->store_malloc(ctx->spare_edges, &d_edges, (n_edges + 16) * sizeof(uint32_t)) != cudaSuccess) {
         cudaGetLastError();
         return ctx->fail(WK_E_OOM, "store edges");
     }
@@ -916,7 +1018,7 @@ int gbuild_segments(wk_ctx* ctx, Builder& bd, DirItems* D, unsigned long long* s
 
     const uint64_t n_slots = (main_buckets + n_ext) * kAssoc;
     Slot* d_slots = nullptr;
-    if (wk::ctx_malloc(ctx, &d_slots, std::max<uint64_t>(n_slots, kAssoc) * sizeof(Slot)) != cudaSuccess) {
+    if (ctx->store_malloc(ctx->spare_slots, &d_slots, std::max<uint64_t>(n_slots, kAssoc) * sizeof(Slot)) != cudaSuccess) {
         cudaGetLastError();
         return ctx->fail(WK_E_OOM, "store slots");
     }
@@ -955,7 +1057,7 @@ int gbuild(wk_ctx* ctx, const uint32_t* d_tr, uint64_t n, double load, bool vers
     uint32_t* part = nullptr;
     unsigned long long* d_count = nullptr;
     uint32_t* d_mm = nullptr;
-    if (!B.get(&hist, (uint64_t)kDigits * gmax) || !B.get(&part, gmax + 2) || !B.get(&d_count, 1) ||
+    if (!B.get(&hist, (uint64_t)kDigits * (gmax + 1)) || !B.get(&part, gmax + 2) || !B.get(&d_count, 1) ||
         !B.get(&d_mm, 8))
         return ctx->fail(WK_E_OOM, "store build scratch");
 
@@ -1041,15 +1143,19 @@ extern "C" int wk_store_build_device(wk_ctx* ctx, const uint32_t* triples, uint6
     WKG_CUDA(ctx, cudaSetDevice(ctx->device));
     WKG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     // the old store goes first: a build needs the room
-    ctx->drop_store();
+    ctx->drop_store(true);
     ctx->release_serve();   // (a build needs the room)
+    struct DropSpare {      // what the build did not use
+        wk_ctx* c;
+        ~DropSpare() { c->drop_spare(); }
+    } drop_spare{ctx};
     wk::Slot* slots = nullptr;
     uint32_t* edges = nullptr;
     uint64_t n_slots = 0, n_edges = 0;
     std::vector<wk_seg_meta> segs;
     int rc;
     {
-        Bufs B;   // the build's scratch, freed before the store is adopted
+        Bufs B(ctx, n_triples);   // the build's scratch, freed before the store is adopted
         uint32_t* d_tr = nullptr;
         if (!B.get(&d_tr, std::max<uint64_t>(n_triples, 1) * 3)) return ctx->fail(WK_E_OOM, "store build triples");
         if (n_triples)
@@ -1058,6 +1164,7 @@ extern "C" int wk_store_build_device(wk_ctx* ctx, const uint32_t* triples, uint6
         cudaStreamSynchronize(ctx->stream);
     }
     if (rc) {
+        ctx->slots_bytes = ctx->edges_bytes = 0;
         if (slots) cudaFree(slots);
         if (edges) cudaFree(edges);
         return rc;

@@ -55,9 +55,9 @@ __device__ __forceinline__ void flush_range(SegScan* out, uint32_t seg, uint32_t
 // One thread per slot, a warp over shares of 1,024 slots, four slots loaded before any is looked
 // at.  The shares are dealt round: a segment's keys lie together, and with one contiguous share a
 // warp the few warps that met the segments with lists of hundreds of entries (the members of 9,000
-// departments) ran long after the others (1.78 -> 0.49 ms at 500 organisations).  Bound by the read of the table (16 bytes a slot, most of
-// them empty at the default load factor) and by the short lists' sectors.  Lists past kChunkList
-// entries (the type and predicate indexes: 1.5e6 entries in one list at 500 organisations) go to a
+// departments) ran long after the others (1.78 -> 0.49 ms at 500 organisations).  Bound by the read
+// of the table (16 bytes a slot, most of them empty at the default load factor) and by the short
+// lists' sectors.  Lists past kChunkList entries (the type and predicate indexes: 1.5e6 entries in one list at 500 organisations) go to a
 // queue as chunks that a second kernel checks with every warp; walked by the one warp that met
 // them, they took 21 of the 22 ms this check cost on that store.
 constexpr int kScanUnroll = 4;

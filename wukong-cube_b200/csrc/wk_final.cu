@@ -6,10 +6,11 @@
 // DISTINCT follows the reference step for step: the rows are sorted by all their columns,
 // compared as signed 32-bit values (ReduceCmp over an int table, sparql.hpp:1403-1417), then
 // of each run of neighbours equal on the required columns the first is kept.  The sort is an
-// LSD radix sort of (packed key, row index) pairs over only the bits in which the rows differ
-// (see "DISTINCT sort" below); rows equal in every column are interchangeable, so the result
-// does not depend on how the reference's std::sort orders them.  A table found to be in that
-// order already (one pass over it, rows_sorted_kernel) skips the sort.
+// LSD radix sort of packed keys over only the bits in which the rows differ (see "DISTINCT sort"
+// below).  Only the columns up to the last required one are looked at: the columns behind it order
+// rows that are equal in all that is output.  Rows equal in every column looked at are
+// interchangeable, so the result does not depend on how the reference's std::sort orders them.  A
+// table found to be in that order already (one pass over it, scan_rows_kernel) skips the sort.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,78 +33,19 @@ constexpr int kFinThreads = 256;
 constexpr int kDigits = 256;
 
 // ---------------------------------------------------------------- DISTINCT sort
-// The sort orders rows by all their columns as signed 32-bit values.  A column is first mapped
+// The sort orders rows by their columns as signed 32-bit values.  A column is first mapped
 // to its offset from the column's smallest value (in signed order), so a column spanning d
 // distinct-order values needs only ceil(log2(d)) bits, and a constant column none.  Columns are
 // packed, last column in the lowest bits, into 64-bit keys ("chunks" of consecutive columns that
 // fit in 64 bits); the LSD sort runs the chunks from the last columns to the first, and within a
-// chunk one stable 8-bit counting pass per byte of the chunk's bits.  Every pass reads the keys
-// and row indices with coalesced loads; the table itself is read once per chunk, to build its
-// keys.
-
-// Smallest and largest value of every column (signed order, stored with the sign bit flipped).
-__global__ void __launch_bounds__(kFinThreads) minmax_kernel(const uint32_t* table, uint64_t elems, int cols,
-                                                             uint32_t* mm /* [2 * cols] */) {
-    __shared__ uint32_t s_lo[64], s_hi[64];
-    for (int c = threadIdx.x; c < cols; c += kFinThreads) {
-        s_lo[c] = 0xFFFFFFFFu;
-        s_hi[c] = 0;
-    }
-    __syncthreads();
-    const uint64_t stride = (uint64_t)gridDim.x * kFinThreads;
-    uint64_t e = blockIdx.x * (uint64_t)kFinThreads + threadIdx.x;
-    int c = (int)(e % cols);
-    const int step = (int)(stride % cols);
-    uint32_t lo = 0xFFFFFFFFu, hi = 0;
-    int cur = c;
-    // eight loads in flight per thread; the host makes the grid's stride a multiple of cols where
-    // it can, so a thread's elements stay in one column and the fold below never runs in the loop
-    constexpr int kPer = 8;
-    for (; e + (kPer - 1) * stride < elems; e += kPer * stride) {
-        uint32_t v[kPer];
-#pragma unroll
-        for (int r = 0; r < kPer; ++r) v[r] = __ldg(table + e + r * stride) ^ 0x80000000u;
-#pragma unroll
-        for (int r = 0; r < kPer; ++r) {
-            if (c != cur) {
-                atomicMin(&s_lo[cur], lo);
-                atomicMax(&s_hi[cur], hi);
-                lo = 0xFFFFFFFFu;
-                hi = 0;
-                cur = c;
-            }
-            lo = min(lo, v[r]);
-            hi = max(hi, v[r]);
-            c += step;
-            if (c >= cols) c -= cols;
-        }
-    }
-    for (; e < elems; e += stride) {
-        const uint32_t v = __ldg(table + e) ^ 0x80000000u;
-        if (c != cur) {   // column changed: fold the run so far into shared memory
-            atomicMin(&s_lo[cur], lo);
-            atomicMax(&s_hi[cur], hi);
-            lo = 0xFFFFFFFFu;
-            hi = 0;
-            cur = c;
-        }
-        lo = min(lo, v);
-        hi = max(hi, v);
-        c += step;
-        if (c >= cols) c -= cols;
-    }
-    if (lo <= hi) {
-        atomicMin(&s_lo[cur], lo);
-        atomicMax(&s_hi[cur], hi);
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < cols; k += kFinThreads) {
-        if (s_lo[k] <= s_hi[k]) {
-            atomicMin(&mm[2 * k], s_lo[k]);
-            atomicMax(&mm[2 * k + 1], s_hi[k]);
-        }
-    }
-}
+// chunk one stable counting pass per byte of the chunk's bits.
+//
+// Where one chunk holds all the columns, the key is the row: the passes move the keys alone (16
+// bytes a row and pass instead of 24), and the compaction compares neighbouring keys and writes the
+// required columns out of them, so no index array is kept and no row is gathered.  Else every
+// pass moves the row indices with the keys, and the table is read once per chunk.
+// Measured on 3,000,000 rows of three columns (63 bits, 39 of them up to the second column), the
+// first two required: 598 -> 265 us a call.
 
 // One chunk's key layout: columns ccol[0..nc), most significant first, ccol[j] in cbits[j]
 // bits above the next, offset by cmin[j].
@@ -129,20 +71,32 @@ __global__ void __launch_bounds__(kFinThreads) key_kernel(const uint32_t* table,
     }
 }
 
-// *flag = 1 when some row is greater than the next one, every column compared as a signed 32-bit
-// value in column order (ReduceCmp).  A table already in that order is what the sort would
-// return (rows equal in every column are interchangeable), so the sort is skipped for it: the
-// exploration writes rows in input order and each row's new column from a sorted list, so a
-// table started from an index or a constant with unique rows comes out in this order.
+// One pass over the rows: *flag = 0 (all ones before) when some row is greater than the next one,
+// its first `cmp` columns compared as signed 32-bit values in column order (ReduceCmp), and the
+// smallest and largest value of each of these columns (in signed order, stored with the sign bit
+// flipped; the largest as its complement, so that both begin as all ones).  A table already in that
+// order is what the sort would return (rows equal in these columns are interchangeable), so the
+// sort is skipped for it: the exploration writes rows in input order and each row's new column
+// from a sorted list, so a table started from an index or a constant with unique rows comes out in
+// this order.
 // A CTA stages `tile_rows` consecutive rows and the row after them in shared memory with
-// coalesced loads, eight in flight per thread, then each thread compares one row with the next
-// out of shared memory; a CTA that finds a pair out of order stops.
+// coalesced loads, eight in flight per thread, then each thread compares rows with the next ones
+// and takes the columns' extremes out of shared memory.  Bound by the read of the table: 14.9 us at
+// 36 MB, where two kernels that each read it took 22.
 constexpr int kCheckWords = 8192;   // 32 KiB of rows per tile
 
-__global__ void __launch_bounds__(kFinThreads) rows_sorted_kernel(const uint32_t* table, int cols, uint32_t n,
-                                                                  uint32_t tile_rows, unsigned* flag) {
+__global__ void __launch_bounds__(kFinThreads) scan_rows_kernel(const uint32_t* table, int cols, int cmp,
+                                                                uint32_t n, uint32_t tile_rows, unsigned* flag,
+                                                                uint32_t* mm /* [2 * cmp] */) {
     __shared__ uint32_t s_t[kCheckWords];
+    __shared__ uint32_t s_lo[32], s_hi[32];
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        s_lo[threadIdx.x] = 0xFFFFFFFFu;
+        s_hi[threadIdx.x] = 0;
+    }
     const uint32_t pairs = n - 1;   // pair i is rows (i, i + 1); n >= 2
+    bool bad = false;
     for (uint64_t t0 = (uint64_t)blockIdx.x * tile_rows; t0 < pairs; t0 += (uint64_t)gridDim.x * tile_rows) {
         const uint32_t here = (uint32_t)min((uint64_t)tile_rows, pairs - t0);   // pairs of this tile
         const uint32_t words = (here + 1) * (uint32_t)cols;                     // <= kCheckWords
@@ -154,26 +108,40 @@ __global__ void __launch_bounds__(kFinThreads) rows_sorted_kernel(const uint32_t
 #pragma unroll
             for (int r = 0; r < kPer; ++r) v[r] = __ldg(src + w + r * kFinThreads);
 #pragma unroll
-            for (int r = 0; r < kPer; ++r) s_t[w + r * kFinThreads] = v[r];
+            for (int r = 0; r < kPer; ++r) s_t[w + r * kFinThreads] = v[r] ^ 0x80000000u;
         }
-        for (; w < words; w += kFinThreads) s_t[w] = __ldg(src + w);
+        for (; w < words; w += kFinThreads) s_t[w] = __ldg(src + w) ^ 0x80000000u;
         __syncthreads();
-        bool bad = false;
-        for (uint32_t i = threadIdx.x; i < here && !bad; i += kFinThreads) {
+        for (uint32_t i = threadIdx.x; i < here; i += kFinThreads) {
             const uint32_t* r = s_t + i * cols;
-            for (int c = 0; c < cols; ++c) {
-                const int32_t x = (int32_t)r[c], y = (int32_t)r[cols + c];
+            for (int c = 0; c < cmp; ++c) {
+                const uint32_t x = r[c], y = r[cols + c];
                 if (x != y) {
-                    bad = x > y;
+                    bad |= x > y;
                     break;
                 }
             }
         }
-        // also the barrier before the next tile overwrites s_t
-        if (__syncthreads_or(bad)) {
-            if (threadIdx.x == 0) atomicOr(flag, 1u);
-            return;
+        for (int c = 0; c < cmp; ++c) {
+            uint32_t lo = 0xFFFFFFFFu, hi = 0;
+            for (uint32_t i = threadIdx.x; i <= here; i += kFinThreads) {
+                const uint32_t x = s_t[i * cols + c];
+                lo = min(lo, x);
+                hi = max(hi, x);
+            }
+            lo = __reduce_min_sync(kFull, lo);
+            hi = __reduce_max_sync(kFull, hi);
+            if (lane == 0 && lo <= hi) {
+                atomicMin(&s_lo[c], lo);
+                atomicMax(&s_hi[c], hi);
+            }
         }
+        __syncthreads();   // before the next tile overwrites s_t
+    }
+    if (__syncthreads_or(bad) && threadIdx.x == 0) *flag = 0;
+    if ((int)threadIdx.x < cmp && s_lo[threadIdx.x] <= s_hi[threadIdx.x]) {
+        atomicMin(&mm[2 * threadIdx.x], s_lo[threadIdx.x]);
+        atomicMin(&mm[2 * threadIdx.x + 1], ~s_hi[threadIdx.x]);
     }
 }
 
@@ -184,6 +152,7 @@ struct SortPass {
     uint32_t* idx_out;
     int shift;
     uint32_t n;
+    uint32_t per_cta;        // elements of a CTA
     uint32_t* hist;          // [kDigits][grid]: digit-major, so one scan gives the offsets
     uint32_t* dtot;          // [kDigits]: elements of each digit
 };
@@ -195,8 +164,10 @@ __device__ __forceinline__ void chunk(uint32_t n, uint32_t* lo, uint32_t* hi) {
     *hi = min(n, *lo + c);
 }
 
-__global__ void __launch_bounds__(kFinThreads) iota_kernel(uint32_t* idx, uint32_t n) {
-    for (uint32_t i = blockIdx.x * kFinThreads + threadIdx.x; i < n; i += gridDim.x * kFinThreads) idx[i] = i;
+template <class A>
+__device__ __forceinline__ void span(const A& a, uint32_t* lo, uint32_t* hi) {
+    *lo = (uint32_t)min((uint64_t)a.n, (uint64_t)blockIdx.x * a.per_cta);
+    *hi = (uint32_t)min((uint64_t)a.n, (uint64_t)*lo + a.per_cta);
 }
 
 // Digit counts of each CTA's chunk.  A thread loads eight keys before it counts any of them, so
@@ -207,7 +178,7 @@ __global__ void __launch_bounds__(kFinThreads) hist_kernel(const SortPass a) {
     s_h[threadIdx.x] = 0;
     __syncthreads();
     uint32_t lo, hi;
-    chunk(a.n, &lo, &hi);
+    span(a, &lo, &hi);
     uint64_t i = lo + threadIdx.x;
     for (; i + (kPer - 1) * kFinThreads < hi; i += kPer * kFinThreads) {
         unsigned long long k[kPer];
@@ -251,14 +222,24 @@ __global__ void __launch_bounds__(kFinThreads) digit_rows_kernel(uint32_t* hist,
     uint32_t* row = hist + (size_t)blockIdx.x * grid;
     if (threadIdx.x == 0) s_carry = 0;
     __syncthreads();
-    for (uint32_t b0 = 0; b0 < grid; b0 += kFinThreads) {
-        const uint32_t b = b0 + threadIdx.x;
-        const uint64_t x = b < grid ? row[b] : 0;
-        const uint64_t ex = block_exclusive_sum<kFinThreads>(x, s_warp);
+    constexpr uint32_t kPer = 4;   // a row of a full grid in one round
+    for (uint32_t b0 = 0; b0 < grid; b0 += kPer * kFinThreads) {
+        const uint32_t b = b0 + kPer * threadIdx.x;
+        uint32_t x[kPer], sum = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kPer; ++j) x[j] = b + j < grid ? row[b + j] : 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kPer; ++j) sum += x[j];
+        const uint64_t ex = block_exclusive_sum<kFinThreads>(sum, s_warp);
         const uint64_t carry = s_carry;
-        if (b < grid) row[b] = (uint32_t)(carry + ex);
+        uint32_t at = (uint32_t)(carry + ex);
+#pragma unroll
+        for (uint32_t j = 0; j < kPer; ++j) {
+            if (b + j < grid) row[b + j] = at;
+            at += x[j];
+        }
         __syncthreads();
-        if (threadIdx.x == kFinThreads - 1) s_carry = carry + ex + x;
+        if (threadIdx.x == kFinThreads - 1) s_carry = carry + ex + sum;
         __syncthreads();
     }
     if (threadIdx.x == 0) dtot[blockIdx.x] = (uint32_t)s_carry;
@@ -266,85 +247,260 @@ __global__ void __launch_bounds__(kFinThreads) digit_rows_kernel(uint32_t* hist,
 
 // Stable scatter of 2,048-element tiles: warp w of the CTA takes elements [w * 256, w * 256 + 256)
 // of the tile in 8 rounds of 32 consecutive ones, so the warp's rounds follow the elements'
-// order.  Within a round, an element's rank among the lanes with its digit comes from a match,
-// and the warp's running count of each digit (shared memory, updated by one lane per digit)
-// gives its place in the warp; one barrier then turns the warps' counts into per-warp digit
-// offsets.  The tile is placed in shared memory sorted by digit (stable), and then written out
-// in that order, consecutive threads on consecutive elements, so each digit's run goes to
-// global memory in contiguous, coalesced stores.  Built for 4 CTAs per SM (64 registers, no
-// spills; 34.9 KB of shared memory each), so the pass's 4 CTAs per SM run in one wave.
+// order.  Within a round, an element's rank among the lanes with its digit comes from a mask per
+// digit in shared memory, into which the lanes set their bits (a match takes time with the number of
+// different digits, 32 us a pass of eight bits where one with a third of the digits took 17; eight
+// ballots were bound by their own pipe at 24), and the warp's running count of each digit (updated
+// by one lane per digit) gives its place in the warp; one barrier then turns the warps' counts into
+// per-warp digit offsets.  The tile is placed in shared memory sorted by digit (stable), and then
+// written out in that order, consecutive threads on consecutive elements, so each digit's run goes
+// to global memory in contiguous, coalesced stores.  With the row indices: 4 CTAs per SM (64
+// registers, no spills; 43 KB of shared memory each), so the pass's 4 CTAs per SM run in one wave.
+// Keys alone: 5 CTAs per SM, each over whole tiles.  Bound by the shared-memory chain within a tile
+// and its barriers at this number of warps: 35 us a pass with the indices and the match, 22 with
+// keys alone and the masks, at 3,000,000 rows.
 constexpr int kScatterPer = 8;                                // elements per thread per tile
 constexpr int kScatterTile = kFinThreads * kScatterPer;       // 2,048
 
-__global__ void __launch_bounds__(kFinThreads, 4) scatter_kernel(const SortPass a) {
+template <bool kIdx>
+__global__ void __launch_bounds__(kFinThreads, kIdx ? 4 : 5) scatter_kernel(const SortPass a) {
     constexpr int kWarps = kFinThreads / 32;
-    __shared__ uint32_t s_run[kDigits];
     __shared__ uint32_t s_cnt[kWarps][kDigits];
-    __shared__ uint32_t s_tbase[kDigits];
+    __shared__ uint32_t s_peers[kWarps][kDigits];
+    __shared__ uint32_t s_off[kDigits];
     __shared__ unsigned long long s_key[kScatterTile];
-    __shared__ uint32_t s_idx[kScatterTile];
+    __shared__ uint32_t s_idx[kIdx ? kScatterTile : 1];
     __shared__ uint64_t s_warp[kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // thread d: digit d's first place for this CTA = the elements of smaller digits plus the
     // digit-d elements of the CTAs before this one
     const uint32_t smaller = (uint32_t)block_exclusive_sum<kFinThreads>(a.dtot[threadIdx.x], s_warp);
-    s_run[threadIdx.x] = smaller + a.hist[threadIdx.x * gridDim.x + blockIdx.x];
+    uint32_t run = smaller + a.hist[threadIdx.x * gridDim.x + blockIdx.x];
     uint32_t lo, hi;
-    chunk(a.n, &lo, &hi);
-    for (uint32_t base = lo; base < hi; base += kScatterTile) {
+    span(a, &lo, &hi);
+    for (int w = 0; w < kWarps; ++w) s_peers[w][threadIdx.x] = 0;
+    for (uint64_t base = lo; base < hi; base += kScatterTile) {
         for (int w = 0; w < kWarps; ++w) s_cnt[w][threadIdx.x] = 0;
         __syncthreads();
         unsigned long long key[kScatterPer];
-        uint32_t row[kScatterPer], dg[kScatterPer], at[kScatterPer];
-        const uint32_t wbase = base + (uint32_t)warp * (32 * kScatterPer);
+        [[maybe_unused]] uint32_t row[kScatterPer];
+        uint32_t dg[kScatterPer], at[kScatterPer];
+        const uint64_t wbase = base + (uint32_t)warp * (32 * kScatterPer);
 #pragma unroll
         for (int r = 0; r < kScatterPer; ++r) {
-            const uint32_t i = wbase + r * 32 + lane;
+            const uint64_t i = wbase + r * 32 + lane;
             const bool live = i < hi;
             key[r] = live ? a.key_in[i] : 0;
-            row[r] = live ? a.idx_in[i] : 0;
-            dg[r] = live ? (uint32_t)(key[r] >> a.shift) & 0xFFu : kDigits + lane;   // lone sentinel
+            if constexpr (kIdx) row[r] = live ? a.idx_in[i] : 0;
+            dg[r] = live ? (uint32_t)(key[r] >> a.shift) & 0xFFu : (uint32_t)kDigits;
         }
 #pragma unroll
         for (int r = 0; r < kScatterPer; ++r) {
-            const unsigned peers = __match_any_sync(0xffffffffu, dg[r]);
-            const int rank = __popc(peers & ((1u << lane) - 1));
             const bool live = dg[r] < kDigits;
+            if (live) atomicOr(&s_peers[warp][dg[r]], 1u << lane);
+            __syncwarp();
+            const unsigned peers = live ? s_peers[warp][dg[r]] : 0;   // the lanes with this lane's digit
+            const int rank = __popc(peers & ((1u << lane) - 1));
             at[r] = live ? s_cnt[warp][dg[r]] + rank : 0;
             __syncwarp();
-            if (live && rank == 0) s_cnt[warp][dg[r]] += __popc(peers);
+            if (live && rank == 0) {
+                s_cnt[warp][dg[r]] += __popc(peers);
+                s_peers[warp][dg[r]] = 0;
+            }
             __syncwarp();
         }
         __syncthreads();
-        uint32_t tile_cnt = 0;   // per digit (thread = digit): prefix over the warps
-        for (int w = 0; w < kWarps; ++w) {
-            const uint32_t c = s_cnt[w][threadIdx.x];
-            s_cnt[w][threadIdx.x] = tile_cnt;
-            tile_cnt += c;
-        }
-        // the tile sorted by digit in shared memory: digit d's elements start at s_tbase[d]
+        uint32_t cnt[kWarps], tile_cnt = 0;   // per digit (thread = digit): prefix over the warps
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) cnt[w] = s_cnt[w][threadIdx.x];
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) tile_cnt += cnt[w];
+        // the tile sorted by digit in shared memory: digit d's elements start at tbase, warp w's
+        // at s_cnt[w][d]; s_off[d] takes a place in the tile to its place in the output
         const uint32_t tbase = (uint32_t)block_exclusive_sum<kFinThreads>(tile_cnt, s_warp);
-        s_tbase[threadIdx.x] = tbase;
+        s_off[threadIdx.x] = run - tbase;
+        run += tile_cnt;
+        uint32_t wat = tbase;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            s_cnt[w][threadIdx.x] = wat;
+            wat += cnt[w];
+        }
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kScatterPer; ++r) {
             if (dg[r] >= kDigits) continue;
-            const uint32_t lp = s_tbase[dg[r]] + s_cnt[warp][dg[r]] + at[r];
+            const uint32_t lp = s_cnt[warp][dg[r]] + at[r];
             s_key[lp] = key[r];
-            s_idx[lp] = row[r];
+            if constexpr (kIdx) s_idx[lp] = row[r];
         }
         __syncthreads();
         // consecutive threads write consecutive elements: each digit's run goes out contiguous
-        const uint32_t m = min((uint32_t)kScatterTile, hi - base);
+        const uint32_t m = (uint32_t)min((uint64_t)kScatterTile, hi - base);
         for (uint32_t j = threadIdx.x; j < m; j += kFinThreads) {
             const unsigned long long k = s_key[j];
             const uint32_t d = (uint32_t)(k >> a.shift) & 0xFFu;
-            const uint32_t pos = s_run[d] + (j - s_tbase[d]);
+            const uint32_t pos = s_off[d] + j;
             a.key_out[pos] = k;
-            a.idx_out[pos] = s_idx[j];
+            if constexpr (kIdx) a.idx_out[pos] = s_idx[j];
         }
         __syncthreads();
-        s_run[threadIdx.x] += tile_cnt;
+    }
+}
+
+// ---- one chunk holds all the columns looked at: keys alone
+
+// The rows' keys and the first pass's digit counts, a CTA over the span it has in that pass: the
+// table is read once, eight rows in flight per thread.
+__global__ void __launch_bounds__(kFinThreads) key_hist_kernel(const uint32_t* table, int cols,
+                                                               const __grid_constant__ ChunkDesc cd, const SortPass a,
+                                                               unsigned long long* keys) {
+    constexpr int kPer = 8;
+    __shared__ uint32_t s_h[kDigits];
+    s_h[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t lo, hi;
+    span(a, &lo, &hi);
+    for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += kPer * kFinThreads) {
+        unsigned long long k[kPer];
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) k[r] = 0;
+        for (int j = 0; j < cd.nc; ++j) {
+            const int c = cd.ccol[j], bits = cd.cbits[j];
+            const uint32_t lowest = cd.cmin[j];
+            uint32_t v[kPer];
+#pragma unroll
+            for (int r = 0; r < kPer; ++r) {
+                const uint64_t i = i0 + r * kFinThreads;
+                v[r] = i < hi ? __ldg(table + i * cols + c) : 0;
+            }
+#pragma unroll
+            for (int r = 0; r < kPer; ++r)
+                k[r] = (k[r] << bits) | (unsigned long long)((v[r] ^ 0x80000000u) - lowest);
+        }
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+            const uint64_t i = i0 + r * kFinThreads;
+            if (i >= hi) continue;
+            keys[i] = k[r];
+            atomicAdd(&s_h[(uint32_t)k[r] & 0xFFu], 1u);
+        }
+    }
+    __syncthreads();
+    a.hist[threadIdx.x * gridDim.x + blockIdx.x] = s_h[threadIdx.x];
+}
+
+// The required columns of a key: column k is the `bits[k]` bits at `shift[k]`, above `lowest[k]`.
+struct KeyCols {
+    int n;
+    unsigned long long mask;   // their bits: neighbours that differ in none of them are one row
+    int shift[32], bits[32];
+    uint32_t lowest[32];
+};
+
+struct KeyRuns {
+    const unsigned long long* keys;   // sorted
+    uint32_t n;
+    uint32_t per_cta;                 // keys of a CTA
+    uint32_t* part;                   // [grid + 1] kept keys per CTA, then their exclusive scan
+};
+
+__device__ __forceinline__ bool starts_key_run(const KeyRuns& a, const KeyCols& kc, uint32_t i) {
+    return i == 0 || ((a.keys[i] ^ a.keys[i - 1]) & kc.mask) != 0;
+}
+
+__global__ void __launch_bounds__(kFinThreads) key_count_kernel(const KeyRuns a, const __grid_constant__ KeyCols kc) {
+    __shared__ uint64_t s_warp[kFinThreads / 32];
+    uint32_t lo, hi;
+    span(a, &lo, &hi);
+    uint64_t c = 0;
+#pragma unroll 4
+    for (uint64_t i = (uint64_t)lo + threadIdx.x; i < hi; i += kFinThreads) c += starts_key_run(a, kc, (uint32_t)i);
+    const uint64_t ex = block_exclusive_sum<kFinThreads>(c, s_warp);
+    if (threadIdx.x == kFinThreads - 1) a.part[blockIdx.x] = (uint32_t)(ex + c);
+}
+
+// Kept key number r goes to output row r - start where that lies in [0, count).  A warp takes four
+// runs of 32 keys a round, so one scan serves 1,024 keys; a round's kept keys are packed in shared
+// memory and written out column by column, consecutive threads on consecutive words.
+// The rows kept (*total) are known on the device only: a result that does not fit `cap` words is
+// left out whole, and the host, which reads *total, makes room and runs this again.
+__global__ void __launch_bounds__(kFinThreads) key_write_kernel(const KeyRuns a, const __grid_constant__ KeyCols kc,
+                                                                const uint32_t* total, uint64_t offset,
+                                                                int64_t limit, uint32_t* out, uint64_t cap,
+                                                                uint64_t* out_rows) {
+    constexpr int kPer = 4;
+    __shared__ uint32_t s_n[kFinThreads / 32];
+    __shared__ unsigned long long s_key[kPer * kFinThreads];
+    __shared__ uint4 s_col[32];   // a column's shift, mask, smallest value
+    if (threadIdx.x < 32)
+        s_col[threadIdx.x] = make_uint4(kc.shift[threadIdx.x],
+                                        kc.bits[threadIdx.x] ? 0xFFFFFFFFu >> (32 - kc.bits[threadIdx.x]) : 0,
+                                        kc.lowest[threadIdx.x], 0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t m = *total, start = min(offset, m);
+    const uint64_t count = limit < 0 ? m - start : min((uint64_t)limit, m - start);
+    if (count * kc.n > cap) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *out_rows = count;
+    uint32_t lo, hi;
+    span(a, &lo, &hi);
+    uint64_t carry = a.part[blockIdx.x];
+    for (uint64_t base = lo; base < hi; base += kPer * kFinThreads) {
+        unsigned long long key[kPer];
+        unsigned m32[kPer];
+        uint32_t mine = 0;
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+            const uint64_t i = base + (warp * kPer + r) * 32 + lane;
+            key[r] = i < hi ? a.keys[i] : 0;
+        }
+        const uint64_t w0 = base + warp * kPer * 32;   // the key before the warp's
+        unsigned long long before = lane == 0 && w0 > 0 && w0 < hi ? a.keys[w0 - 1] : 0;
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+            const uint64_t i = w0 + r * 32 + lane;
+            const unsigned long long up = __shfl_up_sync(kFull, key[r], 1);
+            const unsigned long long prev = lane == 0 ? before : up;
+            before = __shfl_sync(kFull, key[r], 31);
+            m32[r] = __ballot_sync(kFull, i < hi && (i == 0 || ((key[r] ^ prev) & kc.mask) != 0));
+            mine += __popc(m32[r]);
+        }
+        // the warp's kept keys go before those of the warps behind it
+        if (lane == 0) s_n[warp] = mine;
+        __syncthreads();
+        uint32_t at = 0, kept = 0;
+#pragma unroll
+        for (int w = 0; w < kFinThreads / 32; ++w) {
+            if (w < warp) at += s_n[w];
+            kept += s_n[w];
+        }
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+            if (m32[r] >> lane & 1u) s_key[at + __popc(m32[r] & ((1u << lane) - 1))] = key[r];
+            at += __popc(m32[r]);
+        }
+        __syncthreads();
+        // the packed keys [from, to) are output rows carry + from - start ...
+        const uint32_t from = carry < start ? (uint32_t)min((uint64_t)kept, start - carry) : 0;
+        const uint32_t to = (uint32_t)min((uint64_t)kept, start + count > carry ? start + count - carry : 0);
+        if (from < to) {
+            uint32_t* dst = out + (carry + from - start) * kc.n;
+            const uint32_t words = (to - from) * kc.n, n = (uint32_t)kc.n;
+            uint32_t j = threadIdx.x / n, c = threadIdx.x - j * n;
+            const uint32_t dj = kFinThreads / n, dc = kFinThreads - dj * n;
+            for (uint32_t e = threadIdx.x; e < words; e += kFinThreads) {
+                const uint4 col = s_col[c];
+                dst[e] = (((uint32_t)(s_key[from + j] >> col.x) & col.y) + col.z) ^ 0x80000000u;
+                j += dj;
+                c += dc;
+                if (c >= n) {
+                    c -= n;
+                    ++j;
+                }
+            }
+        }
+        carry += kept;
+        __syncthreads();
     }
 }
 
@@ -498,14 +654,16 @@ __global__ void __launch_bounds__(kFinThreads) bound_place_kernel(const BoundArg
 }  // namespace
 
 cudaError_t final_kernel_attrs() {
-    cudaError_t e = use_max_shared_carveout(iota_kernel);
-    if (e == cudaSuccess) e = use_max_shared_carveout(minmax_kernel);
+    cudaError_t e = use_max_shared_carveout(scan_rows_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(key_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(hist_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(scan_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(digit_rows_kernel);
-    if (e == cudaSuccess) e = use_max_shared_carveout(rows_sorted_kernel);
-    if (e == cudaSuccess) e = use_max_shared_carveout(scatter_kernel);
+    if (e == cudaSuccess) e = use_max_shared_carveout(scatter_kernel<true>);
+    if (e == cudaSuccess) e = use_max_shared_carveout(scatter_kernel<false>);
+    if (e == cudaSuccess) e = use_max_shared_carveout(key_hist_kernel);
+    if (e == cudaSuccess) e = use_max_shared_carveout(key_count_kernel);
+    if (e == cudaSuccess) e = use_max_shared_carveout(key_write_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(unique_count_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(unique_place_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(project_kernel);
@@ -550,6 +708,13 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
     if (R >= (1ull << 32)) return ctx->fail(WK_E_CAPACITY, "table too long for the post-pattern stage");
     const uint32_t n = (uint32_t)R;
     const int grid = std::max(1, std::min<int>(ctx->sm_count * 4, (int)((n + 2047) / 2048)));
+    // the passes over keys alone: whole tiles for each CTA, and one wave of CTAs (a part
+    // that ends within a tile leaves the rest of the CTA idle in it)
+    const uint32_t tiles = (uint32_t)(((uint64_t)n + kScatterTile - 1) / kScatterTile);
+    const uint32_t cta_tiles = (tiles + ctx->sm_count * 5 - 1) / (ctx->sm_count * 5);
+    const int kgrid1 = (int)((tiles + cta_tiles - 1) / cta_tiles);
+    const int hgrid = std::max(grid, kgrid1);        // the histogram's rows
+    const int pgrid1 = std::max(grid, ctx->sm_count * 8);   // the CTA counts
     // scratch: the required columns, two index arrays, two key arrays (DISTINCT only), the
     // digit histogram, the CTA counts and the distinct total, the column ranges, the digit totals
     const bool sort = distinct && n > 1;
@@ -557,8 +722,8 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
     const size_t idx_bytes = ((2 * (size_t)n * 4) + 255) & ~(size_t)255;
     // the two key arrays; once the sort is done the same room holds the table in sorted order
     const size_t key_bytes = sort ? std::max(2 * (size_t)n * 8, (size_t)n * cols * 4) : 0;
-    const size_t bytes = keep_bytes + idx_bytes + key_bytes + (size_t)kDigits * grid * 4 +
-                         ((size_t)grid + 2) * 4 + (size_t)cols * 8 + (size_t)kDigits * 4 + 64;
+    const size_t bytes = keep_bytes + idx_bytes + key_bytes + (size_t)kDigits * hgrid * 4 +
+                         ((size_t)pgrid1 + 2) * 4 + (size_t)cols * 8 + (size_t)kDigits * 4 + 64;
     // the context keeps the scratch between calls (grown, never shrunk): an allocation and a
     // cudaFree per call would cost more than the stage's own kernels
     int src = ctx->final_scratch_reserve(bytes);
@@ -574,48 +739,113 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
     unsigned long long* key0 = reinterpret_cast<unsigned long long*>(scratch + keep_bytes + idx_bytes);
     unsigned long long* key1 = key0 + (sort ? n : 0);
     uint32_t* hist = reinterpret_cast<uint32_t*>(scratch + keep_bytes + idx_bytes + key_bytes);
-    uint32_t* part = hist + (size_t)kDigits * grid;
-    uint32_t* d_total = part + grid + 1;
+    uint32_t* part = hist + (size_t)kDigits * hgrid;
+    uint32_t* d_total = part + pgrid1 + 1;
     uint32_t* d_mm = d_total + 1;
     uint32_t* dtot = d_mm + 2 * (size_t)cols;
-    cudaError_t e = cudaMemcpyAsync(d_keep, keep_cols, (size_t)n_keep * 4, cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return done(ctx->cuda_fail(e, "post-pattern columns"));
+    cudaError_t e = cudaSuccess;
     const uint32_t* idx = nullptr;   // null: rows in table order
     const uint32_t* table_src = in->d;   // the rows idx refers to (the sorted copy after a sort)
     uint64_t m = n;
+    // the columns up to the last required one order and tell apart all that is output
+    int cmp = 0;
+    for (int k = 0; k < n_keep; ++k) cmp = std::max(cmp, keep_cols[k] + 1);
     bool in_order = false;
-    if (sort) {   // a table already in the sort's order keeps it (d_total is free until the scan)
-        unsigned h_flag = 1;
-        if ((e = cudaMemsetAsync(d_total, 0, 4, s)) == cudaSuccess) {
-            const uint32_t tile_rows = (uint32_t)(kCheckWords / cols - 1);   // cols <= 32: >= 255 rows
-            const int cgrid = (int)std::max<uint64_t>(
-                1, std::min<uint64_t>((uint64_t)ctx->sm_count * 6, ((uint64_t)n - 1 + tile_rows - 1) / tile_rows));
-            rows_sorted_kernel<<<cgrid, kFinThreads, 0, s>>>(in->d, cols, n, tile_rows, d_total);
+    std::vector<uint32_t> mm(2 * (size_t)cols);
+    if (sort) {   // a table already in the sort's order keeps it; else each column's range, in signed order
+        const uint32_t max_rows = (uint32_t)(kCheckWords / cols - 1);   // cols <= 32: >= 255 rows
+        const uint64_t ctas = (uint64_t)ctx->sm_count * 6, turns = (n - 1 + ctas * max_rows - 1) / (ctas * max_rows);
+        const uint32_t tile_rows = (uint32_t)std::max<uint64_t>(255, (n - 1 + ctas * turns - 1) / (ctas * turns));
+        const int cgrid = (int)std::min<uint64_t>(ctas, ((uint64_t)n - 1 + tile_rows - 1) / tile_rows);
+        // (d_total is free until the scan: the order check's word, with the ranges behind it)
+        if ((e = cudaMemsetAsync(d_total, 0xFF, (1 + mm.size()) * 4, s)) == cudaSuccess) {
+            scan_rows_kernel<<<cgrid, kFinThreads, 0, s>>>(in->d, cols, cmp, n, tile_rows, d_total, d_mm);
             e = cudaGetLastError();
         }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&h_flag, d_total, 4, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(ctx->h_small, d_total, (1 + mm.size()) * 4, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return done(ctx->cuda_fail(e, "order check"));
-        in_order = h_flag == 0;
+        in_order = ctx->h_small[0] != 0;
+        for (int c = 0; c < cols; ++c) {
+            mm[2 * c] = ctx->h_small[1 + 2 * c];
+            mm[2 * c + 1] = ~ctx->h_small[2 + 2 * c];
+        }
+        int bits = 0;
+        for (int c = 0; c < cmp; ++c)
+            if (mm[2 * c] < mm[2 * c + 1]) bits += 32 - __builtin_clz(mm[2 * c + 1] - mm[2 * c]);
+        // one key per row holds all that matters of it (bits > 0: rows equal in these columns are in order)
+        if (!in_order && bits <= 64 && n_keep <= 32) {
+            ChunkDesc cd{};
+            KeyCols kc{};
+            kc.n = n_keep;
+            std::vector<int> shift_of(cmp, 0), bits_of(cmp, 0);
+            int left = bits;
+            for (int c = 0; c < cmp; ++c) {
+                if (mm[2 * c] >= mm[2 * c + 1]) continue;   // constant: orders nothing
+                bits_of[c] = 32 - __builtin_clz(mm[2 * c + 1] - mm[2 * c]);
+                left -= bits_of[c];
+                shift_of[c] = left;
+                cd.ccol[cd.nc] = c;
+                cd.cbits[cd.nc] = bits_of[c];
+                cd.cmin[cd.nc++] = mm[2 * c];
+            }
+            for (int k = 0; k < n_keep; ++k) {
+                const int c = keep_cols[k];
+                kc.shift[k] = shift_of[c];
+                kc.bits[k] = bits_of[c];
+                kc.lowest[k] = mm[2 * c];
+                if (bits_of[c]) kc.mask |= (unsigned long long)(0xFFFFFFFFu >> (32 - bits_of[c])) << shift_of[c];
+            }
+            unsigned long long *ka = key0, *kb = key1;
+            for (int shift = 0; shift < bits; shift += 8) {
+                SortPass p{ka, nullptr, kb, nullptr, shift, n, cta_tiles * kScatterTile, hist, dtot};
+                if (shift == 0)
+                    key_hist_kernel<<<kgrid1, kFinThreads, 0, s>>>(in->d, cols, cd, p, ka);
+                else
+                    hist_kernel<<<kgrid1, kFinThreads, 0, s>>>(p);
+                digit_rows_kernel<<<kDigits, kFinThreads, 0, s>>>(hist, (uint32_t)kgrid1, dtot);
+                scatter_kernel<false><<<kgrid1, kFinThreads, 0, s>>>(p);
+                std::swap(ka, kb);
+            }
+            // whole rounds of key_write_kernel for each CTA, and one wave of CTAs
+            const uint32_t rounds = (uint32_t)(((uint64_t)n + 1023) / 1024);
+            const uint32_t cta_rounds = (rounds + ctx->sm_count * 8 - 1) / (ctx->sm_count * 8);
+            const int ugrid = (int)((rounds + cta_rounds - 1) / cta_rounds);
+            KeyRuns u{ka, n, cta_rounds * 1024, part};
+            key_count_kernel<<<ugrid, kFinThreads, 0, s>>>(u, kc);
+            scan_kernel<<<1, 1024, 0, s>>>(part, (uint32_t)ugrid, d_total);
+            // written right away where the room that `out` has turns out to be enough
+            auto write = [&] {
+                key_write_kernel<<<ugrid, kFinThreads, 0, s>>>(u, kc, d_total, (uint64_t)offset, limit, out->d,
+                                                               out->cap, out->d_rows);
+                return cudaGetLastError();
+            };
+            out->written();
+            if ((e = write()) != cudaSuccess) return done(ctx->cuda_fail(e, "distinct launches"));
+            if ((e = cudaMemcpyAsync(ctx->h_small, d_total, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+                (e = cudaStreamSynchronize(s)) != cudaSuccess)
+                return done(ctx->cuda_fail(e, "distinct count"));
+            m = ctx->h_small[0];
+            const uint64_t start = std::min<uint64_t>((uint64_t)offset, m);
+            const uint64_t count = limit < 0 ? m - start : std::min<uint64_t>((uint64_t)limit, m - start);
+            if (!out->d || count * n_keep > out->cap) {
+                const int rc = ctx->table_reserve(out, std::max<uint64_t>(count * n_keep, 1));
+                if (rc) return done(rc);
+                if ((e = write()) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
+                    return done(ctx->cuda_fail(e, "distinct rows"));
+            }
+            out->cols = n_keep;
+            out->rows = count;
+            out->rows_known = true;
+            return WK_SUCCESS;
+        }
     }
+    e = cudaMemcpyAsync(d_keep, keep_cols, (size_t)n_keep * 4, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return done(ctx->cuda_fail(e, "post-pattern columns"));
     if (sort) {
         const uint32_t* sorted = nullptr;   // the sorted row order (null: the table's own)
         if (!in_order) {
-            // each column's range, in signed order
-            std::vector<uint32_t> mm(2 * (size_t)cols);
-            for (int c = 0; c < cols; ++c) {
-                mm[2 * c] = 0xFFFFFFFFu;
-                mm[2 * c + 1] = 0;
-            }
-            if ((e = cudaMemcpyAsync(d_mm, mm.data(), mm.size() * 4, cudaMemcpyHostToDevice, s)) != cudaSuccess)
-                return done(ctx->cuda_fail(e, "column ranges"));
-            int mgrid = std::max(1, std::min(ctx->sm_count * 8, (int)(((uint64_t)n * cols + 255) / 256)));
-            if (mgrid >= cols) mgrid -= mgrid % cols;   // stride a multiple of cols: one column per thread
-            minmax_kernel<<<mgrid, kFinThreads, 0, s>>>(in->d, (uint64_t)n * cols, cols, d_mm);
-            if ((e = cudaGetLastError()) != cudaSuccess ||
-                (e = cudaMemcpyAsync(mm.data(), d_mm, mm.size() * 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-                (e = cudaStreamSynchronize(s)) != cudaSuccess)
-                return done(ctx->cuda_fail(e, "column ranges"));
             // chunks of columns, last column first; a constant column orders nothing and is left out
             std::vector<ChunkDesc> chunks;
             std::vector<int> chunk_bits;
@@ -632,7 +862,7 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
                 cur = ChunkDesc{};
                 cur_bits = 0;
             };
-            for (int c = cols - 1; c >= 0; --c) {
+            for (int c = cmp - 1; c >= 0; --c) {
                 const uint32_t lo = mm[2 * c], hi = mm[2 * c + 1];
                 if (lo >= hi) continue;
                 const int b = 32 - __builtin_clz(hi - lo);
@@ -652,19 +882,15 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
             for (size_t k = 0; k < chunks.size(); ++k) {
                 key_kernel<<<kgrid, kFinThreads, 0, s>>>(in->d, cols, chunks[k], sorted, n, ka, ia);
                 for (int shift = 0; shift < chunk_bits[k]; shift += 8) {
-                    SortPass p{ka, ia, kb, ib, shift, n, hist, dtot};
+                    SortPass p{ka, ia, kb, ib, shift, n, (uint32_t)(((uint64_t)n + grid - 1) / grid), hist, dtot};
                     hist_kernel<<<grid, kFinThreads, 0, s>>>(p);
                     digit_rows_kernel<<<kDigits, kFinThreads, 0, s>>>(hist, (uint32_t)grid, dtot);
-                    scatter_kernel<<<grid, kFinThreads, 0, s>>>(p);
+                    scatter_kernel<true><<<grid, kFinThreads, 0, s>>>(p);
                     std::swap(ka, kb);
                     std::swap(ia, ib);
                 }
                 sorted = ia;
                 std::swap(ia, ib);   // the next chunk's keys go to the other index array
-            }
-            if (!sorted) {   // every column constant: every row is equal, the table order stands
-                iota_kernel<<<kgrid, kFinThreads, 0, s>>>(idx0, n);
-                sorted = idx0;
             }
         }
         uint32_t* kept = sorted == idx0 ? idx1 : idx0;

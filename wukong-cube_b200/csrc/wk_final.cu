@@ -18,6 +18,7 @@
 
 #include "wk_ctx.h"
 #include "wk_device.cuh"
+#include "wk_radix.cuh"
 
 namespace wk {
 namespace {
@@ -30,7 +31,7 @@ using namespace dev;
     } while (0)
 
 constexpr int kFinThreads = 256;
-constexpr int kDigits = 256;
+constexpr int kDigits = radix::kDigits;
 
 // ---------------------------------------------------------------- DISTINCT sort
 // The sort orders rows by their columns as signed 32-bit values.  A column is first mapped
@@ -156,7 +157,7 @@ struct SortPass {
     uint32_t* hist;          // [kDigits][grid]: digit-major, so one scan gives the offsets
     uint32_t* dtot;          // [kDigits]: elements of each digit
 };
-static_assert(kFinThreads == kDigits, "the counting passes give each digit one thread");
+static_assert(kFinThreads == radix::kThreads);
 
 __device__ __forceinline__ void chunk(uint32_t n, uint32_t* lo, uint32_t* hi) {
     const uint32_t c = (n + gridDim.x - 1) / gridDim.x;
@@ -211,141 +212,20 @@ __global__ void __launch_bounds__(1024) scan_kernel(uint32_t* v, uint32_t n, uin
     if (threadIdx.x == 0 && total) *total = (uint32_t)s_carry;
 }
 
-// Offsets of a counting pass: digit d of CTA b starts at the elements of smaller digits plus the
-// digit-d elements of CTAs before b.  CTA d of this launch scans digit d's row of hist (one
-// contiguous row of `grid` words, digit-major) in place into exclusive offsets within the digit,
-// with coalesced loads, and writes the digit's total to dtot[d]; each scatter CTA then adds the
-// elements of smaller digits (an exclusive scan of dtot) itself.
-__global__ void __launch_bounds__(kFinThreads) digit_rows_kernel(uint32_t* hist, uint32_t grid, uint32_t* dtot) {
-    __shared__ uint64_t s_warp[kFinThreads / 32];
-    __shared__ uint64_t s_carry;
-    uint32_t* row = hist + (size_t)blockIdx.x * grid;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    constexpr uint32_t kPer = 4;   // a row of a full grid in one round
-    for (uint32_t b0 = 0; b0 < grid; b0 += kPer * kFinThreads) {
-        const uint32_t b = b0 + kPer * threadIdx.x;
-        uint32_t x[kPer], sum = 0;
-#pragma unroll
-        for (uint32_t j = 0; j < kPer; ++j) x[j] = b + j < grid ? row[b + j] : 0;
-#pragma unroll
-        for (uint32_t j = 0; j < kPer; ++j) sum += x[j];
-        const uint64_t ex = block_exclusive_sum<kFinThreads>(sum, s_warp);
-        const uint64_t carry = s_carry;
-        uint32_t at = (uint32_t)(carry + ex);
-#pragma unroll
-        for (uint32_t j = 0; j < kPer; ++j) {
-            if (b + j < grid) row[b + j] = at;
-            at += x[j];
-        }
-        __syncthreads();
-        if (threadIdx.x == kFinThreads - 1) s_carry = carry + ex + sum;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) dtot[blockIdx.x] = (uint32_t)s_carry;
-}
-
-// Stable scatter of 2,048-element tiles: warp w of the CTA takes elements [w * 256, w * 256 + 256)
-// of the tile in 8 rounds of 32 consecutive ones, so the warp's rounds follow the elements'
-// order.  Within a round, an element's rank among the lanes with its digit comes from a mask per
-// digit in shared memory, into which the lanes set their bits (a match takes time with the number of
-// different digits, 32 us a pass of eight bits where one with a third of the digits took 17; eight
-// ballots were bound by their own pipe at 24), and the warp's running count of each digit (updated
-// by one lane per digit) gives its place in the warp; one barrier then turns the warps' counts into
-// per-warp digit offsets.  The tile is placed in shared memory sorted by digit (stable), and then
-// written out in that order, consecutive threads on consecutive elements, so each digit's run goes
-// to global memory in contiguous, coalesced stores.  With the row indices: 4 CTAs per SM (64
-// registers, no spills; 43 KB of shared memory each), so the pass's 4 CTAs per SM run in one wave.
-// Keys alone: 5 CTAs per SM, each over whole tiles.  Bound by the shared-memory chain within a tile
-// and its barriers at this number of warps: 35 us a pass with the indices and the match, 22 with
-// keys alone and the masks, at 3,000,000 rows.
-constexpr int kScatterPer = 8;                                // elements per thread per tile
-constexpr int kScatterTile = kFinThreads * kScatterPer;       // 2,048
-
+// The scatter of a pass (radix_scatter).  With the row indices: 4 CTAs per SM (64 registers, no
+// spills; 43 KB of shared memory each), so the pass's 4 CTAs per SM run in one wave.  Keys alone:
+// 5 CTAs per SM, each over whole tiles.
 template <bool kIdx>
 __global__ void __launch_bounds__(kFinThreads, kIdx ? 4 : 5) scatter_kernel(const SortPass a) {
-    constexpr int kWarps = kFinThreads / 32;
-    __shared__ uint32_t s_cnt[kWarps][kDigits];
-    __shared__ uint32_t s_peers[kWarps][kDigits];
-    __shared__ uint32_t s_off[kDigits];
-    __shared__ unsigned long long s_key[kScatterTile];
-    __shared__ uint32_t s_idx[kIdx ? kScatterTile : 1];
-    __shared__ uint64_t s_warp[kWarps];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ radix::Tile<kIdx> s_tile;
     // thread d: digit d's first place for this CTA = the elements of smaller digits plus the
     // digit-d elements of the CTAs before this one
-    const uint32_t smaller = (uint32_t)block_exclusive_sum<kFinThreads>(a.dtot[threadIdx.x], s_warp);
-    uint32_t run = smaller + a.hist[threadIdx.x * gridDim.x + blockIdx.x];
+    const uint32_t smaller = (uint32_t)block_exclusive_sum<kFinThreads>(a.dtot[threadIdx.x], s_tile.warp);
+    const uint32_t first = smaller + a.hist[threadIdx.x * gridDim.x + blockIdx.x];
     uint32_t lo, hi;
     span(a, &lo, &hi);
-    for (int w = 0; w < kWarps; ++w) s_peers[w][threadIdx.x] = 0;
-    for (uint64_t base = lo; base < hi; base += kScatterTile) {
-        for (int w = 0; w < kWarps; ++w) s_cnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        unsigned long long key[kScatterPer];
-        [[maybe_unused]] uint32_t row[kScatterPer];
-        uint32_t dg[kScatterPer], at[kScatterPer];
-        const uint64_t wbase = base + (uint32_t)warp * (32 * kScatterPer);
-#pragma unroll
-        for (int r = 0; r < kScatterPer; ++r) {
-            const uint64_t i = wbase + r * 32 + lane;
-            const bool live = i < hi;
-            key[r] = live ? a.key_in[i] : 0;
-            if constexpr (kIdx) row[r] = live ? a.idx_in[i] : 0;
-            dg[r] = live ? (uint32_t)(key[r] >> a.shift) & 0xFFu : (uint32_t)kDigits;
-        }
-#pragma unroll
-        for (int r = 0; r < kScatterPer; ++r) {
-            const bool live = dg[r] < kDigits;
-            if (live) atomicOr(&s_peers[warp][dg[r]], 1u << lane);
-            __syncwarp();
-            const unsigned peers = live ? s_peers[warp][dg[r]] : 0;   // the lanes with this lane's digit
-            const int rank = __popc(peers & ((1u << lane) - 1));
-            at[r] = live ? s_cnt[warp][dg[r]] + rank : 0;
-            __syncwarp();
-            if (live && rank == 0) {
-                s_cnt[warp][dg[r]] += __popc(peers);
-                s_peers[warp][dg[r]] = 0;
-            }
-            __syncwarp();
-        }
-        __syncthreads();
-        uint32_t cnt[kWarps], tile_cnt = 0;   // per digit (thread = digit): prefix over the warps
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) cnt[w] = s_cnt[w][threadIdx.x];
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) tile_cnt += cnt[w];
-        // the tile sorted by digit in shared memory: digit d's elements start at tbase, warp w's
-        // at s_cnt[w][d]; s_off[d] takes a place in the tile to its place in the output
-        const uint32_t tbase = (uint32_t)block_exclusive_sum<kFinThreads>(tile_cnt, s_warp);
-        s_off[threadIdx.x] = run - tbase;
-        run += tile_cnt;
-        uint32_t wat = tbase;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            s_cnt[w][threadIdx.x] = wat;
-            wat += cnt[w];
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kScatterPer; ++r) {
-            if (dg[r] >= kDigits) continue;
-            const uint32_t lp = s_cnt[warp][dg[r]] + at[r];
-            s_key[lp] = key[r];
-            if constexpr (kIdx) s_idx[lp] = row[r];
-        }
-        __syncthreads();
-        // consecutive threads write consecutive elements: each digit's run goes out contiguous
-        const uint32_t m = (uint32_t)min((uint64_t)kScatterTile, hi - base);
-        for (uint32_t j = threadIdx.x; j < m; j += kFinThreads) {
-            const unsigned long long k = s_key[j];
-            const uint32_t d = (uint32_t)(k >> a.shift) & 0xFFu;
-            const uint32_t pos = s_off[d] + j;
-            a.key_out[pos] = k;
-            if constexpr (kIdx) a.idx_out[pos] = s_idx[j];
-        }
-        __syncthreads();
-    }
+    radix::radix_scatter<kIdx>(s_tile, a.key_in, a.idx_in, a.key_out, a.idx_out, lo, hi, first,
+                        [&](unsigned long long k, uint32_t) { return (uint32_t)(k >> a.shift) & 0xFFu; });
 }
 
 // ---- one chunk holds all the columns looked at: keys alone
@@ -658,7 +538,7 @@ cudaError_t final_kernel_attrs() {
     if (e == cudaSuccess) e = use_max_shared_carveout(key_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(hist_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(scan_kernel);
-    if (e == cudaSuccess) e = use_max_shared_carveout(digit_rows_kernel);
+    if (e == cudaSuccess) e = use_max_shared_carveout(radix::digit_rows_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(scatter_kernel<true>);
     if (e == cudaSuccess) e = use_max_shared_carveout(scatter_kernel<false>);
     if (e == cudaSuccess) e = use_max_shared_carveout(key_hist_kernel);
@@ -710,10 +590,8 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
     const int grid = std::max(1, std::min<int>(ctx->sm_count * 4, (int)((n + 2047) / 2048)));
     // the passes over keys alone: whole tiles for each CTA, and one wave of CTAs (a part
     // that ends within a tile leaves the rest of the CTA idle in it)
-    const uint32_t tiles = (uint32_t)(((uint64_t)n + kScatterTile - 1) / kScatterTile);
-    const uint32_t cta_tiles = (tiles + ctx->sm_count * 5 - 1) / (ctx->sm_count * 5);
-    const int kgrid1 = (int)((tiles + cta_tiles - 1) / cta_tiles);
-    const int hgrid = std::max(grid, kgrid1);        // the histogram's rows
+    const radix::Split ksplit = radix::split(n, (uint64_t)ctx->sm_count * 5);
+    const int hgrid = std::max(grid, ksplit.grid);        // the histogram's rows
     const int pgrid1 = std::max(grid, ctx->sm_count * 8);   // the CTA counts
     // scratch: the required columns, two index arrays, two key arrays (DISTINCT only), the
     // digit histogram, the CTA counts and the distinct total, the column ranges, the digit totals
@@ -799,13 +677,13 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
             }
             unsigned long long *ka = key0, *kb = key1;
             for (int shift = 0; shift < bits; shift += 8) {
-                SortPass p{ka, nullptr, kb, nullptr, shift, n, cta_tiles * kScatterTile, hist, dtot};
+                SortPass p{ka, nullptr, kb, nullptr, shift, n, ksplit.per_cta, hist, dtot};
                 if (shift == 0)
-                    key_hist_kernel<<<kgrid1, kFinThreads, 0, s>>>(in->d, cols, cd, p, ka);
+                    key_hist_kernel<<<ksplit.grid, kFinThreads, 0, s>>>(in->d, cols, cd, p, ka);
                 else
-                    hist_kernel<<<kgrid1, kFinThreads, 0, s>>>(p);
-                digit_rows_kernel<<<kDigits, kFinThreads, 0, s>>>(hist, (uint32_t)kgrid1, dtot);
-                scatter_kernel<false><<<kgrid1, kFinThreads, 0, s>>>(p);
+                    hist_kernel<<<ksplit.grid, kFinThreads, 0, s>>>(p);
+                radix::digit_rows_kernel<<<kDigits, kFinThreads, 0, s>>>(hist, (uint32_t)ksplit.grid, dtot);
+                scatter_kernel<false><<<ksplit.grid, kFinThreads, 0, s>>>(p);
                 std::swap(ka, kb);
             }
             // whole rounds of key_write_kernel for each CTA, and one wave of CTAs
@@ -884,7 +762,7 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
                 for (int shift = 0; shift < chunk_bits[k]; shift += 8) {
                     SortPass p{ka, ia, kb, ib, shift, n, (uint32_t)(((uint64_t)n + grid - 1) / grid), hist, dtot};
                     hist_kernel<<<grid, kFinThreads, 0, s>>>(p);
-                    digit_rows_kernel<<<kDigits, kFinThreads, 0, s>>>(hist, (uint32_t)grid, dtot);
+                    radix::digit_rows_kernel<<<kDigits, kFinThreads, 0, s>>>(hist, (uint32_t)grid, dtot);
                     scatter_kernel<true><<<grid, kFinThreads, 0, s>>>(p);
                     std::swap(ka, kb);
                     std::swap(ia, ib);

@@ -31,13 +31,15 @@
 
 #include "wk_ctx.h"
 #include "wk_device.cuh"
+#include "wk_radix.cuh"
 
 namespace wk {
 namespace {
 using namespace dev;
 
 constexpr int kT = 256;       // threads per CTA of every build kernel
-constexpr int kDigits = 256;  // 8-bit radix digits
+constexpr int kDigits = radix::kDigits;
+static_assert(kT == radix::kThreads);
 
 __device__ __forceinline__ void span_of(uint64_t n, uint64_t* lo, uint64_t* hi) {
     const uint64_t c = (n + gridDim.x - 1) / gridDim.x;
@@ -125,13 +127,19 @@ struct Pass {
     unsigned long long* k_out;
     uint32_t* v_out;
     uint64_t n;
+    uint64_t per_cta;   // items of a CTA
     int shift;
     int from_value;
     uint32_t* hist;   // [kDigits][grid], digit-major; then each digit's total [kDigits]
 };
 
-__device__ __forceinline__ uint32_t digit(const Pass& a, uint64_t i) {
-    return a.from_value ? (a.v_in[i] >> a.shift) & 0xFFu : (uint32_t)(a.k_in[i] >> a.shift) & 0xFFu;
+__device__ __forceinline__ uint32_t digit(const Pass& a, unsigned long long k, uint32_t v) {
+    return a.from_value ? (v >> a.shift) & 0xFFu : (uint32_t)(k >> a.shift) & 0xFFu;
+}
+
+__device__ __forceinline__ void span_of(const Pass& a, uint64_t* lo, uint64_t* hi) {
+    *lo = min(a.n, (uint64_t)blockIdx.x * a.per_cta);
+    *hi = min(a.n, *lo + a.per_cta);
 }
 
 __global__ void __launch_bounds__(kT) hist_kernel(const Pass a) {
@@ -139,12 +147,15 @@ __global__ void __launch_bounds__(kT) hist_kernel(const Pass a) {
     s_h[threadIdx.x] = 0;
     __syncthreads();
     uint64_t lo, hi;
-    span_of(a.n, &lo, &hi);
+    span_of(a, &lo, &hi);
     constexpr int kU = 8;   // digits loaded together, then counted
     for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += kU * kT) {
         uint32_t d[kU];
 #pragma unroll
-        for (int u = 0; u < kU; ++u) d[u] = i0 + u * kT < hi ? digit(a, i0 + u * kT) : 0xFFFFFFFFu;
+        for (int u = 0; u < kU; ++u) {
+            const uint64_t i = i0 + u * kT;
+            d[u] = i >= hi ? kDigits : a.from_value ? digit(a, 0, a.v_in[i]) : digit(a, a.k_in[i], 0);
+        }
 #pragma unroll
         for (int u = 0; u < kU; ++u)
             if (d[u] < kDigits) atomicAdd(&s_h[d[u]], 1u);
@@ -171,68 +182,17 @@ __global__ void __launch_bounds__(1024) scan32_kernel(uint32_t* v, uint32_t n) {
     }
 }
 
-// One CTA per digit scans that digit's row of the histogram (one word per CTA of the pass) in place
-// and leaves the digit's total behind the rows; the scatter CTAs add the smaller digits' totals
-// themselves (4.9 us; one CTA over all the rows took 224 us, three quarters of a pass at 6e6 items).
-__global__ void __launch_bounds__(kT) digit_rows_kernel(uint32_t* hist, uint32_t grid) {
-    __shared__ uint64_t s_warp[kT / 32];
-    __shared__ uint64_t s_carry;
-    uint32_t* row = hist + (size_t)blockIdx.x * grid;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
-    for (uint32_t b0 = 0; b0 < grid; b0 += kT) {
-        const uint32_t b = b0 + threadIdx.x;
-        const uint64_t x = b < grid ? row[b] : 0;
-        const uint64_t ex = block_exclusive_sum<kT>(x, s_warp);
-        const uint64_t carry = s_carry;
-        if (b < grid) row[b] = (uint32_t)(carry + ex);
-        __syncthreads();
-        if (threadIdx.x == kT - 1) s_carry = carry + ex + x;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) hist[(size_t)kDigits * grid + blockIdx.x] = (uint32_t)s_carry;
-}
-
-__global__ void __launch_bounds__(kT) scatter_kernel(const Pass a) {
-    __shared__ uint64_t s_warp[kT / 32];
-    __shared__ uint32_t s_run[kDigits];
-    __shared__ uint32_t s_cnt[kT / 32][kDigits];
-    __shared__ uint32_t s_tile[kDigits];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    static_assert(kT == kDigits, "one thread per digit");
-    s_run[threadIdx.x] = a.hist[threadIdx.x * gridDim.x + blockIdx.x] +
-                         (uint32_t)block_exclusive_sum<kT>(a.hist[(size_t)kDigits * gridDim.x + threadIdx.x], s_warp);
+// With the values: 4 CTAs per SM (41 KB of shared memory each).  Tiles of 256 items written from
+// their own threads, with a match per item, took 72 us a pass over 6e6 items; staged ones take 48.
+__global__ void __launch_bounds__(kT, 4) scatter_kernel(const Pass a) {
+    __shared__ radix::Tile<true> s_tile;
+    const uint32_t smaller =
+        (uint32_t)block_exclusive_sum<kT>(a.hist[(size_t)kDigits * gridDim.x + threadIdx.x], s_tile.warp);
     uint64_t lo, hi;
-    span_of(a.n, &lo, &hi);
-    for (uint64_t base = lo; base < hi; base += kT) {
-        for (int w = 0; w < kT / 32; ++w) s_cnt[w][threadIdx.x] = 0;
-        __syncthreads();
-        const uint64_t i = base + threadIdx.x;
-        const bool live = i < hi;
-        const uint32_t dg = live ? digit(a, i) : kDigits + lane;   // lone sentinel
-        const unsigned peers = __match_any_sync(0xffffffffu, dg);
-        const int rank = __popc(peers & ((1u << lane) - 1));
-        if (live && rank == 0) s_cnt[warp][dg] = __popc(peers);
-        __syncthreads();
-        {
-            uint32_t acc = 0;
-            for (int w = 0; w < kT / 32; ++w) {
-                const uint32_t c = s_cnt[w][threadIdx.x];
-                s_cnt[w][threadIdx.x] = acc;
-                acc += c;
-            }
-            s_tile[threadIdx.x] = acc;
-        }
-        __syncthreads();
-        if (live) {
-            const uint32_t at = s_run[dg] + s_cnt[warp][dg] + rank;
-            a.k_out[at] = a.k_in[i];
-            a.v_out[at] = a.v_in[i];
-        }
-        __syncthreads();
-        s_run[threadIdx.x] += s_tile[threadIdx.x];
-        __syncthreads();
-    }
+    span_of(a, &lo, &hi);
+    radix::radix_scatter<true>(s_tile, a.k_in, a.v_in, a.k_out, a.v_out, lo, hi,
+                               smaller + a.hist[threadIdx.x * gridDim.x + blockIdx.x],
+                               [&](unsigned long long k, uint32_t v) { return digit(a, k, v); });
 }
 
 // ---------------------------------------------------------------- compaction
@@ -500,7 +460,7 @@ cudaError_t gbuild_kernel_attrs() {
     if (e == cudaSuccess) e = use_max_shared_carveout(hist_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(scatter_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(scan32_kernel);
-    if (e == cudaSuccess) e = use_max_shared_carveout(digit_rows_kernel);
+    if (e == cudaSuccess) e = use_max_shared_carveout(radix::digit_rows_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(compact_count_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(compact_place_kernel);
     if (e == cudaSuccess) e = use_max_shared_carveout(values_kernel);
@@ -640,14 +600,15 @@ struct Builder {
              int vbits, uint32_t* hist, int* where) {
         *where = 0;
         if (n < 2) return WK_SUCCESS;
-        const int grid = grid_for(n);
+        const wk::radix::Split sp = wk::radix::split(n, (uint64_t)sm * 4);
         unsigned long long *ka = k, *kb = k2;
         uint32_t *va = v, *vb = v2;
         auto pass = [&](int shift, int from_value) {
-            wk::Pass p{ka, va, kb, vb, n, shift, from_value, hist};
-            wk::hist_kernel<<<grid, wk::kT, 0, s>>>(p);
-            wk::digit_rows_kernel<<<wk::kDigits, wk::kT, 0, s>>>(hist, (uint32_t)grid);
-            wk::scatter_kernel<<<grid, wk::kT, 0, s>>>(p);
+            wk::Pass p{ka, va, kb, vb, n, sp.per_cta, shift, from_value, hist};
+            wk::hist_kernel<<<sp.grid, wk::kT, 0, s>>>(p);
+            wk::radix::digit_rows_kernel<<<wk::kDigits, wk::kT, 0, s>>>(hist, (uint32_t)sp.grid,
+                                                                        hist + (size_t)wk::kDigits * sp.grid);
+            wk::scatter_kernel<<<sp.grid, wk::kT, 0, s>>>(p);
             std::swap(ka, kb);
             std::swap(va, vb);
             *where ^= 1;

@@ -27,7 +27,8 @@ CU_SOURCES = ["wk_kernels.cu", "wk_explore.cu", "wk_batch.cu", "wk_serve.cu", "w
               "wk_final.cu", "wk_versatile.cu", "wk_gbuild.cu", "wk_dir.cu", "wk_pipe.cu", "wk_level.cu"]
 CPP_SOURCES = ["wk_ctx.cpp", "wk_gstore.cpp", "wk_synth.cpp", "wk_tune.cpp", "wk_loader.cpp"]
 HEADERS = ["wk_format.h", "wk_internal.h", "wk_kernels.h", "wk_ctx.h", "wk_batch.h",
-           "wk_device.cuh", "wk_explore.h", "wk_flat.h", "wk_versatile.h", "wk_dir.h", "wk_pipe.h", "wk_level.h"]
+           "wk_device.cuh", "wk_explore.h", "wk_flat.h", "wk_versatile.h", "wk_dir.h", "wk_pipe.h", "wk_level.h",
+           "wk_radix.cuh"]
 
 
 def _run(cmd):

@@ -10,15 +10,17 @@
 //
 // One launch per pass: CTAs claim chunks of consecutive rows (two per CTA on a large input) from a
 // device counter.  A chunk's warps first count: each runs free over its own rows, 32 at a time, one
-// per lane and kPipeRows per thread with their lookups in flight together.  Then one decoupled
+// per lane and two or four per thread with their lookups in flight together.  Then one decoupled
 // look-back gives the chunk its output position, and the warps write, through shared memory so that
 // stores are coalesced whatever the row width.  A chunk of up to four rounds (1.2 M rows on 148 SMs)
-// keeps what it counted, as far as the columns it appends fit; a larger one runs its surviving rows again from L2, which is cheaper than
-// the alternatives measured: a look-back per round put every warp behind the slowest of a wave
-// (triangle at 10,000 organisations: 288 us against 190), and positions kept in memory (count,
-// place and expand launches per step, the form before) cost 32 bytes a row and step (390 us).
-// What bounds it now: issue (about 90 instructions a row and step) and the latency of the lookups;
-// DRAM runs at a fifth of its rate.
+// keeps what it counted, as far as the columns it appends fit; a larger one runs its surviving rows
+// again from L2, which is cheaper than the alternatives measured: a look-back per round put every
+// warp behind the slowest of a wave (triangle at 10,000 organisations: 288 us against 190), and
+// positions kept in memory (count, place and expand launches per step, the form before) cost 32
+// bytes a row and step (390 us).  What bounds it: issue and the latency of the lookups; DRAM runs at
+// a fifth of its rate.  Every lane of a round loads, a lost row's from the first place of the array
+// it reads: a branch per lookup was 43 branches and 368 instructions per 32 rows of the triangle's
+// three steps, 204 us; without them 152, and 119 with four rows per thread.
 // Rows come out row-major, then in list order, as the CPU engine appends them (sparql.hpp:328-370).
 // A row whose list is longer than the slice threshold goes to the slice queue that idle CTAs drain,
 // so a hub vertex is spread over the device.
@@ -42,17 +44,22 @@ using namespace dev;
 constexpr int kPipeThreads = 256;
 constexpr int kPipeWarps = kPipeThreads / 32;
 // Rows per thread in flight x CTAs per SM (registers), kernel us of the star at 1,000 organisations /
-// the star over a Zipf graph of 3,001 / the triangle at 10,000 / 1 M rows expanded / 2.5 M rows
-// filtered: 2 x 4 (64) 31/77/190/96/122; 4 x 4 37/84/201/99/114; 4 x 3 (80) 34/79/279/101/114;
-// 2 x 5 (48) 38/90/199/99/124; 1 x 6 (40) 49/93/207/111/129; 1 x 8 (32) 54/100/329/132/266.
-constexpr int kPipeRows = 2;           // rows per thread in flight: a round is 32 * kPipeRows per warp
+// the star over a Zipf graph of 3,001 / 1 M rows expanded, which end with a last step, and the
+// triangle at 10,000 / 2.5 M rows filtered, which do not: 2 x 4 (64) 32/64/84, 152/120; 3 x 4 33/61/95,
+// 133/122; 4 x 4 43/90/118, 118/122; 4 x 3 (80) 29/60/93, 208/114; 2 x 5 (48) 36/106/116, 158/131;
+// 2 x 3 32/72/92, 285/119; 1 x 6 (40) 39/104/163, 354/148.  A last step's lists take the registers,
+// and so do a table's columns, whose loads hold a filter either way.
+template <bool kLast, bool kList>
+constexpr int kPipeRows = !kLast && kList ? 4 : 2;   // rows per thread: a round is 32 times that per warp
 constexpr int kMaxGroups = kPipeMaxTileRows / kPipeThreads;   // 32-row groups of a warp's chunk
-constexpr int kMaxRounds = kMaxGroups / kPipeRows;
 constexpr int kPipeCtas = 4;           // CTAs per SM: 64 registers a thread
 constexpr int kStageWords = 512;       // output words staged per warp
 constexpr int kKeepRounds = 4;         // rounds of a chunk whose counted lists are kept for writing
-constexpr int kHeldSlots = 12;         // words per thread for held columns (columns x rows x rounds)
-static_assert(kHeldSlots >= (kMaxPipeCols + 1) * kPipeRows, "one round's columns are always held");
+template <bool kLast>
+constexpr int kHeldSlots = kLast ? 12 : 16;   // words a thread holds: columns x rows x rounds
+static_assert(kHeldSlots<true> >= (kMaxPipeCols + 1) * kPipeRows<true, true> &&
+                  kHeldSlots<false> >= (kMaxPipeCols + 1) * kPipeRows<false, true>,
+              "one round's columns are always held");
 constexpr uint32_t kLaneList = 16;     // a warp with no longer list writes a row's outputs by its lane
 constexpr uint32_t kWarpList = 256;    // a warp with a longer list than this writes row by row
 
@@ -83,6 +90,7 @@ static_assert(sizeof(StepRow) == 48, "StepRow is three 16-byte words");
 template <bool kList>
 struct Rows {
     const uint32_t* src;    // a table: row 0 (row k is 32 * k rows on)
+    const uint32_t* safe;   // its first row, read in the place of a row that is not there
     int w_in;               // columns read from src (0 for a list)
     uint32_t* held;         // held column j of row k: held[j * stride + k * kPipeThreads]
     int stride;
@@ -91,6 +99,11 @@ struct Rows {
     }
     __device__ __forceinline__ uint32_t col(int k, int c) const {
         return kList || c >= w_in ? at(k, c) : __ldg(src + 32 * k * w_in + c);
+    }
+    // the same, of a row that is there only if `live` (else any word)
+    __device__ __forceinline__ uint32_t col_if(bool live, int k, int c) const {
+        if (kList || c >= w_in) return at(k, c);
+        return __ldg((live ? src + 32 * k * w_in : safe) + c);
     }
     // the same of lane `of`
     __device__ __forceinline__ uint32_t col_of(int k, int c, int of) const {
@@ -108,16 +121,19 @@ __device__ __forceinline__ uint64_t slow_word(const PipeArgs& a, const PipeOp& o
     const uint64_t key = o.type_index ? make_key(0, cur, kIn) : make_key(cur, o.pid, o.dir);
     return sg.num_buckets && key ? thread_probe(a.store, key, bucket_of(key, sg), &a.ctl->err) : 0;
 }
+template <int K>
 struct SlowWords {
-    uint64_t p[kPipeRows];
+    uint64_t p[K];
 };
+template <int K>
 struct SlowIds {
-    uint32_t id[kPipeRows];
+    uint32_t id[K];
 };
-__device__ __noinline__ SlowWords slow_words(const PipeArgs& a, const PipeOp& o, SlowIds cur, unsigned live) {
-    SlowWords w;
+template <int K>
+__device__ __noinline__ SlowWords<K> slow_words(const PipeArgs& a, const PipeOp& o, SlowIds<K> cur, unsigned live) {
+    SlowWords<K> w;
 #pragma unroll
-    for (int k = 0; k < kPipeRows; ++k) w.p[k] = live >> k & 1 ? slow_word(a, o, cur.id[k]) : 0;
+    for (int k = 0; k < K; ++k) w.p[k] = live >> k & 1 ? slow_word(a, o, cur.id[k]) : 0;
     return w;
 }
 
@@ -140,85 +156,123 @@ __device__ __forceinline__ OneList one_list(const PipeArgs& a, const SegDesc& sg
 
 // found[k]: target[k] in the list edges[off, off + deg) of the rows in `look`, short lists by quads
 // as thread_member does, every row's quad in flight together.
-__device__ __forceinline__ void pipe_member(const PipeArgs& a, const uint64_t (&off)[kPipeRows],
-                                            const uint32_t (&deg)[kPipeRows], const uint32_t (&target)[kPipeRows],
-                                            const bool (&look)[kPipeRows], bool (&found)[kPipeRows]) {
-    constexpr int K = kPipeRows;
-    bool more = false, quads[K];
+template <int K>
+__device__ __forceinline__ void pipe_member(const PipeArgs& a, const uint64_t (&off)[K],
+                                            const uint32_t (&deg)[K], const uint32_t (&target)[K],
+                                            const bool (&look)[K], bool (&found)[K]) {
+    bool more = false, slow = false, quads[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
         quads[k] = look[k] && deg[k] <= kQuadList && !(off[k] & kInlineTag);
-        found[k] = false;
-        if (look[k] && !quads[k])
-            found[k] = thread_member(a.store.edges, off[k], deg[k], target[k], a.sorted_lists != 0);
+        found[k] = look[k] && (off[k] & kInlineTag) && (uint32_t)off[k] == target[k];
+        slow |= look[k] && !quads[k] && !(off[k] & kInlineTag);
         more |= quads[k];
+    }
+    if (slow) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (look[k] && !quads[k] && !(off[k] & kInlineTag))
+                found[k] = thread_member(a.store.edges, off[k], deg[k], target[k], a.sorted_lists != 0);
     }
     for (int q = 0; more; q += 4) {
         uint4 x[K];
         more = false;
-#pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (quads[k]) x[k] = __ldg(reinterpret_cast<const uint4*>(a.store.edges) + (off[k] >> 2) + (q >> 2));
+        const uint4* e4 = reinterpret_cast<const uint4*>(a.store.edges) + (q >> 2);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            if (!quads[k]) continue;
+            // (a row without a quad here reads the first one: the array is padded)
+            const uint4* p = reinterpret_cast<const uint4*>(a.store.edges);
+            if (quads[k]) p = e4 + (off[k] >> 2);
+            x[k] = __ldg(p);
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
             const int lo = (int)(off[k] & 3), hi = lo + (int)deg[k];
             const uint32_t t = target[k];
-            found[k] = (x[k].x == t && q >= lo) || (x[k].y == t && q + 1 >= lo && q + 1 < hi) ||
-                       (x[k].z == t && q + 2 >= lo && q + 2 < hi) || (x[k].w == t && q + 3 >= lo && q + 3 < hi);
-            quads[k] = !found[k] && q + 4 < hi;
+            const bool here = quads[k] & (((x[k].x == t) & (q >= lo)) | ((x[k].y == t) & (q + 1 >= lo) & (q + 1 < hi)) |
+                                          ((x[k].z == t) & (q + 2 >= lo) & (q + 2 < hi)) |
+                                          ((x[k].w == t) & (q + 3 >= lo) & (q + 3 < hi)));
+            found[k] |= here;
+            quads[k] = quads[k] & !here & (q + 4 < hi);
             more |= quads[k];
         }
     }
 }
 
+// Directory lookup of a round: has[k] stays where cur[k] has a key, and at[k] is then the place of its
+// word (0 elsewhere, so that every lane may load).  Every lane loads: a load per lane that needs one
+// was a branch each, 43 a row group in the triangle and a third of its instructions.
+template <int K>
+__device__ __forceinline__ void dir_places(const StepRow& s, const uint32_t (&cur)[K],
+                                           bool (&has)[K], uint32_t (&at)[K]) {
+    const uint2* dir = s.dir;
+    const uint32_t lo = s.vid_lo, span = s.vid_span;
+    uint2 b[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const uint32_t id = cur[k] - lo;
+        has[k] = has[k] & (id < span);
+        b[k] = __ldg(dir + (has[k] ? id >> 5 : 0u));
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const uint32_t id = cur[k] - lo;
+        has[k] = has[k] & dir_has(b[k], id);
+        at[k] = has[k] ? dir_place(b[k], id) : 0u;
+    }
+}
+
 // Lists of cur[k] in the step's segment for the live rows (deg 0 elsewhere).
+template <int K>
 __device__ __forceinline__ void pipe_lists(const PipeArgs& a, const StepRow& s, const PipeOp& o,
-                                           const uint32_t (&cur)[kPipeRows], const bool (&live)[kPipeRows],
-                                           uint64_t (&off)[kPipeRows], uint32_t (&deg)[kPipeRows]) {
-    constexpr int K = kPipeRows;
+                                           const uint32_t (&cur)[K], const bool (&live)[K],
+                                           uint64_t (&off)[K], uint32_t (&deg)[K]) {
     uint64_t p[K];
     bool zero = false;
 #pragma unroll
     for (int k = 0; k < K; ++k) zero |= live[k] && cur[k] == 0;
     if (s.how <= kHowWord && !zero) {
-        uint2 b[K];
-        const uint2* dir = s.dir;
-        const uint32_t lo = s.vid_lo, span = s.vid_span;
+        uint32_t at[K];
+        bool has[K];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const uint32_t id = cur[k] - lo;
-            b[k] = make_uint2(0, 0);
-            if (live[k] && id < span) b[k] = __ldg(dir + (id >> 5));
-        }
-        const bool values = s.how == kHowValue;
+        for (int k = 0; k < K; ++k) has[k] = live[k];
+        dir_places(s, cur, has, at);
+        if (s.how == kHowValue) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const uint32_t id = cur[k] - lo;
-            p[k] = 0;
-            if (!dir_has(b[k], id)) continue;
-            const uint32_t at = dir_place(b[k], id);
-            p[k] = values ? make_inline_ptr(__ldg(static_cast<const uint32_t*>(s.words) + at))
-                          : __ldg(static_cast<const unsigned long long*>(s.words) + at);
+            for (int k = 0; k < K; ++k) {
+                const uint64_t e = make_inline_ptr(__ldg(static_cast<const uint32_t*>(s.words) + at[k]));
+                p[k] = has[k] ? e : 0;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const uint64_t e = __ldg(static_cast<const unsigned long long*>(s.words) + at[k]);
+                p[k] = has[k] ? e : 0;
+            }
         }
     } else {
         unsigned m = 0;
-        SlowIds ids;
+        SlowIds<K> ids;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             m |= (unsigned)live[k] << k;
             ids.id[k] = cur[k];
         }
-        const SlowWords w = slow_words(a, o, ids, m);
+        const SlowWords<K> w = slow_words<K>(a, o, ids, m);
 #pragma unroll
         for (int k = 0; k < K; ++k) p[k] = w.p[k];
     }
+    bool corrupt = false;   // (list_of_ptr, without its branches)
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        uint64_t d;
-        list_of_ptr(p[k], a.store.n_edges, &a.ctl->err, &off[k], &d);
-        deg[k] = (uint32_t)d;
+        const bool one = ptr_is_inline(p[k]);
+        deg[k] = (uint32_t)ptr_size(p[k]);
+        off[k] = one ? kInlineTag | (uint32_t)(p[k] >> kNbitsSize) : ptr_off(p[k]);
+        const bool bad = !one & (off[k] + deg[k] > a.store.n_edges);
+        corrupt |= bad & (deg[k] != 0);
+        if (bad) deg[k] = 0;
     }
+    if (corrupt) atomicOr(&a.ctl->err, kErrCorrupt);
 }
 
 // Bytes and list entries the steps run one launch each would account for (StepCtl), of a thread's
@@ -229,10 +283,9 @@ struct Acc {
 
 // The steps of the pass over a round; `live` keeps the rows that survive.  Without `test`: rows known
 // to survive, of which only the appended columns are wanted.
-template <bool kList>
+template <bool kList, int K>
 __device__ __forceinline__ void pipe_ops(const PipeArgs& a, const StepRow* steps, const Rows<kList>& v,
-                                         bool (&live)[kPipeRows], bool test, Acc* acc) {
-    constexpr int K = kPipeRows;
+                                         bool (&live)[K], bool test, Acc* acc) {
     int w = a.w_in;   // columns of a row at this step
 #pragma unroll 1
     for (int i = 0; i < a.n_ops; ++i) {
@@ -242,8 +295,8 @@ __device__ __forceinline__ void pipe_ops(const PipeArgs& a, const StepRow* steps
         uint32_t cur[K], n_in = 0, sd = 0;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            cur[k] = kBlankId;
-            if (live[k]) cur[k] = v.col(k, s.col);
+            const uint32_t x = v.col_if(live[k], k, s.col);
+            cur[k] = live[k] ? x : kBlankId;
         }
         bool zero = false;
 #pragma unroll
@@ -254,39 +307,25 @@ __device__ __forceinline__ void pipe_ops(const PipeArgs& a, const StepRow* steps
         }
         if (how == kHowValue && !zero) {
             // every list has one entry and the directory holds it (a blank id is outside it)
-            const uint2* dir = s.dir;
-            const uint32_t lo = s.vid_lo, span = s.vid_span;
-            uint2 b[K];
-            uint32_t e[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const uint32_t id = cur[k] - lo;
-                live[k] = live[k] && id < span;
-                if (live[k]) b[k] = __ldg(dir + (id >> 5));
-            }
+            uint32_t at[K], e[K];
+            dir_places(s, cur, live, at);
             const uint32_t* words = static_cast<const uint32_t*>(s.words);
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const uint32_t id = cur[k] - lo;
-                live[k] = live[k] && dir_has(b[k], id);
-                if (live[k]) e[k] = __ldg(words + dir_place(b[k], id));
-            }
+            for (int k = 0; k < K; ++k) e[k] = __ldg(words + at[k]);
             if (acc) {
 #pragma unroll
                 for (int k = 0; k < K; ++k) sd += live[k];
             }
             if (op == kXK2U) {
 #pragma unroll
-                for (int k = 0; k < K; ++k)
-                    if (live[k]) v.at(k, w) = e[k];
+                for (int k = 0; k < K; ++k) v.at(k, w) = e[k];   // (a lost row's word is not read)
             } else if (op == kXK2K) {
 #pragma unroll
-                for (int k = 0; k < K; ++k)
-                    if (live[k]) live[k] = e[k] == v.col(k, s.tcol);
+                for (int k = 0; k < K; ++k) live[k] = live[k] & (e[k] == v.col_if(live[k], k, s.tcol));
             } else {
                 const uint32_t target = s.end_const;
 #pragma unroll
-                for (int k = 0; k < K; ++k) live[k] = live[k] && e[k] == target;
+                for (int k = 0; k < K; ++k) live[k] = live[k] & (e[k] == target);
             }
         } else {
             uint64_t off[K];
@@ -319,7 +358,7 @@ __device__ __forceinline__ void pipe_ops(const PipeArgs& a, const StepRow* steps
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
                     target[k] = how == kHowOne ? cur[k] : s.end_const;
-                    if (op == kXK2K && live[k]) target[k] = v.col(k, s.tcol);
+                    if (op == kXK2K) target[k] = v.col_if(live[k], k, s.tcol);
                 }
                 pipe_member(a, off, deg, target, live, found);
 #pragma unroll
@@ -339,16 +378,15 @@ __device__ __forceinline__ void pipe_ops(const PipeArgs& a, const StepRow* steps
 }
 
 // Count and list of the last step for a round.
-template <bool kList>
+template <bool kList, int K>
 __device__ __forceinline__ void pipe_last(const PipeArgs& a, const StepRow& s, const Rows<kList>& v,
-                                          bool (&live)[kPipeRows], int w, uint32_t (&cnt)[kPipeRows],
-                                          uint64_t (&off)[kPipeRows], Acc* acc) {
-    constexpr int K = kPipeRows;
+                                          bool (&live)[K], int w, uint32_t (&cnt)[K],
+                                          uint64_t (&off)[K], Acc* acc) {
     uint32_t cur[K];
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        cur[k] = kBlankId;
-        if (live[k]) cur[k] = v.col(k, s.col);
+        const uint32_t x = v.col_if(live[k], k, s.col);
+        cur[k] = live[k] ? x : kBlankId;
         live[k] = live[k] && cur[k] != kBlankId && !(a.last.type_index && cur[k] >= (1u << kNbitsIdx));
     }
     pipe_lists(a, s, a.last, cur, live, off, cnt);
@@ -374,7 +412,7 @@ __device__ __forceinline__ void flush_words(uint32_t* dst, const uint32_t* s, ui
 // list.
 template <bool kLast, bool kList>
 __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __grid_constant__ PipeArgs a) {
-    constexpr int K = kPipeRows;
+    constexpr int K = kPipeRows<kLast, kList>, kMaxRounds = kMaxGroups / K;
     extern __shared__ __align__(16) unsigned char smem[];   // pipe_smem_bytes
     // the lists of the kept rounds and their counts, then positions (a last step)
     uint64_t* const s_off = reinterpret_cast<uint64_t*>(smem);
@@ -473,9 +511,10 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __g
 
     Rows<kList> v;
     v.w_in = kList ? 0 : a.w_in;
+    v.safe = in;
     // small chunks keep what they count; the rows of a larger one are run again to be written
     const int held_cols = w_row - v.w_in;
-    const bool keep = rounds <= (kLast ? kKeepRounds : kMaxRounds) && held_cols * K * rounds <= kHeldSlots;
+    const bool keep = rounds <= (kLast ? kKeepRounds : kMaxRounds) && held_cols * K * rounds <= kHeldSlots<kLast>;
     v.stride = (keep ? rounds : 1) * K * kPipeThreads;
     bool live[K];
     uint32_t done = 0;   // chunks this CTA has written
@@ -538,7 +577,11 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __g
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
                     live[k] = k < n_groups && (mask >> k & 1) && r0 + 32 * k < R;
-                    if (kList && live[k]) v.at(k, 0) = in ? __ldg(v.src + 32 * k) : only;
+                    if (kList) {
+                        uint32_t x = only;
+                        if (in) x = __ldg(live[k] ? v.src + 32 * k : in);
+                        v.at(k, 0) = x;
+                    }
                 }
                 // (rows known to survive: only their appended columns are wanted)
                 if (kLast || count || w_row > a.w_in)
@@ -775,8 +818,8 @@ PipeKernel pipe_kernel_of(int k) {
 }  // namespace
 
 static size_t pipe_smem_bytes(bool last) {
-    return (last ? kKeepRounds * kPipeRows * kPipeThreads * 12 : 0) + kPipeWarps * kStageWords * 4 +
-           kHeldSlots * kPipeThreads * 4;
+    return (last ? kKeepRounds * kPipeRows<true, false> * kPipeThreads * 12 : 0) + kPipeWarps * kStageWords * 4 +
+           (last ? kHeldSlots<true> : kHeldSlots<false>) * kPipeThreads * 4;
 }
 static bool kernel_has_last(int k) { return k >= 2; }
 

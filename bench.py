@@ -44,20 +44,18 @@ import numpy as np  # noqa: E402
 METRIC = "light-query QPS at p99 latency; heavy-query ms; vs plain per-query GPU path"
 
 # DRAM bytes (read + write) per input row of the dominant batch level, from one ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum, one pass) of level 3 of a replay of the
-# 16,384-query batch on the 1,000-organisation graph: 103,307,264 B + 18,270,720 B for
-# 2,617,493 input rows, with the knobs the autotuner picks (one thread per row, 32-row slices,
-# flat passes for levels 0 and 1).  Scaled by the dominant level's input rows; on the larger
-# graph fewer sectors hit in L2, so the scaled figure is a lower bound there.
-LEVEL_TRAFFIC_PER_ROW = (103307264 + 18270720) / 2617493
-# DRAM bytes (read + write) per input row of the heavy triangle's flat steps, from one ncu
-# capture (dram__bytes_read.sum + dram__bytes_write.sum, one pass) of its launches on the
-# 2,000-organisation graph (4.2 GB store, 1,821,743 input rows per step), the count launch plus
-# place and expand: the known_to_known step (degreeFrom) and the one-to-one known_to_unknown step
-# (memberOf).  Scaled by the dominant heavy step's input rows.
+# (dram__bytes_read.sum + dram__bytes_write.sum) of the third fused level of a 16,384-query batch
+# on the 2,000-organisation graph: 37,519,400 B + 2,610,688 B for 1,405,738 input rows.  Scaled by
+# the dominant level's input rows; on the larger graph fewer sectors hit in L2, so the scaled
+# figure is a lower bound there.
+LEVEL_TRAFFIC_PER_ROW = (37519400 + 2610688) / 1405738
+# DRAM bytes (read + write) per input row of the heavy triangle's steps run one per launch, from
+# one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) on the 2,000-organisation graph
+# (4.2 GB store, 1,806,383 input rows per step): the known_to_known step (degreeFrom) and the
+# one-to-one known_to_unknown step (memberOf).  Scaled by the dominant heavy step's input rows.
 HEAVY_TRAFFIC_PER_ROW = {
-    "known_to_known": (221116672 + 3919872 + 7783168) / 1821743,
-    "known_to_unknown": (207086336 + 8665088 + 11008 + 23040) / 1821743,
+    "known_to_known": (31024640 + 512) / 1806383,
+    "known_to_unknown": (16579072 + 2304) / 1806383,
 }
 
 
@@ -576,8 +574,9 @@ def run_ours(args, world, rank, local_rank):
         return max(s["distinct_keys"] / rr_peak, s["alg_bytes"] / (peak * 1e9))
 
     def random_roofline(s):
-        return {"bound": "one random read per distinct probed key at the measured random-read "
-                         "rate, or the algorithmic bytes at the copy bandwidth, whichever is longer",
+        return {"bound": "hash probes: one random read per distinct probed key at the measured random-read "
+                         "rate, or the algorithmic bytes at the copy bandwidth, whichever is longer "
+                         "(lookups by vertex directory share lines between keys and may pass it)",
                 "distinct_keys": s["distinct_keys"], "peak_reads_per_s": rr_peak,
                 "peak_bytes_per_s": peak * 1e9, "bound_ms": bound_s(s) * 1000.0,
                 "kernel_ms": s["ms"], "frac": bound_s(s) / (s["ms"] / 1000.0)}
@@ -588,7 +587,8 @@ def run_ours(args, world, rank, local_rank):
         h["frac_of_bound"] = h["bound_ms"] / sum(s["ms"] for s in h["profile"])
     flat_mask = tune.get("batch_flat", 0)
     dom_k = levels.index(dom)
-    dom_kernel = ("flat passes (batch level %d)" if (flat_mask >> dom_k) & 1
+    dom_kernel = ("level_kernel (fused batch level %d)" if not flat_mask else
+                  "flat passes (batch level %d)" if (flat_mask >> dom_k) & 1
                   else "explore_kernel (batch level %d)") % dom_k
 
     lat = sorted(step_ms)
@@ -617,8 +617,8 @@ def run_ours(args, world, rank, local_rank):
                          "frac": achieved / peak, "traffic": LEVEL_TRAFFIC_PER_ROW * dom["rows_in"],
                          "traffic_rate": dram_rate(LEVEL_TRAFFIC_PER_ROW * dom["rows_in"], dom["ms"], peak),
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of "
-                                           "batch level 3 on the 1,000-organisation graph (1 pass; "
-                                           "46.4 B per input row) x this launch's input rows",
+                                           "the third fused level on the 2,000-organisation graph "
+                                           "(28.5 B per input row) x this launch's input rows",
                          "peak_source": src,
                          "kernel": dom_kernel,
                          "algorithmic_bytes": dom["alg_bytes"], "kernel_ms": dom["ms"],
@@ -634,11 +634,10 @@ def run_ours(args, world, rank, local_rank):
                                                           hdom["ms"], peak)
                                                 if hdom["kind"] in HEAVY_TRAFFIC_PER_ROW else None),
                                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of "
-                                                 "the triangle's flat launches on the 2,000-organisation "
+                                                 "the triangle's steps on the 2,000-organisation "
                                                  "graph (1 pass; B per input row of this step's kind) x "
                                                  "this step's input rows",
-                               "kernel": "single-query " + hdom["kind"] + " step (tile launch or "
-                                         "flat pipeline, whichever the device picked)",
+                               "kernel": "pipe_kernel (single-query " + hdom["kind"] + " step, one per launch)",
                                "algorithmic_bytes": hdom["alg_bytes"], "kernel_ms": hdom["ms"],
                                "random_reads": random_roofline(hdom)},
             "random_read_peak": {"value": rr_peak, "unit": "reads/s",
@@ -648,8 +647,8 @@ def run_ours(args, world, rank, local_rank):
             "batch_other_ms": overheads,
             "autotune": tune,
             "serving": serving,
-            # per batch: one launch per level (three where the level runs the flat passes),
-            # result scan, gather
+            # per batch: one launch per level (three where the level runs the flat passes; fused
+            # levels are fewer than the patterns), result scan, gather
             "gpu_launches": args.steps * (sum(3 if (tune.get("batch_flat", 0) >> k) & 1 else 1
                                               for k in range(len(levels))) + 2),
             "clocks": clk.summary()}

@@ -453,12 +453,14 @@ int wk_debug_device_allocs(uint64_t* count);
  *           CTA (block-per-row) instead of by the CTA that probed it (group-per-row); 8 to
  *           2^23, default 128;
  *   knob 3: the same for batches and serving;
- *   knob 4: single-query steps of index-start plans (and single steps) whose input has at
- *           least this many rows run as the flat count / scan / expand pipeline instead of the
- *           tile launch; 0 never does (default 65,536);
- *   knob 5: a mask over batch levels; level k runs as the flat passes when bit k is set (one
- *           thread per row, full occupancy, output rows split evenly over the grid) and as
- *           the tile launch otherwise (default 0: all tile launches);
+ *   knob 4: single steps whose input has at least this many rows run as a fused pass instead of
+ *           the tile launch; whole plans run as fused passes (a run of steps per launch) unless it
+ *           is 0, which never does (default 65,536);
+ *   knob 5: a mask over batch levels; with a bit set, a batch runs one level per pattern, level k
+ *           as the flat passes when bit k is set (one thread per row, full occupancy, output rows
+ *           split evenly over the grid) and as the tile launch otherwise.  0 (the default) runs
+ *           fused levels, each query's steps up to the next one that multiplies rows, on a store
+ *           with vertex directories, and tile launches on one without;
  *   knob 6: polls a bounded device-side wait on another CTA (a tile's look-back, a CTA waiting
  *           for the long-list slice queue) makes before it gives up and the call returns
  *           WK_E_TIMEOUT; 0 restores the default (2^24).  A few polls make the waits run out,

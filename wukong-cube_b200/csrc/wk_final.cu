@@ -699,6 +699,10 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
                                                                out->cap, out->d_rows);
                 return cudaGetLastError();
             };
+            if (!out->d || !out->d_rows) {   // (a table that an earlier call could not grow)
+                const int rc = ctx->table_reserve(out, 1);
+                if (rc) return done(rc);
+            }
             out->written();
             if ((e = write()) != cudaSuccess) return done(ctx->cuda_fail(e, "distinct launches"));
             if ((e = cudaMemcpyAsync(ctx->h_small, d_total, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
@@ -707,7 +711,7 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
             m = ctx->h_small[0];
             const uint64_t start = std::min<uint64_t>((uint64_t)offset, m);
             const uint64_t count = limit < 0 ? m - start : std::min<uint64_t>((uint64_t)limit, m - start);
-            if (!out->d || count * n_keep > out->cap) {
+            if (count * n_keep > out->cap) {
                 const int rc = ctx->table_reserve(out, std::max<uint64_t>(count * n_keep, 1));
                 if (rc) return done(rc);
                 if ((e = write()) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)

@@ -3,10 +3,12 @@
 // gpu_hash.cu:96-326).
 //
 // Knobs (wk_ctx_tune_set): lanes per probe group (1 / 2 / 4 / 8 lanes: one thread per row
-// reading the home sector, or a group reading 32 / 64 / 128 bytes of a bucket per request) and the slice threshold (lists longer than it are written
-// block-per-row as slices by every CTA, shorter ones group-per-row by the CTA that probed them),
-// and for batches the mask of levels that run as the flat passes instead of the tile launch
-// (chosen greedily level by level after the tile settings).
+// reading the home sector, or a group reading 32 / 64 / 128 bytes of a bucket per request) and the
+// slice threshold (lists longer than it are written block-per-row as slices by every CTA, shorter
+// ones group-per-row by the CTA that probed them),
+// and for batches the mask of levels that run as the flat passes (chosen greedily level by level
+// after the settings without a mask: fused levels on a store with vertex directories, which leave
+// the lanes aside, tile launches on one without).
 // Constant-start queries are timed as one batch replayed from its CUDA graph (CUDA events on
 // the context stream); index-start queries step by step through wk_query_profile, so lanes are
 // chosen per (step kind, input columns).  Everything goes through the public entry points, so
@@ -147,7 +149,7 @@ extern "C" int wk_ctx_autotune(wk_ctx* ctx, const wk_query* queries, uint32_t n,
         if ((rc = time_batch(ctx, light, iters, s, ev, &best))) return rc;
         out->batch_ms_default = best;
         int bl = out->batch_lanes, bs = out->batch_slice_rows, bf = 0;
-        // every tile setting (all levels on the tile launch) ...
+        // every setting without a mask ...
         if ((rc = wk_ctx_tune_set(ctx, WK_KNOB_BATCH_FLAT, 0))) return rc;
         best = 1e30;
         for (int l : kLanes)

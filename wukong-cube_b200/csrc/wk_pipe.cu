@@ -54,6 +54,20 @@ constexpr int kPipeRows = !kLast && kList ? 4 : 2;   // rows per thread: a round
 constexpr int kMaxGroups = kPipeMaxTileRows / kPipeThreads;   // 32-row groups of a warp's chunk
 constexpr int kPipeCtas = 4;           // CTAs per SM: 64 registers a thread
 constexpr int kStageWords = 512;       // output words staged per warp
+constexpr int kMaxTableCols = 32;      // columns of the widest table (wk_config::max_cols)
+// Output rows of `cols` words staged at once where they are spread over the lanes: one to four for
+// each lane, or, for rows so wide that the stage holds fewer than 32 (from 17 columns on), as many as
+// it holds.  Never none: the loop over a warp's output rows advances by it.
+__host__ __device__ constexpr uint32_t spread_rows(int cols) {
+    const uint32_t fit = (uint32_t)(kStageWords / cols);
+    return fit >= 128 ? 128 : fit >= 32 ? fit & ~31u : fit;
+}
+constexpr bool spread_ends() {
+    for (int c = 1; c <= kMaxTableCols; ++c)
+        if (spread_rows(c) < 1 || spread_rows(c) * c > (uint32_t)kStageWords) return false;
+    return true;
+}
+static_assert(spread_ends(), "the stage holds a row of any table");
 constexpr int kKeepRounds = 4;         // rounds of a chunk whose counted lists are kept for writing
 template <bool kLast>
 constexpr int kHeldSlots = kLast ? 12 : 16;   // words a thread holds: columns x rows x rounds
@@ -697,7 +711,7 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __g
                     n += __shfl_sync(kFull, st, 31);
                 }
                 __syncwarp();
-                const uint32_t fit = min(kStageWords / wo / 32, 4) * 32;   // output rows staged at once
+                const uint32_t fit = spread_rows(wo);   // output rows staged at once
                 for (uint32_t c0 = 0; c0 < n; c0 += fit) {
                     const uint32_t c1 = min(n, c0 + fit);
                     int row[4];

@@ -975,7 +975,9 @@ static int build_directories(wk_ctx* ctx, const std::vector<wk::SegScan>& of_seg
         const uint64_t n = sums[b1 / wk::kDirScanBlocks] - sums[ds[k].block0 / wk::kDirScanBlocks];
         at[k + 1] = at[k] + (n * (ds[k].seg.dir_values ? 4 : 8) + 15) / 16 * 16;
     }
-    if (wk::dev_malloc(&words, std::max<uint64_t>(at.back(), 16)) != cudaSuccess) {
+    // (a lookup that finds no key still loads its segment's first word, so one lies behind the last
+    // segment too: its keys may all have empty lists, which are no keys to a step)
+    if (wk::dev_malloc(&words, at.back() + 16) != cudaSuccess) {
         cudaGetLastError();
         return drop(WK_SUCCESS);
     }

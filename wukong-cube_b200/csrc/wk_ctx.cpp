@@ -201,6 +201,9 @@ void wk_ctx::drop_store(bool spare) {
     n_slots = n_edges = n_inline = 0;
     n_pseg = 0;
     has_dir = no_fuse = false;
+    segs.clear();
+    index = wk::SegIndex{};
+    index_ptr.clear();
     seg_desc.clear();
     seg_longest.clear();
 }
@@ -1696,6 +1699,9 @@ extern "C" int wk_query_enqueue(wk_ctx* ctx, const wk_query* q, int32_t mode) {
         if (!steps.empty()) final_table(ctx, query_passes(ctx, steps))->cols = steps.back().out_cols;
         return WK_SUCCESS;
     }
+    // (after a load that failed there is nothing to look up, and what is left of the tables of the
+    // store before must not reach a launch)
+    if (!steps.empty() && !ctx->has_store) return ctx->fail(WK_E_NOSTORE, "no store uploaded");
     return enqueue_plan(ctx, steps, query_passes(ctx, steps), *q);
 }
 

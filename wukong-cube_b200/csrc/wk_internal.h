@@ -41,8 +41,8 @@ struct SegIndex {
     int32_t find(uint64_t vid, uint32_t pid, int dir) const {
         if (dir < 0 || dir > 1) return -1;
         if (vid == 0) return index_seg[dir];
-        if (pid >= (1u << kNbitsIdx)) return -1;
-        return normal[(size_t)pid * 2 + dir];
+        const size_t i = (size_t)pid * 2 + dir;
+        return i < normal.size() ? normal[i] : -1;   // (empty before build)
     }
 };
 

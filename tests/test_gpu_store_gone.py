@@ -48,3 +48,31 @@ def test_enqueue_before_any_store(stores):
     q = workloads.heavy_star(stores["v"])
     with wk.Context(0) as ctx:
         assert wk.lib().wk_query_enqueue(ctx.h, q.as_c(), wk.MODE_RESIDENT) == wk.E_NOSTORE
+
+
+def test_batch_replay(stores):
+    """The last batch's graph launches on the store and the scratch of its time: not once they are gone."""
+    v, o = stores["v"], stores["o"]
+    inst = {t: stores["g"].get_index(t, wk.IN) for t in range(v["t_org"], v["t_doc"] + 1)}
+    qs = workloads.light_queries(v, inst, 50, seed=2)
+    with wk.Context(0) as ctx:
+        ctx.upload_gstore(stores["g"])
+        ctx.batch_device(qs)
+        ctx.batch_replay()
+        ctx.check()
+        ctx.upload_gstore(stores["g"])
+        assert wk.lib().wk_batch_replay(ctx.h) == wk.E_BADARG
+        for q, (t, st) in zip(qs, ctx.batch(qs)):
+            assert st == 0 and np.array_equal(oracle.sorted_rows(t), oracle.sorted_rows(o.run(q.flat(), q.nvars)[1]))
+        ctx.batch_replay()
+        ctx.check()
+        big = ctx.table(np.full((1 << 22, 1), 1 << 17, np.uint32), capacity=1 << 23)   # more tiles than the scratch has words
+        out = ctx.table(capacity=1 << 27)                                              # and more slices
+        ctx.known_to_const(big, 0, 1 << 17, v["p_takes"], wk.OUT, out)
+        ctx.known_to_unknown(big, 0, v["p_takes"], wk.OUT, out)
+        rc = wk.lib().wk_batch_replay(ctx.h)
+        assert rc == wk.E_BADARG
+        ctx.check()
+        big.free(), out.free()
+        _lose_store(ctx, stores)
+        assert wk.lib().wk_batch_replay(ctx.h) == wk.E_BADARG

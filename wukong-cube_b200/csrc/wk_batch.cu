@@ -157,6 +157,8 @@ struct BatchState {
     // graph of the launch sequence for one batch shape
     cudaGraphExec_t exec = nullptr;
     std::string shape;
+    uint64_t store_gen = 0;               // the store and the context's scratch it launches on
+    void *status = nullptr, *heavy = nullptr;
 };
 
 // Places in the plan block of a batch of n queries in L levels: each query's level count and final
@@ -607,6 +609,9 @@ int launch_batch(wk_ctx* ctx, BatchState* b, const Plan& P) {
         cudaGraphDestroy(g);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "batch instantiate");
         b->shape = shape;
+        b->store_gen = ctx->store_gen;
+        b->status = ctx->d_status;
+        b->heavy = ctx->d_heavy;
     }
     WKB_CUDA(ctx, cudaGraphLaunch(b->exec, ctx->stream));
     return WK_SUCCESS;
@@ -851,6 +856,8 @@ extern "C" int wk_batch_replay(wk_ctx* ctx) {
     std::lock_guard<std::mutex> lk(ctx->mu);
     BatchState* b = (BatchState*)ctx->batch;
     if (!b || !b->exec) return ctx->fail(WK_E_BADARG, "no batch has run on this context");
+    if (b->store_gen != ctx->store_gen || b->status != ctx->d_status || b->heavy != ctx->d_heavy)
+        return ctx->fail(WK_E_BADARG, "the store or the scratch that the last batch ran on is gone: run it again");
     WKB_CUDA(ctx, cudaGraphLaunch(b->exec, ctx->stream));
     return WK_SUCCESS;
 }

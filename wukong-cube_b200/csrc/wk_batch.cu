@@ -315,7 +315,7 @@ int build_plan(wk_ctx* ctx, BatchState* b, const wk_query* queries, uint32_t n, 
     const int max_cols = ctx->cfg.max_cols;
     const bool versatile = ctx->versatile;
     // fused levels look vertices up in directories; a store without them keeps a pattern per level
-    P.fused = ctx->has_dir && !ctx->no_fuse && !ctx->batch_flat;
+    P.fused = ctx->has_dir && !ctx->batch_flat;
     int steps_max = 0;
 #pragma omp parallel if (n >= 2048)
     {
@@ -648,7 +648,6 @@ int run_batch(wk_ctx* ctx, BatchState* b, const wk_query* queries, uint32_t n, P
         ctx->clear_ctl_err();
         if (err & wk::kErrCorrupt) return ctx->fail(WK_E_CORRUPT, "key table chain out of range");
         if (err & wk::kErrTimeout) return ctx->fail(WK_E_TIMEOUT, "batch look-back timed out");
-        if (err & wk::kErrUnfuse) ctx->no_fuse = true;   // vid 0 in the store's lists
         uint64_t rows = b->rows_cap, res = b->result_cap;
         if (err & (wk::kErrOverflow | wk::kErrStatus)) rows = std::max<uint64_t>(rows * 2, need + need / 4);
         if (total_elems > res) res = total_elems + total_elems / 4 + 1024;

@@ -200,7 +200,7 @@ void wk_ctx::drop_store(bool spare) {
     d_dir_words = nullptr;
     n_slots = n_edges = n_inline = 0;
     n_pseg = 0;
-    has_dir = no_fuse = false;
+    has_dir = zero_ids = false;
     segs.clear();
     index = wk::SegIndex{};
     index_ptr.clear();
@@ -497,18 +497,22 @@ bool is_filter(const PlanStep& s) {
     return s.kind == PlanStep::kK2K || s.kind == PlanStep::kK2C || s.kind == PlanStep::kC2K ||
            s.kind == PlanStep::kI2K;
 }
-// known_to_unknown whose lists all have at most one entry
+// known_to_unknown whose lists all have at most one entry, the predicate's index list among them
+// where the store's own rows may hold vertex 0
 bool is_functional(const wk_ctx* ctx, const PlanStep& s) {
     if (s.kind != PlanStep::kK2U || (s.pid == kTypeId && s.dir == kIn)) return false;
     const uint32_t id = ctx->seg_id(1, s.pid, s.dir);
-    return id == 0 || ctx->seg_longest[id - 1] <= 1;
+    if (id && ctx->seg_longest[id - 1] > 1) return false;
+    if (!ctx->zero_ids) return true;
+    auto it = ctx->index_ptr.find(s.pid * 2 + (uint32_t)s.dir);
+    return it != ctx->index_ptr.end() && ptr_size(it->second) <= 1;
 }
 
 }  // namespace
 
 bool step_gives_one(const wk_ctx* ctx, const PlanStep& s) { return is_filter(s) || is_functional(ctx, s); }
 
-std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>& steps, bool fuse) {
+std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>& steps) {
     std::vector<PlanPass> out;
     const int n = (int)steps.size();
     for (int i = 0; i < n;) {
@@ -517,18 +521,16 @@ std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>
         int ops = 0, cols = 0;
         bool pipe = false;
         for (; j < n && !is_start(steps[j]) && !is_versatile_step(steps[j].kind); ++j) {
-            const bool func = is_functional(ctx, steps[j]) && fuse;
-            if (is_filter(steps[j]) || func) {
-                if (ops == kMaxPipeOps || (func && cols == kMaxPipeCols)) break;
-                ++ops;
-                cols += func;
+            const bool func = is_functional(ctx, steps[j]);
+            if (!func && !is_filter(steps[j])) {   // a step that multiplies rows ends the pass
                 pipe = true;
-                if (fuse) continue;
-            } else {
-                pipe = true;   // a step that multiplies rows ends the pass
+                ++j;
+                break;
             }
-            ++j;
-            break;
+            if (ops == kMaxPipeOps || (func && cols == kMaxPipeCols)) break;
+            ++ops;
+            cols += func;
+            pipe = true;
         }
         if (!pipe) j = i + 1;
         out.push_back(PlanPass{i, j - i, pipe});
@@ -715,6 +717,7 @@ int wk::ctx_make_child(wk_ctx* parent, const CtaUse& beside_use, int beside_ctas
     ctx->index = parent->index;
     ctx->seg_desc = parent->seg_desc;
     ctx->seg_longest = parent->seg_longest;
+    ctx->zero_ids = parent->zero_ids;
     ctx->index_ptr = parent->index_ptr;
     ctx->d_segs = parent->d_segs;
     ctx->has_dir = parent->has_dir;
@@ -1084,21 +1087,27 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
         }
         ctx->n_inline = found.n_inline;
         e = cudaMemsetAsync(&scan.d->n_inline, 0, sizeof(scan.d->n_inline), s);
-        if (e == cudaSuccess) e = launch_inline(ctx->dev_store(), &scan.d->n_inline, ctx->d_inline_orig, ctx->sm_count, s);
+        if (e == cudaSuccess) e = launch_inline(ctx->dev_store(), scan.d, ctx->d_inline_orig, ctx->sm_count, s);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "one-entry lists");
     }
     std::vector<SegScan> of_seg(n_segs, no_key);
     std::vector<PredSeg> ps(np);   // which segment each entry belongs to
     if (np) WK_CUDA(ctx, cudaMemcpy(ps.data(), ctx->d_pseg, np * sizeof(PredSeg), cudaMemcpyDeviceToHost));
-    for (uint32_t i = 0; i < np; ++i) of_seg[ps[i].seg_no] = hv[i];
+    // (a predicate and direction met in several segments: the scan's findings are at the first entry)
+    for (uint32_t i = 0, first = 0; i < np; ++i) {
+        if (ps[i].key != ps[first].key) first = i;
+        of_seg[ps[i].seg_no] = hv[first];
+    }
     ctx->seg_longest.clear();
     for (auto& x : of_seg) ctx->seg_longest.push_back(x.longest);
     if (!(found.flags & kStoreBadChain)) {
         rc = build_directories(ctx, of_seg, scan.d);
         if (rc) return rc;
     }
-    e = cudaStreamSynchronize(s);
+    e = cudaMemcpyAsync(&found.flags, &scan.d->flags, sizeof(found.flags), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "one-entry lists");
+    ctx->zero_ids = (found.flags & kStoreZeroId) != 0;
     ctx->has_store = true;
     return WK_SUCCESS;
 }
@@ -1474,13 +1483,12 @@ static std::string plan_key(const std::vector<wk::PlanStep>& steps, const wk_que
     put(&ctx->d_flat, sizeof(ctx->d_flat));
     put(&ctx->flat_cap_rows, sizeof(ctx->flat_cap_rows));
     put(&ctx->flat_min_rows, sizeof(ctx->flat_min_rows));
-    put(&ctx->no_fuse, sizeof(ctx->no_fuse));
     return k;
 }
 
 // The launches of a plan run back to back: fused passes, or (knob 4 at 0) one launch per step.
 static std::vector<wk::PlanPass> query_passes(const wk_ctx* ctx, const std::vector<wk::PlanStep>& steps) {
-    if (ctx->flat_min_rows) return wk::plan_passes(ctx, steps, !ctx->no_fuse);
+    if (ctx->flat_min_rows) return wk::plan_passes(ctx, steps);
     std::vector<wk::PlanPass> out;
     for (size_t i = 0; i < steps.size(); ++i) out.push_back(wk::PlanPass{(int)i, 1, false});
     return out;
@@ -1512,7 +1520,7 @@ static int enqueue_plan(wk_ctx* ctx, const std::vector<wk::PlanStep>& steps, con
                         const wk_query& q) {
     for (size_t i = 0; i < passes.size(); ++i) {
         const wk_table* in = i ? &ctx->rbuf[(i - 1) & 1] : nullptr;
-        int rc = wk::enqueue_pass(ctx, steps, passes[i], in, &ctx->rbuf[i & 1], q.mt_tid, q.mt_factor, !ctx->no_fuse,
+        int rc = wk::enqueue_pass(ctx, steps, passes[i], in, &ctx->rbuf[i & 1], q.mt_tid, q.mt_factor, true,
                                   ctx->stream);
         if (rc) return rc;
     }
@@ -1597,7 +1605,6 @@ static int query_run(wk_ctx* ctx, const wk_query* q, int32_t mode, const wk_tabl
             if (rc) return rc;
             if (err & wk::kErrCorrupt) return ctx->fail(WK_E_CORRUPT, "key table chain out of range");
             if (err & wk::kErrTimeout) return ctx->fail(WK_E_TIMEOUT, "tile look-back timed out");
-            if (err & wk::kErrUnfuse) ctx->no_fuse = true;   // vid 0 in the store's lists
             if (err & (wk::kErrOverflow | wk::kErrStatus)) {
                 int wmax = 1;
                 for (auto& s : steps) wmax = std::max(wmax, s.out_cols);
@@ -1767,8 +1774,7 @@ extern "C" int wk_query_profile(wk_ctx* ctx, const wk_query* q, int32_t iters, w
             wk_table* o = &ctx->rbuf[i & 1];
             WK_CUDA(ctx, cudaMemsetAsync(&ctx->d_ctl->sum_deg, 0, 16, ctx->stream));
             WK_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
-            rc = wk::enqueue_pass(ctx, steps, pass_of(i), in, o, q->mt_tid, q->mt_factor, !ctx->no_fuse, ctx->stream,
-                                  true);
+            rc = wk::enqueue_pass(ctx, steps, pass_of(i), in, o, q->mt_tid, q->mt_factor, true, ctx->stream, true);
             if (rc) return rc;
             WK_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
             WK_CUDA(ctx, cudaEventSynchronize(e1));

@@ -96,7 +96,7 @@ struct wk_ctx {
     wk::SegIndex index;
     std::vector<wk::SegDesc> seg_desc;   // of each segment, with its directory
     std::vector<uint32_t> seg_longest;   // entries of each segment's longest list
-    bool no_fuse = false;                // a query met vid 0 in a functional step (kErrUnfuse)
+    bool zero_ids = false;               // a list of the store holds id 0 (see step_gives_one)
     wk::SegDesc* d_segs = nullptr;       // DevStore::segs: an absent segment, then seg_desc
     wk::DirBlock* d_dir_blocks = nullptr;   // vertex directories (wk_dir.cu)
     void* d_dir_words = nullptr;
@@ -267,12 +267,14 @@ struct PlanPass {
     int first, n;
     bool pipe;
 };
-// Whether a step gives each row at most one output row: a filter, or known_to_unknown on a
-// predicate whose lists all have at most one entry.
+// Whether a step of a plan gives each row at most one output row: a filter, or known_to_unknown on a
+// predicate whose lists all have at most one entry.  A row's vertex comes from the store's lists; where
+// one of those holds id 0, which names the predicate's index list, that list counts among them.
 bool step_gives_one(const wk_ctx* ctx, const PlanStep& s);
-// The passes of a plan; `fuse` false: one step each (a start list still joins its first step).
-std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>& steps, bool fuse);
-// Enqueue one pass reading `in` (null when it starts the plan) into `out`.  `fuse` as above;
+// The passes of a plan.
+std::vector<PlanPass> plan_passes(const wk_ctx* ctx, const std::vector<PlanStep>& steps);
+// Enqueue one pass reading `in` (null when it starts the plan) into `out`.  `fuse` false: every
+// known_to_unknown step multiplies rows (a single step over a caller's table with vertex 0 in it);
 // `account`: the steps' bytes and list entries are added to the control block (a profile).
 int enqueue_pass(wk_ctx* ctx, const std::vector<PlanStep>& steps, const PlanPass& p, const wk_table* in, wk_table* out,
                  int32_t mt_tid, int32_t mt_factor, bool fuse, cudaStream_t s, bool account = false);

@@ -130,7 +130,8 @@ store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, SegSc
                     } else if (sz <= kSerialList) {
                         uint32_t prev = 0;
                         const int n = (int)sz;
-                        for (int e0 = 0; n > 1 && e0 < n; e0 += 8) {   // eight entries in flight
+                        // (a one-entry list of the plain type is read when it goes into its slot)
+                        for (int e0 = 0; (n > 1 || sl[u].ptr >> 62) && e0 < n; e0 += 8) {   // eight entries in flight
                             uint32_t x[8];
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
@@ -139,6 +140,7 @@ store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, SegSc
                             for (int j = 0; j < 8; ++j) {
                                 if (e0 + j >= n) continue;
                                 if (e0 + j && prev >= x[j]) flags |= kStoreUnsorted;
+                                if (x[j] == 0) flags |= kStoreZeroId;
                                 prev = x[j];
                             }
                         }
@@ -165,11 +167,15 @@ store_scan_kernel(const DevStore st, const PredSeg* pseg, uint32_t n_pseg, SegSc
                         for (uint32_t c = lane; c < nc && at + c < max_chunks; c += 32)
                             chunks[at + c] = make_ulonglong2(0, 0);
                     }
-                    bool bad = false;
+                    bool bad = false, zero = false;
 #pragma unroll 8
-                    for (uint64_t e = 1 + lane; e < n; e += 32)
-                        bad |= __ldg(st.edges + o + e - 1) >= __ldg(st.edges + o + e);
+                    for (uint64_t e = 1 + lane; e < n; e += 32) {
+                        const uint32_t x = __ldg(st.edges + o + e - 1), y = __ldg(st.edges + o + e);
+                        bad |= x >= y;
+                        zero |= x == 0 || y == 0;
+                    }
                     if (bad) flags |= kStoreUnsorted;
+                    if (zero) flags |= kStoreZeroId;
                 }
             }
         }
@@ -187,14 +193,19 @@ chunk_check_kernel(const uint32_t* edges, const ulonglong2* chunks, uint32_t max
     const uint32_t n = min(out->n_chunks, max_chunks);
     const int lane = threadIdx.x & 31;
     const uint32_t warps = gridDim.x * (kLoadThreads / 32);
-    bool bad = false;
+    bool bad = false, zero = false;
     for (uint32_t i = blockIdx.x * (kLoadThreads / 32) + threadIdx.x / 32; i < n; i += warps) {
         const ulonglong2 c = chunks[i];
         const uint32_t* p = edges + c.x;
 #pragma unroll 8
-        for (uint64_t e = 1 + lane; e < c.y; e += 32) bad |= __ldg(p + e - 1) >= __ldg(p + e);
+        for (uint64_t e = 1 + lane; e < c.y; e += 32) {
+            const uint32_t x = __ldg(p + e - 1), y = __ldg(p + e);
+            bad |= x >= y;
+            zero |= x == 0 || y == 0;
+        }
     }
-    if (__any_sync(kFull, bad) && lane == 0) atomicOr(&out->flags, (unsigned)kStoreUnsorted);
+    const unsigned flags = (__any_sync(kFull, bad) ? kStoreUnsorted : 0u) | (__any_sync(kFull, zero) ? kStoreZeroId : 0u);
+    if (flags && lane == 0) atomicOr(&out->flags, flags);
 }
 
 // One-entry lists into their keys' own pointer words (see kInlinePtrType): for every data slot
@@ -202,9 +213,10 @@ chunk_check_kernel(const uint32_t* edges, const ulonglong2* chunks, uint32_t max
 // `orig` (slot index, pointer word; wk_store_export puts them back) and the slot's pointer word
 // becomes the entry with the inline type.  The places in `orig` are taken a warp at a time.
 __global__ void __launch_bounds__(kLoadThreads)
-inline_kernel(Slot* slots, uint64_t n_slots, const uint32_t* edges, uint64_t n_edges, unsigned long long* n,
+inline_kernel(Slot* slots, uint64_t n_slots, const uint32_t* edges, uint64_t n_edges, StoreScan* out,
               uint64_t* orig) {
     const int lane = threadIdx.x & 31;
+    bool zero = false;
     const uint64_t stride = (uint64_t)gridDim.x * kLoadThreads * kScanUnroll;
     for (uint64_t b = ((uint64_t)blockIdx.x * kLoadThreads + (threadIdx.x & ~31)) * kScanUnroll; b < n_slots;
          b += stride) {
@@ -227,7 +239,7 @@ inline_kernel(Slot* slots, uint64_t n_slots, const uint32_t* edges, uint64_t n_e
         }
         if (!total) continue;
         unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(n, (unsigned long long)total);
+        if (lane == 0) at = atomicAdd(&out->n_inline, (unsigned long long)total);
         at = __shfl_sync(kFull, at, 0);
 #pragma unroll
         for (int u = 0; u < kScanUnroll; ++u) {
@@ -235,11 +247,14 @@ inline_kernel(Slot* slots, uint64_t n_slots, const uint32_t* edges, uint64_t n_e
                 const uint64_t i = b + 32 * u + lane;
                 const uint64_t k = at + __popc(m[u] & ((1u << lane) - 1));
                 *reinterpret_cast<ulonglong2*>(orig + 2 * k) = make_ulonglong2(i, sl[u].ptr);
-                slots[i].ptr = make_inline_ptr(__ldg(edges + ptr_off(sl[u].ptr)));
+                const uint32_t entry = __ldg(edges + ptr_off(sl[u].ptr));
+                zero |= entry == 0;
+                slots[i].ptr = make_inline_ptr(entry);
             }
             at += __popc(m[u]);
         }
     }
+    if (zero) atomicOr(&out->flags, (unsigned)kStoreZeroId);
 }
 
 // Every key a probe of its segment finds, from the segment's main buckets: f(vid, pointer word).
@@ -384,9 +399,9 @@ cudaError_t launch_store_scan(const DevStore& st, const PredSeg* pseg, uint32_t 
     return cudaGetLastError();
 }
 
-cudaError_t launch_inline(const DevStore& st, unsigned long long* n, uint64_t* orig, int sm_count, cudaStream_t s) {
+cudaError_t launch_inline(const DevStore& st, StoreScan* out, uint64_t* orig, int sm_count, cudaStream_t s) {
     inline_kernel<<<load_grid(sm_count), kLoadThreads, 0, s>>>(const_cast<Slot*>(st.slots), st.n_buckets * kAssoc,
-                                                               st.edges, st.n_edges, n, orig);
+                                                               st.edges, st.n_edges, out, orig);
     return cudaGetLastError();
 }
 

@@ -16,6 +16,7 @@ enum : uint32_t {
     kStoreInlineType = 4u, // a pointer word already carries the inline type
     kStoreBadChain = 8u,   // a chain link past the slot array, or a chain that does not end
     kStoreDupKey = 16u,    // a key twice in one chain
+    kStoreZeroId = 32u,    // a list holds id 0, which as a row's vertex names an index list
 };
 struct StoreScan {
     unsigned long long n_inline;   // keys whose list has one entry
@@ -40,8 +41,8 @@ struct SegScan {
 cudaError_t launch_store_scan(const DevStore& st, const PredSeg* pseg, uint32_t n_pseg, SegScan* per_seg,
                               StoreScan* out, ulonglong2* chunks, uint32_t max_chunks, int sm_count, cudaStream_t s);
 // One-entry lists into their keys' pointer words; the original words (slot index, word) go to
-// orig, counted in *n (0 on entry).
-cudaError_t launch_inline(const DevStore& st, unsigned long long* n, uint64_t* orig, int sm_count, cudaStream_t s);
+// orig, counted in out->n_inline (0 on entry).  (Their entries are looked at here, all others by the scan.)
+cudaError_t launch_inline(const DevStore& st, StoreScan* out, uint64_t* orig, int sm_count, cudaStream_t s);
 
 // A segment whose directory is built: its main buckets (disjoint from every other's), the keys'
 // predicate and direction, and where its blocks start among all blocks.

@@ -14,7 +14,8 @@ enum : uint32_t {
     kErrCorrupt = 4u,    // a key-table chain left the slot array or exceeded the hop limit
     kErrStatus = 8u,     // more tiles than the status array holds (host grows it and reruns)
     kErrResult = 16u,    // a result gather did not fit its buffer (host grows it and reruns)
-    kErrUnfuse = 32u,    // a step taken for functional gave a row several (host reruns unfused)
+    kErrUnfuse = 32u,    // a step taken for functional gave a row of a caller's table several (host
+                         // reruns it as one that multiplies rows)
 };
 
 // Per-stream control block of the single-pass scan.  Kernels that use it reset the tile and

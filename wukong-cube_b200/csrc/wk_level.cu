@@ -171,7 +171,6 @@ __device__ __forceinline__ uint32_t level_row(const LevelArgs& a, const SegDir* 
             cnt = (uint32_t)deg;
             ++w;
         } else if (s.op == kXK2U) {
-            if (deg > 1) atomicOr(&a.ctl->err, kErrUnfuse);   // (vid 0 only)
             cnt = deg ? 1 : 0;
             if (deg) app[(w - run.cin) * kLevThreads] = list_at(a.store.edges, *off, 0);
             ++w;

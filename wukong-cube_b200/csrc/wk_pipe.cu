@@ -27,8 +27,10 @@
 //
 // Sizes are read on the device, so passes chain without a host round trip and can be captured.
 // An output that does not fit sets kErrOverflow and the rows needed.  A row whose vertex is 0 names
-// an index list; where that gives a functional step more than one row the launch sets kErrUnfuse
-// and the host runs the plan with every such step as a pass of its own.
+// an index list.  A plan's rows hold it only where the store's own lists do, which is found when the
+// store is loaded, and its steps are then taken for what they are; a single step over a caller's table,
+// whose rows may hold anything, sets kErrUnfuse where the list has more than one entry, and the host
+// runs it again as a step that multiplies rows.
 #include <cuda_runtime.h>
 
 #include <algorithm>

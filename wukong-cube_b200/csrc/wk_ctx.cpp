@@ -1203,7 +1203,7 @@ extern "C" int wk_table_upload(wk_ctx* ctx, wk_table* t, const uint32_t* host, u
 }
 
 int wk::table_rows(wk_ctx* ctx, const wk_table* t, uint64_t* rows) {
-    if (!t->rows_known) {
+    if (!t->rows_known || t->replayed) {
         WK_CUDA(ctx, cudaMemcpyAsync(ctx->h_rows, t->d_rows, 8, cudaMemcpyDeviceToHost, ctx->stream));
         WK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         t->rows = ctx->h_rows[0];
@@ -1709,6 +1709,10 @@ extern "C" int wk_query_enqueue(wk_ctx* ctx, const wk_query* q, int32_t mode) {
     // (after a load that failed there is nothing to look up, and what is left of the tables of the
     // store before must not reach a launch)
     if (!steps.empty() && !ctx->has_store) return ctx->fail(WK_E_NOSTORE, "no store uploaded");
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    WK_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone)
+        for (auto& t : ctx->rbuf) t.replayed = true;
     return enqueue_plan(ctx, steps, query_passes(ctx, steps), *q);
 }
 

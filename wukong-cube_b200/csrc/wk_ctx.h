@@ -24,6 +24,8 @@ struct wk_table {
     // such launch goes through written()), so that it is not read again.
     mutable bool rows_known = false;
     mutable uint64_t rows = 0;
+    // A caller's own captured graph writes the table, whenever it is replayed: nothing is kept then.
+    bool replayed = false;
     void written() { rows_known = false; }
 };
 

@@ -607,9 +607,10 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
     int src = ctx->final_scratch_reserve(bytes);
     if (src) return src;
     char* scratch = static_cast<char*>(ctx->d_final_scratch);
-    auto done = [&](int rc) {
-        cudaStreamSynchronize(s);
-        return rc;
+    auto done = [&](int rc) {   // after what was enqueued; a success is one only if that was
+        const cudaError_t w = cudaStreamSynchronize(s);
+        if (w != cudaSuccess) cudaGetLastError();   // (reported here, not by the next launch)
+        return rc == WK_SUCCESS && w != cudaSuccess ? ctx->cuda_fail(w, "post-pattern stage") : rc;
     };
     int32_t* d_keep = reinterpret_cast<int32_t*>(scratch);
     uint32_t* idx0 = reinterpret_cast<uint32_t*>(scratch + keep_bytes);
@@ -809,9 +810,11 @@ extern "C" int wk_table_final_process(wk_ctx* ctx, const wk_table* in, const int
     project_kernel<<<pgrid, kFinThreads, 0, s>>>(table_src, cols, d_keep, n_keep, idx, start, count, out->d,
                                                  out->d_rows);
     if ((e = cudaGetLastError()) != cudaSuccess) return done(ctx->cuda_fail(e, "projection launch"));
+    const int wrc = done(WK_SUCCESS);
+    if (wrc) return wrc;
     out->rows = count;
     out->rows_known = true;
-    return done(WK_SUCCESS);
+    return WK_SUCCESS;
 }
 
 extern "C" int wk_table_filter_bound(wk_ctx* ctx, const wk_table* in, const int32_t* bound_cols,
@@ -847,8 +850,9 @@ extern "C" int wk_table_filter_bound(wk_ctx* ctx, const wk_table* in, const int3
     if (src) return src;
     char* scratch = static_cast<char*>(ctx->d_final_scratch);
     auto done = [&](int code) {
-        cudaStreamSynchronize(s);
-        return code;
+        const cudaError_t w = cudaStreamSynchronize(s);
+        if (w != cudaSuccess) cudaGetLastError();
+        return code == WK_SUCCESS && w != cudaSuccess ? ctx->cuda_fail(w, "filter stage") : code;
     };
     int32_t* d_cols = reinterpret_cast<int32_t*>(scratch);
     uint32_t* part = reinterpret_cast<uint32_t*>(scratch + 256);

@@ -169,6 +169,7 @@ void wk_ctx::drop_store(bool spare) {
     ++store_gen;
     has_store = false;
     drop_spare();
+    release_serve();   // (what follows needs the room, for its own scratch too)
     if (!borrowed_store) {
         // A store built again in the same context mostly needs the same arrays (freeing and mapping
         // them took most of a small build); they are kept for it when a build's scratch, a few times

@@ -1105,7 +1105,6 @@ extern "C" int wk_store_build_device(wk_ctx* ctx, const uint32_t* triples, uint6
     WKG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     // the old store goes first: a build needs the room
     ctx->drop_store(true);
-    ctx->release_serve();   // (a build needs the room)
     struct DropSpare {      // what the build did not use
         wk_ctx* c;
         ~DropSpare() { c->drop_spare(); }

@@ -467,8 +467,10 @@ struct HeavyLanes {
 };
 
 // Device bytes of serving buffers a context keeps between runs (two default arenas and their
-// owners fit); larger ones go back at the end of the run.  Allocating and freeing them cost 30 to
-// 300 ms a run, many times a burst's own work.
+// owners fit), as long as the device has seven times as much free besides; others go back at the
+// end of the run.  Allocating and freeing them cost 30 to 300 ms a run, many times a burst's own
+// work.  What is kept goes back when an allocation of the context fails, with its store, and with the
+// context.
 constexpr uint64_t kKeepServeBytes = 4ull << 30;
 
 }  // namespace
@@ -778,6 +780,9 @@ extern "C" int wk_serve_run_open_loop(wk_ctx* ctx, const wk_serve_config* cfg_in
         finished.clear();
         ++iter;
     }
-    if (S.kept_bytes() <= wk::kKeepServeBytes) ctx->serve = kept.release();
+    size_t free_b = 0, total_b = 0;
+    if (S.kept_bytes() <= wk::kKeepServeBytes && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
+        S.kept_bytes() <= free_b / 7)
+        ctx->serve = kept.release();
     return WK_SUCCESS;
 }

@@ -90,7 +90,7 @@ extern "C" int wk_measure_random_reads(wk_ctx* ctx, uint64_t region_bytes, int32
         if (sink) cudaFree(sink);
         return rc;
     };
-    if (wk::dev_malloc(&buf, region_bytes) != cudaSuccess || wk::dev_malloc(&sink, 4) != cudaSuccess) {
+    if (wk::ctx_malloc(ctx, &buf, region_bytes) != cudaSuccess || wk::ctx_malloc(ctx, &sink, 4) != cudaSuccess) {
         cudaGetLastError();
         return done(ctx->fail(WK_E_OOM, "random-read calibration buffer"));
     }

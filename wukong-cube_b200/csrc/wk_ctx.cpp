@@ -506,7 +506,7 @@ bool is_functional(const wk_ctx* ctx, const PlanStep& s) {
     if (id && ctx->seg_longest[id - 1] > 1) return false;
     if (!ctx->zero_ids) return true;
     auto it = ctx->index_ptr.find(s.pid * 2 + (uint32_t)s.dir);
-    return it != ctx->index_ptr.end() && ptr_size(it->second) <= 1;
+    return it != ctx->index_ptr.end() && it->second.probed && ptr_size(it->second.ptr) <= 1;
 }
 
 }  // namespace
@@ -554,10 +554,10 @@ int enqueue_pass(wk_ctx* ctx, const std::vector<PlanStep>& steps, const PlanPass
         a.from_list = 1;
         a.src_key = index ? make_key(0, st.start_const, st.dir) : make_key(st.start_const, st.pid, st.dir);
         auto it = ctx->index_ptr.find(st.start_const * 2 + (uint32_t)st.dir);
-        if (index && it != ctx->index_ptr.end()) {
+        if (index && it != ctx->index_ptr.end() && it->second.probed) {
             a.src_known = 1;
-            a.src_off = ptr_off(it->second);
-            a.src_len = ptr_size(it->second);
+            a.src_off = ptr_off(it->second.ptr);
+            a.src_len = ptr_size(it->second.ptr);
         }
         a.src_seg = index ? ctx->seg_of(0, st.start_const, st.dir) : ctx->seg_of(st.start_const, st.pid, st.dir);
         a.mt_tid = index ? mt_tid : 0;
@@ -1026,23 +1026,50 @@ int wk::store_adopt(wk_ctx* ctx, Slot* d_slots, uint64_t n_slots, uint32_t* d_ed
         // projects from
         ctx->index_ptr.clear();
         const uint64_t nb = n_slots / wk::kAssoc;
-        std::vector<wk::Slot> bk;
         for (int d = 0; d < 2; ++d) {
             const int32_t i = ctx->index.index_seg[d];
             if (i < 0) continue;
             const wk_seg_meta& m = segs[i];
             const uint64_t ranges[2][2] = {{m.bucket_start, m.num_buckets}, {m.ext_start, m.ext_num}};
-            for (auto& r : ranges) {
-                if (!r[1] || r[0] >= nb || r[1] > nb - r[0]) continue;
-                bk.resize(r[1] * wk::kAssoc);
-                WK_CUDA(ctx, cudaMemcpy(bk.data(), d_slots + r[0] * wk::kAssoc, bk.size() * sizeof(wk::Slot),
-                                        cudaMemcpyDeviceToHost));
-                for (size_t k = 0; k < bk.size(); ++k) {
-                    const uint64_t key = bk[k].key;
-                    if (k % wk::kAssoc == wk::kAssoc - 1 || key == 0 || wk::key_vid(key) != 0) continue;
-                    ctx->index_ptr.emplace(wk::key_pid(key) * 2 + wk::key_dir(key), bk[k].ptr);
-                }
+            std::vector<wk::Slot> bk[2];
+            for (int r = 0; r < 2; ++r) {
+                if (!ranges[r][1] || ranges[r][0] >= nb || ranges[r][1] > nb - ranges[r][0]) continue;
+                bk[r].resize(ranges[r][1] * wk::kAssoc);
+                WK_CUDA(ctx, cudaMemcpy(bk[r].data(), d_slots + ranges[r][0] * wk::kAssoc,
+                                        bk[r].size() * sizeof(wk::Slot), cudaMemcpyDeviceToHost));
             }
+            // the slot that a start's probe of `key` ends at, walked as the start list's launch walks (the
+            // whole bucket, then its chain unless a slot is empty); null where it finds none, or follows
+            // a chain out of the copies
+            auto probe = [&](uint64_t key) -> const wk::Slot* {
+                const wk::SegDesc& sg = ctx->seg_desc[i];
+                uint64_t b = sg.bucket_start + wk::mod_barrett(wk::hash_u64(key), sg.num_buckets, sg.magic);
+                for (uint64_t hop = 0; hop <= ranges[0][1] + ranges[1][1]; ++hop) {
+                    const wk::Slot* s = nullptr;
+                    for (int r = 0; r < 2; ++r)
+                        if (b >= ranges[r][0] && (b - ranges[r][0]) * wk::kAssoc < bk[r].size())
+                            s = bk[r].data() + (b - ranges[r][0]) * wk::kAssoc;
+                    if (!s) return nullptr;
+                    bool empty = s[wk::kAssoc - 1].key == 0;
+                    for (int k = 0; k < wk::kAssoc - 1; ++k) {
+                        if (s[k].key == key) return s + k;
+                        empty |= s[k].key == 0;
+                    }
+                    if (empty) return nullptr;
+                    b = wk::key_vid(s[wk::kAssoc - 1].key);
+                }
+                return nullptr;
+            };
+            for (auto& r : bk)
+                for (size_t k = 0; k < r.size(); ++k) {
+                    const uint64_t key = r[k].key;
+                    if (k % wk::kAssoc == wk::kAssoc - 1 || key == 0 || wk::key_vid(key) != 0 ||
+                        wk::key_dir(key) != (uint32_t)d)
+                        continue;
+                    const wk::Slot* s = probe(key);
+                    ctx->index_ptr.emplace(wk::key_pid(key) * 2 + wk::key_dir(key),
+                                           wk_ctx::IndexList{s ? s->ptr : r[k].ptr, s != nullptr});
+                }
         }
     }
     // one pass over the slots: are all lists inside the edge array, ascending and unique (which
@@ -1506,7 +1533,7 @@ static int plan_scratch(wk_ctx* ctx, const std::vector<wk::PlanStep>& steps) {
     if (!steps.empty() && steps[0].kind == wk::PlanStep::kIndex) {
         auto it = ctx->index_ptr.find(steps[0].start_const * 2 + (uint32_t)steps[0].dir);
         if (it != ctx->index_ptr.end()) {
-            int rc = ctx->ensure_status(wk::ptr_size(it->second) / wk::kPipeMaxTileRows + 4ull * wk::pipe_grid(ctx->sm_count));
+            int rc = ctx->ensure_status(wk::ptr_size(it->second.ptr) / wk::kPipeMaxTileRows + 4ull * wk::pipe_grid(ctx->sm_count));
             if (rc) return rc;
         }
     }

@@ -109,7 +109,11 @@ struct wk_ctx {
     bool versatile = false;           // the store holds the vertex-predicate lists
     wk::PredSeg* d_pseg = nullptr;    // predicate segments by pid * 2 + dir (versatile steps)
     uint32_t n_pseg = 0;
-    std::map<uint32_t, uint64_t> index_ptr;   // tpid * 2 + dir -> pointer word of its index list
+    struct IndexList {
+        uint64_t ptr;    // pointer word
+        bool probed;     // a probe of the key ends at it (else the word is only good for an estimate)
+    };
+    std::map<uint32_t, IndexList> index_ptr;   // tpid * 2 + dir -> its index list
     uint64_t* d_inline_orig = nullptr;   // (slot index, original pointer word) of every slot
     uint64_t n_inline = 0;               // whose one-entry list is kept in the slot itself
     bool borrowed_store = false;   // a serving lane: the store belongs to its parent context

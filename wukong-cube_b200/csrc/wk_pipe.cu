@@ -153,14 +153,39 @@ __device__ __noinline__ SlowWords<K> slow_words(const PipeArgs& a, const PipeOp&
     return w;
 }
 
+// Pointer word of a start's key, found as the start list's own launch (list_kernel) finds it: anywhere
+// in a bucket, and past it only where none of its slots is empty.
+__device__ __noinline__ uint64_t start_word(const DevStore& st, uint64_t key, uint64_t bucket, unsigned* err) {
+    for (int hop = 0; hop < kMaxProbeIters; ++hop) {
+        if (bucket >= st.n_buckets) break;
+        const Slot* b = st.slots + bucket * kAssoc;
+        ulonglong2 s[kAssoc];
+#pragma unroll
+        for (int i = 0; i < kAssoc; i += 2) load_sector(b + i, &s[i], &s[i + 1]);
+        bool empty = s[kAssoc - 1].x == 0;   // (no chain)
+#pragma unroll
+        for (int i = 0; i < kAssoc - 1; ++i) {
+            if (s[i].x == key) return s[i].y;
+            empty |= s[i].x == 0;
+        }
+        if (empty) return 0;
+        bucket = key_vid(s[kAssoc - 1].x);
+    }
+    atomicOr(err, kErrCorrupt);
+    return 0;
+}
+
 // The one list of a step (or of the start), worked out once per CTA.
 struct OneList {
     uint64_t off, deg;
 };
-__device__ __forceinline__ OneList one_list(const PipeArgs& a, const SegDesc& sg, uint64_t key, uint32_t mt) {
+__device__ __forceinline__ OneList one_list(const PipeArgs& a, const SegDesc& sg, uint64_t key, uint32_t mt,
+                                            bool start) {
     OneList l{0, 0};
     if (sg.num_buckets == 0 || key == 0) return l;
-    list_of_ptr(hash_lookup(a.store, sg, key, &a.ctl->err), a.store.n_edges, &a.ctl->err, &l.off, &l.deg);
+    const uint64_t p = start ? start_word(a.store, key, bucket_of(key, sg), &a.ctl->err)
+                             : hash_lookup(a.store, sg, key, &a.ctl->err);
+    list_of_ptr(p, a.store.n_edges, &a.ctl->err, &l.off, &l.deg);
     if (mt) {
         uint64_t lo, hi;
         mt_slice(mt, l.deg, &lo, &hi);
@@ -457,7 +482,7 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __g
         s.col = o.cs;
         s.tcol = o.ce;
         if (o.op == kXC2K || o.op == kXI2K) {
-            const OneList l = one_list(a, o.seg, o.start_key, o.op == kXI2K ? o.mt : 0);
+            const OneList l = one_list(a, o.seg, o.start_key, o.op == kXI2K ? o.mt : 0, false);
             s.how = kHowOne;
             s.col = o.ce;
             s.one_off = l.off;
@@ -473,7 +498,7 @@ __global__ void __launch_bounds__(kPipeThreads, kPipeCtas) pipe_kernel(const __g
     if (kList) {
         if (threadIdx.x == kPipeThreads - 1) {
             s_src = OneList{a.src_off, a.src_len};
-            if (!a.src_known) s_src = one_list(a, a.src_seg, a.src_key, 0);
+            if (!a.src_known) s_src = one_list(a, a.src_seg, a.src_key, 0, true);
         }
         __syncthreads();
         const uint64_t sz = s_src.deg;

@@ -128,7 +128,7 @@ uint64_t plan_projection(const wk_ctx* ctx, const std::vector<PlanStep>& plan) {
         switch (s.kind) {
             case PlanStep::kIndex: {
                 auto it = ctx->index_ptr.find(s.start_const * 2 + (uint32_t)s.dir);
-                rows = it == ctx->index_ptr.end() ? 0.0 : (double)ptr_size(it->second);
+                rows = it == ctx->index_ptr.end() ? 0.0 : (double)ptr_size(it->second.ptr);
                 break;
             }
             case PlanStep::kConst: rows = mean_deg(s.pid, s.dir); break;

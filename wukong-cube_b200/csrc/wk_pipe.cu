@@ -159,17 +159,18 @@ __device__ __noinline__ uint64_t start_word(const DevStore& st, uint64_t key, ui
     for (int hop = 0; hop < kMaxProbeIters; ++hop) {
         if (bucket >= st.n_buckets) break;
         const Slot* b = st.slots + bucket * kAssoc;
-        ulonglong2 s[kAssoc];
-#pragma unroll
-        for (int i = 0; i < kAssoc; i += 2) load_sector(b + i, &s[i], &s[i + 1]);
-        bool empty = s[kAssoc - 1].x == 0;   // (no chain)
-#pragma unroll
-        for (int i = 0; i < kAssoc - 1; ++i) {
-            if (s[i].x == key) return s[i].y;
-            empty |= s[i].x == 0;
+        bool empty = false;
+        uint64_t link = 0;
+        for (int i = 0; i < kAssoc; i += 2) {
+            ulonglong2 s0, s1;
+            load_sector(b + i, &s0, &s1);
+            if (s0.x == key) return s0.y;
+            link = s1.x;
+            empty |= s0.x == 0 || link == 0;   // (slot 7 empty: no chain)
+            if (i + 1 < kAssoc - 1 && s1.x == key) return s1.y;
         }
         if (empty) return 0;
-        bucket = key_vid(s[kAssoc - 1].x);
+        bucket = key_vid(link);
     }
     atomicOr(err, kErrCorrupt);
     return 0;

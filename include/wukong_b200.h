@@ -451,8 +451,9 @@ int wk_debug_device_allocs(uint64_t* count);
  *   knob 1: the same for batches and serving;
  *   knob 2: the list length above which a row's output is written as 2,048-row slices by every
  *           CTA (block-per-row) instead of by the CTA that probed it (group-per-row); 8 to
- *           2^23, default 128;
- *   knob 3: the same for batches and serving;
+ *           2^23, default 128.  A fused pass writes lists of up to 256 entries by their warp, but
+ *           for those past the threshold that share 64 rows with a longer one;
+ *   knob 3: the same for batches (fused levels too, exactly) and serving;
  *   knob 4: single steps whose input has at least this many rows run as a fused pass instead of
  *           the tile launch; whole plans run as fused passes (a run of steps per launch) unless it
  *           is 0, which never does (default 65,536);

@@ -37,7 +37,6 @@ constexpr int kGroups = 4;            // 32-row groups of a warp's chunk at most
 constexpr int kStageWords = 512;      // output words staged per warp
 constexpr int kStageRows = 128;       // and their rows' owners
 constexpr uint32_t kLaneList = 16;    // a warp with no longer list writes a row's outputs by its lane
-constexpr uint32_t kSliceList = 64;   // lists past this are written as slices by any CTA (knob 3 unset)
 
 // The directory half of a SegDesc; segments past kSmemSegs are read where they are.
 struct SegDir {
@@ -217,7 +216,7 @@ __global__ void __launch_bounds__(kLevThreads, kLevCtas) level_kernel(const __gr
     // no chunk for this CTA: it leaves, and the others count without it
     const unsigned active = (unsigned)min((unsigned long long)gridDim.x, (unsigned long long)ntiles);
     if (blockIdx.x >= active) return;
-    const uint32_t thr = a.slice_rows ? min(max(a.slice_rows, (uint32_t)kMinSliceRows), 1u << 23) : kSliceList;
+    const uint32_t thr = a.slice_rows ? min(max(a.slice_rows, (uint32_t)kMinSliceRows), 1u << 23) : (uint32_t)kHeavyRows;
     const unsigned long long spin = a.spin_limit ? a.spin_limit : kDefaultSpinLimit;
     const int wo = a.w_out;
     uint32_t* const stage = S.stage[warp];
@@ -315,7 +314,7 @@ __global__ void __launch_bounds__(kLevThreads, kLevCtas) level_kernel(const __gr
                     w_row += (__ldg(reinterpret_cast<const uint32_t*>(a.steps + run.first + i) + 5) & 0xFF) == kXK2U;
             }
             const uint32_t mx = __reduce_max_sync(kFull, cnt);
-            if (mx <= kLaneList) {
+            if (mx <= min(kLaneList, thr)) {
                 // short lists: each lane lays its row's outputs out in the stage, as many rows as fit
                 // at a time
                 const uint32_t n = (uint32_t)n_all, s0 = (uint32_t)st, fit = min(kStageWords / wo, kStageRows);

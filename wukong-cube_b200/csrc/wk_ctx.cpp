@@ -996,11 +996,35 @@ static int build_directories(wk_ctx* ctx, const std::vector<wk::SegScan>& of_seg
     if (e != cudaSuccess) return drop(ctx->cuda_fail(e, "vertex directories"));
     ctx->d_dir_blocks = blocks;
     ctx->d_dir_words = words;
+    ctx->dir_bytes = n_blocks * sizeof(wk::DirBlock) + at.back() + 16;
     blocks = nullptr;
     words = nullptr;
     ctx->has_dir = true;
     for (size_t k = 0; k < ds.size(); ++k) ctx->seg_desc[which[k]] = ds[k].seg;
     return drop(store_tables(ctx));
+}
+
+bool wk_ctx::drop_directories(size_t bytes) {
+    size_t free_b = 0, total_b = 0;
+    if (!has_dir || borrowed_store || serving || rbuf[0].replayed ||
+        cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b + dir_bytes)
+        return false;
+    if (cudaDeviceSynchronize() != cudaSuccess) return false;
+    for (wk_ctx* lane : lanes) wk_ctx_destroy(lane);   // (the next serving run makes them again)
+    lanes.clear();
+    drop_graphs();   // captured passes hold their segments' directories
+    for (auto& d : seg_desc) {
+        d.dir = nullptr;
+        d.dir_words = nullptr;
+        d.vid_lo = d.vid_span = d.dir_values = 0;
+    }
+    has_dir = false;
+    if (store_tables(this) != WK_SUCCESS) return false;   // (the directories stay, for who reads the old tables)
+    cudaFree(d_dir_blocks);
+    cudaFree(d_dir_words);
+    d_dir_blocks = nullptr;
+    d_dir_words = nullptr;
+    return true;
 }
 
 // Make device arrays the context's store: segment lookup, predicate segment table, the list

@@ -102,7 +102,9 @@ struct wk_ctx {
     wk::SegDesc* d_segs = nullptr;       // DevStore::segs: an absent segment, then seg_desc
     wk::DirBlock* d_dir_blocks = nullptr;   // vertex directories (wk_dir.cu)
     void* d_dir_words = nullptr;
+    size_t dir_bytes = 0;
     bool has_dir = false;                // some segment has a directory
+    bool serving = false;                // a serving run is on: its lanes read the store as it is
     uint64_t store_gen = 0;              // stores this context has held (captured launches hold
                                          // the addresses of theirs)
     bool has_store = false;
@@ -214,6 +216,9 @@ struct wk_ctx {
     // device has plenty of room).
     void drop_store(bool spare = false);
     void drop_spare();
+    // Give the vertex directories back to an allocation of `bytes` (lookups go by hash from then on);
+    // false where it would not fit all the same, or something running or captured may still read them.
+    bool drop_directories(size_t bytes);
     struct Spare {
         void* p = nullptr;
         size_t bytes = 0;
@@ -235,7 +240,8 @@ namespace wk {
 // that one copy brings all of them.
 constexpr size_t kCtlBlockBytes = sizeof(StepCtl) + 2 * sizeof(uint64_t);
 constexpr uint64_t kSmallElems = 4096;
-// dev_malloc that gives the kept serving buffers back and tries again when the device is full.
+// dev_malloc that gives back what the context only keeps to be faster, and tries again, when the
+// device is full: the kept serving buffers, then the vertex directories.
 template <class T>
 cudaError_t ctx_malloc(wk_ctx* ctx, T** p, size_t bytes) {
     cudaError_t e = dev_malloc(p, bytes);
@@ -243,6 +249,10 @@ cudaError_t ctx_malloc(wk_ctx* ctx, T** p, size_t bytes) {
         cudaGetLastError();
         ctx->release_serve();
         e = dev_malloc(p, bytes);
+    }
+    if (e != cudaSuccess && ctx->has_dir) {
+        cudaGetLastError();
+        if (ctx->drop_directories(bytes)) e = dev_malloc(p, bytes);
     }
     return e;
 }

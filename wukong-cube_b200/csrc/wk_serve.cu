@@ -503,6 +503,11 @@ extern "C" int wk_serve_run_open_loop(wk_ctx* ctx, const wk_serve_config* cfg_in
     std::lock_guard<std::mutex> lk(ctx->mu);
     if (!ctx->has_store) return ctx->fail(WK_E_NOSTORE, "no store uploaded");
     if (n == 0) return WK_SUCCESS;
+    struct Serving {
+        wk_ctx* c;
+        explicit Serving(wk_ctx* ctx) : c(ctx) { c->serving = true; }
+        ~Serving() { c->serving = false; }
+    } serving(ctx);
     // the buffers kept from the run before; a run that fails gives them back
     std::unique_ptr<wk::Serve> kept(static_cast<wk::Serve*>(ctx->serve));
     ctx->serve = nullptr;

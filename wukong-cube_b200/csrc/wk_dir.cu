@@ -275,6 +275,9 @@ __device__ __forceinline__ void dir_walk(const DevStore& st, const DirSeg* segs,
         uint64_t bucket = home;
         int hop = 0;
         for (; hop < kMaxProbeIters; ++hop) {
+            // (a chain this long may be one that does not end; where one has been found there is no
+            // directory, so the walks of a store full of them are cut short)
+            if (hop >= 64 && *(volatile unsigned*)flags & kStoreBadChain) return;
             if (bucket >= st.n_buckets) {
                 atomicOr(flags, kStoreBadChain);
                 break;

@@ -154,8 +154,6 @@ struct wk_ctx {
     // CUDA graphs of resident query plans
     struct GraphEntry {
         cudaGraphExec_t exec = nullptr;
-        const wk_table* final_table = nullptr;
-        uint64_t cap0 = 0, cap1 = 0;
     };
     std::map<std::string, GraphEntry> graphs;
 

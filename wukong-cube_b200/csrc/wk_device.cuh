@@ -1,7 +1,7 @@
 // Device-side building blocks shared by the single-query and the batched step kernels:
 // bounded mbarrier waits and TMA bulk copies, the sector-granular group probe of the key table,
-// the block scan, the warp-parallel decoupled look-back, 16-byte stores from shared memory,
-// list membership and the self-resetting exit protocol of a launch.
+// the lookup by vertex directory, the block scan, the warp-parallel decoupled look-back, the slice
+// queue of long lists, list membership and the self-resetting exit protocol of a launch.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -16,7 +16,6 @@ constexpr int kMaxProbeIters = 1 << 14;                   // chain walk limit
 constexpr unsigned long long kFlagAgg = 1, kFlagPrefix = 2;
 constexpr unsigned long long kValMask = (1ull << 46) - 1;
 constexpr unsigned kTmaWaitLimit = 1u << 24;              // mbarrier polls before giving up
-constexpr int kChunkBytes = 32 * 1024;                    // staging of one output chunk
 constexpr int kLinear = 8;                                // list entries checked by ballot
 
 static_assert(kTileRows % kStepThreads == 0, "rows per thread");
@@ -247,10 +246,8 @@ __device__ __forceinline__ void group_probe(const DevStore& st, const uint64_t (
 }
 
 // Probe one key by one thread: the home bucket's slots two at a time (one 32-byte sector),
-// then the chain through slot 7.  Returns the pointer word, 0 when absent.  `first` skips the
-// home bucket's slots a caller has already compared (0 or an even slot).
-__device__ __forceinline__ uint64_t thread_probe(const DevStore& st, uint64_t key, uint64_t bucket,
-                                                 unsigned* err, int first = 0) {
+// then the chain through slot 7.  Returns the pointer word, 0 when absent.
+__device__ __forceinline__ uint64_t thread_probe(const DevStore& st, uint64_t key, uint64_t bucket, unsigned* err) {
     for (int hop = 0; hop < kMaxProbeIters; ++hop) {
         if (bucket >= st.n_buckets) {
             atomicOr(err, kErrCorrupt);
@@ -259,7 +256,6 @@ __device__ __forceinline__ uint64_t thread_probe(const DevStore& st, uint64_t ke
         const Slot* b = st.slots + bucket * kAssoc;
 #pragma unroll
         for (int s = 0; s < kAssoc - 1; s += 2) {
-            if (hop == 0 && s < first) continue;
             ulonglong2 s0, s1;
             load_sector(b + s, &s0, &s1);   // both slots: one 32-byte sector
             if (s0.x == key) return s0.y;
@@ -509,27 +505,6 @@ __device__ __forceinline__ unsigned long long claim_slice(StepCtl* ctl, const He
         }
         if (spins > 32) __nanosleep(64);
     }
-}
-
-// Copy `count` words from shared memory to global memory with 16-byte stores where aligned.
-__device__ __forceinline__ void store_words(uint32_t* dst, const uint32_t* src, uint64_t count) {
-    const uintptr_t addr = reinterpret_cast<uintptr_t>(dst);
-    uint64_t head = ((16 - (addr & 15)) & 15) >> 2;
-    if (head > count) head = count;
-    if (threadIdx.x < head) dst[threadIdx.x] = src[threadIdx.x];
-    const uint64_t nvec = (count - head) >> 2;
-    uint4* dv = reinterpret_cast<uint4*>(dst + head);
-    const uint32_t* sv = src + head;
-    for (uint64_t v = threadIdx.x; v < nvec; v += blockDim.x) {
-        uint4 x;
-        x.x = sv[4 * v];
-        x.y = sv[4 * v + 1];
-        x.z = sv[4 * v + 2];
-        x.w = sv[4 * v + 3];
-        dv[v] = x;
-    }
-    const uint64_t done = head + (nvec << 2);
-    if (threadIdx.x < count - done) dst[done + threadIdx.x] = src[done + threadIdx.x];
 }
 
 // The last CTA to leave resets the tile/exit counters and advances the epoch; when the 16-bit

@@ -69,7 +69,7 @@ typedef struct wk_serve wk_serve;
 /* Device context configuration.  Zero fields take defaults. */
 typedef struct wk_config {
     int32_t device;                   /* CUDA device ordinal */
-    int32_t max_cols;                 /* widest result table accepted (default 64) */
+    int32_t max_cols;                 /* widest result table accepted (at most, and by default, 32) */
     uint64_t rbuf_bytes;              /* initial size of each of the two ping-pong result
                                          buffers (GPUMem rbuf, gpu_mem.hpp:53-60); they grow */
     uint64_t working_set_cap_bytes;   /* serving admission cap (default 40 GiB) */
@@ -264,8 +264,9 @@ int wk_store_build_device(wk_ctx* ctx, const uint32_t* triples, uint64_t n_tripl
 int wk_store_export(wk_ctx* ctx, void* slots, uint64_t slots_cap, uint32_t* edges, uint64_t edges_cap,
                     wk_seg_meta* segs, uint32_t segs_cap, uint64_t* n_slots, uint64_t* n_edges, uint32_t* n_segs);
 /* Device bytes held by the store (slots + edges + segment table).  The lookup tables derived from
- * it at load time (vertex directories, at most a quarter of the then free memory; the original
- * words of one-entry lists) are not counted. */
+ * it at load time (vertex directories, at most a quarter of the then free memory, which an allocation
+ * of the context that has no other room takes back; the original words of one-entry lists) are not
+ * counted. */
 int wk_store_bytes(const wk_ctx* ctx, uint64_t* bytes);
 
 /* ---------------------------------------------------------------- result tables */
@@ -501,9 +502,10 @@ int wk_ctx_autotune(wk_ctx* ctx, const wk_query* queries, uint32_t n, int32_t it
 int wk_measure_random_reads(wk_ctx* ctx, uint64_t region_bytes, int32_t iters, double* reads_per_s);
 
 /* ---------------------------------------------------------------- batching
- * Run n planned queries together: all queries advance one pattern per level inside one
- * persistent kernel fed by a device work queue, levels replayed from a CUDA graph.  No
- * counterpart in the reference (it runs one query per GPU agent at a time). */
+ * Run n planned queries together: all queries advance level by level, a level being one persistent
+ * launch fed by a device work queue, and the levels are replayed from a CUDA graph.  On a store with
+ * vertex directories a level runs each query's steps up to the next one that multiplies rows, else
+ * one pattern.  No counterpart in the reference (it runs one query per GPU agent at a time). */
 int wk_batch_execute(wk_ctx* ctx, const wk_query* queries, uint32_t n, uint32_t* host_out,
                      uint64_t cap_elems, wk_qresult* results);
 /* A stream of batches: queries[0..n) run as consecutive batches of `batch` queries (0: 16,384)
@@ -518,7 +520,8 @@ int wk_batch_execute_stream(wk_ctx* ctx, const wk_query* queries, uint32_t n, ui
 int wk_batch_execute_device(wk_ctx* ctx, const wk_query* queries, uint32_t n,
                             uint64_t* total_rows);
 /* Replay the last batch of this context on its stream and return without waiting (for
- * device-side timing of an identical batch; errors surface through wk_ctx_check). */
+ * device-side timing of an identical batch; errors surface through wk_ctx_check).  WK_E_BADARG
+ * when none has run, or when the store or the scratch that it ran on is gone. */
 int wk_batch_replay(wk_ctx* ctx);
 /* Per-level profile of a batch: each level launch between CUDA events on the context stream,
  * averaged over `iters` runs after one warm-up; out[k].kind = 5, followed by three entries
@@ -529,7 +532,10 @@ int wk_batch_profile(wk_ctx* ctx, const wk_query* queries, uint32_t n, int32_t i
 /* ---------------------------------------------------------------- serving
  * Continuous batching over an open-loop arrival schedule (no reference counterpart; shaped
  * like ConsoleProxy::run_query_emu, console_proxy.hpp:287-439).  arrival_us[i] is when
- * query i arrives, relative to the start of the run; results are copied to host_out. */
+ * query i arrives, relative to the start of the run; results are copied to host_out.
+ * The run's table arenas (up to 4 GiB, and only where the device has seven times as much free
+ * besides) stay with the context for its next run; an allocation of the context that needs their
+ * room, a load, and wk_ctx_destroy give them back. */
 int wk_serve_run_open_loop(wk_ctx* ctx, const wk_serve_config* cfg, const wk_query* queries,
                            uint32_t n, const double* arrival_us, uint32_t* host_out,
                            uint64_t cap_elems, wk_qresult* results);

@@ -9,13 +9,14 @@
 //
 // A launch is shaped like the fused pass of a single query (wk_pipe.cu): CTAs claim chunks of
 // consecutive rows (1,024 on a large level, fewer as long as there is a CTA for more), count, take a
-// decoupled look-back, and write what they counted, short lists through shared memory.  One row per thread: rows of different queries run different steps, and a warp's 32
-// rows mostly belong to one or two queries.  Rows whose lists are longer than the slice threshold go
-// to the slice queue that CTAs without work drain.
+// decoupled look-back, and write what they counted, short lists through shared memory.  One row per
+// thread: rows of different queries run different steps, and a warp's 32 rows mostly belong to one or
+// two queries.  Rows whose lists are longer than the slice threshold go to the slice queue that CTAs
+// without work drain (128 entries unless knob 3 says otherwise; 64 took the same time).
 //
 // What bounds it: a chunk waits for the counts of the chunks before it (11 us of a chunk's 40 on the
 // last level of 16,384 light queries over 2,000 organisations), and the chain of a row's dependent
-// reads; DRAM and issue are a quarter used.  Levels of that batch, us: 37 + 125 + 173 + 147, against 46
+// reads; issue is a quarter used, DRAM less than a tenth.  Levels of that batch, us: 37 + 125 + 173 + 147, against 46
 // + 123 + 105 + 114 + 82 + 66 for a launch per pattern; 64 queries 88 against 145.  Measured without
 // gain: two or four rows per thread where a warp's rows are one query's, chunks of 256 or 512 rows
 // (191 and 152 against 147 on the last level), three or five CTAs per SM, descriptors a step ahead.

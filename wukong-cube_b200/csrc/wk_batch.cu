@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kScanThreads) result_scan_kernel(const ResultS
 
 // Copy each query's final table (stride of its level) into the compact result buffer.
 __global__ void __launch_bounds__(256) gather_kernel(const GatherArgs a) {
-    if (a.n == 0) return;
+    if (a.n == 0 || (a.ctl->err & kErrTimeout)) return;   // (after a wait that gave up there is no result)
     if (a.res_off[a.n] > a.out_cap) {   // the host grows the buffer and reruns
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&a.ctl->err, kErrOverflow);
         return;

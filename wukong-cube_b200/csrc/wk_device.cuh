@@ -511,9 +511,13 @@ __device__ __forceinline__ unsigned long long claim_slice(StepCtl* ctl, const He
 // epoch wraps it clears the status array first so no stale word can match the next epoch.
 // `tags` / `tag_stride` / `n_tags`: epoch-tagged words of the long-list slice queue, cleared with
 // the status array when the epoch wraps.  n_ctas: how many CTAs of the launch get here.
+// owned_rows: the row count of an output whose rows name their owner query.  After a wait that gave up
+// some of them may not have been written, and the next level would read whatever is there as owners:
+// their count goes past every capacity, so it does no work (as after an overflow).
+constexpr uint64_t kRowsGaveUp = 1ull << 62;
 __device__ void exit_protocol(StepCtl* ctl, unsigned long long* status, unsigned epoch,
                               unsigned* tags, unsigned tag_stride, unsigned long long n_tags,
-                              unsigned n_ctas = gridDim.x) {
+                              unsigned n_ctas = gridDim.x, uint64_t* owned_rows = nullptr) {
     __shared__ int s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -523,6 +527,7 @@ __device__ void exit_protocol(StepCtl* ctl, unsigned long long* status, unsigned
     }
     __syncthreads();
     if (!s_last) return;
+    if (owned_rows && threadIdx.x == 0 && (*(volatile unsigned*)&ctl->err & kErrTimeout)) *owned_rows = kRowsGaveUp;
     unsigned next = epoch + 1;
     if (next > 0xFFFFu) {
         for (unsigned long long i = threadIdx.x; i < ctl->status_cap; i += blockDim.x) status[i] = 0;

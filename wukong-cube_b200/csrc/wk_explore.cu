@@ -615,7 +615,8 @@ __global__ void __launch_bounds__(kStepThreads, explore_min_blocks(L)) explore_k
         atomicAdd(&a.ctl->sum_deg, acc_sd);
     }
     exit_protocol(a.ctl, a.status, epoch, a.heavy ? &a.heavy[0].tag : nullptr,
-                  sizeof(HeavyItem) / sizeof(uint32_t), a.heavy ? a.heavy_cap : 0);
+                  sizeof(HeavyItem) / sizeof(uint32_t), a.heavy ? a.heavy_cap : 0, gridDim.x,
+                  a.owner_out ? a.out_rows : nullptr);
 }
 
 template <int L>

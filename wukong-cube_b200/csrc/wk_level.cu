@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kLevThreads, kLevCtas) level_kernel(const __gr
         }
     }
     exit_protocol(a.ctl, a.status, epoch, a.heavy ? &a.heavy[0].tag : nullptr, sizeof(HeavyItem) / sizeof(uint32_t),
-                  a.heavy ? a.heavy_cap : 0, active);
+                  a.heavy ? a.heavy_cap : 0, active, a.out_rows);
 }
 
 }  // namespace

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(256)
 finish_gather_kernel(const uint32_t* fin_slots, const uint32_t* fin_cols, uint32_t n_fin,
                      const unsigned long long* qfirst, const uint64_t* fin_off,
                      const uint32_t* arena, int w, uint32_t* out, uint64_t out_cap, StepCtl* ctl) {
-    if (n_fin == 0) return;
+    if (n_fin == 0 || (ctl->err & kErrTimeout)) return;   // (after a wait that gave up there is no result)
     if (fin_off[n_fin] > out_cap) {   // the host grows the buffer and reruns the iteration
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&ctl->err, kErrResult);
         return;

@@ -44,3 +44,22 @@ def test_levels_after_a_wait_that_ran_out(built, levels):
         got = ctx.serve(qs, np.zeros(len(qs)))
         for k, w in want.items():
             assert got[k][1] == 0 and np.array_equal(oracle.sorted_rows(got[k][0]), w)
+
+
+def test_the_limit_holds_for_a_batch_that_ran_before(built):
+    """The captured launches of a batch follow knob 6: the same batch with the limit at two polls and with
+    the default again."""
+    tr, v = wk.synth_generate(30, seed=2)
+    g = wk.GStore(tr)
+    inst = {t: g.get_index(t, wk.IN) for t in range(v["t_org"], v["t_doc"] + 1)}
+    qs = workloads.light_queries(v, inst, 3000, seed=11)
+    with wk.Context(0) as ctx:
+        ctx.upload_gstore(g)
+        ctx.batch_device(qs)
+        codes = []
+        for _ in range(4):
+            ctx.tune_set(wk.KNOB_SPIN_LIMIT, 2)
+            codes.append(_codes(lambda: ctx.batch_device(qs)))
+            ctx.tune_set(wk.KNOB_SPIN_LIMIT, 0)
+            ctx.batch_device(qs)
+        assert wk.E_TIMEOUT in codes

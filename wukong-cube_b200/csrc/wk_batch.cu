@@ -594,6 +594,7 @@ int launch_batch(wk_ctx* ctx, BatchState* b, const Plan& P) {
     put(&ctx->batch_lanes, 4);
     put(&ctx->batch_slice_rows, 4);
     put(&ctx->batch_flat, 4);
+    put(&ctx->spin_limit, 8);
     put(&b->d_flat, sizeof(void*));
     put(&ctx->store_gen, 8);
     if (shape != b->shape || !b->exec) {

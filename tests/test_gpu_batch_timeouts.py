@@ -19,7 +19,7 @@ def _codes(call):
         return e.code
 
 
-@pytest.mark.parametrize("levels", ["fused", "a pattern each"])
+@pytest.mark.parametrize("levels", ["fused", "a pattern each", "flat after tiles"])
 def test_levels_after_a_wait_that_ran_out(built, levels):
     tr, v = wk.synth_generate(30, seed=2)
     g = wk.GStore(tr)
@@ -29,7 +29,7 @@ def test_levels_after_a_wait_that_ran_out(built, levels):
     want = {k: oracle.sorted_rows(o.run(qs[k].flat(), qs[k].nvars)[1]) for k in range(0, len(qs) - 1, 37)}
     with wk.Context(0) as ctx:
         ctx.upload_gstore(g)
-        ctx.tune_set(wk.KNOB_BATCH_FLAT, 0 if levels == "fused" else 1 << 15)
+        ctx.tune_set(wk.KNOB_BATCH_FLAT, {"fused": 0, "a pattern each": 1 << 15, "flat after tiles": 0b111100}[levels])
         seen = set()
         for turn in range(6):
             ctx.tune_set(wk.KNOB_SPIN_LIMIT, 2)

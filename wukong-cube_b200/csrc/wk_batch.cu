@@ -49,6 +49,8 @@ __global__ void __launch_bounds__(kScanThreads) result_scan_kernel(const ResultS
     __shared__ uint64_t s_warp[kScanThreads / 32];
     const uint32_t n = a.n;
     const uint32_t t0 = blockIdx.x * kScanThreads;
+    // (read here by the thread that writes the total, so that the scan hides it)
+    const unsigned err = t0 + threadIdx.x + 1 == n ? *(volatile unsigned*)&a.ctl->err : 0;
     // eight queries per thread at a time: their step counts, then their row counts and widths,
     // are loaded together (one dependent round trip per eight queries, not per query)
     uint64_t before = 0;
@@ -82,12 +84,13 @@ __global__ void __launch_bounds__(kScanThreads) result_scan_kernel(const ResultS
     }
     const uint64_t ex = dev::block_exclusive_sum<kScanThreads>(elems, s_warp);
     if (q < n) a.res_off[q] = s_base + ex;
-    if (n > 0 ? q == n - 1 : q == 0) a.res_off[n] = s_base + ex + elems;
+    // (after a wait that gave up there is no result: a total past every capacity, so nothing is gathered)
+    if (n > 0 ? q == n - 1 : q == 0) a.res_off[n] = err & kErrTimeout ? ~0ull : s_base + ex + elems;
 }
 
 // Copy each query's final table (stride of its level) into the compact result buffer.
 __global__ void __launch_bounds__(256) gather_kernel(const GatherArgs a) {
-    if (a.n == 0 || (a.ctl->err & kErrTimeout)) return;   // (after a wait that gave up there is no result)
+    if (a.n == 0) return;
     if (a.res_off[a.n] > a.out_cap) {   // the host grows the buffer and reruns
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&a.ctl->err, kErrOverflow);
         return;
@@ -542,6 +545,7 @@ int enqueue_batch(wk_ctx* ctx, BatchState* b, const Plan& P, ProfHooks* ph = nul
     }
     wk::ResultScanArgs ra{};
     ra.n = n;
+    ra.ctl = ctx->d_ctl;
     ra.nsteps = reinterpret_cast<const uint32_t*>(b->d_plan);
     ra.qfirst = b->d_qfirst;
     ra.qcount = b->d_qcount;

@@ -11,6 +11,7 @@ namespace wk {
 constexpr int kMaxBatchLevels = 16;
 
 struct ResultScanArgs {
+    const StepCtl* ctl;
     uint32_t n;
     const uint32_t* nsteps;              // [n] patterns per query (0 = failed / empty plan)
     const unsigned long long* qfirst;    // [levels][n]

@@ -197,6 +197,42 @@ void free_state(BatchState* b) {
         if (e_ != cudaSuccess) return (ctx)->cuda_fail(e_, #call); \
     } while (0)
 
+struct Plan {
+    uint32_t n = 0;
+    int levels = 0;                     // launches
+    bool fused = false;
+    size_t up_bytes = 0;                // of the plan block
+    int width[kMaxBatchLevels] = {0};
+    std::vector<int32_t> status;
+    std::vector<wk::PlanStep> steps;    // [n][kMaxBatchLevels]
+    std::vector<uint8_t> nsteps;        // [n]
+    std::vector<uint32_t> first;        // [n] each query's first step (fused)
+    const PlanLayout layout() const { return PlanLayout(n, levels, fused); }
+};
+
+// Host-side state kept between batch calls of a context: the plans (their arrays are large,
+// and touching fresh pages for them cost 0.4 ms per 16,384-query batch) and the pipelined
+// path's streams and events (creating them cost 0.17 ms per call).  Calls on one context are
+// serialised by its mutex, so one set serves every call.
+struct BatchHost {
+    Plan plan[2];
+    cudaStream_t copy_stream = nullptr, upload_stream = nullptr;
+    cudaEvent_t ready[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
+    cudaEvent_t uploaded[2] = {nullptr, nullptr};
+    ~BatchHost() {
+        for (int k = 0; k < 2; ++k)
+            for (cudaEvent_t e : {ready[k], copied[k], uploaded[k]})
+                if (e) cudaEventDestroy(e);
+        if (copy_stream) cudaStreamDestroy(copy_stream);
+        if (upload_stream) cudaStreamDestroy(upload_stream);
+    }
+};
+
+BatchHost* batch_host(wk_ctx* ctx) {
+    if (!ctx->batch_host) ctx->batch_host = new BatchHost();
+    return (BatchHost*)ctx->batch_host;
+}
+
 int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, int steps, uint64_t rows_cap, int w,
                  uint64_t result_cap) {
     rows_cap = (rows_cap + 15) & ~15ull;   // keeps every level region 16-byte aligned
@@ -209,8 +245,12 @@ int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, int steps, 
     rows_cap = std::max(rows_cap, b->rows_cap);
     w = std::max(w, b->w_cap);
     result_cap = std::max(result_cap, b->result_cap);
-    // every stream, the pipelined path's copy stream too, may still read the old buffers
-    WKB_CUDA(ctx, cudaDeviceSynchronize());
+    // the context's streams, the pipelined path's copy stream too, may still read the old buffers (a
+    // device-wide wait would end another thread's capture)
+    const BatchHost* h = (const BatchHost*)ctx->batch_host;
+    WKB_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (h && h->copy_stream) WKB_CUDA(ctx, cudaStreamSynchronize(h->copy_stream));
+    if (h && h->upload_stream) WKB_CUDA(ctx, cudaStreamSynchronize(h->upload_stream));
     free_state(b);
     auto dm = [&](void** p, size_t bytes) {
         if (wk::ctx_malloc(ctx, p, std::max<size_t>(bytes, 16)) != cudaSuccess) {
@@ -250,19 +290,6 @@ int ensure_state(wk_ctx* ctx, BatchState* b, uint32_t n, int levels, int steps, 
     return WK_SUCCESS;
 }
 
-struct Plan {
-    uint32_t n = 0;
-    int levels = 0;                     // launches
-    bool fused = false;
-    size_t up_bytes = 0;                // of the plan block
-    int width[kMaxBatchLevels] = {0};
-    std::vector<int32_t> status;
-    std::vector<wk::PlanStep> steps;    // [n][kMaxBatchLevels]
-    std::vector<uint8_t> nsteps;        // [n]
-    std::vector<uint32_t> first;        // [n] each query's first step (fused)
-    const PlanLayout layout() const { return PlanLayout(n, levels, fused); }
-};
-
 // The levels of one query's steps: fused runs (one level starts the rows, then as many steps per
 // level as give a row at most one output row and one that multiplies rows), with `put(level, first
 // step, steps, last)` for each.  Returns how many.
@@ -281,29 +308,6 @@ int query_levels(const wk_ctx* ctx, const wk::PlanStep* st, int ns, Put put) {
         i = j;
     }
     return level;
-}
-
-// Host-side state kept between batch calls of a context: the plans (their arrays are large,
-// and touching fresh pages for them cost 0.4 ms per 16,384-query batch) and the pipelined
-// path's streams and events (creating them cost 0.17 ms per call).  Calls on one context are
-// serialised by its mutex, so one set serves every call.
-struct BatchHost {
-    Plan plan[2];
-    cudaStream_t copy_stream = nullptr, upload_stream = nullptr;
-    cudaEvent_t ready[2] = {nullptr, nullptr}, copied[2] = {nullptr, nullptr};
-    cudaEvent_t uploaded[2] = {nullptr, nullptr};
-    ~BatchHost() {
-        for (int k = 0; k < 2; ++k)
-            for (cudaEvent_t e : {ready[k], copied[k], uploaded[k]})
-                if (e) cudaEventDestroy(e);
-        if (copy_stream) cudaStreamDestroy(copy_stream);
-        if (upload_stream) cudaStreamDestroy(upload_stream);
-    }
-};
-
-BatchHost* batch_host(wk_ctx* ctx) {
-    if (!ctx->batch_host) ctx->batch_host = new BatchHost();
-    return (BatchHost*)ctx->batch_host;
 }
 
 // Resolve every query (host threads, no allocation per query) and fill the pinned descriptor

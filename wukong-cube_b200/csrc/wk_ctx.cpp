@@ -177,7 +177,9 @@ void wk_ctx::drop_store(bool spare) {
         size_t free_b = 0, total_b = 0;
         if (spare && d_slots && slots_bytes && edges_bytes && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess &&
             slots_bytes + edges_bytes <= free_b / 8) {
-            cudaDeviceSynchronize();   // (as freeing them would: other streams' work on the old store)
+            // the context's work on the old store (its lanes are gone; a device-wide wait would end
+            // another thread's capture)
+            cudaStreamSynchronize(stream);
             spare_slots = Spare{d_slots, slots_bytes};
             spare_edges = Spare{d_edges, edges_bytes};
             d_slots = nullptr;
@@ -1009,7 +1011,7 @@ bool wk_ctx::drop_directories(size_t bytes) {
     if (!has_dir || borrowed_store || serving || rbuf[0].replayed ||
         cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || bytes > free_b + dir_bytes)
         return false;
-    if (cudaDeviceSynchronize() != cudaSuccess) return false;
+    if (cudaStreamSynchronize(stream) != cudaSuccess) return false;
     for (wk_ctx* lane : lanes) wk_ctx_destroy(lane);   // (the next serving run makes them again)
     lanes.clear();
     drop_graphs();   // captured passes hold their segments' directories
